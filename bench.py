@@ -36,7 +36,7 @@ import time
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
-SPMV_KERNEL = "bicg_spmv_omega"
+SPMV_KERNEL = "rb_spmv_omega"
 # DRAM bytes (read + write) that ncu measured for one launch of a kernel
 # against its algorithmic bytes, on the FP64 2 x 2 block layout of the
 # two-phase 128x128x48 case (profiles/solver_kernels_twophase_128x128x48.md,
@@ -55,9 +55,11 @@ TRAFFIC_RATIO = {
 # to residual and Jacobian assembly.
 KRYLOV_KERNELS = {"bicg_p", "bicg_spmv_alpha", "bicg_s", "bicg_spmv_omega", "bicg_xr", "bilu_lower", "bilu_upper",
                   "mg_residual", "mg_restrict", "mg_correct", "mg_prolong", "mg_tail", "mg_dense_apply",
+                  "rb_pre", "rb_y", "rb_res", "rb_restrict", "rb_post", "rb_fin", "rb_dense", "rb_tail",
+                  "rb_spmv_y", "rb_spmv_alpha", "rb_spmv_omega",
                   "residual", "add_float", "sumsq"}
 SETUP_KERNELS = {"bicg_init", "gather_values", "mg_galerkin", "mg_ap_values", "bilu_factor", "mg_dense_inverse",
-                 "to_float", "permute", "unpermute"}
+                 "to_float", "permute", "unpermute", "mg_strength", "rb_init", "rb_solution"}
 
 
 def parse():

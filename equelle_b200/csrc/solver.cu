@@ -32,7 +32,11 @@
 // Preconditioner "multigrid" (default; see the analysis section below):
 // geometric-aggregation V-cycle with these block ILU(0) sweeps as smoothers,
 // which keeps the iteration count of the elliptic pressure part from growing
-// with the grid; "ilu0": the staged block ILU(0) alone.
+// with the grid; "ilu0": the staged block ILU(0) alone.  Where every level
+// takes two colours (the cell graphs of Cartesian grids, FP64 vectors),
+// BiCGStab and the cycle run on the black half alone (twocolour.cuh); the
+// kernels over stages below serve the other orderings, FP32 vectors
+// ("refine"), patterns of more colours and "ilu0".
 //
 // Precision "mixed": BiCGStab and every vector in FP64, the preconditioner's
 // matrices (level matrices, block ILU(0) factors, coarsest inverse) stored
@@ -417,31 +421,6 @@ __global__ void gather_values_kernel(const double* __restrict__ src, const int* 
     {
         const int e = map[p];
         dst[p] = e >= 0 ? src[e] : 0.0;
-    }
-}
-
-// The same gather, one block row per thread over its slots: a thread's
-// loads stay in the few Jacobian rows of its block row (the unknowns of one
-// cell), which L1 then serves, and a warp's stores at one slot position are
-// one contiguous segment.
-template <int BB>
-__global__ void gather_rows_kernel(int nb, const int* __restrict__ slice_ptr, const double* __restrict__ src,
-                                   const int* __restrict__ map, double* __restrict__ dst)
-{
-    // every lane of the last slice, also past the last row (its slots are
-    // padding: zero)
-    GRID_STRIDE(r, ((int64_t)nb + 31) & ~(int64_t)31)
-    {
-        const int R = (int)r, lane = R & 31;
-        const int s0 = slice_ptr[R >> 5], width = (slice_ptr[(R >> 5) + 1] - s0) >> 5;
-        for (int k = 0; k < width; ++k) {
-            const int64_t q = (int64_t)(s0 + (k << 5) + lane) * BB;
-#pragma unroll
-            for (int e = 0; e < BB; ++e) {
-                const int j = map[q + e];
-                dst[q + e] = j >= 0 ? src[j] : 0.0;
-            }
-        }
     }
 }
 
@@ -1107,22 +1086,37 @@ __global__ void sumsq_kernel(const double* __restrict__ a, int n, double* partia
 }
 
 // ---- multilevel preconditioner kernels -------------------------------------
-// Coarse-level values: each entry of the coarse pattern is the sum of the
-// finer level's values that aggregate onto it (Galerkin product R A R^T with
-// a 0/1 aggregation R), gathered in ascending fine-entry order, and stored
-// at its value position gpos[c] (the other positions, padding and entries a
-// block does not have, are zeroed beforehand).
-__global__ void galerkin_kernel(int64_t nnz_c, const int* __restrict__ gptr, const int* __restrict__ gidx,
-                                const int* __restrict__ gpos, const double* __restrict__ fine,
-                                double* __restrict__ coarse)
+// Strengths of the couplings by direction (see direction_strengths).
+__global__ void direction_strength_kernel(int nb, int bs, SellView m, const double* __restrict__ a,
+                                          const int* __restrict__ perm, int nx, int ny, int nc, double* partials,
+                                          unsigned int* counter, double* out)
 {
-    GRID_STRIDE(c, nnz_c)
+    double d[3] = {0.0, 0.0, 0.0};
+    const int bb = bs * bs;
+    GRID_STRIDE(r, nb)
     {
-        double s = 0.0;
-        const int k1 = gptr[c + 1];
-        for (int k = gptr[c]; k < k1; ++k) s += fine[gidx[k]];
-        coarse[gpos[c]] = s;
+        const int R = (int)r, lane = R & 31, sb = m.slice_ptr[R >> 5], len = m.len[R];
+        const int u = perm[R * bs], comp = u / nc, cell = u - comp * nc;
+        const int i = cell % nx, j = (cell / nx) % ny, k = cell / (nx * ny);
+        for (int c = 0; c < bs; ++c) {
+            double s[3] = {0.0, 0.0, 0.0}, diag = 0.0;
+            for (int t = 0; t < len; ++t) {
+                const int q = sb + (t << 5) + lane, v = perm[m.col[q] * bs], vcomp = v / nc, vcell = v - vcomp * nc;
+                if (vcomp != comp) continue;
+                const double x = fabs(a[(size_t)q * bb + c * bs + c]);
+                if (vcell == cell) diag = x;
+                else s[vcell / (nx * ny) != k ? 2 : (vcell / nx) % ny != j ? 1 : 0] += x;
+            }
+            const double sum = s[0] + s[1] + s[2];
+            if (!(sum > 0.0) || !(diag > 0.0) || !isfinite(sum / diag)) continue;
+            const double w = fmin(1.0, sum / diag) / sum;
+            for (int e = 0; e < 3; ++e) d[e] += w * s[e];
+        }
+        (void)i;
     }
+    double s[3];
+    if (grid_sum<3>(d, partials, counter, s))
+        for (int e = 0; e < 3; ++e) out[e] = s[e];
 }
 
 template <int B, int KM, class T, class M>
@@ -1195,9 +1189,11 @@ __global__ void mg_correct_kernel(int nb, int r_zero, SellView ap, const M* __re
     }
 }
 
-// Values of A P: slot q of A P is the sum, value by value, of the A slots
-// gidx[gptr[q] .. gptr[q + 1]) (ascending); padding slots get 0.
-__global__ void ap_values_kernel(int64_t slots, int bb, const int* __restrict__ gptr, const int* __restrict__ gidx,
+// Sums of a level's blocks, value by value: slot q of the result is the sum
+// of the slots gidx[gptr[q] .. gptr[q + 1]) of `a` (ascending); padding slots
+// get 0.  The values of A P, and those of the next coarser level (Galerkin
+// product R A R^T with a 0/1 aggregation R).
+__global__ void slot_sums_kernel(int64_t slots, int bb, const int* __restrict__ gptr, const int* __restrict__ gidx,
                                  const double* __restrict__ a, double* __restrict__ ap)
 {
     GRID_STRIDE(i, slots * bb)
@@ -1363,6 +1359,7 @@ constexpr int kTailSmem = 200 * 1024;
 template <class T, class M>
 struct TailLevel {
     int nb = 0, n = 0, coarsest = 0;
+    double alpha = 1.0;          // factor of the correction from the next level
     TailLocal so{};              // shared memory layout (levels >= local_first)
     SellView m{};                // slices of uniform width m.width
     const M* a = nullptr;
@@ -1384,7 +1381,6 @@ struct TailParams {
     int ncopies = 0;
     PrefetchRegion reg[kMaxPrefetch];
     TailCopy copies[kMaxCopies];
-    double alpha = 1.0;          // coarse-correction factor
     long long* trace = nullptr;  // SM clock after each step (linsolver_tail_trace)
 };
 
@@ -1542,7 +1538,7 @@ __device__ void local_cycle(const TailParams<T, M>& p, int lf, unsigned char* sm
     for (--l; l >= lf; --l) {
         const TailLevel<T, M>& G = p.lv[l];
         const LocalView<T, M> V = local_view(G, sm);
-        prolong_rows<B, T, false>(G.nb, V.aggb, local_view(p.lv[l + 1], sm).z, V.z, p.alpha, tid, nth);
+        prolong_rows<B, T, false>(G.nb, V.aggb, local_view(p.lv[l + 1], sm).z, V.z, G.alpha, tid, nth);
         __syncthreads();
         residual_rows<B, KM, T, M, false, true>(G.nb, 0, V.m, V.a, V.z, V.r, V.t, tid, nth);
         __syncthreads();
@@ -1609,13 +1605,15 @@ __global__ void __launch_bounds__(kTailThreads)
         const TailLevel<T, M>& L = p.lv[l];
         const T* r = l == 0 ? r_top : L.r;
         T* z = l == 0 ? z_top : L.z;
-        prolong_rows<B, T, true>(L.nb, L.aggb, p.lv[l + 1].z, z, p.alpha, tid, nth);
+        prolong_rows<B, T, true>(L.nb, L.aggb, p.lv[l + 1].z, z, L.alpha, tid, nth);
         tail_step(trace, tk);
         residual_rows<B, KM, T, M, true, U>(L.nb, 0, L.m, L.a, z, r, L.t, tid, nth);
         tail_step(trace, tk);
         tail_ilu<B, KM, T, M>(L, L.t, L.w, z, tid, nth, trace, tk);
     }
 }
+
+#include "twocolour.cuh"
 
 }  // namespace
 
@@ -1624,11 +1622,14 @@ __global__ void __launch_bounds__(kTailThreads)
 //
 // Multilevel preconditioner (the default when the system is laid out as
 // `ncomp` blocks of one unknown per grid cell, as newtonSolve and
-// newtonSolveSystem stack them): geometric aggregation of 2x2x2 cells per
-// unknown block, Galerkin coarse matrices R A R^T, a V(1,1) cycle with one
-// block ILU(0) sweep before and after the coarse correction on every level,
-// and a dense inverse on the coarsest level (<= 128 unknowns).  Otherwise
-// plain block ILU(0).
+// newtonSolveSystem stack them): geometric aggregation of cells per unknown
+// block, in pairs along the directions that are strong enough (kSemiCoarsen),
+// Galerkin coarse matrices R A R^T, a V cycle with a block ILU(0) sweep after
+// the coarse correction on every level and one before it where the aggregates
+// are more than pairs (after pairing along the strong direction alone, the
+// sweep before it changes the iteration count by less than one in seventeen),
+// and a dense inverse on the coarsest level (<= 128 unknowns).  The analysis
+// works on the block graph; otherwise plain block ILU(0).
 // ---------------------------------------------------------------------------
 struct HostCsr {
     int n = 0;
@@ -1647,7 +1648,15 @@ struct Level {
     // (algorithmic bytes of the sweeps)
     std::vector<int64_t> stage_lower, stage_upper;
     Buf perm;                      // permuted unknown position -> natural unknown
-    Buf gptr, gidx, gpos;          // Galerkin gather from the finer level's values (levels > 0)
+    Buf gptr, gidx;                // Galerkin sums: the finer level's slots of each slot (levels > 0)
+    double alpha = 1.0;            // factor of the correction from the next coarser level
+    // two-colour form: red block rows, whether the level pre-smooths, and
+    // its block rows by aggregate (next coarser block row): the black ones
+    // (members_b, gb per aggregate, -1 past the last) and all (members_a, ga)
+    int nr = 0;
+    bool pre = true;
+    int gb = 0, ga = 0;
+    Buf members_b, members_a;
     Buf aggb;                      // coarse block row of each block row (next coarser level)
     // A P (see mg_correct_kernel), in the same sliced layout: slots, the
     // longest row, slices, coarse block columns, row lengths, and the A slots
@@ -1660,9 +1669,9 @@ struct Level {
     {
         return SellView{ap_sp->as<int>(), ap_col->as<int>(), ap_len->as<int>(), ap_len->as<int>(), 0};
     }
-    // host copies of the slices, columns and row lengths while the
-    // hierarchy is built
-    std::vector<int> h_sp, h_col, h_len;
+    // host copies of the slices, columns, row lengths and coarse block rows
+    // while the hierarchy is built
+    std::vector<int> h_sp, h_col, h_len, h_aggb;
     Buf mptr, midx;                // aggregate members (unknown positions) of each coarse unknown
     Buf mpad;                      // the same, kMembers per coarse unknown, -1 past the last (or none)
     int64_t sell_size = 0;         // slots of the block sliced ELL layout
@@ -1687,7 +1696,7 @@ struct SolverAnalysis {
     bool natural = false;
     bool ok = true;  // every row has a diagonal entry (1 x 1 blocks)
     bool multigrid = false;
-    double mg_alpha = 1.0;  // coarse-grid correction factor
+    bool two_colour = false;  // every level but the coarsest has two stages (twocolour.cuh)
     std::vector<Level> levels;
     Buf vmap;        // level-0 value <- Jacobian entry (-1: zero)
     Buf vec64, vec32, scal, partials, counter, factor_status;
@@ -1784,6 +1793,12 @@ inline int find_small(const int* v, int len, int key)
     return (k < len && v[k] == key) ? k : len;
 }
 
+// Loops of the analysis over fewer rows run on one thread: waking a team for
+// each of the many small loops of a small hierarchy costs more than the loops
+// (heat 64x64, whole analysis: 1.0 ms on one thread), and far more when the
+// host's cores are busy with other runtimes.
+constexpr int kSerialRows = 8192;
+
 // Builds the CSR pattern whose row r is the sorted, repeat-free union of
 // the columns that gather(r, buf) writes into buf (at most `cap` of them).
 // Two passes over the rows, each parallel over rows.
@@ -1792,7 +1807,7 @@ void build_rows(int nrows, int cap, HostCsr& out, Gather gather)
 {
     out.n = nrows;
     out.ptr.assign(nrows + 1, 0);
-#pragma omp parallel
+#pragma omp parallel if (nrows > kSerialRows)
     {
         std::vector<int> buf(cap > 0 ? cap : 1);
 #pragma omp for schedule(static)
@@ -1800,7 +1815,7 @@ void build_rows(int nrows, int cap, HostCsr& out, Gather gather)
     }
     for (int r = 0; r < nrows; ++r) out.ptr[r + 1] += out.ptr[r];
     out.col.resize(out.ptr[nrows] > 0 ? out.ptr[nrows] : 1);
-#pragma omp parallel
+#pragma omp parallel if (nrows > kSerialRows)
     {
         std::vector<int> buf(cap > 0 ? cap : 1);
 #pragma omp for schedule(static)
@@ -1818,23 +1833,12 @@ inline int max_row(const HostCsr& A)
     return m;
 }
 
-// Lays out the matrix with pattern `A` (natural unknown numbering, rows with
-// ascending columns) in blocks of `bs` unknowns: block row of unknown u is
-// u % nb and its component u / nb (nb = n / bs).  Orders the block rows by
-// stage and builds the block sliced ELL pattern (each row with its diagonal
-// block).  Returns the unknown permutation (position -> natural unknown),
-// its inverse, and for every entry of `A` its position in the level's value
-// array.  With `uniform`, every slice is as wide as the longest row.
-void order_level(Core& c, const HostCsr& A, bool natural, int bs, bool uniform, Level& L, std::vector<int>& perm,
-                 std::vector<int>& iperm, std::vector<int>& vpos, bool& ok)
+// Block graph of the pattern `A` of a system of blocks of `bs` unknowns
+// (natural block numbering: unknown u is component u / nb of block u % nb,
+// nb = n / bs), rows sorted, with the diagonal.
+HostCsr block_graph(const HostCsr& A, int bs)
 {
-    const int n = A.n;
-    const int nb = n / bs;
-    const int bb = bs * bs;
-    const int64_t nnz = A.ptr[n];
-    const auto t0 = std::chrono::steady_clock::now();
-    auto ms = [&] { return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count(); };
-    // block graph (natural block numbering), sorted, with the diagonal
+    const int nb = A.n / bs;
     HostCsr G;
     build_rows(nb, bs * max_row(A) + 1, G, [&](int R, int* buf) {
         int len = 0;
@@ -1849,116 +1853,84 @@ void order_level(Core& c, const HostCsr& A, bool natural, int bs, bool uniform, 
         buf[len++] = R;
         return len;
     });
-    if (bs == 1) {
-        bool all = true;
-#pragma omp parallel for reduction(&& : all) schedule(static)
-        for (int u = 0; u < n; ++u) {
-            bool has = false;
-            for (int e = A.ptr[u]; e < A.ptr[u + 1]; ++e) has = has || A.col[e] == u;
-            all = all && has;
-        }
-        if (!all) ok = false;
-    }
-    const double tg = ms();
+    return G;
+}
+
+// Lays out a level with block graph G (natural block numbering) in blocks of
+// `bs` unknowns: orders the block rows by stage and builds the block sliced
+// ELL pattern.  Fills the permutation of the block rows (pb: position ->
+// natural, ipb: its inverse) and, for every entry of G, its slot.  With
+// `uniform`, every slice is as wide as the longest row.
+void order_level(Core& c, const HostCsr& G, bool natural, int bs, bool uniform, Level& L, std::vector<int>& pb,
+                 std::vector<int>& ipb, std::vector<int>& slot)
+{
+    const int nb = G.n;
+    const int n = nb * bs;
+    const int bb = bs * bs;
+    const auto t0 = std::chrono::steady_clock::now();
+    auto ms = [&] { return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count(); };
     const std::vector<int> key = stage_keys(G, natural);
     const double tk = ms();
     const int nst = nb > 0 ? *std::max_element(key.begin(), key.end()) + 1 : 0;
     L.stage_ptr.assign(nst + 1, 0);
     for (int R = 0; R < nb; ++R) L.stage_ptr[key[R] + 1]++;
     for (int s = 0; s < nst; ++s) L.stage_ptr[s + 1] += L.stage_ptr[s];
-    std::vector<int> pb(nb), ipb(nb);
+    pb.assign(nb, 0);
+    ipb.assign(nb, 0);
     {
         std::vector<int> pos(L.stage_ptr.begin(), L.stage_ptr.end() - 1);
         for (int R = 0; R < nb; ++R) pb[pos[key[R]]++] = R;
     }
     for (int R = 0; R < nb; ++R) ipb[pb[R]] = R;
-    perm.assign(n, 0);
-    iperm.assign(n, 0);
-#pragma omp parallel for schedule(static)
-    for (int R = 0; R < nb; ++R)
-        for (int cc = 0; cc < bs; ++cc) {
-            perm[R * bs + cc] = cc * nb + pb[R];
-            iperm[cc * nb + pb[R]] = R * bs + cc;
-        }
-    const double tp = ms();
-    // permuted block rows: sorted permuted columns
-    std::vector<int> pptr(nb + 1, 0), pcol(G.ptr[nb] > 0 ? G.ptr[nb] : 1);
-    for (int R = 0; R < nb; ++R) pptr[R + 1] = pptr[R] + (G.ptr[pb[R] + 1] - G.ptr[pb[R]]);
-#pragma omp parallel for schedule(static)
-    for (int R = 0; R < nb; ++R) {
-        const int o = pb[R];
-        int w = pptr[R];
-        for (int e = G.ptr[o]; e < G.ptr[o + 1]; ++e) pcol[w++] = ipb[G.col[e]];
-        std::sort(pcol.begin() + pptr[R], pcol.begin() + pptr[R + 1]);
-    }
-    const double tc = ms();
-    // block sliced ELL, 32 block rows per slice
+    // block sliced ELL, 32 block rows per slice, a row's blocks in ascending
+    // order of their position
     const int nsl = (nb + 31) / 32;
     std::vector<int> sp(nsl + 1, 0), len(nb > 0 ? nb : 1), dk(nb > 0 ? nb : 1);
-    int wmax = 0;
-    for (int R = 0; R < nb; ++R) wmax = std::max(wmax, pptr[R + 1] - pptr[R]);
+    const int wmax = max_row(G);
+    for (int R = 0; R < nb; ++R) len[R] = G.ptr[pb[R] + 1] - G.ptr[pb[R]];
     for (int sl = 0; sl < nsl; ++sl) {
         int w = 0;
-        for (int R = sl * 32; R < std::min(nb, sl * 32 + 32); ++R) w = std::max(w, pptr[R + 1] - pptr[R]);
+        for (int R = sl * 32; R < std::min(nb, sl * 32 + 32); ++R) w = std::max(w, len[R]);
         sp[sl + 1] = sp[sl] + 32 * (uniform ? wmax : w);
     }
     L.width = uniform ? wmax : 0;
     const int64_t size = sp[nsl];
     if (size * bb >= (int64_t)INT_MAX) fail(EQG_ERR_UNSUPPORTED, "linear system too large for 32-bit value offsets");
     std::vector<int> scol(size > 0 ? size : 1, 0);
-    int kmax = 0;
-#pragma omp parallel for reduction(max : kmax) schedule(static)
-    for (int R = 0; R < nb; ++R) {
-        const int base = sp[R / 32] + (R % 32);
-        len[R] = pptr[R + 1] - pptr[R];
-        kmax = std::max(kmax, len[R]);
-        const int w = (sp[R / 32 + 1] - sp[R / 32]) / 32;
-        dk[R] = -1;
-        for (int k = 0; k < w; ++k) {
-            if (k < len[R]) {
-                scol[base + 32 * k] = pcol[pptr[R] + k];
-                if (pcol[pptr[R] + k] == R) dk[R] = k;
-            } else {
-                scol[base + 32 * k] = R;  // padding: a valid column, values 0, never read by the kernels
+    slot.assign(G.ptr[nb] > 0 ? G.ptr[nb] : 1, 0);
+#pragma omp parallel if (nb > kSerialRows)
+    {
+        std::vector<std::pair<int, int>> row(wmax > 0 ? wmax : 1);  // (column's position, entry of G)
+#pragma omp for schedule(static)
+        for (int R = 0; R < nb; ++R) {
+            const int o = pb[R], e0 = G.ptr[o], rl = len[R];
+            for (int k = 0; k < rl; ++k) row[k] = {ipb[G.col[e0 + k]], e0 + k};
+            std::sort(row.begin(), row.begin() + rl);
+            const int base = sp[R / 32] + (R % 32);
+            const int w = (sp[R / 32 + 1] - sp[R / 32]) / 32;
+            dk[R] = -1;
+            for (int k = 0; k < rl; ++k) {
+                scol[base + 32 * k] = row[k].first;
+                slot[row[k].second] = base + 32 * k;
+                if (row[k].first == R) dk[R] = k;
             }
+            for (int k = rl; k < w; ++k) scol[base + 32 * k] = R;  // padding: a valid column, values 0
         }
     }
-    L.kmax = kmax;
+    L.kmax = wmax;
     const double ts = ms();
-    // value position of every scalar entry of A, block row by block row
-    vpos.assign(nnz > 0 ? nnz : 1, -1);
-#pragma omp parallel for schedule(static)
-    for (int Rn = 0; Rn < nb; ++Rn) {
-        const int R = ipb[Rn];
-        const int* row = pcol.data() + pptr[R];
-        const int rl = pptr[R + 1] - pptr[R];
-        for (int cu = 0; cu < bs; ++cu) {
-            const int u = cu * nb + Rn;
-            for (int e = A.ptr[u]; e < A.ptr[u + 1]; ++e) {
-                int cell = A.col[e], cv = 0;  // column = cv nb + cell, cv < bs (no division)
-                while (cell >= nb) {
-                    cell -= nb;
-                    ++cv;
-                }
-                const int k = find_small(row, rl, ipb[cell]);
-                const int64_t slot0 = sp[R / 32] + 32 * k;
-                vpos[e] = (int)((slot0 + R % 32) * bb + cu * bs + cv);
-            }
-        }
-    }
-    const double tv = ms();
+    std::vector<int> perm(n > 0 ? n : 1);
+#pragma omp parallel for schedule(static) if (nb > kSerialRows)
+    for (int R = 0; R < nb; ++R)
+        for (int cc = 0; cc < bs; ++cc) perm[R * bs + cc] = cc * nb + pb[R];
     L.n = n;
     L.nb = nb;
     L.bs = bs;
-    L.nnz = nnz;
     L.sell_size = size;
     L.vals = size * bb;
-    L.blocks = pptr[nb];
+    L.blocks = G.ptr[nb];
     L.sell_ptr = upload_ints(c, sp);
     L.sell_col = upload_ints(c, scol);
-    L.h_sp = sp;
-    L.h_col = scol;
-    L.h_len = len;
     L.sell_len = upload_ints(c, len);
     L.sell_dk = upload_ints(c, dk);
     {
@@ -1972,15 +1944,17 @@ void order_level(Core& c, const HostCsr& A, bool natural, int bs, bool uniform, 
                 L.stage_upper[st] += std::max(0, len[R] - d - 1);
             }
     }
+    L.h_sp = std::move(sp);
+    L.h_col = std::move(scol);
+    L.h_len = std::move(len);
     const size_t nv = (size_t)(L.vals > 0 ? L.vals : 1);
     L.as64 = c.allocN<double>(nv);
     L.lus64 = c.allocN<double>(nv);
     L.perm = upload_ints(c, perm);
     L.v64 = c.allocN<double>((size_t)4 * (n > 0 ? n : 1));
     if (c.verbose > 2 && nb > 100000)
-        std::printf("        ordering of %d block rows: %.1f ms (block graph %.1f, stages %.1f, permutation %.1f, "
-                    "sorted columns %.1f, slices %.1f, value positions %.1f, uploads %.1f)\n",
-                    nb, ms(), tg, tk - tg, tp - tk, tc - tp, ts - tc, tv - ts, ms() - tv);
+        std::printf("        ordering of %d block rows: %.1f ms (stages %.1f, slices %.1f, uploads %.1f)\n", nb, ms(),
+                    tk, ts - tk, ms() - ts);
 }
 
 // A P of level L (see mg_correct_kernel): for every block row, its coarse
@@ -1995,7 +1969,7 @@ void build_ap(Core& c, Level& L, const std::vector<int>& aggb)
     std::vector<int> alen(nb > 0 ? nb : 1, 0);
     std::unique_ptr<int[]> rowq(new int[(size_t)nb * W]);  // coarse columns of each row, ascending
     int kmax = 0;
-#pragma omp parallel for reduction(max : kmax) schedule(static)
+#pragma omp parallel for reduction(max : kmax) schedule(static) if (nb > kSerialRows)
     for (int R = 0; R < nb; ++R) {
         const int base = L.h_sp[R / 32] + (R % 32);
         int q[64];
@@ -2019,7 +1993,7 @@ void build_ap(Core& c, Level& L, const std::vector<int>& aggb)
     }
     const int64_t slots = asp[nsl];
     std::vector<int> acol(slots > 0 ? slots : 1, 0), cnt(slots + 1, 0);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (nb > kSerialRows)
     for (int R = 0; R < nb; ++R) {
         const int abase = asp[R / 32] + (R % 32);
         const int w = (asp[R / 32 + 1] - asp[R / 32]) / 32;
@@ -2034,7 +2008,7 @@ void build_ap(Core& c, Level& L, const std::vector<int>& aggb)
     }
     for (int64_t q = 0; q < slots; ++q) cnt[q + 1] += cnt[q];
     std::vector<int> gidx(cnt[slots] > 0 ? cnt[slots] : 1);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (nb > kSerialRows)
     for (int R = 0; R < nb; ++R) {
         const int abase = asp[R / 32] + (R % 32);
         const int base = L.h_sp[R / 32] + (R % 32);
@@ -2059,7 +2033,78 @@ void build_ap(Core& c, Level& L, const std::vector<int>& aggb)
     L.ap64 = c.allocN<double>((size_t)(slots > 0 ? slots : 1) * L.bs * L.bs);
 }
 
-std::shared_ptr<SolverAnalysis> analyse(Core& c, const Pattern& p, bool natural, bool allow_multigrid)
+// What the sweeps over stages need of a level besides its matrix: the
+// aggregate members by unknown, and A P on levels above ap_rows unknowns.
+void stage_members(Core& c, Level& L, const Level& C, int ap_rows)
+{
+    const int bs = L.bs;
+    std::vector<int> mptr(C.n + 1, 0), midx(L.n > 0 ? L.n : 1);
+    for (int R = 0; R < L.nb; ++R)
+        for (int cc = 0; cc < bs; ++cc) mptr[L.h_aggb[R] * bs + cc + 1]++;
+    int max_members = 0;
+    for (int P = 0; P < C.n; ++P) {
+        max_members = std::max(max_members, mptr[P + 1]);
+        mptr[P + 1] += mptr[P];
+    }
+    {
+        std::vector<int> pos(mptr.begin(), mptr.end() - 1);
+        for (int R = 0; R < L.nb; ++R)
+            for (int cc = 0; cc < bs; ++cc) midx[pos[L.h_aggb[R] * bs + cc]++] = R * bs + cc;
+    }
+    L.mptr = upload_ints(c, mptr);
+    L.midx = upload_ints(c, midx);
+    if (max_members <= kMembers) {
+        std::vector<int> mpad((size_t)C.n * kMembers, -1);
+#pragma omp parallel for schedule(static) if (C.n > kSerialRows)
+        for (int P = 0; P < C.n; ++P)
+            for (int k = mptr[P]; k < mptr[P + 1]; ++k) mpad[(size_t)P * kMembers + (k - mptr[P])] = midx[k];
+        L.mpad = upload_ints(c, mpad);
+    }
+    if (L.n > ap_rows) build_ap(c, L, L.h_aggb);
+}
+
+// Level 0's matrix from the Jacobian's values.
+void gather_level0(Core& c, const SolverAnalysis& an, const double* jval)
+{
+    const Level& L0 = an.levels[0];
+    launch(c, "gather_values", [&] {
+        gather_values_kernel<<<blocksFor(L0.vals), kThreads, 0, c.stream>>>(jval, an.vmap->as<int>(),
+                                                                            L0.as64->as<double>(), L0.vals);
+    }, 12.0 * L0.vals + 8.0 * an.nnz);
+}
+
+// Mean share of the same-component couplings of a block row that each
+// direction of the level-0 grid has, weighted by how strongly the row is
+// coupled at all (shares of the diagonal, at most 1): the strengths the
+// aggregation follows.
+void direction_strengths(Core& c, const Level& L, double (&s)[3])
+{
+    const int nblk = blocksFor(L.nb, kThreads, kRedBlocks);
+    Buf part = c.allocN<double>((size_t)nblk * 3 + 3);
+    Buf counter = c.allocN<unsigned int>(1);
+    EQG_CUDA(cudaMemsetAsync(counter->ptr, 0, sizeof(unsigned int), c.stream));
+    double* out = part->as<double>() + (size_t)nblk * 3;
+    launch(c, "mg_strength", [&] {
+        direction_strength_kernel<<<nblk, kThreads, 0, c.stream>>>(
+            L.nb, L.bs, L.view(), L.as64->as<double>(), L.perm->as<int>(), c.nx, c.ny, c.nc, part->as<double>(),
+            counter->as<unsigned int>(), out);
+    });
+    EQG_CUDA(cudaMemcpyAsync(c.pinned, out, 3 * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    c.sync();
+    for (int d = 0; d < 3; ++d) s[d] = c.pinned[d];
+}
+
+// Levels are coarsened only along the directions at least 1 / kSemiCoarsen
+// as strong as the strongest one: the point smoothers do not reduce error
+// that varies slowly along a strong direction and quickly along a weak one.
+// BiCGStab iterations of a two-phase solve on 48 x 48 x 32 cells of 10 x 10 x
+// 2 m (strengths 25 : 1 : 1): 38 with 2 x 2 x 2 aggregates on every level, 21
+// with one z-pairing level first, 17 with two (then 2 x 2 x 2 at 6.25 : 1),
+// 18 with three.  At 4 : 1 one z-pairing level and none are equal.
+constexpr double kSemiCoarsen = 6.5;
+
+std::shared_ptr<SolverAnalysis> analyse(Core& c, const Pattern& p, bool natural, bool allow_multigrid,
+                                        const double* jval)
 {
     const auto t_start = std::chrono::steady_clock::now();
     auto since = [&] {
@@ -2099,189 +2144,203 @@ std::shared_ptr<SolverAnalysis> analyse(Core& c, const Pattern& p, bool natural,
         (!natural && fp64_vectors && (ncomp == 2 || ncomp == 3) && c.param_i("linsolver_block", 1) != 0) ? ncomp
                                                                                                           : 1;
 
-    std::vector<int> perm, iperm, vpos;
     an->levels.emplace_back();
     const double t_copy = since();
     // levels small enough for the fused coarse cycle get slices of uniform width
     const int fuse_rows = c.param_i("linsolver_mg_fuse_rows", 40000);
     const int ap_rows = c.param_i("linsolver_mg_ap_rows", 40000);
-    order_level(c, A, natural, bs, n <= fuse_rows, an->levels[0], perm, iperm, vpos, an->ok);
-    const double t_level0 = since();
+    HostCsr fine = block_graph(A, bs);
+    std::vector<int> pb, ipb, slot;
+    order_level(c, fine, natural, bs, n <= fuse_rows, an->levels[0], pb, ipb, slot);
+    an->levels[0].nnz = p.nnz;
     {
+        // value position of every Jacobian entry; with 1 x 1 blocks every row
+        // must have its diagonal entry (the graph's is always there)
+        const int nb = fine.n, bb = bs * bs;
         std::vector<int> vmap(an->levels[0].vals > 0 ? an->levels[0].vals : 1, -1);
-#pragma omp parallel for schedule(static)
-        for (int64_t e = 0; e < p.nnz; ++e) vmap[vpos[e]] = (int)e;
+        bool all = true;
+#pragma omp parallel for schedule(static) reduction(&& : all) if (nb > kSerialRows)
+        for (int Rn = 0; Rn < nb; ++Rn) {
+            const int* row = fine.col.data() + fine.ptr[Rn];
+            const int rl = fine.ptr[Rn + 1] - fine.ptr[Rn];
+            for (int cu = 0; cu < bs; ++cu) {
+                const int u = cu * nb + Rn;
+                bool has = bs > 1;
+                for (int e = A.ptr[u]; e < A.ptr[u + 1]; ++e) {
+                    int cell = A.col[e], cv = 0;  // column = cv nb + cell, cv < bs (no division)
+                    while (cell >= nb) {
+                        cell -= nb;
+                        ++cv;
+                    }
+                    has = has || cell == Rn;
+                    const int64_t q = slot[fine.ptr[Rn] + find_small(row, rl, cell)];
+                    vmap[q * bb + cu * bs + cv] = e;
+                }
+                all = all && has;
+            }
+        }
+        an->ok = all;
         an->vmap = upload_ints(c, vmap);
     }
+    const double t_level0 = since();
     an->multigrid = mg_wanted && an->ok;
-    an->mg_alpha = c.param_d("linsolver_mg_alpha", c.nz > 1 ? kMgAlpha3d : kMgAlpha2d);
-    an->levels[0].cx = c.nx;
-    an->levels[0].cy = c.ny;
-    an->levels[0].cz = c.nz;
     if (an->multigrid) {
-        // the finer level in its natural ordering, with its permutation and
-        // value positions (level 0: the Jacobian pattern itself)
-        const HostCsr* finep = &A;
-        const std::vector<int>* fpermp = &perm;
-        const std::vector<int>* fvposp = &vpos;
-        HostCsr owned;
-        std::vector<int> owned_perm, owned_vpos;
+        double strength[3] = {1.0, 1.0, 1.0};
+        if ((c.nx > 1) + (c.ny > 1) + (c.nz > 1) > 1) {
+            gather_level0(c, *an, jval);
+            direction_strengths(c, an->levels[0], strength);
+        }
+        int dims[3] = {c.nx, c.ny, c.nz};
+        const int ncn = fine.n / c.nc;  // nodes of the block graph per cell (1 with blocks of all components)
         for (;;) {
             const double tl0 = since();
-            const HostCsr& fine = *finep;
-            const std::vector<int>& fperm = *fpermp;
-            const std::vector<int>& fvpos = *fvposp;
             Level& F = an->levels.back();
-            const int fcx = F.cx, fcy = F.cy, fcz = F.cz;
-            const int fcells = fcx * fcy * fcz;
-            const int ccx = (fcx + 1) / 2, ccy = (fcy + 1) / 2, ccz = fcz > 1 ? (fcz + 1) / 2 : 1;
-            const int ccells = ccx * ccy * ccz;
-            const int nc_unk = ncomp * ccells;
-            // aggregate of every fine unknown (natural indices)
-            std::vector<int> agg_nat(fine.n);
-#pragma omp parallel for schedule(static)
+            // aggregates: pairs of cells along every direction strong enough
+            int f[3], cdims[3];
+            double top = 0.0;
+            for (int d = 0; d < 3; ++d)
+                if (dims[d] > 1) top = std::max(top, strength[d]);
+            int cut = 0;
+            for (int d = 0; d < 3; ++d) {
+                f[d] = dims[d] > 1 && !(strength[d] * kSemiCoarsen < top) ? 2 : 1;
+                cdims[d] = (dims[d] + f[d] - 1) / f[d];
+                cut += f[d] == 2;
+            }
+            // couplings of a coarse cell: twice as many fine ones per other
+            // direction that was paired
+            for (int d = 0; d < 3; ++d) strength[d] *= std::ldexp(1.0, cut - (f[d] == 2));
+            F.alpha = c.param_d("linsolver_mg_alpha", cut == 2 && c.nz == 1 ? kMgAlpha2d : kMgAlpha3d);
+            F.pre = cut > 1;
+            const int fcells = dims[0] * dims[1] * dims[2], ccells = cdims[0] * cdims[1] * cdims[2];
+            const int ncb = ncn * ccells;  // coarse block rows
+            std::vector<int> agg(fine.n);
+#pragma omp parallel for schedule(static) if (fine.n > kSerialRows)
             for (int u = 0; u < fine.n; ++u) {
                 const int comp = u / fcells, cell = u - comp * fcells;
-                const int i = cell % fcx, j = (cell / fcx) % fcy, k = cell / (fcx * fcy);
-                agg_nat[u] = comp * ccells + (i / 2) + ccx * ((j / 2) + ccy * (fcz > 1 ? k / 2 : 0));
+                const int i = cell % dims[0], j = (cell / dims[0]) % dims[1], k = cell / (dims[0] * dims[1]);
+                agg[u] = comp * ccells + i / f[0] + cdims[0] * (j / f[1] + cdims[1] * (k / f[2]));
             }
-            // members of every coarse unknown (natural indices, ascending)
-            std::vector<int> nmptr(nc_unk + 1, 0), nmidx(fine.n);
-            for (int u = 0; u < fine.n; ++u) nmptr[agg_nat[u] + 1]++;
-            for (int U = 0; U < nc_unk; ++U) nmptr[U + 1] += nmptr[U];
+            // members of every coarse node (natural numbering, ascending)
+            std::vector<int> nptr(ncb + 1, 0), nidx(fine.n);
+            for (int u = 0; u < fine.n; ++u) nptr[agg[u] + 1]++;
+            for (int U = 0; U < ncb; ++U) nptr[U + 1] += nptr[U];
             {
-                std::vector<int> pos(nmptr.begin(), nmptr.end() - 1);
-                for (int u = 0; u < fine.n; ++u) nmidx[pos[agg_nat[u]]++] = u;
+                std::vector<int> pos(nptr.begin(), nptr.end() - 1);
+                for (int u = 0; u < fine.n; ++u) nidx[pos[agg[u]]++] = u;
             }
             int max_members = 0;
-            for (int U = 0; U < nc_unk; ++U) max_members = std::max(max_members, nmptr[U + 1] - nmptr[U]);
-            // coarse pattern (natural ordering, sorted rows)
-            HostCsr C;
-            build_rows(nc_unk, max_members * max_row(fine) + 1, C, [&](int U, int* buf) {
+            for (int U = 0; U < ncb; ++U) max_members = std::max(max_members, nptr[U + 1] - nptr[U]);
+            HostCsr coarse;
+            build_rows(ncb, max_members * max_row(fine) + 1, coarse, [&](int U, int* buf) {
                 int len = 0;
-                for (int m = nmptr[U]; m < nmptr[U + 1]; ++m) {
-                    const int u = nmidx[m];
-                    for (int e = fine.ptr[u]; e < fine.ptr[u + 1]; ++e) buf[len++] = agg_nat[fine.col[e]];
+                for (int m = nptr[U]; m < nptr[U + 1]; ++m) {
+                    const int u = nidx[m];
+                    for (int e = fine.ptr[u]; e < fine.ptr[u + 1]; ++e) buf[len++] = agg[fine.col[e]];
                 }
                 return len;
             });
             an->levels.emplace_back();
             Level& Lc = an->levels.back();
             Level& Lf = an->levels[an->levels.size() - 2];
-            Lc.cx = ccx;
-            Lc.cy = ccy;
-            Lc.cz = ccz;
-            std::vector<int> cperm, ciperm, cvpos;
-            bool cok = true;
+            std::vector<int> cpb, cipb, cslot;
             const double tl1 = since();
-            order_level(c, C, natural, bs, nc_unk <= fuse_rows, Lc, cperm, ciperm, cvpos, cok);
+            order_level(c, coarse, natural, bs, ncb * bs <= fuse_rows, Lc, cpb, cipb, cslot);
+            Lc.nnz = (int64_t)coarse.ptr[ncb] * bs * bs;
             const double tl2 = since();
-            if (!cok) fail(EQG_ERR_DEVICE, "coarse level without a diagonal entry");
-            // aggregation in permuted positions, and aggregate members
-            std::vector<int> aggp(fine.n);
-#pragma omp parallel for schedule(static)
-            for (int pf = 0; pf < fine.n; ++pf) aggp[pf] = ciperm[agg_nat[fperm[pf]]];
-            std::vector<int> mptr(nc_unk + 1, 0), midx(fine.n);
-            for (int pf = 0; pf < fine.n; ++pf) mptr[aggp[pf] + 1]++;
-            for (int P = 0; P < nc_unk; ++P) mptr[P + 1] += mptr[P];
+            // coarse block row of every fine one, and the members of every
+            // coarse block row, in positions (ascending)
+            Lf.h_aggb.resize(fine.n);
+#pragma omp parallel for schedule(static) if (fine.n > kSerialRows)
+            for (int R = 0; R < fine.n; ++R) Lf.h_aggb[R] = cipb[agg[pb[R]]];
+            Lf.aggb = upload_ints(c, Lf.h_aggb);
+            Lf.nr = Lf.stage_ptr.size() > 1 ? Lf.stage_ptr[1] : 0;
             {
-                std::vector<int> pos(mptr.begin(), mptr.end() - 1);
-                for (int pf = 0; pf < fine.n; ++pf) midx[pos[aggp[pf]]++] = pf;
-            }
-            {
-                // per block row: unknown R*bs + c aggregates onto coarse R'*bs + c
-                std::vector<int> aggb(Lf.nb);
-                bool whole = true;
-#pragma omp parallel for schedule(static) reduction(&& : whole)
+                auto pow2 = [](int v) {
+                    int g = 1;
+                    while (g < v) g *= 2;
+                    return g;
+                };
+                std::vector<int> nblack(ncb, 0);
+                for (int R = Lf.nr; R < Lf.nb; ++R) nblack[Lf.h_aggb[R]]++;
+                Lf.ga = pow2(max_members);
+                Lf.gb = pow2(*std::max_element(nblack.begin(), nblack.end()));
+                std::vector<int> ma((size_t)ncb * Lf.ga, -1), mb((size_t)ncb * Lf.gb, -1), na(ncb, 0);
+                std::fill(nblack.begin(), nblack.end(), 0);
                 for (int R = 0; R < Lf.nb; ++R) {
-                    aggb[R] = aggp[R * bs] / bs;
-                    for (int cc = 0; cc < bs; ++cc) whole = whole && aggp[R * bs + cc] == aggb[R] * bs + cc;
+                    const int P = Lf.h_aggb[R];
+                    ma[(size_t)P * Lf.ga + na[P]++] = R;
+                    if (R >= Lf.nr) mb[(size_t)P * Lf.gb + nblack[P]++] = R;
                 }
-                if (!whole) fail(EQG_ERR_DEVICE, "aggregation splits a block");
-                Lf.aggb = upload_ints(c, aggb);
-                if (Lf.n > ap_rows) build_ap(c, Lf, aggb);
-            }
-            Lf.h_sp.clear();
-            Lf.h_col.clear();
-            Lf.h_len.clear();
-            Lf.mptr = upload_ints(c, mptr);
-            Lf.midx = upload_ints(c, midx);
-            if (max_members <= kMembers) {
-                std::vector<int> mpad((size_t)nc_unk * kMembers, -1);
-#pragma omp parallel for schedule(static)
-                for (int P = 0; P < nc_unk; ++P)
-                    for (int k = mptr[P]; k < mptr[P + 1]; ++k) mpad[(size_t)P * kMembers + (k - mptr[P])] = midx[k];
-                Lf.mpad = upload_ints(c, mpad);
+                Lf.members_a = upload_ints(c, ma);
+                Lf.members_b = upload_ints(c, mb);
             }
             const double tl3 = since();
-            // Galerkin gather: for every coarse entry, the value positions of
-            // the fine entries that aggregate onto it, in ascending fine-entry
-            // order.  A coarse row's entries come only from its members' rows,
-            // so both passes run per coarse row.
-            const int64_t fnnz = fine.ptr[fine.n];
-            const int cnnz = C.ptr[nc_unk];
-            std::vector<int> gptr(cnnz + 1, 0), gidx(fnnz > 0 ? fnnz : 1);
-#pragma omp parallel for schedule(static)
-            for (int U = 0; U < nc_unk; ++U) {
-                const int* row = C.col.data() + C.ptr[U];
-                const int rl = C.ptr[U + 1] - C.ptr[U];
-                for (int m = nmptr[U]; m < nmptr[U + 1]; ++m) {
-                    const int u = nmidx[m];
-                    for (int e = fine.ptr[u]; e < fine.ptr[u + 1]; ++e)
-                        gptr[C.ptr[U] + find_small(row, rl, agg_nat[fine.col[e]]) + 1]++;
-                }
-            }
-            for (int k = 0; k < cnnz; ++k) gptr[k + 1] += gptr[k];
-#pragma omp parallel
+            // Galerkin sums R A R^T with 0/1 aggregation: for every coarse
+            // slot, the fine slots that aggregate onto it, in ascending order
+            // of the fine (row, column).  A coarse row's entries come only
+            // from its members' rows, so both passes run per coarse row.
+            std::vector<int> gptr(Lc.sell_size + 1, 0), gidx(fine.ptr[fine.n] > 0 ? fine.ptr[fine.n] : 1);
+            auto coarse_slot = [&](int U, int fe) {
+                const int e0 = coarse.ptr[U];
+                return cslot[e0 + find_small(coarse.col.data() + e0, coarse.ptr[U + 1] - e0, agg[fine.col[fe]])];
+            };
+#pragma omp parallel for schedule(static) if (ncb > kSerialRows)
+            for (int U = 0; U < ncb; ++U)
+                for (int m = nptr[U]; m < nptr[U + 1]; ++m)
+                    for (int e = fine.ptr[nidx[m]]; e < fine.ptr[nidx[m] + 1]; ++e) gptr[coarse_slot(U, e) + 1]++;
+            for (int64_t k = 0; k < Lc.sell_size; ++k) gptr[k + 1] += gptr[k];
+#pragma omp parallel if (ncb > kSerialRows)
             {
-                std::vector<int> pos;
+                std::vector<int> pos(max_row(coarse));
 #pragma omp for schedule(static)
-                for (int U = 0; U < nc_unk; ++U) {
-                    const int* row = C.col.data() + C.ptr[U];
-                    const int rl = C.ptr[U + 1] - C.ptr[U];
-                    pos.assign(gptr.begin() + C.ptr[U], gptr.begin() + C.ptr[U + 1]);
-                    for (int m = nmptr[U]; m < nmptr[U + 1]; ++m) {
-                        const int u = nmidx[m];
-                        for (int e = fine.ptr[u]; e < fine.ptr[u + 1]; ++e)
-                            gidx[pos[find_small(row, rl, agg_nat[fine.col[e]])]++] = fvpos[e];
-                    }
+                for (int U = 0; U < ncb; ++U) {
+                    const int e0 = coarse.ptr[U], rl = coarse.ptr[U + 1] - e0;
+                    for (int k = 0; k < rl; ++k) pos[k] = gptr[cslot[e0 + k]];
+                    for (int m = nptr[U]; m < nptr[U + 1]; ++m)
+                        for (int e = fine.ptr[nidx[m]]; e < fine.ptr[nidx[m] + 1]; ++e)
+                            gidx[pos[find_small(coarse.col.data() + e0, rl, agg[fine.col[e]])]++] = slot[e];
                 }
             }
             Lc.gptr = upload_ints(c, gptr);
             Lc.gidx = upload_ints(c, gidx);
-            Lc.gpos = upload_ints(c, cvpos);
-            Lc.nnz = cnnz;
             if (c.verbose > 2)
-                std::printf("        coarse level of %d unknowns: %.1f ms (pattern %.1f, ordering %.1f, aggregation "
-                            "and A P %.1f, Galerkin lists %.1f)\n",
-                            nc_unk, since() - tl0, tl1 - tl0, tl2 - tl1, tl3 - tl2, since() - tl3);
-            if (nc_unk <= coarsest || (ccx == 1 && ccy == 1 && ccz == 1)) {
-                if (nc_unk > kCoarsest) {
+                std::printf("        coarse level of %d unknowns (%dx%dx%d aggregates): %.1f ms (pattern %.1f, ordering "
+                            "%.1f, members %.1f, Galerkin lists %.1f)\n",
+                            ncb * bs, f[0], f[1], f[2], since() - tl0, tl1 - tl0, tl2 - tl1, tl3 - tl2, since() - tl3);
+            for (int d = 0; d < 3; ++d) dims[d] = cdims[d];
+            if (ncb * bs <= coarsest || ccells == 1) {
+                if (ncb * bs > kCoarsest) {
                     an->multigrid = false;  // cannot coarsen further and too large to invert
                     an->levels.resize(1);
                     break;
                 }
                 Lc.coarsest = true;
-                Lc.inv64 = c.allocN<double>((size_t)nc_unk * nc_unk);
+                Lc.inv64 = c.allocN<double>((size_t)ncb * bs * ncb * bs);
                 break;
             }
-            owned = std::move(C);
-            owned_perm = std::move(cperm);
-            owned_vpos = std::move(cvpos);
-            finep = &owned;
-            fpermp = &owned_perm;
-            fvposp = &owned_vpos;
+            fine = std::move(coarse);
+            pb = std::move(cpb);
+            ipb = std::move(cipb);
+            slot = std::move(cslot);
         }
     }
     if (an->multigrid) {
+        const int nl = (int)an->levels.size();
+        // the two-colour form (twocolour.cuh): two stages on every level but
+        // the coarsest, FP64 vectors, the default ordering
+        an->two_colour = !natural && fp64_vectors;
+        for (const Level& L : an->levels)
+            if (!L.coarsest && (L.stage_ptr.size() != 3 || L.gb > kMembers || L.ga > kMembers)) an->two_colour = false;
+        // otherwise the sweeps over stages, with their own member lists
+        if (!an->two_colour)
+            for (int l = 0; l + 1 < nl; ++l) stage_members(c, an->levels[l], an->levels[l + 1], ap_rows);
         // fuse the levels of at most linsolver_mg_fuse_rows unknowns (0: none):
         // from the first level from which on every level is that small, has
         // slices of uniform width, at most kTailStages stages and aggregates
         // of at most kMembers members (the coarsest needs none of these)
-        const int nl = (int)an->levels.size();
         auto fusable = [&](const Level& L) {
             return L.coarsest || (L.n <= fuse_rows && L.width > 0 && (int)L.stage_ptr.size() - 1 <= kTailStages &&
-                                  L.mpad);
+                                  (an->two_colour || L.mpad));
         };
         for (int l = nl - 1; l >= 0 && nl - l <= kMaxTail && fusable(an->levels[l]); --l)
             if (!an->levels[l].coarsest) an->tail_first = l;
@@ -2290,13 +2349,15 @@ std::shared_ptr<SolverAnalysis> analyse(Core& c, const Pattern& p, bool natural,
                 if (!an->levels[l].coarsest) an->tail_kmax = std::max(an->tail_kmax, an->levels[l].kmax);
     }
     for (auto& L : an->levels) {
-        L.h_sp.clear();
-        L.h_col.clear();
-        L.h_len.clear();
+        L.h_sp = L.h_col = L.h_len = L.h_aggb = std::vector<int>();
     }
-    an->vec64 = c.allocN<double>((size_t)10 * vec_stride(n));
+    // the right-hand side and the BiCGStab vectors, of the black half alone in
+    // the two-colour form
+    const Level& L0 = an->levels[0];
+    an->vec64 = c.allocN<double>(an->two_colour ? vec_stride(n) + 10 * vec_stride((L0.nb - L0.nr) * bs)
+                                                : 10 * vec_stride(n));
     an->scal = c.alloc(sizeof(KScal));
-    an->partials = c.allocN<double>((size_t)kRedBlocks * 2);
+    an->partials = c.allocN<double>((size_t)kRedBlocks * 3);
     an->counter = c.allocN<unsigned int>(1);
     an->factor_status = c.allocN<int>(1);
     EQG_CUDA(cudaMemsetAsync(an->counter->ptr, 0, sizeof(unsigned int), c.stream));
@@ -2375,14 +2436,13 @@ constexpr int pc_mode()
     return sizeof(T) == sizeof(float) ? 1 : (sizeof(M) == sizeof(float) ? 2 : 0);
 }
 
-// Cluster size for mg_tail_kernel<B, KM, T, M>: linsolver_mg_cluster
+// Cluster size for a fused coarse cycle's kernel: linsolver_mg_cluster
 // (default 16, at most 16), reduced until the device reports that it can
 // schedule one cluster of that size.
-template <int B, int KM, class T, class M>
-int tail_cluster_size(Core& c)
+template <class Kernel>
+int tail_cluster_size(Core& c, Kernel kern)
 {
     int want = std::min(16, std::max(1, c.param_i("linsolver_mg_cluster", 16)));
-    auto kern = mg_tail_kernel<B, KM, T, M>;
     if (want > 8) EQG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     EQG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem));
     for (; want > 1; want /= 2) {
@@ -2485,6 +2545,65 @@ int plan_local(Core& c, const SolverAnalysis& an, int& bytes, TailParams<T, M>* 
     return lf;
 }
 
+// plan_local for the two-colour form.
+template <class M>
+int plan_rb_local(Core& c, const SolverAnalysis& an, int& bytes, RbTailParams<M>* p)
+{
+    const int nlev = (int)an.levels.size() - an.tail_first;
+    bytes = 0;
+    if (an.tail_first < 0 || an.tail_kmax > 16 || !c.param_i("linsolver_mg_local", 1)) return nlev;
+    int off = 0, copies = 0, lf = nlev;
+    auto place = [&](int64_t b) {
+        const int o = off;
+        off += (int)((b + 15) & ~(int64_t)15);
+        return o;
+    };
+    for (int i = nlev - 1; i >= 1; --i) {
+        const Level& L = an.levels[an.tail_first + i];
+        const int off0 = off;
+        RbLocal o{};
+        struct Piece {
+            const void* src;
+            int dst;
+            int64_t bytes;
+        } piece[5];
+        int np = 0;
+        auto copied = [&](const void* src, int64_t b) {
+            piece[np] = Piece{src, place(b), b};
+            return piece[np++].dst;
+        };
+        if (L.vals * (int64_t)sizeof(M) > kTailSmem) break;
+        o.r = place((int64_t)L.n * sizeof(double));
+        if (L.coarsest) {
+            o.inv = copied(level_inv<M>(L), (int64_t)L.n * L.n * sizeof(M));
+        } else {
+            const bool black = L.pre;
+            const Level& C = an.levels[an.tail_first + i + 1];
+            o.w = place((int64_t)L.n * sizeof(double));
+            o.a = copied(level_a<M>(L), L.vals * (int64_t)sizeof(M));
+            o.lu = copied(level_lu<M>(L), L.vals * (int64_t)sizeof(M));
+            o.col = copied(L.sell_col->ptr, L.sell_size * 4);
+            o.len = copied(L.sell_len->ptr, (int64_t)L.nb * 4);
+            o.list = copied((black ? L.members_b : L.members_a)->ptr, (int64_t)C.nb * (black ? L.gb : L.ga) * 4);
+        }
+        if (off > kTailSmem || copies + np > kMaxCopies) {
+            off = off0;
+            break;
+        }
+        copies += np;
+        lf = i;
+        if (p) {
+            p->lv[i].so = o;
+            for (int k = 0; k < np; ++k)
+                p->copies[p->ncopies++] = TailCopy{piece[k].src, piece[k].dst, (int)piece[k].bytes};
+        }
+    }
+    if (lf == nlev) return nlev;
+    bytes = off;
+    if (p) p->local_first = lf;
+    return lf;
+}
+
 // Algorithmic bytes of the solver launches (reported with kernel timings):
 // every matrix block the step needs read once (its B^2 values and 4-byte
 // column), 4 bytes of row data per block row read (its length or diagonal
@@ -2528,10 +2647,54 @@ void prepare_tail(Core& c, SolverAnalysis& an)
     const int mode = pc_mode<T, M>();
     int& cl = an.tail_cluster[mode];
     const int bs = an.levels[an.tail_first].bs;
-    if (!cl) WITH_BS(bs, WITH_KMAX(an.tail_kmax, cl = tail_cluster_size<BS, KK, T, M>(c)));
     int bytes = 0;
+    if constexpr (sizeof(T) == sizeof(double)) {
+        if (an.two_colour) {
+            if (!cl) WITH_BS(bs, WITH_KMAX(an.tail_kmax, cl = tail_cluster_size(c, rb_tail_kernel<BS, KK, M>)));
+            an.tail_local[mode] = plan_rb_local<M>(c, an, bytes, nullptr);
+            an.last_mode = mode;
+            return;
+        }
+    }
+    if (!cl) WITH_BS(bs, WITH_KMAX(an.tail_kmax, cl = tail_cluster_size(c, mg_tail_kernel<BS, KK, T, M>)));
     an.tail_local[mode] = plan_local<T, M>(c, an, bytes, nullptr);
     an.last_mode = mode;
+}
+
+// Launch of a fused coarse cycle: one cluster of `cl` blocks.
+struct TailLaunch {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    TailLaunch(Core& c, int cl, int smem)
+    {
+        if (cl <= 0) fail(EQG_ERR_DEVICE, "fused coarse cycle launched before its cluster size was chosen");
+        cfg.gridDim = dim3(cl);
+        cfg.blockDim = dim3(kTailThreads);
+        cfg.dynamicSmemBytes = (size_t)smem;
+        cfg.stream = c.stream;
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = cl;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = c.pdl_launch ? 2 : 1;
+    }
+};
+
+// Algorithmic bytes of a fused cycle: every fused level's matrix, factors and
+// index arrays once (the data the bulk prefetch fetches) and four vectors.
+template <class T, class M>
+double tail_bytes(const SolverAnalysis& an)
+{
+    double b = 0.0;
+    for (size_t l = an.tail_first; l < an.levels.size(); ++l) {
+        const Level& L = an.levels[l];
+        b += (L.coarsest ? (double)L.n * L.n : 2.0 * L.vals) * sizeof(M) + 4.0 * L.sell_size + 8.0 * L.nb +
+             4.0 * L.n * sizeof(T);
+    }
+    return b;
 }
 
 // z = V-cycle(r) from level tail_first down, as one mg_tail_kernel launch.
@@ -2560,6 +2723,7 @@ void launch_tail(Core& c, const SolverAnalysis& an, const T* r, T* z, const KSca
         t.nb = L.nb;
         t.n = L.n;
         t.coarsest = L.coarsest ? 1 : 0;
+        t.alpha = L.alpha;
         t.m = L.view();
         t.a = level_a<M>(L);
         t.nstages = (int)L.stage_ptr.size() - 1;
@@ -2577,37 +2741,13 @@ void launch_tail(Core& c, const SolverAnalysis& an, const T* r, T* z, const KSca
         t.w = level_vec<T>(L, 3);
     }
     if (an.tail_trace) p.trace = an.tail_trace->as<long long>();
-    p.alpha = an.mg_alpha;
     p.local_first = p.nlev;
     int smem = 0;
     if (an.tail_local[pc_mode<T, M>()] < p.nlev) plan_local<T, M>(c, an, smem, &p);
-    const int cl = an.tail_cluster[pc_mode<T, M>()];
-    if (cl <= 0) fail(EQG_ERR_DEVICE, "fused coarse cycle launched before its cluster size was chosen");
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[2];
-    cfg.gridDim = dim3(cl);
-    cfg.blockDim = dim3(kTailThreads);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = c.stream;
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = cl;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = c.pdl_launch ? 2 : 1;
-    // algorithmic bytes: every fused level's matrix, factors and index
-    // arrays once (the data the bulk prefetch fetches) and its four vectors
-    double tail_bytes = 0.0;
-    for (size_t l = an.tail_first; l < an.levels.size(); ++l) {
-        const Level& L = an.levels[l];
-        tail_bytes += (L.coarsest ? (double)L.n * L.n : 2.0 * L.vals) * sizeof(M) + 4.0 * L.sell_size +
-                      8.0 * L.nb + 4.0 * L.n * sizeof(T);
-    }
+    TailLaunch cfg(c, an.tail_cluster[pc_mode<T, M>()], smem);
     WITH_BS(an.levels[an.tail_first].bs, WITH_KMAX(an.tail_kmax, launch(c, "mg_tail", [&] {
-                EQG_CUDA(cudaLaunchKernelEx(&cfg, mg_tail_kernel<BS, KK, T, M>, p, r, z, sc, skip_if_s));
-            }, tail_bytes)));
+                EQG_CUDA(cudaLaunchKernelEx(&cfg.cfg, mg_tail_kernel<BS, KK, T, M>, p, r, z, sc, skip_if_s));
+            }, tail_bytes<T, M>(an))));
 }
 
 // Prints the steps of the last fused coarse cycle (linsolver_tail_trace=1):
@@ -2629,7 +2769,24 @@ void report_tail_trace(Core& c, const SolverAnalysis& an)
     };
     const int lf = an.tail_first + an.tail_local[an.last_mode];  // first shared-memory level (last + 1: none)
     int l = an.tail_first;
-    for (; l < lf; ++l) {
+    if (an.two_colour) {
+        auto name = [&](int k, const char* what) { names.push_back("L" + std::to_string(k) + "." + what); };
+        for (; l < lf && l < last; ++l) {
+            if (an.levels[l].pre) {
+                name(l, "pre");
+                name(l, "y");
+            }
+            name(l, an.levels[l].pre ? "residual" : "restrict");
+        }
+        name(l, l == lf ? "shared" : "dense");
+        for (--l; l >= an.tail_first; --l) {
+            name(l, "y");
+            if (l == 0) break;
+            name(l, "post");
+            name(l, "fin");
+        }
+    }
+    for (; !an.two_colour && l < lf; ++l) {
         if (an.levels[l].coarsest || l == last) {
             names.push_back("L" + std::to_string(l) + ".dense");
             break;
@@ -2638,10 +2795,10 @@ void report_tail_trace(Core& c, const SolverAnalysis& an)
         names.push_back("L" + std::to_string(l) + ".residual");
         if (l + 1 < lf) names.push_back("L" + std::to_string(l) + ".restrict");
     }
-    if (l == lf && lf <= last)
+    if (!an.two_colour && l == lf && lf <= last)
         names.push_back("L" + std::to_string(lf - 1) + ".restrict+L" + std::to_string(lf) + "-L" +
                         std::to_string(last) + ".shared");
-    for (--l; l >= an.tail_first; --l) {
+    for (--l; !an.two_colour && l >= an.tail_first; --l) {
         names.push_back("L" + std::to_string(l) + ".prolong");
         names.push_back("L" + std::to_string(l) + ".residual");
         ilu(l);
@@ -2761,16 +2918,159 @@ void vcycle(Core& c, const SolverAnalysis& an, size_t l, const T* r, T* z, const
         WITH_BS(L.bs, WITH_KMAX(L.ap_kmax, launch(c, "mg_correct", [&] {
                     launch_k(c, mg_correct_kernel<BS, KK, T, M>, blocksFor(L.nb, L.threads), L.threads, L.nb, r_zero,
                              L.ap_view(),
-                             level_ap<M>(L), (const int*)L.aggb->as<int>(), (const T*)zc, z, t, an.mg_alpha, sc, skip);
+                             level_ap<M>(L), (const int*)L.aggb->as<int>(), (const T*)zc, z, t, L.alpha, sc, skip);
                 }, bytes)));
     } else {
         WITH_BS(L.bs, launch(c, "mg_prolong", [&] {
                     launch_k(c, mg_prolong_kernel<BS, T>, blocksFor(L.nb, L.threads), L.threads, L.nb,
-                             (const int*)L.aggb->as<int>(), (const T*)zc, z, an.mg_alpha, sc, skip);
+                             (const int*)L.aggb->as<int>(), (const T*)zc, z, L.alpha, sc, skip);
                 }, 4.0 * L.nb + (double)C.n * sizeof(T) + 2.0 * L.n * sizeof(T)));
         level_residual<T, M>(c, L, z, r, t, 0, sc, skip);
     }
     ilu_apply<T, M>(c, L, t, w, z, sc, skip);
+}
+
+// ---- the two-colour cycle (twocolour.cuh) ---------------------------------------
+// The pieces of one level: right-hand side, iterate and work vector by block
+// row.  Level 0 works on the caller's black vectors (`in`, `out`), whose red
+// right-hand side is zero.
+template <class M>
+struct RbVectors {
+    const double *r, *r_red;
+    double *z, *y;
+    const int* list;  // members restricted to the next level
+    int g;
+    UpView up;
+    RbVectors(const SolverAnalysis& an, size_t l, const double* in, double* out)
+    {
+        const Level& L = an.levels[l];
+        const int64_t red = (int64_t)L.nr * L.bs;
+        double* v0 = level_vec<double>(L, 0);
+        r = l == 0 ? in - red : v0;
+        r_red = l == 0 ? nullptr : r;
+        z = l == 0 ? out - red : level_vec<double>(L, 1);
+        y = l == 0 ? v0 : z;
+        const bool black = L.pre || l == 0;
+        list = L.coarsest ? nullptr : (black ? L.members_b : L.members_a)->as<int>();
+        g = black ? L.gb : L.ga;
+        if (l > 0) {
+            const Level& F = an.levels[l - 1];
+            up.list = F.members_b->as<int>();
+            up.g = F.gb;
+            up.add = F.pre ? 1 : 0;
+            up.alpha = F.alpha;
+            up.w = l == 1 ? out - (int64_t)F.nr * F.bs : level_vec<double>(F, 1);
+        }
+    }
+};
+
+template <class M>
+void launch_rb_tail(Core& c, const SolverAnalysis& an, const double* in, double* out, const KScal* sc, int skip)
+{
+    RbTailParams<M> p;
+    auto region = [&](const void* ptr, int64_t bytes) {
+        if (p.nregions < kMaxPrefetch && bytes >= 16) p.reg[p.nregions++] = PrefetchRegion{ptr, (unsigned long long)bytes};
+    };
+    for (size_t l = an.tail_first; l < an.levels.size(); ++l) {
+        const Level& L = an.levels[l];
+        const RbVectors<M> v(an, l, in, out);
+        RbTailLevel<M>& t = p.lv[p.nlev++];
+        t.nb = L.nb;
+        t.nr = L.nr;
+        t.n = L.n;
+        t.coarsest = L.coarsest ? 1 : 0;
+        t.pre = L.pre ? 1 : 0;
+        t.m = L.view();
+        t.r = v.r;
+        t.r_red = v.r_red;
+        t.rw = const_cast<double*>(v.r);
+        t.z = v.z;
+        t.y = v.y;
+        t.list = v.list;
+        t.g = v.g;
+        t.up = v.up;
+        if (L.coarsest) {
+            t.inv = level_inv<M>(L);
+            region(t.inv, (int64_t)L.n * L.n * (int64_t)sizeof(M));
+        } else {
+            t.a = level_a<M>(L);
+            t.lu = level_lu<M>(L);
+            region(L.sell_col->ptr, L.sell_size * 4);
+            region(L.sell_len->ptr, (int64_t)L.nb * 4);
+            region(t.a, L.vals * (int64_t)sizeof(M));
+            region(t.lu, L.vals * (int64_t)sizeof(M));
+            region(t.list, (int64_t)an.levels[l + 1].nb * t.g * 4);
+        }
+    }
+    if (an.tail_trace) p.trace = an.tail_trace->as<long long>();
+    p.local_first = p.nlev;
+    int smem = 0;
+    if (an.tail_local[pc_mode<double, M>()] < p.nlev) plan_rb_local<M>(c, an, smem, &p);
+    TailLaunch cfg(c, an.tail_cluster[pc_mode<double, M>()], smem);
+    WITH_BS(an.levels[an.tail_first].bs, WITH_KMAX(an.tail_kmax, launch(c, "rb_tail", [&] {
+                EQG_CUDA(cudaLaunchKernelEx(&cfg.cfg, rb_tail_kernel<BS, KK, M>, p, sc, skip));
+            }, tail_bytes<double, M>(an))));
+}
+
+// out = V-cycle(in) on the black rows, from level l down.
+template <class M>
+void rb_cycle(Core& c, const SolverAnalysis& an, size_t l, const double* in, double* out, const KScal* sc, int skip)
+{
+    if ((int)l == an.tail_first) {
+        launch_rb_tail<M>(c, an, in, out, sc, skip);
+        return;
+    }
+    const Level& L = an.levels[l];
+    const RbVectors<M> v(an, l, in, out);
+    if (L.coarsest) {
+        WITH_BS(L.bs, launch(c, "rb_dense", [&] {
+                    launch_k(c, rb_dense_kernel<BS, M>, 1, 1024, L.n, level_inv<M>(L), v.r, v.up, sc, skip);
+                }, (double)L.n * L.n * sizeof(M) + 2.0 * L.n * sizeof(double)));
+        return;
+    }
+    const Level& C = an.levels[l + 1];
+    double* rc = level_vec<double>(C, 0);
+    const M* a = level_a<M>(L);
+    const M* lu = level_lu<M>(L);
+    const int nr = L.nr, nk = L.nb - L.nr, nt = L.threads;
+    // algorithmic bytes: the stored blocks of a half, row lengths, diagonal
+    // blocks, and every vector element read or written once
+    const double row = 8.0 * L.bs, diag = (double)sizeof(M) * L.bs * L.bs;
+    const double half_u = block_bytes<M>(L, L.stage_upper[0]) + 4.0 * nr, half_l = block_bytes<M>(L, L.stage_lower[1]) + 4.0 * nk;
+    const double red = l == 0 ? 0.0 : row * nr;  // the red right-hand side
+    auto y_rows = [&] {
+        WITH_BS(L.bs, WITH_KMAX(L.kmax, launch(c, "rb_y", [&] {
+                    launch_k(c, rb_y_kernel<BS, KK, M>, blocksFor(nr, nt), nt, nr, L.view(), lu, v.r_red,
+                             (const double*)v.z, v.y, sc, skip);
+                }, half_u + red + row * (nr + nk))));
+    };
+    if (L.pre) {
+        WITH_BS(L.bs, WITH_KMAX(L.kmax, launch(c, "rb_pre", [&] {
+                    launch_k(c, rb_pre_kernel<BS, KK, M>, blocksFor(nk + 31, nt), nt, nr, L.nb, L.view(), lu, v.r,
+                             v.r_red, v.z, sc, skip);
+                }, (l == 0 ? 0.0 : half_l) + red + (diag + 2 * row) * nk)));
+        y_rows();
+        WITH_BS(L.bs, WITH_KMAX(L.kmax, launch(c, "rb_res", [&] {
+                    launch_k(c, rb_res_kernel<BS, KK, M>, blocksFor((int64_t)C.nb * v.g, nt), nt, C.nb, v.g, v.list,
+                             L.view(), a, lu, v.r, (const double*)v.y, (const double*)v.z, rc, sc, skip);
+                }, half_l + (diag + 2 * row) * nk + row * nr + (4.0 * v.g + row) * C.nb)));
+    } else {
+        WITH_BS(L.bs, launch(c, "rb_restrict", [&] {
+                    launch_k(c, rb_restrict_kernel<BS>, blocksFor(C.nb, nt), nt, C.nb, v.g, v.list, v.r, rc, sc, skip);
+                }, row * nk + red + (4.0 * v.g + row) * C.nb));
+    }
+    rb_cycle<M>(c, an, l + 1, in, out, sc, skip);
+    y_rows();
+    const double to_fine = v.up.w ? 4.0 * v.up.g + row * v.up.g * (v.up.add ? 2.0 : 1.0) : 0.0;
+    WITH_BS(L.bs, WITH_KMAX(L.kmax, launch(c, "rb_post", [&] {
+                launch_k(c, rb_post_kernel<BS, KK, M>, blocksFor(nk + 31, nt), nt, nr, L.nb, L.view(), a, lu, v.r,
+                         (const double*)v.y, v.z, v.up, sc, skip);
+            }, half_l + (2 * diag + 3 * row + to_fine) * nk + row * nr)));
+    if (v.up.w == nullptr) return;
+    WITH_BS(L.bs, WITH_KMAX(L.kmax, launch(c, "rb_fin", [&] {
+                launch_k(c, rb_fin_kernel<BS, KK, M>, blocksFor(nr, nt), nt, nr, L.view(), lu, v.r,
+                         (const double*)v.z, v.up, sc, skip);
+            }, half_u + (diag + row + to_fine) * nr + row * nk)));
 }
 
 template <class T, class M>
@@ -2857,8 +3157,9 @@ void tune_file_write(const std::string& path)
     std::rename(tmp.c_str(), path.c_str());
 }
 
-template <class T, class M>
-void autotune(Core& c, SolverAnalysis& an, const T* b, T* out, const KScal* sc)
+// apply() applies the preconditioner once.
+template <class T, class M, class Apply>
+void autotune(Core& c, SolverAnalysis& an, Apply&& apply)
 {
     const int mode = pc_mode<T, M>();
     if (an.tuned[mode]) return;
@@ -2879,6 +3180,7 @@ void autotune(Core& c, SolverAnalysis& an, const T* b, T* out, const KScal* sc)
     key << prop.name << "; n " << an.n << "; nnz " << an.nnz << "; bs " << an.levels[0].bs << "; levels";
     for (auto& L : an.levels) key << " " << L.n;
     key << "; fused from " << an.tail_first << "; precision " << mode;
+    if (an.two_colour) key << "; two colours";
     std::string file = c.param_s("linsolver_tune_file", "");
     if (file.empty() && std::getenv("EQG_TUNE_FILE")) file = std::getenv("EQG_TUNE_FILE");
     {
@@ -2902,11 +3204,11 @@ void autotune(Core& c, SolverAnalysis& an, const T* b, T* out, const KScal* sc)
     EQG_CUDA(cudaEventCreate(&e0));
     EQG_CUDA(cudaEventCreate(&e1));
     auto measure = [&] {
-        precondition<T, M>(c, an, b, out, sc, 0);
+        apply();
         float best = 1e30f;
         for (int rep = 0; rep < 2; ++rep) {
             EQG_CUDA(cudaEventRecord(e0, c.stream));
-            for (int k = 0; k < 4; ++k) precondition<T, M>(c, an, b, out, sc, 0);
+            for (int k = 0; k < 4; ++k) apply();
             EQG_CUDA(cudaEventRecord(e1, c.stream));
             EQG_CUDA(cudaEventSynchronize(e1));
             float ms = 0.f;
@@ -2962,63 +3264,19 @@ void autotune(Core& c, SolverAnalysis& an, const T* b, T* out, const KScal* sc)
     if (!file.empty()) tune_file_write(file);
 }
 
-// BiCGStab on the permuted system with values a; v.b holds the right-hand
-// side.
-template <class T>
-SolveResult bicgstab(Core& c, SolverAnalysis& an, const T* a, Vecs<T> v, double tol, int max_iter, int check_every,
-                     bool pc32 = false)
+// Runs `iteration` (the launches of one BiCGStab iteration) until the device
+// status says to stop; `slot`: the analysis' graph to use.
+template <class Iteration>
+SolveResult run_iterations(Core& c, SolverAnalysis& an, int slot, double tol, int max_iter, int check_every,
+                           Iteration&& iteration)
 {
-    const int n = an.n;
-    const Level& L0 = an.levels[0];
     KScal* sc = an.scal->as<KScal>();
-    double* part = an.partials->as<double>();
-    unsigned int* cnt = an.counter->as<unsigned int>();
-    const int nb = blocksFor(n, kThreads, kRedBlocks);
-    const int nbr = blocksFor(L0.nb, kThreads, kRedBlocks);
-    const double vb = (double)n * sizeof(T);  // one vector
-    const double spmv_bytes = block_bytes<T>(L0, L0.blocks) + 4.0 * L0.nb + 3.0 * vb;
-    launch(c, "bicg_init", [&] {
-        bicg_init_kernel<T><<<nb, kThreads, 0, c.stream>>>(v.b, v.r, v.rhat, v.p, v.v, v.x, n, part, cnt, sc, tol * tol);
-    }, 6.0 * vb);
-    auto iteration = [&] {
-        launch(c, "bicg_p", [&] {
-            launch_k(c, bicg_p_kernel<T>, blocksFor(n), kThreads, (const T*)v.r, (const T*)v.v, v.p, n,
-                     (const KScal*)sc);
-        }, 4.0 * vb);
-        apply_pc<T>(c, an, v.p, v.ph, sc, 0, pc32);
-        WITH_BS(L0.bs, WITH_KMAX(L0.kmax, launch(c, "bicg_spmv_alpha", [&] {
-                    launch_k(c, bicg_spmv_alpha_kernel<BS, KK, T>, nbr, kThreads, L0.view(), a, (const T*)v.ph,
-                             (const T*)v.rhat, v.v, L0.nb, part, cnt, sc);
-                }, spmv_bytes)));
-        launch(c, "bicg_s", [&] {
-            launch_k(c, bicg_s_kernel<T>, nb, kThreads, (const T*)v.r, (const T*)v.v, v.s, n, part, cnt, sc);
-        }, 3.0 * vb);
-        apply_pc<T>(c, an, v.s, v.sh, sc, 1, pc32);
-        WITH_BS(L0.bs, WITH_KMAX(L0.kmax, launch(c, "bicg_spmv_omega", [&] {
-                    launch_k(c, bicg_spmv_omega_kernel<BS, KK, T>, nbr, kThreads, L0.view(), a, (const T*)v.sh,
-                             (const T*)v.s, v.t, L0.nb, part, cnt, sc);
-                }, spmv_bytes)));
-        launch(c, "bicg_xr", [&] {
-            launch_k(c, bicg_xr_kernel<T>, nb, kThreads, (const T*)v.ph, (const T*)v.sh, (const T*)v.s,
-                     (const T*)v.t, (const T*)v.rhat, v.x, v.r, n, part, cnt, sc);
-        }, 8.0 * vb);
-    };
-    // launch shapes of the preconditioner, once per analysis and precision
-    // (before the graph capture below)
-    if (an.multigrid || an.levels[0].n > 0) {
-        if constexpr (sizeof(T) == sizeof(double)) {
-            if (pc32) autotune<double, float>(c, an, v.b, v.ph, sc);
-            else autotune<double, double>(c, an, v.b, v.ph, sc);
-        } else {
-            autotune<float, float>(c, an, v.b, v.ph, sc);
-        }
-    }
     // Graph of `check_every` iterations, captured once per analysis and
     // precision; kernel arguments are fixed (buffers of the analysis,
     // scalars in device memory).  Kernel timing (time_kernel) needs one
     // event pair per launch, so timed runs launch eagerly.
     const bool graphs = c.timed_kernel.empty() && c.param_i("linsolver_graphs", 1) != 0;
-    SolverAnalysis::IterGraph& g = an.graph[sizeof(T) == sizeof(double) ? (pc32 ? 2 : 0) : 1];
+    SolverAnalysis::IterGraph& g = an.graph[slot];
     if (graphs && (!g.exec || g.chunk != check_every)) {
         if (g.exec) {
             cudaGraphExecDestroy(g.exec);
@@ -3067,6 +3325,122 @@ SolveResult bicgstab(Core& c, SolverAnalysis& an, const T* a, Vecs<T> v, double 
     res.iterations = h.iterations;
     const double b2 = tol > 0 ? h.thr / (tol * tol) : 0.0;
     res.rel_residual = b2 > 0 ? std::sqrt(h.rr / b2) : 0.0;
+    return res;
+}
+
+// BiCGStab on the permuted system with values a; v.b holds the right-hand
+// side.
+template <class T>
+SolveResult bicgstab(Core& c, SolverAnalysis& an, const T* a, Vecs<T> v, double tol, int max_iter, int check_every,
+                     bool pc32 = false)
+{
+    const int n = an.n;
+    const Level& L0 = an.levels[0];
+    KScal* sc = an.scal->as<KScal>();
+    double* part = an.partials->as<double>();
+    unsigned int* cnt = an.counter->as<unsigned int>();
+    const int nb = blocksFor(n, kThreads, kRedBlocks);
+    const int nbr = blocksFor(L0.nb, kThreads, kRedBlocks);
+    const double vb = (double)n * sizeof(T);  // one vector
+    const double spmv_bytes = block_bytes<T>(L0, L0.blocks) + 4.0 * L0.nb + 3.0 * vb;
+    launch(c, "bicg_init", [&] {
+        bicg_init_kernel<T><<<nb, kThreads, 0, c.stream>>>(v.b, v.r, v.rhat, v.p, v.v, v.x, n, part, cnt, sc, tol * tol);
+    }, 6.0 * vb);
+    auto iteration = [&] {
+        launch(c, "bicg_p", [&] {
+            launch_k(c, bicg_p_kernel<T>, blocksFor(n), kThreads, (const T*)v.r, (const T*)v.v, v.p, n,
+                     (const KScal*)sc);
+        }, 4.0 * vb);
+        apply_pc<T>(c, an, v.p, v.ph, sc, 0, pc32);
+        WITH_BS(L0.bs, WITH_KMAX(L0.kmax, launch(c, "bicg_spmv_alpha", [&] {
+                    launch_k(c, bicg_spmv_alpha_kernel<BS, KK, T>, nbr, kThreads, L0.view(), a, (const T*)v.ph,
+                             (const T*)v.rhat, v.v, L0.nb, part, cnt, sc);
+                }, spmv_bytes)));
+        launch(c, "bicg_s", [&] {
+            launch_k(c, bicg_s_kernel<T>, nb, kThreads, (const T*)v.r, (const T*)v.v, v.s, n, part, cnt, sc);
+        }, 3.0 * vb);
+        apply_pc<T>(c, an, v.s, v.sh, sc, 1, pc32);
+        WITH_BS(L0.bs, WITH_KMAX(L0.kmax, launch(c, "bicg_spmv_omega", [&] {
+                    launch_k(c, bicg_spmv_omega_kernel<BS, KK, T>, nbr, kThreads, L0.view(), a, (const T*)v.sh,
+                             (const T*)v.s, v.t, L0.nb, part, cnt, sc);
+                }, spmv_bytes)));
+        launch(c, "bicg_xr", [&] {
+            launch_k(c, bicg_xr_kernel<T>, nb, kThreads, (const T*)v.ph, (const T*)v.sh, (const T*)v.s,
+                     (const T*)v.t, (const T*)v.rhat, v.x, v.r, n, part, cnt, sc);
+        }, 8.0 * vb);
+    };
+    // launch shapes of the preconditioner, once per analysis and precision
+    // (before the graph capture below)
+    if (an.multigrid || an.levels[0].n > 0) {
+        if constexpr (sizeof(T) == sizeof(double)) {
+            if (pc32) autotune<double, float>(c, an, [&] { precondition<double, float>(c, an, v.b, v.ph, sc, 0); });
+            else autotune<double, double>(c, an, [&] { precondition<double, double>(c, an, v.b, v.ph, sc, 0); });
+        } else {
+            autotune<float, float>(c, an, [&] { precondition<float, float>(c, an, v.b, v.ph, sc, 0); });
+        }
+    }
+    return run_iterations(c, an, sizeof(T) == sizeof(double) ? (pc32 ? 2 : 0) : 1, tol, max_iter, check_every, iteration);
+}
+
+// BiCGStab on the black half of the system (twocolour.cuh), M the type of
+// the preconditioner's matrices.  `b`: the right-hand side in block-row order;
+// the solution goes to `xout` in the natural order.
+template <class M>
+SolveResult bicgstab_rb(Core& c, SolverAnalysis& an, const double* b, double* xout, double tol, int max_iter,
+                        int check_every)
+{
+    const Level& L0 = an.levels[0];
+    const int nr = L0.nr, nk = L0.nb - L0.nr, n = nk * L0.bs;
+    const Vecs<double> v = vecs<double>(an.vec64->as<double>() + vec_stride(an.n), n);
+    KScal* sc = an.scal->as<KScal>();
+    double* part = an.partials->as<double>();
+    unsigned int* cnt = an.counter->as<unsigned int>();
+    const double* a = L0.as64->as<double>();
+    const double* lu = L0.lus64->as<double>();
+    double* y = level_vec<double>(L0, 0);
+    const int nbv = blocksFor(n, kThreads, kRedBlocks), nbk = blocksFor(nk + 31, kThreads, kRedBlocks);
+    const double vb = 8.0 * n, yb = 8.0 * nr * L0.bs, diag = 8.0 * L0.bs * L0.bs;
+    const double half_u = block_bytes<double>(L0, L0.stage_upper[0]) + 4.0 * nr;
+    const double half_l = block_bytes<double>(L0, L0.stage_lower[1]) + 4.0 * nk;
+    WITH_BS(L0.bs, WITH_KMAX(L0.kmax, launch(c, "rb_init", [&] {
+                rb_init_kernel<BS, KK><<<blocksFor(L0.nb, kThreads, kRedBlocks), kThreads, 0, c.stream>>>(
+                    nr, L0.nb, L0.view(), lu, b, v.r, v.rhat, v.p, v.v, v.x, part, cnt, sc, tol * tol);
+            }, half_l + vb * 6.0 + yb)));
+    auto product = [&](const double* z, const double* h, double* out, bool omega) {
+        WITH_BS(L0.bs, WITH_KMAX(L0.kmax, launch(c, "rb_spmv_y", [&] {
+                    launch_k(c, rb_y_kernel<BS, KK, double>, blocksFor(nr, L0.threads), L0.threads, nr, L0.view(), lu,
+                             (const double*)nullptr, z - (int64_t)nr * L0.bs, y, (const KScal*)sc, (int)omega);
+                }, half_u + vb + yb)));
+        WITH_BS(L0.bs, WITH_KMAX(L0.kmax, launch(c, omega ? "rb_spmv_omega" : "rb_spmv_alpha", [&] {
+                    launch_k(c, omega ? rb_spmv_kernel<BS, KK, true> : rb_spmv_kernel<BS, KK, false>, nbk, kThreads,
+                             nr, L0.nb, L0.view(), a, lu, z, (const double*)y, h, out, part, cnt, sc);
+                }, half_l + diag * nk + yb + 3.0 * vb)));
+    };
+    auto iteration = [&] {
+        launch(c, "bicg_p", [&] {
+            launch_k(c, bicg_p_kernel<double>, blocksFor(n), kThreads, (const double*)v.r, (const double*)v.v, v.p, n,
+                     (const KScal*)sc);
+        }, 4.0 * vb);
+        rb_cycle<M>(c, an, 0, v.p, v.ph, sc, 0);
+        product(v.ph, v.rhat, v.v, false);
+        launch(c, "bicg_s", [&] {
+            launch_k(c, bicg_s_kernel<double>, nbv, kThreads, (const double*)v.r, (const double*)v.v, v.s, n, part, cnt,
+                     sc);
+        }, 3.0 * vb);
+        rb_cycle<M>(c, an, 0, v.s, v.sh, sc, 1);
+        product(v.sh, v.s, v.t, true);
+        launch(c, "bicg_xr", [&] {
+            launch_k(c, bicg_xr_kernel<double>, nbv, kThreads, (const double*)v.ph, (const double*)v.sh,
+                     (const double*)v.s, (const double*)v.t, (const double*)v.rhat, v.x, v.r, n, part, cnt, sc);
+        }, 8.0 * vb);
+    };
+    autotune<double, M>(c, an, [&] { rb_cycle<M>(c, an, 0, v.r, v.ph, sc, 0); });
+    const SolveResult res =
+        run_iterations(c, an, sizeof(M) == sizeof(double) ? 0 : 2, tol, max_iter, check_every, iteration);
+    WITH_BS(L0.bs, WITH_KMAX(L0.kmax, launch(c, "rb_solution", [&] {
+                rb_solution_kernel<BS, KK><<<blocksFor(L0.nb), kThreads, 0, c.stream>>>(
+                    nr, L0.nb, L0.view(), lu, b, v.x, L0.perm->as<int>(), xout);
+            }, half_u + diag * nr + vb + 3.0 * yb + vb)));
     return res;
 }
 
@@ -3122,7 +3496,7 @@ SolveResult solve_with(Core& c, const PatternP& p, std::shared_ptr<SolverAnalysi
     // time per step)
     const int check_every = std::max(1, c.param_i("linsolver_check_every", 4));
 
-    if (!slot || slot->natural != natural) slot = analyse(c, *p, natural, allow_multigrid);
+    if (!slot || slot->natural != natural) slot = analyse(c, *p, natural, allow_multigrid, jval);
     c.pdl_launch = c.param_i("linsolver_pdl", 1) != 0;
     SolverAnalysis& an = *slot;
     SolveResult res;
@@ -3135,41 +3509,22 @@ SolveResult solve_with(Core& c, const PatternP& p, std::shared_ptr<SolverAnalysi
     // level matrices and their factorizations (FP64)
     c.factor_clock.start(c.stream);
     const Level& L0 = an.levels[0];
-    launch(c, "gather_values", [&] {
-        // gather_rows=1: one block row per thread (measured slower on the
-        // 128x128x64 Jacobian: 0.74 against 0.64 ms per gather)
-        if (c.param_i("gather_rows", 0) != 0) {
-            const int* sp = L0.sell_ptr->as<int>();
-            if (L0.bs == 1)
-                gather_rows_kernel<1><<<blocksFor(L0.nb + 32), kThreads, 0, c.stream>>>(L0.nb, sp, jval, an.vmap->as<int>(),
-                                                                                  L0.as64->as<double>());
-            else if (L0.bs == 2)
-                gather_rows_kernel<4><<<blocksFor(L0.nb + 32), kThreads, 0, c.stream>>>(L0.nb, sp, jval, an.vmap->as<int>(),
-                                                                                  L0.as64->as<double>());
-            else
-                gather_rows_kernel<9><<<blocksFor(L0.nb + 32), kThreads, 0, c.stream>>>(L0.nb, sp, jval, an.vmap->as<int>(),
-                                                                                  L0.as64->as<double>());
-        } else {
-            gather_values_kernel<<<blocksFor(L0.vals), kThreads, 0, c.stream>>>(jval, an.vmap->as<int>(),
-                                                                                L0.as64->as<double>(), L0.vals);
-        }
-    }, 12.0 * L0.vals + 8.0 * an.nnz);
+    gather_level0(c, an, jval);
     for (size_t l = 1; l < an.levels.size(); ++l) {
         const Level& F = an.levels[l - 1];
         const Level& C = an.levels[l];
-        EQG_CUDA(cudaMemsetAsync(C.as64->ptr, 0, (size_t)C.vals * sizeof(double), c.stream));
-        // the finer level's entries and their gather indices once, the
-        // coarse entries (list bounds, position, value) once
+        // the finer level's blocks and their slot numbers once, the coarse
+        // blocks (list bounds, values) once
         launch(c, "mg_galerkin", [&] {
-            galerkin_kernel<<<blocksFor(C.nnz), kThreads, 0, c.stream>>>(C.nnz, C.gptr->as<int>(), C.gidx->as<int>(),
-                                                                         C.gpos->as<int>(), F.as64->as<double>(),
-                                                                         C.as64->as<double>());
-        }, 12.0 * F.nnz + 16.0 * C.nnz);
+            slot_sums_kernel<<<blocksFor(C.vals), kThreads, 0, c.stream>>>(C.sell_size, C.bs * C.bs, C.gptr->as<int>(),
+                                                                          C.gidx->as<int>(), F.as64->as<double>(),
+                                                                          C.as64->as<double>());
+        }, block_bytes<double>(F, F.blocks) + 4.0 * C.sell_size + 8.0 * C.vals);
     }
     for (auto& L : an.levels)
         if (L.ap_slots > 0) {
             launch(c, "mg_ap_values", [&] {
-                ap_values_kernel<<<blocksFor(L.ap_slots * L.bs * L.bs), kThreads, 0, c.stream>>>(
+                slot_sums_kernel<<<blocksFor(L.ap_slots * L.bs * L.bs), kThreads, 0, c.stream>>>(
                     L.ap_slots, L.bs * L.bs, L.ap_gptr->as<int>(), L.ap_gidx->as<int>(), L.as64->as<double>(),
                     L.ap64->as<double>());
             }, block_bytes<double>(L, L.blocks) + 8.0 * L.ap_slots + 8.0 * L.bs * L.bs * L.ap_slots);
@@ -3193,6 +3548,7 @@ SolveResult solve_with(Core& c, const PatternP& p, std::shared_ptr<SolverAnalysi
         }
     }
     Vecs<double> v = vecs<double>(an.vec64->as<double>(), n);
+    if (an.two_colour) v.b = an.vec64->as<double>();
     launch(c, "permute",
            [&] { permute_kernel<<<blocksFor(n), kThreads, 0, c.stream>>>(rhs, L0.perm->as<int>(), v.b, n); },
            20.0 * n);
@@ -3218,7 +3574,11 @@ SolveResult solve_with(Core& c, const PatternP& p, std::shared_ptr<SolverAnalysi
     if (fstat) return res;  // zero pivot
     c.krylov_clock.start(c.stream);
 
-    if (!refine) {
+    if (an.two_colour) {
+        res = mixed ? bicgstab_rb<float>(c, an, v.b, xout, tol, max_iter, check_every)
+                    : bicgstab_rb<double>(c, an, v.b, xout, tol, max_iter, check_every);
+        res.sweeps = 1;
+    } else if (!refine) {
         res = bicgstab<double>(c, an, L0.as64->as<double>(), v, tol, max_iter, check_every, mixed);
         res.sweeps = 1;
     } else {
@@ -3270,9 +3630,10 @@ SolveResult solve_with(Core& c, const PatternP& p, std::shared_ptr<SolverAnalysi
     }
     c.krylov_clock.stop(c.stream);
     report_tail_trace(c, an);
-    launch(c, "unpermute",
-           [&] { unpermute_kernel<<<blocksFor(n), kThreads, 0, c.stream>>>(v.x, L0.perm->as<int>(), xout, n); },
-           20.0 * n);
+    if (!an.two_colour)
+        launch(c, "unpermute",
+               [&] { unpermute_kernel<<<blocksFor(n), kThreads, 0, c.stream>>>(v.x, L0.perm->as<int>(), xout, n); },
+               20.0 * n);
     res.block_size = L0.bs;
     res.blocks = L0.blocks;
     return res;

@@ -126,9 +126,10 @@ const char* eqg_backend_name(void);
  * levels up to this size run as one kernel; 0: none), linsolver_mg_cluster
  * (16: thread blocks of that kernel's cluster, at most 16),
  * linsolver_mg_alpha (factor of the coarse-grid correction z += alpha P zc;
- * 1.4 on 3D grids, 1.9 on 2D grids), linsolver_mg_ap_rows (40000: levels
- * with more unknowns correct their residual through A P instead of
- * recomputing r - A z), linsolver_mg_coarsest (128: coarsening stops at
+ * 1.9 for 2 x 2 aggregates of 2D grids, else 1.4), linsolver_mg_ap_rows
+ * (40000: levels with more unknowns correct their residual through A P
+ * instead of recomputing r - A z; where the sweeps run over more than two
+ * stages), linsolver_mg_coarsest (128: coarsening stops at
  * this many unknowns, at most 128; that level is solved with a dense
  * inverse), linsolver_pdl (1: the BiCGStab iteration's kernels
  * as programmatic dependent launches; 0: plain launches), linsolver_mg_local (1: that kernel keeps its coarsest levels in one thread
@@ -150,7 +151,7 @@ const char* eqg_backend_name(void);
  * $EQG_TUNE_FILE, else none), spgemm_plan / span_share / jac_concat /
  * jac_defer / stencil_ops (1; 0 switches off an assembly fast path, for
  * comparisons),
- * gather_rows (0), flush_l2 (0; n: n MB written before each Newton solve's
+ * flush_l2 (0; n: n MB written before each Newton solve's
  * start mark, so that a solve timed between its marks starts with a cold L2),
  * time_kernel
  * (a kernel name, or "*", to time with CUDA events) and device (CUDA device
