@@ -1086,39 +1086,6 @@ __global__ void sumsq_kernel(const double* __restrict__ a, int n, double* partia
 }
 
 // ---- multilevel preconditioner kernels -------------------------------------
-// Strengths of the couplings by direction (see direction_strengths).
-__global__ void direction_strength_kernel(int nb, int bs, SellView m, const double* __restrict__ a,
-                                          const int* __restrict__ perm, int nx, int ny, int nc, double* partials,
-                                          unsigned int* counter, double* out)
-{
-    double d[3] = {0.0, 0.0, 0.0};
-    const int bb = bs * bs;
-    GRID_STRIDE(r, nb)
-    {
-        const int R = (int)r, lane = R & 31, sb = m.slice_ptr[R >> 5], len = m.len[R];
-        const int u = perm[R * bs], comp = u / nc, cell = u - comp * nc;
-        const int i = cell % nx, j = (cell / nx) % ny, k = cell / (nx * ny);
-        for (int c = 0; c < bs; ++c) {
-            double s[3] = {0.0, 0.0, 0.0}, diag = 0.0;
-            for (int t = 0; t < len; ++t) {
-                const int q = sb + (t << 5) + lane, v = perm[m.col[q] * bs], vcomp = v / nc, vcell = v - vcomp * nc;
-                if (vcomp != comp) continue;
-                const double x = fabs(a[(size_t)q * bb + c * bs + c]);
-                if (vcell == cell) diag = x;
-                else s[vcell / (nx * ny) != k ? 2 : (vcell / nx) % ny != j ? 1 : 0] += x;
-            }
-            const double sum = s[0] + s[1] + s[2];
-            if (!(sum > 0.0) || !(diag > 0.0) || !isfinite(sum / diag)) continue;
-            const double w = fmin(1.0, sum / diag) / sum;
-            for (int e = 0; e < 3; ++e) d[e] += w * s[e];
-        }
-        (void)i;
-    }
-    double s[3];
-    if (grid_sum<3>(d, partials, counter, s))
-        for (int e = 0; e < 3; ++e) out[e] = s[e];
-}
-
 template <int B, int KM, class T, class M>
 __global__ void mg_residual_kernel(int nb, int r_zero, SellView m, const M* __restrict__ a, const T* __restrict__ x,
                                    const T* __restrict__ b, T* __restrict__ out, const KScal* sc, int skip_if_s)
@@ -1207,8 +1174,8 @@ __global__ void slot_sums_kernel(int64_t slots, int bb, const int* __restrict__ 
     }
 }
 
-// Inverse of the coarsest matrix (n <= kCoarsest unknowns), one thread block,
-// in place in shared memory: Gauss-Jordan elimination with partial pivoting
+// Inverse of the coarsest matrix (n <= kCoarsest unknowns, dense, row-major),
+// in place, by one thread block in shared memory: Gauss-Jordan elimination with partial pivoting
 // (Numerical Recipes, gaussj, row pivots only).  Per pivot k: a warp finds
 // the largest |a_rk|, r >= k (the lowest r among equals) while every thread
 // copies column k; rows k and p are swapped and row k is divided by the
@@ -1218,27 +1185,30 @@ __global__ void slot_sums_kernel(int64_t slots, int bb, const int* __restrict__ 
 // is written out.  A zero or non-finite pivot sets *status.
 constexpr int kCoarsest = 128;
 
+// The dense matrix of a level in the block sliced layout; `dense` is zero
+// beforehand.
 template <int B>
-__global__ void __launch_bounds__(1024) dense_inverse_kernel(int nb, SellView m, const double* __restrict__ a,
-                                                             double* __restrict__ inv, int* status)
+__global__ void dense_fill_kernel(int nb, SellView m, const double* __restrict__ a, double* __restrict__ dense)
 {
-    constexpr int BB = B * B;
-    extern __shared__ __align__(16) double dsm[];
     const int n = nb * B;
+    GRID_STRIDE(r, nb)
+    {
+        const int R = (int)r, lane = R & 31, sb = m.slice_ptr[R >> 5];
+        for (int k = 0; k < m.len[R]; ++k) {
+            const int q = sb + (k << 5) + lane, J = m.col[q];
+            for (int e = 0; e < B * B; ++e) dense[(R * B + e / B) * n + J * B + e % B] = a[(size_t)q * B * B + e];
+        }
+    }
+}
+
+__global__ void __launch_bounds__(1024) dense_inverse_kernel(int n, double* __restrict__ a, int* status)
+{
+    extern __shared__ __align__(16) double dsm[];
     double* w = dsm;                  // n x n, row-major
     double* colk = dsm + n * n;       // column k before the row swap
     __shared__ int piv_row;
     __shared__ int perm[kCoarsest];   // row swapped with k at step k
-    for (int i = threadIdx.x; i < n * n; i += blockDim.x) w[i] = 0.0;
-    __syncthreads();
-    for (int R = threadIdx.x; R < nb; R += blockDim.x) {
-        const int lane = R & 31, sb = m.slice_ptr[R >> 5];
-        for (int k = 0; k < m.len[R]; ++k) {
-            const int J = m.col[sb + (k << 5) + lane];
-            for (int i = 0; i < B; ++i)
-                for (int j = 0; j < B; ++j) w[(R * B + i) * n + J * B + j] = a[(size_t)(sb + (k << 5) + lane) * BB + i * B + j];
-        }
-    }
+    for (int i = threadIdx.x; i < n * n; i += blockDim.x) w[i] = a[i];
     __syncthreads();
     for (int k = 0; k < n; ++k) {
         for (int r = threadIdx.x; r < n; r += blockDim.x) colk[r] = w[r * n + k];
@@ -1301,7 +1271,7 @@ __global__ void __launch_bounds__(1024) dense_inverse_kernel(int nb, SellView m,
     __syncthreads();
     for (int i = threadIdx.x; i < n * n; i += blockDim.x) {
         const int r = i / n, j = i - r * n;
-        inv[i] = w[r * n + src[j]];
+        a[i] = w[r * n + src[j]];
     }
 }
 
@@ -1623,13 +1593,16 @@ __global__ void __launch_bounds__(kTailThreads)
 // Multilevel preconditioner (the default when the system is laid out as
 // `ncomp` blocks of one unknown per grid cell, as newtonSolve and
 // newtonSolveSystem stack them): geometric aggregation of cells per unknown
-// block, in pairs along the directions that are strong enough (kSemiCoarsen),
-// Galerkin coarse matrices R A R^T, a V cycle with a block ILU(0) sweep after
-// the coarse correction on every level and one before it where the aggregates
-// are more than pairs (after pairing along the strong direction alone, the
-// sweep before it changes the iteration count by less than one in seventeen),
-// and a dense inverse on the coarsest level (<= 128 unknowns).  The analysis
-// works on the block graph; otherwise plain block ILU(0).
+// block, Galerkin coarse matrices R A R^T, a V cycle with a block ILU(0) sweep
+// before and after the coarse correction, and a dense inverse on the coarsest
+// level (<= 128 unknowns); otherwise plain block ILU(0).  The two-colour form
+// (twocolour.cuh) needs nothing from the host: its hierarchy follows from the
+// grid, and the device maps the Jacobian's entries.  It pairs cells along the
+// directions that are strong enough only (kSemiCoarsen), and smooths before
+// the correction only where the aggregates are more than pairs (after pairing
+// along the strong direction alone, that sweep changes the iteration count by
+// less than one in seventeen).  Everything else works on the block graph on
+// the host.
 // ---------------------------------------------------------------------------
 struct HostCsr {
     int n = 0;
@@ -1650,13 +1623,6 @@ struct Level {
     Buf perm;                      // permuted unknown position -> natural unknown
     Buf gptr, gidx;                // Galerkin sums: the finer level's slots of each slot (levels > 0)
     double alpha = 1.0;            // factor of the correction from the next coarser level
-    // two-colour form: red block rows, whether the level pre-smooths, and
-    // its block rows by aggregate (next coarser block row): the black ones
-    // (members_b, gb per aggregate, -1 past the last) and all (members_a, ga)
-    int nr = 0;
-    bool pre = true;
-    int gb = 0, ga = 0;
-    Buf members_b, members_a;
     Buf aggb;                      // coarse block row of each block row (next coarser level)
     // A P (see mg_correct_kernel), in the same sliced layout: slots, the
     // longest row, slices, coarse block columns, row lengths, and the A slots
@@ -1690,13 +1656,31 @@ struct Level {
     Buf inv64, inv32;              // coarsest level
 };
 
+// A level of the two-colour form (twocolour.cuh).
+struct RbLevel {
+    RbGrid g;
+    Aggregates agg;          // to the next coarser level
+    int n = 0;               // unknowns
+    int64_t vals = 0;        // values of the matrix (RbMatrix)
+    bool coarsest = false;
+    bool pre = true;         // smooths before the coarse correction
+    double alpha = 1.0;      // factor of the correction from the next coarser level
+    int threads = kThreads;  // threads per block of this level's launch-per-step kernels (autotuned)
+    Buf a64, a32;            // matrix, then its factors
+    Buf inv64, inv32;        // coarsest level
+    Buf v64;                 // right-hand side; red work vector and black iterate
+};
+
 struct SolverAnalysis {
     int n = 0;
     int64_t nnz = 0;
     bool natural = false;
     bool ok = true;  // every row has a diagonal entry (1 x 1 blocks)
     bool multigrid = false;
-    bool two_colour = false;  // every level but the coarsest has two stages (twocolour.cuh)
+    // the two-colour form's levels (twocolour.cuh; none: the levels above),
+    // its block size and number of directions
+    std::vector<RbLevel> rb;
+    int rb_bs = 1, rb_nd = 4;
     std::vector<Level> levels;
     Buf vmap;        // level-0 value <- Jacobian entry (-1: zero)
     Buf vec64, vec32, scal, partials, counter, factor_status;
@@ -2073,35 +2057,7 @@ void gather_level0(Core& c, const SolverAnalysis& an, const double* jval)
     }, 12.0 * L0.vals + 8.0 * an.nnz);
 }
 
-// Mean share of the same-component couplings of a block row that each
-// direction of the level-0 grid has, weighted by how strongly the row is
-// coupled at all (shares of the diagonal, at most 1): the strengths the
-// aggregation follows.
-void direction_strengths(Core& c, const Level& L, double (&s)[3])
-{
-    const int nblk = blocksFor(L.nb, kThreads, kRedBlocks);
-    Buf part = c.allocN<double>((size_t)nblk * 3 + 3);
-    Buf counter = c.allocN<unsigned int>(1);
-    EQG_CUDA(cudaMemsetAsync(counter->ptr, 0, sizeof(unsigned int), c.stream));
-    double* out = part->as<double>() + (size_t)nblk * 3;
-    launch(c, "mg_strength", [&] {
-        direction_strength_kernel<<<nblk, kThreads, 0, c.stream>>>(
-            L.nb, L.bs, L.view(), L.as64->as<double>(), L.perm->as<int>(), c.nx, c.ny, c.nc, part->as<double>(),
-            counter->as<unsigned int>(), out);
-    });
-    EQG_CUDA(cudaMemcpyAsync(c.pinned, out, 3 * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-    c.sync();
-    for (int d = 0; d < 3; ++d) s[d] = c.pinned[d];
-}
-
-// Levels are coarsened only along the directions at least 1 / kSemiCoarsen
-// as strong as the strongest one: the point smoothers do not reduce error
-// that varies slowly along a strong direction and quickly along a weak one.
-// BiCGStab iterations of a two-phase solve on 48 x 48 x 32 cells of 10 x 10 x
-// 2 m (strengths 25 : 1 : 1): 38 with 2 x 2 x 2 aggregates on every level, 21
-// with one z-pairing level first, 17 with two (then 2 x 2 x 2 at 6.25 : 1),
-// 18 with three.  At 4 : 1 one z-pairing level and none are equal.
-constexpr double kSemiCoarsen = 6.5;
+bool rb_analyse(Core& c, SolverAnalysis& an, const Pattern& p, int bs, int coarsest, const double* jval);
 
 std::shared_ptr<SolverAnalysis> analyse(Core& c, const Pattern& p, bool natural, bool allow_multigrid,
                                         const double* jval)
@@ -2119,12 +2075,16 @@ std::shared_ptr<SolverAnalysis> analyse(Core& c, const Pattern& p, bool natural,
     an->n = n;
     an->nnz = p.nnz;
     an->natural = natural;
+    an->scal = c.alloc(sizeof(KScal));
+    an->factor_status = c.allocN<int>(1);
     HostCsr A;
     A.n = n;
-    A.ptr.resize(n + 1);
-    A.col.resize(p.nnz > 0 ? p.nnz : 1);
-    c.copy_to_host(A.ptr.data(), p.rowptr->ptr, (size_t)(n + 1) * 4);
-    if (p.nnz > 0) c.copy_to_host(A.col.data(), p.colind->ptr, (size_t)p.nnz * 4);
+    auto read_pattern = [&] {
+        A.ptr.resize(n + 1);
+        A.col.resize(p.nnz > 0 ? p.nnz : 1);
+        c.copy_to_host(A.ptr.data(), p.rowptr->ptr, (size_t)(n + 1) * 4);
+        if (p.nnz > 0) c.copy_to_host(A.col.data(), p.colind->ptr, (size_t)p.nnz * 4);
+    };
 
     const std::string pre = c.param_s("linsolver_preconditioner", "multigrid");
     if (pre != "multigrid" && pre != "ilu0") fail(EQG_ERR_ARG, "linsolver_preconditioner must be multigrid or ilu0");
@@ -2144,6 +2104,13 @@ std::shared_ptr<SolverAnalysis> analyse(Core& c, const Pattern& p, bool natural,
         (!natural && fp64_vectors && (ncomp == 2 || ncomp == 3) && c.param_i("linsolver_block", 1) != 0) ? ncomp
                                                                                                           : 1;
 
+    // the two-colour form: every unknown of a cell in its block, FP64 vectors,
+    // the default ordering, face neighbours only
+    if (mg_wanted && !natural && fp64_vectors && bs == ncomp && rb_analyse(c, *an, p, bs, coarsest, jval)) {
+        if (c.verbose > 2) std::printf("        linear solver analysis: %.1f ms\n", since());
+        return an;
+    }
+    read_pattern();
     an->levels.emplace_back();
     const double t_copy = since();
     // levels small enough for the fused coarse cycle get slices of uniform width
@@ -2185,32 +2152,18 @@ std::shared_ptr<SolverAnalysis> analyse(Core& c, const Pattern& p, bool natural,
     const double t_level0 = since();
     an->multigrid = mg_wanted && an->ok;
     if (an->multigrid) {
-        double strength[3] = {1.0, 1.0, 1.0};
-        if ((c.nx > 1) + (c.ny > 1) + (c.nz > 1) > 1) {
-            gather_level0(c, *an, jval);
-            direction_strengths(c, an->levels[0], strength);
-        }
         int dims[3] = {c.nx, c.ny, c.nz};
         const int ncn = fine.n / c.nc;  // nodes of the block graph per cell (1 with blocks of all components)
         for (;;) {
             const double tl0 = since();
             Level& F = an->levels.back();
-            // aggregates: pairs of cells along every direction strong enough
+            // aggregates: pairs of cells along every direction
             int f[3], cdims[3];
-            double top = 0.0;
-            for (int d = 0; d < 3; ++d)
-                if (dims[d] > 1) top = std::max(top, strength[d]);
-            int cut = 0;
             for (int d = 0; d < 3; ++d) {
-                f[d] = dims[d] > 1 && !(strength[d] * kSemiCoarsen < top) ? 2 : 1;
+                f[d] = dims[d] > 1 ? 2 : 1;
                 cdims[d] = (dims[d] + f[d] - 1) / f[d];
-                cut += f[d] == 2;
             }
-            // couplings of a coarse cell: twice as many fine ones per other
-            // direction that was paired
-            for (int d = 0; d < 3; ++d) strength[d] *= std::ldexp(1.0, cut - (f[d] == 2));
-            F.alpha = c.param_d("linsolver_mg_alpha", cut == 2 && c.nz == 1 ? kMgAlpha2d : kMgAlpha3d);
-            F.pre = cut > 1;
+            F.alpha = c.param_d("linsolver_mg_alpha", c.nz > 1 ? kMgAlpha3d : kMgAlpha2d);
             const int fcells = dims[0] * dims[1] * dims[2], ccells = cdims[0] * cdims[1] * cdims[2];
             const int ncb = ncn * ccells;  // coarse block rows
             std::vector<int> agg(fine.n);
@@ -2247,33 +2200,11 @@ std::shared_ptr<SolverAnalysis> analyse(Core& c, const Pattern& p, bool natural,
             order_level(c, coarse, natural, bs, ncb * bs <= fuse_rows, Lc, cpb, cipb, cslot);
             Lc.nnz = (int64_t)coarse.ptr[ncb] * bs * bs;
             const double tl2 = since();
-            // coarse block row of every fine one, and the members of every
-            // coarse block row, in positions (ascending)
+            // coarse block row of every fine one, in positions
             Lf.h_aggb.resize(fine.n);
 #pragma omp parallel for schedule(static) if (fine.n > kSerialRows)
             for (int R = 0; R < fine.n; ++R) Lf.h_aggb[R] = cipb[agg[pb[R]]];
             Lf.aggb = upload_ints(c, Lf.h_aggb);
-            Lf.nr = Lf.stage_ptr.size() > 1 ? Lf.stage_ptr[1] : 0;
-            {
-                auto pow2 = [](int v) {
-                    int g = 1;
-                    while (g < v) g *= 2;
-                    return g;
-                };
-                std::vector<int> nblack(ncb, 0);
-                for (int R = Lf.nr; R < Lf.nb; ++R) nblack[Lf.h_aggb[R]]++;
-                Lf.ga = pow2(max_members);
-                Lf.gb = pow2(*std::max_element(nblack.begin(), nblack.end()));
-                std::vector<int> ma((size_t)ncb * Lf.ga, -1), mb((size_t)ncb * Lf.gb, -1), na(ncb, 0);
-                std::fill(nblack.begin(), nblack.end(), 0);
-                for (int R = 0; R < Lf.nb; ++R) {
-                    const int P = Lf.h_aggb[R];
-                    ma[(size_t)P * Lf.ga + na[P]++] = R;
-                    if (R >= Lf.nr) mb[(size_t)P * Lf.gb + nblack[P]++] = R;
-                }
-                Lf.members_a = upload_ints(c, ma);
-                Lf.members_b = upload_ints(c, mb);
-            }
             const double tl3 = since();
             // Galerkin sums R A R^T with 0/1 aggregation: for every coarse
             // slot, the fine slots that aggregate onto it, in ascending order
@@ -2326,21 +2257,14 @@ std::shared_ptr<SolverAnalysis> analyse(Core& c, const Pattern& p, bool natural,
     }
     if (an->multigrid) {
         const int nl = (int)an->levels.size();
-        // the two-colour form (twocolour.cuh): two stages on every level but
-        // the coarsest, FP64 vectors, the default ordering
-        an->two_colour = !natural && fp64_vectors;
-        for (const Level& L : an->levels)
-            if (!L.coarsest && (L.stage_ptr.size() != 3 || L.gb > kMembers || L.ga > kMembers)) an->two_colour = false;
-        // otherwise the sweeps over stages, with their own member lists
-        if (!an->two_colour)
-            for (int l = 0; l + 1 < nl; ++l) stage_members(c, an->levels[l], an->levels[l + 1], ap_rows);
+        for (int l = 0; l + 1 < nl; ++l) stage_members(c, an->levels[l], an->levels[l + 1], ap_rows);
         // fuse the levels of at most linsolver_mg_fuse_rows unknowns (0: none):
         // from the first level from which on every level is that small, has
         // slices of uniform width, at most kTailStages stages and aggregates
         // of at most kMembers members (the coarsest needs none of these)
         auto fusable = [&](const Level& L) {
             return L.coarsest || (L.n <= fuse_rows && L.width > 0 && (int)L.stage_ptr.size() - 1 <= kTailStages &&
-                                  (an->two_colour || L.mpad));
+                                  L.mpad);
         };
         for (int l = nl - 1; l >= 0 && nl - l <= kMaxTail && fusable(an->levels[l]); --l)
             if (!an->levels[l].coarsest) an->tail_first = l;
@@ -2351,15 +2275,9 @@ std::shared_ptr<SolverAnalysis> analyse(Core& c, const Pattern& p, bool natural,
     for (auto& L : an->levels) {
         L.h_sp = L.h_col = L.h_len = L.h_aggb = std::vector<int>();
     }
-    // the right-hand side and the BiCGStab vectors, of the black half alone in
-    // the two-colour form
-    const Level& L0 = an->levels[0];
-    an->vec64 = c.allocN<double>(an->two_colour ? vec_stride(n) + 10 * vec_stride((L0.nb - L0.nr) * bs)
-                                                : 10 * vec_stride(n));
-    an->scal = c.alloc(sizeof(KScal));
-    an->partials = c.allocN<double>((size_t)kRedBlocks * 3);
+    an->vec64 = c.allocN<double>((size_t)10 * vec_stride(n));
+    an->partials = c.allocN<double>((size_t)kRedBlocks * 2);
     an->counter = c.allocN<unsigned int>(1);
-    an->factor_status = c.allocN<int>(1);
     EQG_CUDA(cudaMemsetAsync(an->counter->ptr, 0, sizeof(unsigned int), c.stream));
     c.sync();
     if (c.verbose > 2) {
@@ -2545,65 +2463,6 @@ int plan_local(Core& c, const SolverAnalysis& an, int& bytes, TailParams<T, M>* 
     return lf;
 }
 
-// plan_local for the two-colour form.
-template <class M>
-int plan_rb_local(Core& c, const SolverAnalysis& an, int& bytes, RbTailParams<M>* p)
-{
-    const int nlev = (int)an.levels.size() - an.tail_first;
-    bytes = 0;
-    if (an.tail_first < 0 || an.tail_kmax > 16 || !c.param_i("linsolver_mg_local", 1)) return nlev;
-    int off = 0, copies = 0, lf = nlev;
-    auto place = [&](int64_t b) {
-        const int o = off;
-        off += (int)((b + 15) & ~(int64_t)15);
-        return o;
-    };
-    for (int i = nlev - 1; i >= 1; --i) {
-        const Level& L = an.levels[an.tail_first + i];
-        const int off0 = off;
-        RbLocal o{};
-        struct Piece {
-            const void* src;
-            int dst;
-            int64_t bytes;
-        } piece[5];
-        int np = 0;
-        auto copied = [&](const void* src, int64_t b) {
-            piece[np] = Piece{src, place(b), b};
-            return piece[np++].dst;
-        };
-        if (L.vals * (int64_t)sizeof(M) > kTailSmem) break;
-        o.r = place((int64_t)L.n * sizeof(double));
-        if (L.coarsest) {
-            o.inv = copied(level_inv<M>(L), (int64_t)L.n * L.n * sizeof(M));
-        } else {
-            const bool black = L.pre;
-            const Level& C = an.levels[an.tail_first + i + 1];
-            o.w = place((int64_t)L.n * sizeof(double));
-            o.a = copied(level_a<M>(L), L.vals * (int64_t)sizeof(M));
-            o.lu = copied(level_lu<M>(L), L.vals * (int64_t)sizeof(M));
-            o.col = copied(L.sell_col->ptr, L.sell_size * 4);
-            o.len = copied(L.sell_len->ptr, (int64_t)L.nb * 4);
-            o.list = copied((black ? L.members_b : L.members_a)->ptr, (int64_t)C.nb * (black ? L.gb : L.ga) * 4);
-        }
-        if (off > kTailSmem || copies + np > kMaxCopies) {
-            off = off0;
-            break;
-        }
-        copies += np;
-        lf = i;
-        if (p) {
-            p->lv[i].so = o;
-            for (int k = 0; k < np; ++k)
-                p->copies[p->ncopies++] = TailCopy{piece[k].src, piece[k].dst, (int)piece[k].bytes};
-        }
-    }
-    if (lf == nlev) return nlev;
-    bytes = off;
-    if (p) p->local_first = lf;
-    return lf;
-}
-
 // Algorithmic bytes of the solver launches (reported with kernel timings):
 // every matrix block the step needs read once (its B^2 values and 4-byte
 // column), 4 bytes of row data per block row read (its length or diagonal
@@ -2634,28 +2493,24 @@ void launch_k(Core& c, void (*k)(KArgs...), int grid, int block, Args... args)
     EQG_CUDA(cudaLaunchKernelEx(&cfg, k, args...));
 }
 
+void prepare_tail_trace(Core& c, SolverAnalysis& an)
+{
+    if (!c.param_i("linsolver_tail_trace", 0) || an.tail_trace) return;
+    an.tail_trace = c.allocN<long long>(kTraceMax);
+    EQG_CUDA(cudaMemsetAsync(an.tail_trace->ptr, 0, kTraceMax * sizeof(long long), c.stream));
+}
+
 // Chooses the cluster size of the fused coarse cycle for one precision;
 // called before any stream capture.
 template <class T, class M>
 void prepare_tail(Core& c, SolverAnalysis& an)
 {
     if (an.tail_first < 0) return;
-    if (c.param_i("linsolver_tail_trace", 0) && !an.tail_trace) {
-        an.tail_trace = c.allocN<long long>(kTraceMax);
-        EQG_CUDA(cudaMemsetAsync(an.tail_trace->ptr, 0, kTraceMax * sizeof(long long), c.stream));
-    }
+    prepare_tail_trace(c, an);
     const int mode = pc_mode<T, M>();
     int& cl = an.tail_cluster[mode];
     const int bs = an.levels[an.tail_first].bs;
     int bytes = 0;
-    if constexpr (sizeof(T) == sizeof(double)) {
-        if (an.two_colour) {
-            if (!cl) WITH_BS(bs, WITH_KMAX(an.tail_kmax, cl = tail_cluster_size(c, rb_tail_kernel<BS, KK, M>)));
-            an.tail_local[mode] = plan_rb_local<M>(c, an, bytes, nullptr);
-            an.last_mode = mode;
-            return;
-        }
-    }
     if (!cl) WITH_BS(bs, WITH_KMAX(an.tail_kmax, cl = tail_cluster_size(c, mg_tail_kernel<BS, KK, T, M>)));
     an.tail_local[mode] = plan_local<T, M>(c, an, bytes, nullptr);
     an.last_mode = mode;
@@ -2760,7 +2615,7 @@ void report_tail_trace(Core& c, const SolverAnalysis& an)
     c.sync();
     EQG_CUDA(cudaMemcpy(t.data(), an.tail_trace->ptr, kTraceMax * sizeof(long long), cudaMemcpyDeviceToHost));
     std::vector<std::string> names;
-    const int last = (int)an.levels.size() - 1;
+    const int last = (int)std::max(an.levels.size(), an.rb.size()) - 1;
     auto ilu = [&](int l) {
         const int ns = (int)an.levels[l].stage_ptr.size() - 1;
         for (int s = 1; s < ns; ++s) names.push_back("L" + std::to_string(l) + ".lower" + std::to_string(s));
@@ -2769,14 +2624,14 @@ void report_tail_trace(Core& c, const SolverAnalysis& an)
     };
     const int lf = an.tail_first + an.tail_local[an.last_mode];  // first shared-memory level (last + 1: none)
     int l = an.tail_first;
-    if (an.two_colour) {
+    if (!an.rb.empty()) {
         auto name = [&](int k, const char* what) { names.push_back("L" + std::to_string(k) + "." + what); };
         for (; l < lf && l < last; ++l) {
-            if (an.levels[l].pre) {
+            if (an.rb[l].pre) {
                 name(l, "pre");
                 name(l, "y");
             }
-            name(l, an.levels[l].pre ? "residual" : "restrict");
+            name(l, an.rb[l].pre ? "residual" : "restrict");
         }
         name(l, l == lf ? "shared" : "dense");
         for (--l; l >= an.tail_first; --l) {
@@ -2786,7 +2641,7 @@ void report_tail_trace(Core& c, const SolverAnalysis& an)
             name(l, "fin");
         }
     }
-    for (; !an.two_colour && l < lf; ++l) {
+    for (; an.rb.empty() && l < lf; ++l) {
         if (an.levels[l].coarsest || l == last) {
             names.push_back("L" + std::to_string(l) + ".dense");
             break;
@@ -2795,10 +2650,10 @@ void report_tail_trace(Core& c, const SolverAnalysis& an)
         names.push_back("L" + std::to_string(l) + ".residual");
         if (l + 1 < lf) names.push_back("L" + std::to_string(l) + ".restrict");
     }
-    if (!an.two_colour && l == lf && lf <= last)
+    if (an.rb.empty() && l == lf && lf <= last)
         names.push_back("L" + std::to_string(lf - 1) + ".restrict+L" + std::to_string(lf) + "-L" +
                         std::to_string(last) + ".shared");
-    for (--l; !an.two_colour && l >= an.tail_first; --l) {
+    for (--l; an.rb.empty() && l >= an.tail_first; --l) {
         names.push_back("L" + std::to_string(l) + ".prolong");
         names.push_back("L" + std::to_string(l) + ".residual");
         ilu(l);
@@ -2930,149 +2785,6 @@ void vcycle(Core& c, const SolverAnalysis& an, size_t l, const T* r, T* z, const
     ilu_apply<T, M>(c, L, t, w, z, sc, skip);
 }
 
-// ---- the two-colour cycle (twocolour.cuh) ---------------------------------------
-// The pieces of one level: right-hand side, iterate and work vector by block
-// row.  Level 0 works on the caller's black vectors (`in`, `out`), whose red
-// right-hand side is zero.
-template <class M>
-struct RbVectors {
-    const double *r, *r_red;
-    double *z, *y;
-    const int* list;  // members restricted to the next level
-    int g;
-    UpView up;
-    RbVectors(const SolverAnalysis& an, size_t l, const double* in, double* out)
-    {
-        const Level& L = an.levels[l];
-        const int64_t red = (int64_t)L.nr * L.bs;
-        double* v0 = level_vec<double>(L, 0);
-        r = l == 0 ? in - red : v0;
-        r_red = l == 0 ? nullptr : r;
-        z = l == 0 ? out - red : level_vec<double>(L, 1);
-        y = l == 0 ? v0 : z;
-        const bool black = L.pre || l == 0;
-        list = L.coarsest ? nullptr : (black ? L.members_b : L.members_a)->as<int>();
-        g = black ? L.gb : L.ga;
-        if (l > 0) {
-            const Level& F = an.levels[l - 1];
-            up.list = F.members_b->as<int>();
-            up.g = F.gb;
-            up.add = F.pre ? 1 : 0;
-            up.alpha = F.alpha;
-            up.w = l == 1 ? out - (int64_t)F.nr * F.bs : level_vec<double>(F, 1);
-        }
-    }
-};
-
-template <class M>
-void launch_rb_tail(Core& c, const SolverAnalysis& an, const double* in, double* out, const KScal* sc, int skip)
-{
-    RbTailParams<M> p;
-    auto region = [&](const void* ptr, int64_t bytes) {
-        if (p.nregions < kMaxPrefetch && bytes >= 16) p.reg[p.nregions++] = PrefetchRegion{ptr, (unsigned long long)bytes};
-    };
-    for (size_t l = an.tail_first; l < an.levels.size(); ++l) {
-        const Level& L = an.levels[l];
-        const RbVectors<M> v(an, l, in, out);
-        RbTailLevel<M>& t = p.lv[p.nlev++];
-        t.nb = L.nb;
-        t.nr = L.nr;
-        t.n = L.n;
-        t.coarsest = L.coarsest ? 1 : 0;
-        t.pre = L.pre ? 1 : 0;
-        t.m = L.view();
-        t.r = v.r;
-        t.r_red = v.r_red;
-        t.rw = const_cast<double*>(v.r);
-        t.z = v.z;
-        t.y = v.y;
-        t.list = v.list;
-        t.g = v.g;
-        t.up = v.up;
-        if (L.coarsest) {
-            t.inv = level_inv<M>(L);
-            region(t.inv, (int64_t)L.n * L.n * (int64_t)sizeof(M));
-        } else {
-            t.a = level_a<M>(L);
-            t.lu = level_lu<M>(L);
-            region(L.sell_col->ptr, L.sell_size * 4);
-            region(L.sell_len->ptr, (int64_t)L.nb * 4);
-            region(t.a, L.vals * (int64_t)sizeof(M));
-            region(t.lu, L.vals * (int64_t)sizeof(M));
-            region(t.list, (int64_t)an.levels[l + 1].nb * t.g * 4);
-        }
-    }
-    if (an.tail_trace) p.trace = an.tail_trace->as<long long>();
-    p.local_first = p.nlev;
-    int smem = 0;
-    if (an.tail_local[pc_mode<double, M>()] < p.nlev) plan_rb_local<M>(c, an, smem, &p);
-    TailLaunch cfg(c, an.tail_cluster[pc_mode<double, M>()], smem);
-    WITH_BS(an.levels[an.tail_first].bs, WITH_KMAX(an.tail_kmax, launch(c, "rb_tail", [&] {
-                EQG_CUDA(cudaLaunchKernelEx(&cfg.cfg, rb_tail_kernel<BS, KK, M>, p, sc, skip));
-            }, tail_bytes<double, M>(an))));
-}
-
-// out = V-cycle(in) on the black rows, from level l down.
-template <class M>
-void rb_cycle(Core& c, const SolverAnalysis& an, size_t l, const double* in, double* out, const KScal* sc, int skip)
-{
-    if ((int)l == an.tail_first) {
-        launch_rb_tail<M>(c, an, in, out, sc, skip);
-        return;
-    }
-    const Level& L = an.levels[l];
-    const RbVectors<M> v(an, l, in, out);
-    if (L.coarsest) {
-        WITH_BS(L.bs, launch(c, "rb_dense", [&] {
-                    launch_k(c, rb_dense_kernel<BS, M>, 1, 1024, L.n, level_inv<M>(L), v.r, v.up, sc, skip);
-                }, (double)L.n * L.n * sizeof(M) + 2.0 * L.n * sizeof(double)));
-        return;
-    }
-    const Level& C = an.levels[l + 1];
-    double* rc = level_vec<double>(C, 0);
-    const M* a = level_a<M>(L);
-    const M* lu = level_lu<M>(L);
-    const int nr = L.nr, nk = L.nb - L.nr, nt = L.threads;
-    // algorithmic bytes: the stored blocks of a half, row lengths, diagonal
-    // blocks, and every vector element read or written once
-    const double row = 8.0 * L.bs, diag = (double)sizeof(M) * L.bs * L.bs;
-    const double half_u = block_bytes<M>(L, L.stage_upper[0]) + 4.0 * nr, half_l = block_bytes<M>(L, L.stage_lower[1]) + 4.0 * nk;
-    const double red = l == 0 ? 0.0 : row * nr;  // the red right-hand side
-    auto y_rows = [&] {
-        WITH_BS(L.bs, WITH_KMAX(L.kmax, launch(c, "rb_y", [&] {
-                    launch_k(c, rb_y_kernel<BS, KK, M>, blocksFor(nr, nt), nt, nr, L.view(), lu, v.r_red,
-                             (const double*)v.z, v.y, sc, skip);
-                }, half_u + red + row * (nr + nk))));
-    };
-    if (L.pre) {
-        WITH_BS(L.bs, WITH_KMAX(L.kmax, launch(c, "rb_pre", [&] {
-                    launch_k(c, rb_pre_kernel<BS, KK, M>, blocksFor(nk + 31, nt), nt, nr, L.nb, L.view(), lu, v.r,
-                             v.r_red, v.z, sc, skip);
-                }, (l == 0 ? 0.0 : half_l) + red + (diag + 2 * row) * nk)));
-        y_rows();
-        WITH_BS(L.bs, WITH_KMAX(L.kmax, launch(c, "rb_res", [&] {
-                    launch_k(c, rb_res_kernel<BS, KK, M>, blocksFor((int64_t)C.nb * v.g, nt), nt, C.nb, v.g, v.list,
-                             L.view(), a, lu, v.r, (const double*)v.y, (const double*)v.z, rc, sc, skip);
-                }, half_l + (diag + 2 * row) * nk + row * nr + (4.0 * v.g + row) * C.nb)));
-    } else {
-        WITH_BS(L.bs, launch(c, "rb_restrict", [&] {
-                    launch_k(c, rb_restrict_kernel<BS>, blocksFor(C.nb, nt), nt, C.nb, v.g, v.list, v.r, rc, sc, skip);
-                }, row * nk + red + (4.0 * v.g + row) * C.nb));
-    }
-    rb_cycle<M>(c, an, l + 1, in, out, sc, skip);
-    y_rows();
-    const double to_fine = v.up.w ? 4.0 * v.up.g + row * v.up.g * (v.up.add ? 2.0 : 1.0) : 0.0;
-    WITH_BS(L.bs, WITH_KMAX(L.kmax, launch(c, "rb_post", [&] {
-                launch_k(c, rb_post_kernel<BS, KK, M>, blocksFor(nk + 31, nt), nt, nr, L.nb, L.view(), a, lu, v.r,
-                         (const double*)v.y, v.z, v.up, sc, skip);
-            }, half_l + (2 * diag + 3 * row + to_fine) * nk + row * nr)));
-    if (v.up.w == nullptr) return;
-    WITH_BS(L.bs, WITH_KMAX(L.kmax, launch(c, "rb_fin", [&] {
-                launch_k(c, rb_fin_kernel<BS, KK, M>, blocksFor(nr, nt), nt, nr, L.view(), lu, v.r,
-                         (const double*)v.z, v.up, sc, skip);
-            }, half_u + (diag + row + to_fine) * nr + row * nk)));
-}
-
 template <class T, class M>
 void precondition(Core& c, const SolverAnalysis& an, const T* in, T* out, const KScal* sc, int skip_if_s)
 {
@@ -3165,22 +2877,27 @@ void autotune(Core& c, SolverAnalysis& an, Apply&& apply)
     if (an.tuned[mode]) return;
     an.tuned[mode] = true;
     if (c.param_i("linsolver_autotune", 1) == 0) return;
-    // levels with launch-per-step kernels: all but the fused ones and a
-    // dense coarsest level
-    std::vector<int> lv;
-    for (size_t l = 0; l < an.levels.size(); ++l) {
-        if (an.multigrid && an.tail_first >= 0 && (int)l >= an.tail_first) break;
-        if (an.levels[l].coarsest) break;
-        lv.push_back((int)l);
-        if (!an.multigrid) break;
-    }
+    // the block sizes of the levels with launch-per-step kernels: all but the
+    // fused ones and a dense coarsest level
+    std::vector<int*> lv;
     cudaDeviceProp prop;
     EQG_CUDA(cudaGetDeviceProperties(&prop, c.device));
     std::ostringstream key;
-    key << prop.name << "; n " << an.n << "; nnz " << an.nnz << "; bs " << an.levels[0].bs << "; levels";
-    for (auto& L : an.levels) key << " " << L.n;
+    key << prop.name << "; n " << an.n << "; nnz " << an.nnz << "; bs "
+        << (an.rb.empty() ? an.levels[0].bs : an.rb_bs) << "; levels";
+    auto collect = [&](auto& levels) {
+        bool more = true;
+        for (size_t l = 0; l < levels.size(); ++l) {
+            key << " " << levels[l].n;
+            if (levels[l].coarsest || (an.multigrid && an.tail_first >= 0 && (int)l >= an.tail_first)) more = false;
+            if (more) lv.push_back(&levels[l].threads);
+            if (!an.multigrid) more = false;
+        }
+    };
+    if (an.rb.empty()) collect(an.levels);
+    else collect(an.rb);
     key << "; fused from " << an.tail_first << "; precision " << mode;
-    if (an.two_colour) key << "; two colours";
+    if (!an.rb.empty()) key << "; two colours";
     std::string file = c.param_s("linsolver_tune_file", "");
     if (file.empty() && std::getenv("EQG_TUNE_FILE")) file = std::getenv("EQG_TUNE_FILE");
     {
@@ -3191,7 +2908,7 @@ void autotune(Core& c, SolverAnalysis& an, Apply&& apply)
         }
         auto it = g_tune_cache.find(key.str());
         if (it != g_tune_cache.end() && it->second.threads.size() == lv.size()) {
-            for (size_t i = 0; i < lv.size(); ++i) an.levels[lv[i]].threads = it->second.threads[i];
+            for (size_t i = 0; i < lv.size(); ++i) *lv[i] = it->second.threads[i];
             if (an.tail_first >= 0 && it->second.cluster > 0 && it->second.cluster <= an.tail_cluster[mode])
                 an.tail_cluster[mode] = it->second.cluster;
             return;
@@ -3219,19 +2936,18 @@ void autotune(Core& c, SolverAnalysis& an, Apply&& apply)
     };
     float cur = measure();
     const float first = cur;
-    for (int l : lv) {
-        Level& L = an.levels[l];
-        int best_t = L.threads;
+    for (int* threads : lv) {
+        int best_t = *threads;
         for (int t : {128, 256, 512}) {
             if (t == best_t) continue;
-            L.threads = t;
+            *threads = t;
             const float ms = measure();
             if (ms < cur) {
                 cur = ms;
                 best_t = t;
             }
         }
-        L.threads = best_t;
+        *threads = best_t;
     }
     int& cl = an.tail_cluster[mode];
     if (an.tail_first >= 0 && cl > 1) {
@@ -3252,7 +2968,7 @@ void autotune(Core& c, SolverAnalysis& an, Apply&& apply)
     cudaEventDestroy(e1);
     c.timed_kernel = timed;
     TuneChoice t;
-    for (int l : lv) t.threads.push_back(an.levels[l].threads);
+    for (int* threads : lv) t.threads.push_back(*threads);
     t.cluster = an.tail_first >= 0 ? cl : 0;
     if (c.verbose > 2) {
         std::printf("        autotune: %.3f -> %.3f ms per V-cycle; threads per level:", first / 4, cur / 4);
@@ -3382,68 +3098,6 @@ SolveResult bicgstab(Core& c, SolverAnalysis& an, const T* a, Vecs<T> v, double 
     return run_iterations(c, an, sizeof(T) == sizeof(double) ? (pc32 ? 2 : 0) : 1, tol, max_iter, check_every, iteration);
 }
 
-// BiCGStab on the black half of the system (twocolour.cuh), M the type of
-// the preconditioner's matrices.  `b`: the right-hand side in block-row order;
-// the solution goes to `xout` in the natural order.
-template <class M>
-SolveResult bicgstab_rb(Core& c, SolverAnalysis& an, const double* b, double* xout, double tol, int max_iter,
-                        int check_every)
-{
-    const Level& L0 = an.levels[0];
-    const int nr = L0.nr, nk = L0.nb - L0.nr, n = nk * L0.bs;
-    const Vecs<double> v = vecs<double>(an.vec64->as<double>() + vec_stride(an.n), n);
-    KScal* sc = an.scal->as<KScal>();
-    double* part = an.partials->as<double>();
-    unsigned int* cnt = an.counter->as<unsigned int>();
-    const double* a = L0.as64->as<double>();
-    const double* lu = L0.lus64->as<double>();
-    double* y = level_vec<double>(L0, 0);
-    const int nbv = blocksFor(n, kThreads, kRedBlocks), nbk = blocksFor(nk + 31, kThreads, kRedBlocks);
-    const double vb = 8.0 * n, yb = 8.0 * nr * L0.bs, diag = 8.0 * L0.bs * L0.bs;
-    const double half_u = block_bytes<double>(L0, L0.stage_upper[0]) + 4.0 * nr;
-    const double half_l = block_bytes<double>(L0, L0.stage_lower[1]) + 4.0 * nk;
-    WITH_BS(L0.bs, WITH_KMAX(L0.kmax, launch(c, "rb_init", [&] {
-                rb_init_kernel<BS, KK><<<blocksFor(L0.nb, kThreads, kRedBlocks), kThreads, 0, c.stream>>>(
-                    nr, L0.nb, L0.view(), lu, b, v.r, v.rhat, v.p, v.v, v.x, part, cnt, sc, tol * tol);
-            }, half_l + vb * 6.0 + yb)));
-    auto product = [&](const double* z, const double* h, double* out, bool omega) {
-        WITH_BS(L0.bs, WITH_KMAX(L0.kmax, launch(c, "rb_spmv_y", [&] {
-                    launch_k(c, rb_y_kernel<BS, KK, double>, blocksFor(nr, L0.threads), L0.threads, nr, L0.view(), lu,
-                             (const double*)nullptr, z - (int64_t)nr * L0.bs, y, (const KScal*)sc, (int)omega);
-                }, half_u + vb + yb)));
-        WITH_BS(L0.bs, WITH_KMAX(L0.kmax, launch(c, omega ? "rb_spmv_omega" : "rb_spmv_alpha", [&] {
-                    launch_k(c, omega ? rb_spmv_kernel<BS, KK, true> : rb_spmv_kernel<BS, KK, false>, nbk, kThreads,
-                             nr, L0.nb, L0.view(), a, lu, z, (const double*)y, h, out, part, cnt, sc);
-                }, half_l + diag * nk + yb + 3.0 * vb)));
-    };
-    auto iteration = [&] {
-        launch(c, "bicg_p", [&] {
-            launch_k(c, bicg_p_kernel<double>, blocksFor(n), kThreads, (const double*)v.r, (const double*)v.v, v.p, n,
-                     (const KScal*)sc);
-        }, 4.0 * vb);
-        rb_cycle<M>(c, an, 0, v.p, v.ph, sc, 0);
-        product(v.ph, v.rhat, v.v, false);
-        launch(c, "bicg_s", [&] {
-            launch_k(c, bicg_s_kernel<double>, nbv, kThreads, (const double*)v.r, (const double*)v.v, v.s, n, part, cnt,
-                     sc);
-        }, 3.0 * vb);
-        rb_cycle<M>(c, an, 0, v.s, v.sh, sc, 1);
-        product(v.sh, v.s, v.t, true);
-        launch(c, "bicg_xr", [&] {
-            launch_k(c, bicg_xr_kernel<double>, nbv, kThreads, (const double*)v.ph, (const double*)v.sh,
-                     (const double*)v.s, (const double*)v.t, (const double*)v.rhat, v.x, v.r, n, part, cnt, sc);
-        }, 8.0 * vb);
-    };
-    autotune<double, M>(c, an, [&] { rb_cycle<M>(c, an, 0, v.r, v.ph, sc, 0); });
-    const SolveResult res =
-        run_iterations(c, an, sizeof(M) == sizeof(double) ? 0 : 2, tol, max_iter, check_every, iteration);
-    WITH_BS(L0.bs, WITH_KMAX(L0.kmax, launch(c, "rb_solution", [&] {
-                rb_solution_kernel<BS, KK><<<blocksFor(L0.nb), kThreads, 0, c.stream>>>(
-                    nr, L0.nb, L0.view(), lu, b, v.x, L0.perm->as<int>(), xout);
-            }, half_u + diag * nr + vb + 3.0 * yb + vb)));
-    return res;
-}
-
 void factor_level(Core& c, const Level& L, int* status)
 {
     EQG_CUDA(cudaMemcpyAsync(L.lus64->ptr, L.as64->ptr, (size_t)L.vals * 8, cudaMemcpyDeviceToDevice, c.stream));
@@ -3462,6 +3116,21 @@ void factor_level(Core& c, const Level& L, int* status)
     }
 }
 
+// The n x n matrix `a` inverted in place.
+void dense_inverse(Core& c, int n, double* a, int* status)
+{
+    launch(c, "mg_dense_inverse", [&] {
+        const size_t smem = ((size_t)n * n + n) * sizeof(double);
+        // one value for every call: runtimes on other host threads set the
+        // same attribute, and a smaller value set between this call's set and
+        // its launch would fail it
+        const size_t most = ((size_t)kCoarsest * kCoarsest + kCoarsest) * sizeof(double);
+        EQG_CUDA(cudaFuncSetAttribute(dense_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)std::max(smem, most)));
+        dense_inverse_kernel<<<1, 1024, smem, c.stream>>>(n, a, status);
+    }, 16.0 * n * n);
+}
+
 void to_float(Core& c, const Buf& src, Buf& dst, int64_t n)
 {
     if (!dst) dst = c.allocN<float>((size_t)(n > 0 ? n : 1));
@@ -3473,6 +3142,36 @@ void to_float(Core& c, const Buf& src, Buf& dst, int64_t n)
 }  // namespace
 
 namespace {
+
+#include "twocolour_solve.cuh"
+
+// One solve in the two-colour form.
+SolveResult solve_rb(Core& c, SolverAnalysis& an, const double* jval, const double* rhs, double* xout, bool mixed,
+                     double tol, int max_iter, int check_every)
+{
+    c.factor_clock.start(c.stream);
+    EQG_CUDA(cudaMemsetAsync(an.factor_status->ptr, 0, sizeof(int), c.stream));
+    rb_setup(c, an, jval, mixed);
+    prepare_tail_trace(c, an);
+    if (mixed) prepare_rb_tail<float>(c, an);
+    else prepare_rb_tail<double>(c, an);
+    c.factor_clock.stop(c.stream);
+    int fstat = 0;
+    EQG_CUDA(cudaMemcpyAsync(c.pinned, an.factor_status->ptr, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    c.sync();
+    std::memcpy(&fstat, c.pinned, sizeof(int));
+    SolveResult res;
+    if (fstat) return res;  // zero pivot
+    c.krylov_clock.start(c.stream);
+    res = mixed ? bicgstab_rb<float>(c, an, rhs, xout, tol, max_iter, check_every)
+                : bicgstab_rb<double>(c, an, rhs, xout, tol, max_iter, check_every);
+    res.sweeps = 1;
+    c.krylov_clock.stop(c.stream);
+    report_tail_trace(c, an);
+    res.block_size = an.rb_bs;
+    res.blocks = (int64_t)an.rb[0].g.n * (an.rb_nd + 1);
+    return res;
+}
 
 // One solve with the analysis in `slot` (built on first use; without
 // multigrid when allow_multigrid is false).
@@ -3506,6 +3205,7 @@ SolveResult solve_with(Core& c, const PatternP& p, std::shared_ptr<SolverAnalysi
         res.converged = true;
         return res;
     }
+    if (!an.rb.empty()) return solve_rb(c, an, jval, rhs, xout, mixed, tol, max_iter, check_every);
     // level matrices and their factorizations (FP64)
     c.factor_clock.start(c.stream);
     const Level& L0 = an.levels[0];
@@ -3532,23 +3232,17 @@ SolveResult solve_with(Core& c, const PatternP& p, std::shared_ptr<SolverAnalysi
     EQG_CUDA(cudaMemsetAsync(an.factor_status->ptr, 0, sizeof(int), c.stream));
     for (auto& L : an.levels) {
         if (L.coarsest) {
-            WITH_BS(L.bs, launch(c, "mg_dense_inverse", [&] {
-                const size_t smem = ((size_t)L.n * L.n + L.n) * sizeof(double);
-                // one value for every call: runtimes on other host threads set
-                // the same attribute of the same kernel, and a smaller value
-                // set between this call's set and its launch would fail it
-                const size_t most = ((size_t)kCoarsest * kCoarsest + kCoarsest) * sizeof(double);
-                EQG_CUDA(cudaFuncSetAttribute(dense_inverse_kernel<BS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)std::max(smem, most)));
-                dense_inverse_kernel<BS><<<1, 1024, smem, c.stream>>>(L.nb, L.view(), L.as64->as<double>(),
-                                                                     L.inv64->as<double>(), an.factor_status->as<int>());
-            }, 16.0 * L.n * L.n));
+            EQG_CUDA(cudaMemsetAsync(L.inv64->ptr, 0, (size_t)L.n * L.n * sizeof(double), c.stream));
+            WITH_BS(L.bs, launch(c, "mg_dense_fill", [&] {
+                        dense_fill_kernel<BS><<<blocksFor(L.nb), kThreads, 0, c.stream>>>(
+                            L.nb, L.view(), L.as64->as<double>(), L.inv64->as<double>());
+                    }));
+            dense_inverse(c, L.n, L.inv64->as<double>(), an.factor_status->as<int>());
         } else {
             factor_level(c, L, an.factor_status->as<int>());
         }
     }
     Vecs<double> v = vecs<double>(an.vec64->as<double>(), n);
-    if (an.two_colour) v.b = an.vec64->as<double>();
     launch(c, "permute",
            [&] { permute_kernel<<<blocksFor(n), kThreads, 0, c.stream>>>(rhs, L0.perm->as<int>(), v.b, n); },
            20.0 * n);
@@ -3574,11 +3268,7 @@ SolveResult solve_with(Core& c, const PatternP& p, std::shared_ptr<SolverAnalysi
     if (fstat) return res;  // zero pivot
     c.krylov_clock.start(c.stream);
 
-    if (an.two_colour) {
-        res = mixed ? bicgstab_rb<float>(c, an, v.b, xout, tol, max_iter, check_every)
-                    : bicgstab_rb<double>(c, an, v.b, xout, tol, max_iter, check_every);
-        res.sweeps = 1;
-    } else if (!refine) {
+    if (!refine) {
         res = bicgstab<double>(c, an, L0.as64->as<double>(), v, tol, max_iter, check_every, mixed);
         res.sweeps = 1;
     } else {
@@ -3630,10 +3320,9 @@ SolveResult solve_with(Core& c, const PatternP& p, std::shared_ptr<SolverAnalysi
     }
     c.krylov_clock.stop(c.stream);
     report_tail_trace(c, an);
-    if (!an.two_colour)
-        launch(c, "unpermute",
-               [&] { unpermute_kernel<<<blocksFor(n), kThreads, 0, c.stream>>>(v.x, L0.perm->as<int>(), xout, n); },
-               20.0 * n);
+    launch(c, "unpermute",
+           [&] { unpermute_kernel<<<blocksFor(n), kThreads, 0, c.stream>>>(v.x, L0.perm->as<int>(), xout, n); },
+           20.0 * n);
     res.block_size = L0.bs;
     res.blocks = L0.blocks;
     return res;

@@ -1,20 +1,20 @@
-// Two-colour form of the multigrid-preconditioned BiCGStab (included by
-// solver.cu, inside its anonymous namespace).
+// Two-colour form of the multigrid-preconditioned BiCGStab on the seven-point
+// (five-point) block stencils of Cartesian grids (included by solver.cu,
+// inside its anonymous namespace).
 //
-// On the cell graph of a Cartesian grid every level of the hierarchy takes
-// two colours: the red block rows [0, nr) and the black ones [nr, nb), with
-// no couplings inside a colour.  Red unknowns can then be eliminated exactly,
+// Colouring the cells by the parity of i + j + k, no two cells of a colour
+// are coupled, so the red unknowns can be eliminated exactly,
 //   x_r = D_r^-1 (b_r - U x_b),   S x_b = b_b - L b_r,   S = A_bb - L U,
 // with L = A_br D_r^-1 and U = A_rb the off-diagonal blocks of the block
-// ILU(0) factors and A_bb the black diagonal blocks, so that BiCGStab runs on
-// the black half: vectors of half the length, and S x as two half products
-// (y = -U x, A_bb x + L y) that read each stored block of the factors once.
+// ILU(0) factors, D_r = A_rr, and A_bb the black diagonal blocks, so that
+// BiCGStab runs on the black half: vectors of half the length, and S x as two
+// half products (y = -U x, A_bb x + L y) that read each stored block once.
 // The residual of the whole system is that of its black half (red rows are
 // solved exactly), so the convergence test is unchanged.
 //
-// The V-cycle's block ILU(0) sweeps read the same factors (D_b is the black
-// diagonal block of the factorization, A_bb - the diagonal blocks of L U).
-// With right-hand side (r_r, r_b) and iterate z_b,
+// The V-cycle's block ILU(0) sweeps read the same factors (D_b, the black
+// diagonal block of the factorization, is A_bb less the diagonal blocks of
+// L U).  With right-hand side (r_r, r_b) and iterate z_b,
 //   y   = r_r - U z_b                       (rb_y_rows)
 //   t_b = r_b - A_bb z_b - L y              (the residual; red rows: 0)
 //   z_b += D_b^-1 t_b                       (rb_post_rows)
@@ -22,324 +22,520 @@
 // is one sweep from any z_b: the red part of the iterate is never needed
 // before the last line, the residual of the down-leg is summed straight into
 // the coarse right-hand side (rb_res_rows), and the coarse level's last two
-// steps add alpha times their rows to the fine black rows (scatter_up).  A
-// level with pre-smoothing takes six half products of its factors, one
-// without (Level::pre) three; the level-0 cycle needs no red rows at all.
+// steps add alpha times their rows to the fine black cells (scatter_up).  A
+// level with pre-smoothing (Level::pre) takes six half products of its
+// factors, one without three; level 0 needs no red rows at all.
 //
-// Bound: HBM on the fine levels (the factors, 36 bytes per 2 x 2 FP64 block),
-// latency of dependent steps on the coarse ones.  Measured on one time step
-// against the full-length form over stages (two sweeps, residual, A P up-leg
-// and a full product per application; 2 x 2 x 2 aggregates only): two-phase
-// 128x128x64, 203 BiCGStab iterations of 0.74 ms -> 90 of 0.65 ms (the
-// iterations by aggregation along z alone on the first two levels); 512x512,
-// 53 of 0.50 ms -> 52 of 0.32 ms; 33x31x17, 117 of 0.175 -> 58 of 0.167 ms.
+// Layout: cell c = i + nx (j + ny k) is number c >> 1 of its colour whatever
+// the sides (lines, planes or the whole grid alternate), so a neighbour's
+// place follows from index arithmetic: no column indices, row lengths or
+// slices are stored or waited for, and a step's loads (blocks and gathered
+// vector) are one round trip.  Blocks are stored by direction (W, E, S, N, B,
+// T), each direction contiguous over the rows of a colour: a warp's loads are
+// whole segments.  Couplings that the Jacobian's pattern lacks are zero
+// blocks.
+//
+// Bound: HBM on the fine levels (32 bytes per 2 x 2 FP64 block), latency of
+// dependent steps on the coarse ones.  Measured on one time step, against the
+// full-length form over stages with 2 x 2 x 2 aggregates only and against
+// this form on the block sliced layout (stored columns and lengths): Krylov
+// time of two-phase 128x128x64, 150 (203 iterations) -> 59 -> 51 ms (90; the
+// iterations by pairing along z alone on the first two levels); 512x512, 26.5
+// -> 16.6 -> 11.6 ms; 33x31x17, 20.6 -> 9.7 -> 7.9 ms; impes 97x83x41, 31.6 ->
+// 12.6 -> 10.4 ms.  First step of a new 128x128x64 runtime, with the analysis
+// on the host, then on the device: 526 -> 180 ms.
+
+// Division by a run-time constant, exact for 0 <= n < 2^31: with l =
+// ceil(log2 d) and m = floor(2^(31+l) / d) + 1, floor(n / d) = floor(n m /
+// 2^(31+l)) since m d - 2^(31+l) <= d <= 2^l (Granlund and Montgomery 1994).
+struct FastDiv {
+    unsigned m = 0;
+    int s = 0;  // < 0: d is 1
+    FastDiv() = default;
+    explicit FastDiv(unsigned d)
+    {
+        int l = 0;
+        while ((1ull << l) < d) ++l;
+        m = (unsigned)((1ull << (31 + l)) / d + 1);
+        s = l - 1;
+    }
+    __device__ __forceinline__ int operator()(int n) const { return s < 0 ? n : (int)(__umulhi((unsigned)n, m) >> s); }
+};
+
+// A level's grid of cells.
+struct RbGrid {
+    int nx = 1, ny = 1, nz = 1, n = 1, nr = 1;  // cells, red cells
+    int step = 1;                               // cells of a plane
+    FastDiv by_x, by_plane;
+    RbGrid() = default;
+    RbGrid(int x, int y, int z) : nx(x), ny(y), nz(z), n(x * y * z), nr((n + 1) / 2), step(x * y), by_x(x), by_plane(x * y) {}
+};
+
+struct Cell {
+    int c, i, j, k;
+};
+
+__device__ __forceinline__ Cell cell_at(const RbGrid& g, int c)
+{
+    Cell e;
+    e.c = c;
+    e.k = g.by_plane(c);
+    const int r = c - e.k * g.step;
+    e.j = g.by_x(r);
+    e.i = r - e.j * g.nx;
+    return e;
+}
+
+// Cell number q of a colour (0 red, 1 black): the one of 2 q and 2 q + 1 of
+// that colour.
+__device__ __forceinline__ Cell cell_of(const RbGrid& g, int colour, int q)
+{
+    Cell e = cell_at(g, 2 * q);
+    if (((e.i + e.j + e.k) & 1) != colour) {
+        ++e.c;
+        if (++e.i == g.nx) {
+            e.i = 0;
+            if (++e.j == g.ny) {
+                e.j = 0;
+                ++e.k;
+            }
+        }
+    }
+    return e;
+}
+
+// Whether the cell has a neighbour in direction d, and that neighbour's
+// number in the other colour.
+__device__ __forceinline__ bool neighbour(const RbGrid& g, const Cell& e, int d, int& q)
+{
+    const int off = d < 2 ? 1 : d < 4 ? g.nx : g.step;
+    q = (d & 1 ? e.c + off : e.c - off) >> 1;
+    switch (d) {
+    case 0: return e.i > 0;
+    case 1: return e.i + 1 < g.nx;
+    case 2: return e.j > 0;
+    case 3: return e.j + 1 < g.ny;
+    case 4: return e.k > 0;
+    default: return e.k + 1 < g.nz;
+    }
+}
+
+// The arrays of a level's matrix, one after the other: off-diagonal blocks of
+// the red and of the black cells by direction, diagonal blocks of the red
+// cells and of the black ones, and the factors' black diagonal blocks.  As
+// gathered from the Jacobian: A.  As factored: U (unchanged), L, D_r^-1,
+// A_bb (unchanged), D_b^-1.
+template <class M>
+struct RbMatrix {
+    M *U, *L, *dr, *abb, *db;
+    __host__ __device__ RbMatrix(M* base, int nd, int bb, int n, int nr)
+    {
+        U = base;
+        L = U + (size_t)nd * nr * bb;
+        dr = L + (size_t)nd * (n - nr) * bb;
+        abb = dr + (size_t)nr * bb;
+        db = abb + (size_t)(n - nr) * bb;
+    }
+    static size_t values(int nd, int bb, int n, int nr) { return ((size_t)(nd + 1) * n + (n - nr)) * bb; }
+};
+
+// acc += sum over the neighbours of A_d x_d, directions in order, row q of
+// `rows`; every load is issued before the first sum.
+template <int B, int ND, class M, bool CG>
+__device__ __forceinline__ void stencil_dot(const RbGrid& g, const Cell& e, int q, int rows, const M* __restrict__ a,
+                                            const double* __restrict__ x, double (&acc)[B])
+{
+    constexpr int BB = B * B;
+    M av[ND][BB];
+    double xv[ND][B];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+        int nq;
+        const bool has = neighbour(g, e, d, nq);
+#pragma unroll
+        for (int t = 0; t < BB; ++t) av[d][t] = (M)0;
+#pragma unroll
+        for (int t = 0; t < B; ++t) xv[d][t] = 0.0;
+        if (has) {
+            load_block<BB, M>(a + ((size_t)d * rows + q) * BB, av[d]);
+            load_bvec<B, double, CG>(x, nq, xv[d]);
+        }
+    }
+#pragma unroll
+    for (int d = 0; d < ND; ++d)
+#pragma unroll
+        for (int i = 0; i < B; ++i)
+#pragma unroll
+            for (int j = 0; j < B; ++j) acc[i] = __fma_rn((double)av[d][i * B + j], xv[d][j], acc[i]);
+}
+
+// y = D x of one block.
+template <int B, class M>
+__device__ __forceinline__ void block_mul(const M* __restrict__ a, const double (&x)[B], double (&y)[B])
+{
+    M av[B * B];
+    load_block<B * B, M>(a, av);
+#pragma unroll
+    for (int i = 0; i < B; ++i) {
+        double s = 0.0;
+#pragma unroll
+        for (int j = 0; j < B; ++j) s = __fma_rn((double)av[i * B + j], x[j], s);
+        y[i] = s;
+    }
+}
+
+// Aggregation of a level's cells: pairs along the directions whose shift is
+// 1.  An aggregate has `g` places for black members: the offsets of all
+// paired directions but the first, the first one's follows from the colour.
+struct Aggregates {
+    int sx = 0, sy = 0, sz = 0, g = 1;
+    RbGrid fine, coarse;
+};
+
+// Black member s of the aggregate (i, j, k): its cell, or -1 (outside).
+__device__ __forceinline__ int black_member(const Aggregates& a, int i, int j, int k, int s)
+{
+    i <<= a.sx;
+    j <<= a.sy;
+    k <<= a.sz;
+    if (a.sx) {
+        if (a.sy) {
+            j += s & 1;
+            s >>= 1;
+        }
+        if (a.sz) k += s & 1;
+        i += 1 ^ ((i + j + k) & 1);
+    } else if (a.sy) {
+        if (a.sz) k += s & 1;
+        j += 1 ^ ((i + j + k) & 1);
+    } else {
+        k += 1 ^ ((i + j + k) & 1);
+    }
+    return i < a.fine.nx && j < a.fine.ny && k < a.fine.nz ? i + a.fine.nx * (j + a.fine.ny * k) : -1;
+}
 
 // Where a level's finished rows go: alpha z is added to (add) or stored in
-// the black members, g per block row of this level, of the finer level's z.
+// the black members' z of the finer level.
 struct UpView {
-    const int* list = nullptr;
-    int g = 0;
+    Aggregates agg;
     int add = 0;
     double alpha = 1.0;
-    double* w = nullptr;  // finer level's z, indexed by its block rows; null: no finer level
+    double* w = nullptr;  // null: no finer level
 };
 
 template <int B, bool CG>
-__device__ __forceinline__ void scatter_up(const UpView& u, int R, const double (&z)[B])
+__device__ __forceinline__ void scatter_up(const UpView& u, const Cell& e, const double (&z)[B])
 {
     if (u.w == nullptr) return;
-    for (int s = 0; s < u.g; ++s) {
-        const int m = u.list[R * u.g + s];
-        if (m < 0) continue;
+    for (int s = 0; s < u.agg.g; ++s) {
+        const int c = black_member(u.agg, e.i, e.j, e.k, s);
+        if (c < 0) continue;
         double f[B];
 #pragma unroll
-        for (int c = 0; c < B; ++c) f[c] = 0.0;
-        if (u.add) load_bvec<B, double, CG>(u.w, m, f);
+        for (int t = 0; t < B; ++t) f[t] = 0.0;
+        if (u.add) load_bvec<B, double, CG>(u.w, c >> 1, f);
 #pragma unroll
-        for (int c = 0; c < B; ++c) f[c] += u.alpha * z[c];
-        store_bvec<B, double>(u.w, m, f);
+        for (int t = 0; t < B; ++t) f[t] = __fma_rn(u.alpha, z[t], f[t]);
+        store_bvec<B, double>(u.w, c >> 1, f);
     }
 }
 
-// The steps below are loops over a row range for thread `tid` of `nth`,
-// shared by the one-step kernels and the fused coarse cycle (see
-// mg_tail_kernel), so that both compute every element alike.  Vectors are
-// indexed by block row; r == null stands for a zero red right-hand side.
+// ---- the steps ------------------------------------------------------------------
+// Loops over the rows of a colour for thread `tid` of `nth`, shared by the
+// one-step kernels and the fused coarse cycle (see mg_tail_kernel), so that
+// both compute every element alike (operations written out: the compiler
+// contracted products and sums differently in the shared-memory cycle).  rr, y: red vectors (rr null: zero), rb,
+// z: black ones.
 
-// y_R = r_R - sum U_RJ z_J over the red rows.
-template <int B, int KM, class M, bool CG, bool U>
-__device__ __forceinline__ void rb_y_rows(int nr, const SellView& m, const M* __restrict__ lu, const double* r,
+template <int B, int ND, class M, bool CG>
+__device__ __forceinline__ void red_row(const RbGrid& g, const Cell& e, int q, const M* U, const double* rr,
+                                        const double* z, double (&v)[B])
+{
+    double acc[B];
+#pragma unroll
+    for (int t = 0; t < B; ++t) acc[t] = v[t] = 0.0;
+    if (rr) load_bvec<B, double, CG>(rr, q, v);
+    stencil_dot<B, ND, M, CG>(g, e, q, g.nr, U, z, acc);
+#pragma unroll
+    for (int t = 0; t < B; ++t) v[t] = __dsub_rn(v[t], acc[t]);
+}
+
+// y = rr - U z
+template <int B, int ND, class M, bool CG>
+__device__ __forceinline__ void rb_y_rows(const RbGrid& g, const RbMatrix<const M>& m, const double* rr,
                                           const double* z, double* y, int tid, int nth)
 {
-    for (int R = tid; R < nr; R += nth) {
-        double acc[B];
-#pragma unroll
-        for (int c = 0; c < B; ++c) acc[c] = 0.0;
-        bdot<B, KM, double, M, CG, U>(m, slice_base<U>(m, R), R & 31, 1, m.len[R], lu, z, z, INT_MAX, acc);
+    for (int q = tid; q < g.nr; q += nth) {
         double v[B];
-#pragma unroll
-        for (int c = 0; c < B; ++c) v[c] = 0.0;
-        if (r) load_bvec<B, double, CG>(r, R, v);
-#pragma unroll
-        for (int c = 0; c < B; ++c) v[c] -= acc[c];
-        store_bvec<B, double>(y, R, v);
+        red_row<B, ND, M, CG>(g, cell_of(g, 0, q), q, m.U, rr, z, v);
+        store_bvec<B, double>(y, q, v);
     }
 }
 
-// z_R = D_R^-1 (r_R - sum U_RJ z_J) over the red rows, handed to the finer
-// level (a level's red rows are read by nothing else).
-template <int B, int KM, class M, bool CG, bool U>
-__device__ __forceinline__ void rb_fin_rows(int nr, const SellView& m, const M* __restrict__ lu, const double* r,
+// D_r^-1 (rr - U z), handed to the finer level (nothing else reads it).
+template <int B, int ND, class M, bool CG>
+__device__ __forceinline__ void rb_fin_rows(const RbGrid& g, const RbMatrix<const M>& m, const double* rr,
                                             const double* z, const UpView& up, int tid, int nth)
 {
-    for (int R = tid; R < nr; R += nth) {
-        const int lane = R & 31, sb = slice_base<U>(m, R);
-        double acc[B];
-#pragma unroll
-        for (int c = 0; c < B; ++c) acc[c] = 0.0;
-        bdot<B, KM, double, M, CG, U>(m, sb, lane, 1, m.len[R], lu, z, z, INT_MAX, acc);
+    for (int q = tid; q < g.nr; q += nth) {
+        const Cell e = cell_of(g, 0, q);
         double v[B], x[B];
-        load_bvec<B, double, CG>(r, R, v);
-#pragma unroll
-        for (int c = 0; c < B; ++c) v[c] -= acc[c];
-        bmatvec<B, M>(lu, sb, lane, v, x);
-        scatter_up<B, CG>(up, R, x);
+        red_row<B, ND, M, CG>(g, e, q, m.U, rr, z, v);
+        block_mul<B, M>(m.dr + (size_t)q * B * B, v, x);
+        scatter_up<B, CG>(up, e, x);
     }
 }
 
-// z_R = D_R^-1 (r_R - sum L_RJ y_J) over the black rows, y the red
-// right-hand side (null: zero): the sweep from z = 0.
-template <int B, int KM, class M, bool CG, bool U>
-__device__ __forceinline__ void rb_pre_rows(int nr, int nb, const SellView& m, const M* __restrict__ lu,
-                                            const double* r, const double* y, double* z, int tid, int nth)
+// z = D_b^-1 (rb - L rr): the sweep from z = 0.
+template <int B, int ND, class M, bool CG>
+__device__ __forceinline__ void rb_pre_rows(const RbGrid& g, const RbMatrix<const M>& m, const double* rr,
+                                            const double* rb, double* z, int tid, int nth)
 {
-    for (int R = (nr & ~31) + tid; R < nb; R += nth) {  // whole slices
-        if (R < nr) continue;
-        const int lane = R & 31, sb = slice_base<U>(m, R), d = m.len[R] - 1;
-        double acc[B];
+    const int nk = g.n - g.nr;
+    for (int q = tid; q < nk; q += nth) {
+        double acc[B], v[B], x[B];
 #pragma unroll
-        for (int c = 0; c < B; ++c) acc[c] = 0.0;
-        if (y) bdot<B, KM, double, M, CG, U>(m, sb, lane, 0, d, lu, y, y, INT_MAX, acc);
-        double v[B], x[B];
-        load_bvec<B, double, CG>(r, R, v);
+        for (int t = 0; t < B; ++t) acc[t] = 0.0;
+        if (rr) stencil_dot<B, ND, M, CG>(g, cell_of(g, 1, q), q, nk, m.L, rr, acc);
+        load_bvec<B, double, CG>(rb, q, v);
 #pragma unroll
-        for (int c = 0; c < B; ++c) v[c] -= acc[c];
-        bmatvec<B, M>(lu, sb + (d << 5), lane, v, x);
-        store_bvec<B, double>(z, R, x);
+        for (int t = 0; t < B; ++t) v[t] = __dsub_rn(v[t], acc[t]);
+        block_mul<B, M>(m.db + (size_t)q * B * B, v, x);
+        store_bvec<B, double>(z, q, x);
     }
 }
 
-// t_R = r_R - A_RR z_R - sum L_RJ y_J of one black row.
-template <int B, int KM, class M, bool CG, bool U>
-__device__ __forceinline__ void rb_residual_row(int R, const SellView& m, const M* __restrict__ a,
-                                                const M* __restrict__ lu, const double* r, const double* y,
-                                                const double (&z)[B], double (&t)[B])
+// t = rb - A_bb z - L y of one black row.
+template <int B, int ND, class M, bool CG>
+__device__ __forceinline__ void residual_row(const RbGrid& g, const Cell& e, int q, const RbMatrix<const M>& m,
+                                             const double* rb, const double* y, const double (&z)[B], double (&t)[B])
 {
-    const int lane = R & 31, sb = slice_base<U>(m, R), d = m.len[R] - 1;
     double acc[B], az[B];
 #pragma unroll
     for (int c = 0; c < B; ++c) acc[c] = 0.0;
-    bdot<B, KM, double, M, CG, U>(m, sb, lane, 0, d, lu, y, y, INT_MAX, acc);
-    bmatvec<B, M>(a, sb + (d << 5), lane, z, az);
-    load_bvec<B, double, CG>(r, R, t);
+    load_bvec<B, double, CG>(rb, q, t);
+    block_mul<B, M>(m.abb + (size_t)q * B * B, z, az);
+    stencil_dot<B, ND, M, CG>(g, e, q, g.n - g.nr, m.L, y, acc);
 #pragma unroll
-    for (int c = 0; c < B; ++c) t[c] = (t[c] - az[c]) - acc[c];
+    for (int c = 0; c < B; ++c) t[c] = __dsub_rn(__dsub_rn(t[c], az[c]), acc[c]);
 }
 
-// rc_P = sum of t over the black members of aggregate P, g lanes per
-// aggregate (a power of two; member s of P at list[P g + s], -1 past the
-// last): the lanes' rows are consecutive between neighbouring aggregates, so
-// a warp reads whole segments, and the sum is a butterfly over the g lanes.
-template <int B, int KM, class M, bool CG, bool U>
-__device__ __forceinline__ void rb_res_rows(int ncb, int g, const int* __restrict__ list, const SellView& m,
-                                            const M* __restrict__ a, const M* __restrict__ lu, const double* r,
+// Coarse right-hand side: the sum of t over the black members of each
+// aggregate, g lanes per aggregate in the order of the coarse cells (a
+// member's row follows its neighbour's: whole segments), summed by a
+// butterfly over the g lanes.  rc: red coarse cells, then black ones.
+template <int B, int ND, class M, bool CG>
+__device__ __forceinline__ void rb_res_rows(const Aggregates& a, const RbMatrix<const M>& m, const double* rb,
                                             const double* y, const double* z, double* rc, int tid, int nth)
 {
-    const int items = ncb * g, padded = (items + 31) & ~31;
-    for (int i = tid; i < padded; i += nth) {
-        const int R = i < items ? list[i] : -1;
+    const int items = a.coarse.n * a.g, padded = (items + 31) & ~31, lg = a.g == 4 ? 2 : a.g - 1;
+    for (int it = tid; it < padded; it += nth) {
+        const Cell C = cell_at(a.coarse, it < items ? it >> lg : 0);
+        const int c = it < items ? black_member(a, C.i, C.j, C.k, it & (a.g - 1)) : -1;
         double t[B];
 #pragma unroll
-        for (int c = 0; c < B; ++c) t[c] = 0.0;
-        if (R >= 0) {
+        for (int v = 0; v < B; ++v) t[v] = 0.0;
+        if (c >= 0) {
+            const int q = c >> 1;
             double zv[B];
-            load_bvec<B, double, CG>(z, R, zv);
-            rb_residual_row<B, KM, M, CG, U>(R, m, a, lu, r, y, zv, t);
+            load_bvec<B, double, CG>(z, q, zv);
+            residual_row<B, ND, M, CG>(a.fine, cell_at(a.fine, c), q, m, rb, y, zv, t);
         }
-        for (int o = 1; o < g; o <<= 1)
+        for (int o = 1; o < a.g; o <<= 1)
 #pragma unroll
-            for (int c = 0; c < B; ++c) t[c] += __shfl_xor_sync(0xffffffffu, t[c], o);
-        if (i < items && (i & (g - 1)) == 0) store_bvec<B, double>(rc, i / g, t);
+            for (int v = 0; v < B; ++v) t[v] += __shfl_xor_sync(0xffffffffu, t[v], o);
+        if (it < items && (it & (a.g - 1)) == 0)
+            store_bvec<B, double>(rc, (C.c >> 1) + (((C.i + C.j + C.k) & 1) ? a.coarse.nr : 0), t);
     }
 }
 
-// rc_P = sum of r over the members of aggregate P in `list`, g per aggregate.
+// The same of the right-hand side itself (rr null: zero), for a level
+// without pre-smoothing: pairs, a black member and the red one beside it.
 template <int B, bool CG>
-__device__ __forceinline__ void rb_restrict_rows(int ncb, int g, const int* __restrict__ list, const double* r,
-                                                 double* rc, int tid, int nth)
+__device__ __forceinline__ void rb_restrict_rows(const Aggregates& a, const double* rr, const double* rb, double* rc,
+                                                 int tid, int nth)
 {
-    for (int P = tid; P < ncb; P += nth) {
+    for (int p = tid; p < a.coarse.n; p += nth) {
+        const Cell C = cell_at(a.coarse, p);
         double s[B];
 #pragma unroll
-        for (int c = 0; c < B; ++c) s[c] = 0.0;
-        for (int k = 0; k < g; ++k) {
-            const int m = list[P * g + k];
-            if (m < 0) continue;
+        for (int t = 0; t < B; ++t) s[t] = 0.0;
+        const int i0 = C.i << a.sx, j0 = C.j << a.sy, k0 = C.k << a.sz;
+        for (int o = 0; o < (1 << (a.sx + a.sy + a.sz)); ++o) {
+            const int i = i0 + (a.sx ? o & 1 : 0), j = j0 + (a.sy ? (o >> a.sx) & 1 : 0), k = k0 + (a.sz ? o >> (a.sx + a.sy) : 0);
+            if (i >= a.fine.nx || j >= a.fine.ny || k >= a.fine.nz) continue;
+            const double* r = ((i + j + k) & 1) ? rb : rr;
+            if (!r) continue;
             double v[B];
-            load_bvec<B, double, CG>(r, m, v);
+            load_bvec<B, double, CG>(r, (i + a.fine.nx * (j + a.fine.ny * k)) >> 1, v);
 #pragma unroll
-            for (int c = 0; c < B; ++c) s[c] += v[c];
+            for (int t = 0; t < B; ++t) s[t] += v[t];
         }
-        store_bvec<B, double>(rc, P, s);
+        store_bvec<B, double>(rc, (p >> 1) + (((C.i + C.j + C.k) & 1) ? a.coarse.nr : 0), s);
     }
 }
 
-// z_R += D_R^-1 (r_R - A_RR z_R - sum L_RJ y_J) over the black rows, handed
-// to the finer level.
-template <int B, int KM, class M, bool CG, bool U>
-__device__ __forceinline__ void rb_post_rows(int nr, int nb, const SellView& m, const M* __restrict__ a,
-                                             const M* __restrict__ lu, const double* r, const double* y, double* z,
-                                             const UpView& up, int tid, int nth)
+// z += D_b^-1 (rb - A_bb z - L y), handed to the finer level.
+template <int B, int ND, class M, bool CG>
+__device__ __forceinline__ void rb_post_rows(const RbGrid& g, const RbMatrix<const M>& m, const double* rb,
+                                             const double* y, double* z, const UpView& up, int tid, int nth)
 {
-    for (int R = (nr & ~31) + tid; R < nb; R += nth) {  // whole slices
-        if (R < nr) continue;
+    const int nk = g.n - g.nr;
+    for (int q = tid; q < nk; q += nth) {
+        const Cell e = cell_of(g, 1, q);
         double zv[B], t[B], x[B];
-        load_bvec<B, double, CG>(z, R, zv);
-        rb_residual_row<B, KM, M, CG, U>(R, m, a, lu, r, y, zv, t);
-        bmatvec<B, M>(lu, slice_base<U>(m, R) + ((m.len[R] - 1) << 5), R & 31, t, x);
+        load_bvec<B, double, CG>(z, q, zv);
+        residual_row<B, ND, M, CG>(g, e, q, m, rb, y, zv, t);
+        block_mul<B, M>(m.db + (size_t)q * B * B, t, x);
 #pragma unroll
-        for (int c = 0; c < B; ++c) zv[c] += x[c];
-        store_bvec<B, double>(z, R, zv);
-        scatter_up<B, CG>(up, R, zv);
+        for (int c = 0; c < B; ++c) zv[c] = __dadd_rn(zv[c], x[c]);
+        store_bvec<B, double>(z, q, zv);
+        scatter_up<B, CG>(up, e, zv);
     }
 }
 
-// The coarsest level: z = inv r, a warp per unknown (see dense_rows), handed
-// to the finer level.
+// The coarsest level: inv r, a warp per unknown (see dense_rows; red cells,
+// then black ones), handed to the finer level.
 template <int B, class M, bool CG>
-__device__ __forceinline__ void rb_dense_rows(int n, const M* __restrict__ inv, const double* r, const UpView& up,
-                                              int tid, int nth)
+__device__ __forceinline__ void rb_dense_rows(const RbGrid& g, const M* __restrict__ inv, const double* r,
+                                              const UpView& up, int tid, int nth)
 {
-    const int lane = tid & 31;
+    const int lane = tid & 31, n = g.n * B;
     for (int i = tid >> 5; i < n; i += nth >> 5) {
         double s = 0.0;
-        for (int j = lane; j < n; j += 32) s += (double)inv[i * n + j] * (CG ? __ldcg(r + j) : r[j]);
+        for (int j = lane; j < n; j += 32) s = __fma_rn((double)inv[i * n + j], CG ? __ldcg(r + j) : r[j], s);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         const int P = i / B, c = i - P * B;
-        if (lane < up.g) {
-            const int m = up.list[P * up.g + lane];
-            if (m >= 0) {
-                double* w = up.w + (size_t)m * B + c;
-                const double f = up.add ? (CG ? __ldcg(w) : *w) : 0.0;
-                *w = f + up.alpha * s;
+        if (lane < up.agg.g) {
+            const Cell e = P < g.nr ? cell_of(g, 0, P) : cell_of(g, 1, P - g.nr);
+            const int f = black_member(up.agg, e.i, e.j, e.k, lane);
+            if (f >= 0) {
+                double* w = up.w + (size_t)(f >> 1) * B + c;
+                *w = __fma_rn(up.alpha, s, up.add ? (CG ? __ldcg(w) : *w) : 0.0);
             }
         }
     }
 }
 
 // ---- one step per launch ------------------------------------------------------
-template <int B, int KM, class M>
-__global__ void __launch_bounds__(512) rb_y_kernel(int nr, SellView m, const M* __restrict__ lu, const double* r,
-                                                   const double* z, double* y, const KScal* sc, int skip_if_s)
+template <int B, int ND, class M>
+__global__ void __launch_bounds__(512) rb_y_kernel(RbGrid g, RbMatrix<const M> m, const double* rr, const double* z,
+                                                   double* y, const KScal* sc, int skip_if_s)
 {
     pdl_wait();
     if (mg_skip(sc, skip_if_s)) return;
     THREAD_RANGE;
-    rb_y_rows<B, KM, M, false, false>(nr, m, lu, r, z, y, tid, nth);
+    rb_y_rows<B, ND, M, false>(g, m, rr, z, y, tid, nth);
 }
 
-template <int B, int KM, class M>
-__global__ void __launch_bounds__(512) rb_fin_kernel(int nr, SellView m, const M* __restrict__ lu, const double* r,
-                                                     const double* z, UpView up, const KScal* sc, int skip_if_s)
+template <int B, int ND, class M>
+__global__ void __launch_bounds__(512) rb_fin_kernel(RbGrid g, RbMatrix<const M> m, const double* rr, const double* z,
+                                                     UpView up, const KScal* sc, int skip_if_s)
 {
     pdl_wait();
     if (mg_skip(sc, skip_if_s)) return;
     THREAD_RANGE;
-    rb_fin_rows<B, KM, M, false, false>(nr, m, lu, r, z, up, tid, nth);
+    rb_fin_rows<B, ND, M, false>(g, m, rr, z, up, tid, nth);
 }
 
-template <int B, int KM, class M>
-__global__ void __launch_bounds__(512) rb_pre_kernel(int nr, int nb, SellView m, const M* __restrict__ lu,
-                                                     const double* r, const double* y, double* z, const KScal* sc,
+template <int B, int ND, class M>
+__global__ void __launch_bounds__(512) rb_pre_kernel(RbGrid g, RbMatrix<const M> m, const double* rr, const double* rb,
+                                                     double* z, const KScal* sc, int skip_if_s)
+{
+    pdl_wait();
+    if (mg_skip(sc, skip_if_s)) return;
+    THREAD_RANGE;
+    rb_pre_rows<B, ND, M, false>(g, m, rr, rb, z, tid, nth);
+}
+
+template <int B, int ND, class M>
+__global__ void __launch_bounds__(512) rb_res_kernel(Aggregates a, RbMatrix<const M> m, const double* rb,
+                                                     const double* y, const double* z, double* rc, const KScal* sc,
                                                      int skip_if_s)
 {
     pdl_wait();
     if (mg_skip(sc, skip_if_s)) return;
     THREAD_RANGE;
-    rb_pre_rows<B, KM, M, false, false>(nr, nb, m, lu, r, y, z, tid, nth);
-}
-
-template <int B, int KM, class M>
-__global__ void __launch_bounds__(512) rb_res_kernel(int ncb, int g, const int* __restrict__ list, SellView m,
-                                                     const M* __restrict__ a, const M* __restrict__ lu,
-                                                     const double* r, const double* y, const double* z, double* rc,
-                                                     const KScal* sc, int skip_if_s)
-{
-    pdl_wait();
-    if (mg_skip(sc, skip_if_s)) return;
-    THREAD_RANGE;
-    rb_res_rows<B, KM, M, false, false>(ncb, g, list, m, a, lu, r, y, z, rc, tid, nth);
+    rb_res_rows<B, ND, M, false>(a, m, rb, y, z, rc, tid, nth);
 }
 
 template <int B>
-__global__ void rb_restrict_kernel(int ncb, int g, const int* __restrict__ list, const double* r, double* rc,
-                                   const KScal* sc, int skip_if_s)
+__global__ void __launch_bounds__(512) rb_restrict_kernel(Aggregates a, const double* rr, const double* rb, double* rc,
+                                                          const KScal* sc, int skip_if_s)
 {
     pdl_wait();
     if (mg_skip(sc, skip_if_s)) return;
     THREAD_RANGE;
-    rb_restrict_rows<B, false>(ncb, g, list, r, rc, tid, nth);
+    rb_restrict_rows<B, false>(a, rr, rb, rc, tid, nth);
 }
 
-template <int B, int KM, class M>
-__global__ void __launch_bounds__(512) rb_post_kernel(int nr, int nb, SellView m, const M* __restrict__ a,
-                                                      const M* __restrict__ lu, const double* r, const double* y,
+template <int B, int ND, class M>
+__global__ void __launch_bounds__(512) rb_post_kernel(RbGrid g, RbMatrix<const M> m, const double* rb, const double* y,
                                                       double* z, UpView up, const KScal* sc, int skip_if_s)
 {
     pdl_wait();
     if (mg_skip(sc, skip_if_s)) return;
     THREAD_RANGE;
-    rb_post_rows<B, KM, M, false, false>(nr, nb, m, a, lu, r, y, z, up, tid, nth);
+    rb_post_rows<B, ND, M, false>(g, m, rb, y, z, up, tid, nth);
 }
 
 template <int B, class M>
-__global__ void rb_dense_kernel(int n, const M* __restrict__ inv, const double* r, UpView up, const KScal* sc,
-                                int skip_if_s)
+__global__ void __launch_bounds__(1024) rb_dense_kernel(RbGrid g, const M* __restrict__ inv, const double* r, UpView up,
+                                                        const KScal* sc, int skip_if_s)
 {
     pdl_wait();
     if (mg_skip(sc, skip_if_s)) return;
-    rb_dense_rows<B, M, false>(n, inv, r, up, (int)threadIdx.x, (int)blockDim.x);
+    rb_dense_rows<B, M, false>(g, inv, r, up, (int)threadIdx.x, (int)blockDim.x);
 }
 
 // ---- BiCGStab on the black half ------------------------------------------------
-// g = b_b - L b_r is the first residual; with the vectors' start values, the
-// shadow residual, and the dots of bicg_init (rr of g, thr of the whole b).
-// b is in block-row order; the other vectors hold the black rows only.
-template <int B, int KM>
-__global__ void __launch_bounds__(kThreads) rb_init_kernel(int nr, int nb, SellView m, const double* __restrict__ lu,
+// b (red cells, then black ones) from the natural order, component after
+// component.
+template <int B>
+__global__ void rb_permute_kernel(RbGrid g, const double* __restrict__ rhs, double* __restrict__ b)
+{
+    GRID_STRIDE(c64, g.n)
+    {
+        const Cell e = cell_at(g, (int)c64);
+        const int P = (e.c >> 1) + (((e.i + e.j + e.k) & 1) ? g.nr : 0);
+        double v[B];
+#pragma unroll
+        for (int t = 0; t < B; ++t) v[t] = rhs[(size_t)t * g.n + e.c];
+        store_bvec<B, double>(b, P, v);
+    }
+}
+
+// b_b - L b_r is the first residual; with the vectors' start values, the
+// shadow residual, and the dots of bicg_init (rr of the residual, thr of the
+// whole b).
+template <int B, int ND>
+__global__ void __launch_bounds__(kThreads) rb_init_kernel(RbGrid g, RbMatrix<const double> m,
                                                            const double* __restrict__ b, double* r, double* rhat,
                                                            double* p, double* v, double* x, double* partials,
                                                            unsigned int* counter, KScal* sc, double tol2)
 {
+    const int nk = g.n - g.nr;
+    const double* bb = b + (size_t)g.nr * B;
     double d[3] = {0.0, 0.0, 0.0};
-    GRID_STRIDE(rr, nb)
+    GRID_STRIDE(i64, g.nr)
     {
-        const int R = (int)rr;
-        double bv[B];
-        load_bvec<B, double>(b, R, bv);
+        const int q = (int)i64;
+        double w[B];
+        load_bvec<B, double>(b, q, w);
 #pragma unroll
-        for (int c = 0; c < B; ++c) d[2] += bv[c] * bv[c];
-        if (R < nr) continue;
+        for (int t = 0; t < B; ++t) d[2] += w[t] * w[t];
+        if (q >= nk) continue;
         double acc[B];
 #pragma unroll
-        for (int c = 0; c < B; ++c) acc[c] = 0.0;
-        bdot<B, KM, double, double>(m, m.slice_ptr[R >> 5], R & 31, 0, m.len[R] - 1, lu, b, b, INT_MAX, acc);
-        const int q = R - nr;
+        for (int t = 0; t < B; ++t) acc[t] = 0.0;
+        stencil_dot<B, ND, double, false>(g, cell_of(g, 1, q), q, nk, m.L, b, acc);
+        load_bvec<B, double>(bb, q, w);
 #pragma unroll
-        for (int c = 0; c < B; ++c) {
-            const int64_t i = (int64_t)q * B + c;
-            const double gi = bv[c] - acc[c], hi = shadow_entry(i);
+        for (int t = 0; t < B; ++t) {
+            const int64_t i = (int64_t)q * B + t;
+            const double gi = w[t] - acc[t], hi = shadow_entry(i);
+            d[2] += w[t] * w[t];
             r[i] = gi;
             rhat[i] = hi;
             p[i] = 0.0;
@@ -363,50 +559,48 @@ __global__ void __launch_bounds__(kThreads) rb_init_kernel(int nr, int nb, SellV
     }
 }
 
-// v = S z = A_bb z + L y (y = -U z) over the black rows, with the dots of
-// bicg_spmv_alpha (OMEGA false: alpha = rho_new / (h . v), h the shadow
-// residual) or bicg_spmv_omega (omega = (v . h) / (v . v), h = s).  z, h and
-// v hold the black rows only.
-template <int B, int KM, bool OMEGA>
+// v = S z = A_bb z + L y (y = -U z), with the dots of bicg_spmv_alpha (OMEGA
+// false: alpha = rho_new / (h . v), h the shadow residual) or
+// bicg_spmv_omega (omega = (v . h) / (v . v), h = s).
+template <int B, int ND, bool OMEGA>
 __global__ void __launch_bounds__(kThreads)
-    rb_spmv_kernel(int nr, int nb, SellView m, const double* __restrict__ a, const double* __restrict__ lu,
-                   const double* __restrict__ z, const double* __restrict__ y, const double* __restrict__ h,
-                   double* __restrict__ v, double* partials, unsigned int* counter, KScal* sc)
+    rb_spmv_kernel(RbGrid g, RbMatrix<const double> m, const double* __restrict__ z, const double* __restrict__ y,
+                   const double* __restrict__ h, double* __restrict__ v, double* partials, unsigned int* counter,
+                   KScal* sc)
 {
     pdl_wait();
     if (stopped(sc) || (OMEGA && sc->s_conv)) return;
-    constexpr int ND = OMEGA ? 2 : 1;
-    double d[ND];
+    constexpr int ND_ = OMEGA ? 2 : 1;
+    const int nk = g.n - g.nr;
+    double d[ND_];
 #pragma unroll
-    for (int k = 0; k < ND; ++k) d[k] = 0.0;
-    GRID_STRIDE(i, nb - (nr & ~31))  // whole slices
+    for (int k = 0; k < ND_; ++k) d[k] = 0.0;
+    GRID_STRIDE(q64, nk)
     {
-        const int R = (nr & ~31) + (int)i, q = R - nr;
-        if (q < 0) continue;
-        const int lane = R & 31, sb = m.slice_ptr[R >> 5], dk = m.len[R] - 1;
+        const int q = (int)q64;
         double acc[B], zv[B], az[B], hv[B];
 #pragma unroll
-        for (int c = 0; c < B; ++c) acc[c] = 0.0;
-        bdot<B, KM, double, double>(m, sb, lane, 0, dk, lu, y, y, INT_MAX, acc);
+        for (int t = 0; t < B; ++t) acc[t] = 0.0;
         load_bvec<B, double>(z, q, zv);
-        bmatvec<B, double>(a, sb + (dk << 5), lane, zv, az);
         load_bvec<B, double>(h, q, hv);
+        block_mul<B, double>(m.abb + (size_t)q * B * B, zv, az);
+        stencil_dot<B, ND, double, false>(g, cell_of(g, 1, q), q, nk, m.L, y, acc);
 #pragma unroll
-        for (int c = 0; c < B; ++c) acc[c] += az[c];
+        for (int t = 0; t < B; ++t) acc[t] += az[t];
         store_bvec<B, double>(v, q, acc);
 #pragma unroll
-        for (int c = 0; c < B; ++c) {
-            d[0] += hv[c] * acc[c];
-            if (OMEGA) d[ND - 1] += acc[c] * acc[c];
+        for (int t = 0; t < B; ++t) {
+            d[0] += hv[t] * acc[t];
+            if (OMEGA) d[ND_ - 1] += acc[t] * acc[t];
         }
     }
-    double s[ND];
-    if (grid_sum<ND>(d, partials, counter, s)) {
+    double s[ND_];
+    if (grid_sum<ND_>(d, partials, counter, s)) {
         if (OMEGA) {
             sc->ts = s[0];
-            sc->tt = s[ND - 1];
-            if (s[ND - 1] == 0.0 || !isfinite(s[ND - 1])) sc->status = ST_BREAK;
-            else sc->omega = s[0] / s[ND - 1];
+            sc->tt = s[ND_ - 1];
+            if (s[ND_ - 1] == 0.0 || !isfinite(s[ND_ - 1])) sc->status = ST_BREAK;
+            else sc->omega = s[0] / s[ND_ - 1];
         } else {
             sc->rv = s[0];
             if (s[0] == 0.0 || !isfinite(s[0])) sc->status = ST_BREAK;
@@ -415,60 +609,282 @@ __global__ void __launch_bounds__(kThreads)
     }
 }
 
-// The solution in the natural unknown order: x_b, and x_r = D_r^-1 (b_r - U x_b).
-template <int B, int KM>
-__global__ void __launch_bounds__(kThreads) rb_solution_kernel(int nr, int nb, SellView m,
-                                                               const double* __restrict__ lu,
+// The solution in the natural order: x_b, and x_r = D_r^-1 (b_r - U x_b).
+template <int B, int ND>
+__global__ void __launch_bounds__(kThreads) rb_solution_kernel(RbGrid g, RbMatrix<const double> m,
                                                                const double* __restrict__ b,
-                                                               const double* __restrict__ x,
-                                                               const int* __restrict__ perm, double* __restrict__ out)
+                                                               const double* __restrict__ x, double* __restrict__ out)
 {
-    GRID_STRIDE(rr, nb)
+    const int nk = g.n - g.nr;
+    GRID_STRIDE(q64, g.nr)
     {
-        const int R = (int)rr;
-        double z[B];
-        if (R < nr) {
-            const int lane = R & 31, sb = m.slice_ptr[R >> 5];
-            double acc[B], v[B];
+        const int q = (int)q64;
+        const Cell e = cell_of(g, 0, q);
+        double v[B], z[B];
+        red_row<B, ND, double, false>(g, e, q, m.U, b, x, v);
+        block_mul<B, double>(m.dr + (size_t)q * B * B, v, z);
 #pragma unroll
-            for (int c = 0; c < B; ++c) acc[c] = 0.0;
-            const double* xs = x - (int64_t)nr * B;
-            bdot<B, KM, double, double>(m, sb, lane, 1, m.len[R], lu, xs, xs, INT_MAX, acc);
-            load_bvec<B, double>(b, R, v);
+        for (int t = 0; t < B; ++t) out[(size_t)t * g.n + e.c] = z[t];
+        if (q >= nk) continue;
+        const Cell f = cell_of(g, 1, q);
+        load_bvec<B, double>(x, q, z);
 #pragma unroll
-            for (int c = 0; c < B; ++c) v[c] -= acc[c];
-            bmatvec<B, double>(lu, sb, lane, v, z);
-        } else {
-            load_bvec<B, double>(x, R - nr, z);
+        for (int t = 0; t < B; ++t) out[(size_t)t * g.n + f.c] = z[t];
+    }
+}
+
+// ---- set-up ---------------------------------------------------------------------
+// Where the Jacobian's entries go, one thread per row (component after
+// component): map[position in A] = entry.  bad |= 1: an entry that couples
+// cells which are no neighbours; 2: a row without its diagonal entry.
+__global__ void rb_map_kernel(RbGrid g, int B, int nd, const int* __restrict__ rowptr, const int* __restrict__ colind,
+                              int* __restrict__ map, int* bad)
+{
+    const int nk = g.n - g.nr, bb = B * B;
+    int flags = 0;
+    GRID_STRIDE(u, (int64_t)g.n * B)
+    {
+        const int cu = (int)(u / g.n);
+        const Cell e = cell_at(g, (int)(u - (int64_t)cu * g.n));
+        const int colour = (e.i + e.j + e.k) & 1, q = e.c >> 1, rows = colour ? nk : g.nr;
+        const size_t off = colour ? (size_t)nd * g.nr : 0, dia = (size_t)nd * g.n + (colour ? g.nr : 0);
+        bool has = false;
+        for (int t = rowptr[u]; t < rowptr[u + 1]; ++t) {
+            const int col = colind[t], cv = col / g.n, c = col - cv * g.n, diff = c - e.c;
+            size_t slot;
+            if (diff == 0) {
+                slot = dia + q;
+                has = has || cv == cu;
+            } else {
+                // the direction whose neighbour c is (sides of 1 make two
+                // offsets equal: the one that exists)
+                int d = 0, nq = 0;
+                for (; d < nd; ++d) {
+                    const int o = d < 2 ? 1 : d < 4 ? g.nx : g.step;
+                    if (diff == (d & 1 ? o : -o) && neighbour(g, e, d, nq)) break;
+                }
+                if (d == nd) {
+                    flags |= 1;
+                    continue;
+                }
+                slot = off + (size_t)d * rows + q;
+            }
+            map[slot * bb + cu * B + cv] = t;
         }
+        if (!has) flags |= 2;
+    }
+    if (flags) atomicOr(bad, flags);
+}
+
+// A from the Jacobian's values.  A tile of 32 cells of a colour takes all its
+// directions in turn, so that the sectors of its Jacobian rows, read eight
+// bytes at a time, are read again from L1.
+__global__ void __launch_bounds__(kThreads) rb_gather_kernel(RbGrid g, int bb, int nd, const int* __restrict__ map,
+                                                             const double* __restrict__ j, double* __restrict__ a)
+{
+    const int nk = g.n - g.nr;
+    const int red_tiles = (g.nr + 31) / 32, tiles = red_tiles + (nk + 31) / 32;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const bool red = tile < red_tiles;
+        const int rows = red ? g.nr : nk, q0 = (red ? tile : tile - red_tiles) * 32;
+        const int w = min(32, rows - q0) * bb;
+        for (int x = threadIdx.x; x < w * (nd + 1); x += blockDim.x) {
+            const int d = x / w;
+            const size_t row = d < nd ? (red ? 0 : (size_t)nd * g.nr) + (size_t)d * rows : (size_t)nd * g.n + (red ? 0 : g.nr);
+            const size_t p = (row + q0) * bb + (x - d * w);
+            const int e = map[p];
+            a[p] = e >= 0 ? j[e] : 0.0;
+        }
+    }
+}
+
+// Mean share that each direction has of a cell's couplings of a component
+// with itself, weighted by how strongly the row is coupled at all (shares of
+// its diagonal entry, at most 1).
+__global__ void __launch_bounds__(kThreads) rb_strength_kernel(RbGrid g, int B, int nd, const double* __restrict__ a,
+                                                               double* partials, unsigned int* counter, double* out)
+{
+    const int bb = B * B;
+    const RbMatrix<const double> m(a, nd, bb, g.n, g.nr);
+    double sum[3] = {0.0, 0.0, 0.0};
+    GRID_STRIDE(P64, g.n)
+    {
+        const int P = (int)P64;
+        const bool red = P < g.nr;
+        const int rows = red ? g.nr : g.n - g.nr, q = red ? P : P - g.nr;
+        for (int c = 0; c < B; ++c) {
+            const int e = c * B + c;
+            const double diag = fabs((red ? m.dr : m.abb)[(size_t)q * bb + e]);
+            double s[3] = {0.0, 0.0, 0.0};
+            for (int d = 0; d < nd; ++d) s[d >> 1] += fabs((red ? m.U : m.L)[((size_t)d * rows + q) * bb + e]);
+            const double all = s[0] + s[1] + s[2];
+            if (!(all > 0.0) || !(diag > 0.0) || !isfinite(all / diag)) continue;
+            const double w = fmin(1.0, all / diag) / all;
+            for (int t = 0; t < 3; ++t) sum[t] += w * s[t];
+        }
+    }
+    double s[3];
+    if (grid_sum<3>(sum, partials, counter, s))
+        for (int t = 0; t < 3; ++t) out[t] = s[t];
+}
+
+// The coarse matrix R A R^T of a 0/1 aggregation, one thread per value of a
+// coarse cell: the blocks of its members that cross each of its faces, and
+// its diagonal block with the couplings inside it, summed in the order of
+// the members and directions.
+__global__ void __launch_bounds__(kThreads) rb_galerkin_kernel(Aggregates a, int bb, int nd, const double* __restrict__ fa,
+                                                               double* __restrict__ ca)
+{
+    const RbGrid &f = a.fine, &g = a.coarse;
+    const RbMatrix<const double> F(fa, nd, bb, f.n, f.nr);
+    const RbMatrix<double> G(ca, nd, bb, g.n, g.nr);
+    GRID_STRIDE(x, (int64_t)g.n * bb)
+    {
+        const int c = (int)(x / bb), e = (int)(x - (int64_t)c * bb);
+        const Cell C = cell_at(g, c);
+        const bool red = ((C.i + C.j + C.k) & 1) == 0;
+        const int q = c >> 1, rows = red ? g.nr : g.n - g.nr;
+        double diag = 0.0, off[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        for (int o = 0; o < 8; ++o) {
+            const int dx = o & 1, dy = (o >> 1) & 1, dz = o >> 2;
+            if ((dx && !a.sx) || (dy && !a.sy) || (dz && !a.sz)) continue;
+            Cell m;
+            m.i = (C.i << a.sx) + dx;
+            m.j = (C.j << a.sy) + dy;
+            m.k = (C.k << a.sz) + dz;
+            if (m.i >= f.nx || m.j >= f.ny || m.k >= f.nz) continue;
+            m.c = m.i + f.nx * (m.j + f.ny * m.k);
+            const bool mr = ((m.i + m.j + m.k) & 1) == 0;
+            const int mq = m.c >> 1, mrows = mr ? f.nr : f.n - f.nr;
+            diag += (mr ? F.dr : F.abb)[(size_t)mq * bb + e];
 #pragma unroll
-        for (int c = 0; c < B; ++c) out[perm[R * B + c]] = z[c];
+            for (int d = 0; d < 6; ++d) {
+                if (d >= nd) break;
+                int nq;
+                if (!neighbour(f, m, d, nq)) continue;
+                const double v = (mr ? F.U : F.L)[((size_t)d * mrows + mq) * bb + e];
+                // inside the aggregate: the direction is paired and leads to
+                // the other half
+                const bool inner = d < 2 ? a.sx && dx != (d & 1) : d < 4 ? a.sy && dy != (d & 1) : a.sz && dz != (d & 1);
+                if (inner) diag += v;
+                else off[d] += v;
+            }
+        }
+        (red ? G.dr : G.abb)[(size_t)q * bb + e] = diag;
+#pragma unroll
+        for (int d = 0; d < 6; ++d)
+            if (d < nd) (red ? G.U : G.L)[((size_t)d * rows + q) * bb + e] = off[d];
+    }
+}
+
+// D_r^-1 over the red cells.
+template <int B>
+__global__ void __launch_bounds__(kThreads) rb_factor_red_kernel(RbGrid g, double* __restrict__ dr, int* status)
+{
+    constexpr int BB = B * B;
+    GRID_STRIDE(q, g.nr)
+    {
+        double d[BB];
+#pragma unroll
+        for (int e = 0; e < BB; ++e) d[e] = dr[q * BB + e];
+        if (!invert_block<B>(d)) *status = 1;
+#pragma unroll
+        for (int e = 0; e < BB; ++e) dr[q * BB + e] = d[e];
+    }
+}
+
+// L = A_br D_r^-1 and D_b^-1 = (A_bb - sum L U)^-1 over the black cells: of
+// L U only the diagonal block is in the pattern (block ILU(0)).
+template <int B, int ND>
+__global__ void __launch_bounds__(kThreads) rb_factor_black_kernel(RbGrid g, RbMatrix<double> m, int* status)
+{
+    constexpr int BB = B * B;
+    const int nk = g.n - g.nr;
+    GRID_STRIDE(q64, nk)
+    {
+        const int q = (int)q64;
+        const Cell e = cell_of(g, 1, q);
+        double D[BB];
+#pragma unroll
+        for (int t = 0; t < BB; ++t) D[t] = m.abb[(size_t)q * BB + t];
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+            int nq;
+            if (!neighbour(g, e, d, nq)) continue;
+            double* lp = m.L + ((size_t)d * nk + q) * BB;
+            const double* up = m.U + ((size_t)(d ^ 1) * g.nr + nq) * BB;  // the red cell's block towards this one
+            const double* dp = m.dr + (size_t)nq * BB;
+            double av[BB], dv[BB], uv[BB], l[BB];
+            load_block<BB, double>(lp, av);
+            load_block<BB, double>(dp, dv);
+            load_block<BB, double>(up, uv);
+#pragma unroll
+            for (int i = 0; i < B; ++i)
+#pragma unroll
+                for (int j = 0; j < B; ++j) {
+                    double s = 0.0;
+#pragma unroll
+                    for (int t = 0; t < B; ++t) s += av[i * B + t] * dv[t * B + j];
+                    l[i * B + j] = s;
+                }
+#pragma unroll
+            for (int i = 0; i < B; ++i)
+#pragma unroll
+                for (int j = 0; j < B; ++j) {
+                    double s = 0.0;
+#pragma unroll
+                    for (int t = 0; t < B; ++t) s += l[i * B + t] * uv[t * B + j];
+                    D[i * B + j] -= s;
+                }
+#pragma unroll
+            for (int t = 0; t < BB; ++t) lp[t] = l[t];
+        }
+        if (!invert_block<B>(D)) *status = 1;
+#pragma unroll
+        for (int t = 0; t < BB; ++t) m.db[(size_t)q * BB + t] = D[t];
+    }
+}
+
+// The coarsest matrix, dense and row-major (red cells, then black ones), for
+// dense_inverse_kernel; `dense` is zero beforehand.
+__global__ void rb_dense_fill_kernel(RbGrid g, int B, int nd, const double* __restrict__ a, double* __restrict__ dense)
+{
+    const int bb = B * B, n = g.n * B;
+    const RbMatrix<const double> m(a, nd, bb, g.n, g.nr);
+    GRID_STRIDE(P64, g.n)
+    {
+        const int P = (int)P64;
+        const bool red = P < g.nr;
+        const int rows = red ? g.nr : g.n - g.nr, q = red ? P : P - g.nr;
+        const Cell e = cell_of(g, red ? 0 : 1, q);
+        for (int t = 0; t < bb; ++t)
+            dense[(size_t)(P * B + t / B) * n + P * B + t % B] = (red ? m.dr : m.abb)[(size_t)q * bb + t];
+        for (int d = 0; d < nd; ++d) {
+            int nq;
+            if (!neighbour(g, e, d, nq)) continue;
+            const int Q = red ? g.nr + nq : nq;
+            for (int t = 0; t < bb; ++t)
+                dense[(size_t)(P * B + t / B) * n + Q * B + t % B] = (red ? m.U : m.L)[((size_t)d * rows + q) * bb + t];
+        }
     }
 }
 
 // ---- the coarse end of the cycle in one kernel ----------------------------------
 // As mg_tail_kernel: one thread-block cluster, a cluster barrier between the
 // steps, the coarsest levels in block 0's shared memory.
-struct RbLocal {
-    int a, lu, inv, col, len, list, r, w;
-};
-
 template <class M>
 struct RbTailLevel {
-    int nb = 0, nr = 0, n = 0, coarsest = 0, pre = 1;
-    int g = 0;                   // members per aggregate in `list`
-    SellView m{};
-    const M* a = nullptr;
-    const M* lu = nullptr;
-    const M* inv = nullptr;      // coarsest level
-    const int* list = nullptr;   // members restricted to the next level (black ones when pre)
-    const double* r = nullptr;   // right-hand side by block row
-    const double* r_red = nullptr;  // the same, or null where its red rows are zero
-    double* rw = nullptr;        // where the finer level's restriction writes r
-    double* z = nullptr;         // black rows of the iterate, by block row
-    double* y = nullptr;         // red rows' work vector, by block row
-    UpView up;                   // where its rows go
-    RbLocal so{};
+    RbGrid g;
+    int coarsest = 0, pre = 1;
+    const M* a = nullptr;           // matrix (RbMatrix), or the dense inverse of the coarsest level
+    const double* rr = nullptr;     // right-hand side, red (null: zero) and black
+    const double* rb = nullptr;
+    double* r = nullptr;            // where the finer level's restriction writes it
+    double* z = nullptr;            // black iterate
+    double* y = nullptr;            // red work vector
+    Aggregates agg;                 // to the next level
+    UpView up;                      // where its rows go
+    int so_a = 0, so_r = 0, so_w = 0;  // offsets in block 0's shared memory
 };
 
 template <class M>
@@ -478,90 +894,78 @@ struct RbTailParams {
     int local_first = kMaxTail;
     int nregions = 0;
     int ncopies = 0;
-    PrefetchRegion reg[kMaxPrefetch];
-    TailCopy copies[kMaxCopies];
+    PrefetchRegion reg[kMaxTail];
+    TailCopy copies[kMaxTail];
     long long* trace = nullptr;
 };
 static_assert(sizeof(RbTailParams<double>) <= 4096, "fused cycle parameters exceed 4 KB");
 
-// One level's steps down to its coarse right-hand side; `sync` ends a step.
-template <int B, int KM, class M, bool CG, class Sync>
-__device__ __forceinline__ void rb_down(const RbTailLevel<M>& L, const SellView& m, const M* a, const M* lu,
-                                        const int* list, const double* r, const double* r_red, double* z, double* y,
-                                        int ncb, double* rc, int tid, int nth, Sync&& sync)
+// One level's steps down to the coarse right-hand side rc; sync() ends a step.
+template <int B, int ND, class M, bool CG, class Sync>
+__device__ __forceinline__ void rb_down(const RbTailLevel<M>& L, const RbMatrix<const M>& m, const double* rr,
+                                        const double* rb, double* z, double* y, double* rc, int tid, int nth,
+                                        Sync&& sync)
 {
-    constexpr bool U = KM > 0;
     if (L.pre) {
-        rb_pre_rows<B, KM, M, CG, U>(L.nr, L.nb, m, lu, r, r_red, z, tid, nth);
+        rb_pre_rows<B, ND, M, CG>(L.g, m, rr, rb, z, tid, nth);
         sync();
-        rb_y_rows<B, KM, M, CG, U>(L.nr, m, lu, r_red, z, y, tid, nth);
+        rb_y_rows<B, ND, M, CG>(L.g, m, rr, z, y, tid, nth);
         sync();
-        rb_res_rows<B, KM, M, CG, U>(ncb, L.g, list, m, a, lu, r, y, z, rc, tid, nth);
+        rb_res_rows<B, ND, M, CG>(L.agg, m, rb, y, z, rc, tid, nth);
     } else {
-        rb_restrict_rows<B, CG>(ncb, L.g, list, r, rc, tid, nth);
+        rb_restrict_rows<B, CG>(L.agg, rr, rb, rc, tid, nth);
     }
     sync();
 }
 
-template <int B, int KM, class M, bool CG, class Sync>
-__device__ __forceinline__ void rb_up(const RbTailLevel<M>& L, const SellView& m, const M* a, const M* lu,
-                                      const double* r, const double* r_red, double* z, double* y, const UpView& up,
-                                      int tid, int nth, Sync&& sync)
+template <int B, int ND, class M, bool CG, class Sync>
+__device__ __forceinline__ void rb_up(const RbTailLevel<M>& L, const RbMatrix<const M>& m, const double* rr,
+                                      const double* rb, double* z, double* y, const UpView& up, int tid, int nth,
+                                      Sync&& sync)
 {
-    constexpr bool U = KM > 0;
-    rb_y_rows<B, KM, M, CG, U>(L.nr, m, lu, r_red, z, y, tid, nth);
+    rb_y_rows<B, ND, M, CG>(L.g, m, rr, z, y, tid, nth);
     sync();
-    rb_post_rows<B, KM, M, CG, U>(L.nr, L.nb, m, a, lu, r, y, z, up, tid, nth);
+    rb_post_rows<B, ND, M, CG>(L.g, m, rb, y, z, up, tid, nth);
     if (up.w == nullptr) return;
     sync();
-    rb_fin_rows<B, KM, M, CG, U>(L.nr, m, lu, r, z, up, tid, nth);
+    rb_fin_rows<B, ND, M, CG>(L.g, m, rr, z, up, tid, nth);
     sync();
 }
 
 // The levels from lf on, on block 0 alone, in its shared memory; the
 // correction goes to level lf - 1's z in global memory.
-template <int B, int KM, class M>
+template <int B, int ND, class M>
 __device__ void rb_local_cycle(const RbTailParams<M>& p, int lf, unsigned char* sm)
 {
     const int tid = (int)threadIdx.x, nth = (int)blockDim.x;
     auto sync = [] { __syncthreads(); };
-    auto at_r = [&](int l) { return (double*)(sm + p.lv[l].so.r); };
-    auto at_w = [&](int l) { return (double*)(sm + p.lv[l].so.w); };
-    auto view = [&](int l) {
-        const RbLocal& o = p.lv[l].so;
-        return SellView{nullptr, (const int*)(sm + o.col), (const int*)(sm + o.len), nullptr, p.lv[l].m.width};
+    auto at_r = [&](int l) { return (double*)(sm + p.lv[l].so_r); };
+    auto at_y = [&](int l) { return (double*)(sm + p.lv[l].so_w); };
+    auto at_z = [&](int l) { return at_y(l) + p.lv[l].g.nr * B; };
+    auto matrix = [&](int l) {
+        const RbGrid& g = p.lv[l].g;
+        return RbMatrix<const M>((const M*)(sm + p.lv[l].so_a), ND, B * B, g.n, g.nr);
     };
-    // where level l's rows go: the level above it in shared memory, or
-    // level lf - 1 in global memory
     auto up_of = [&](int l) {
         UpView u = p.lv[l].up;
-        if (l > lf) {
-            u.list = (const int*)(sm + p.lv[l - 1].so.list);
-            if (!p.lv[l - 1].pre) u.list = p.lv[l].up.list;
-            u.w = at_w(l - 1);
-        }
+        if (l > lf) u.w = at_z(l - 1);
         return u;
     };
     asm volatile("cp.async.wait_all;" ::: "memory");
-    for (int i = tid; i < p.lv[lf].n; i += nth) at_r(lf)[i] = __ldcg(p.lv[lf].r + i);
+    for (int i = tid; i < p.lv[lf].g.n * B; i += nth) at_r(lf)[i] = __ldcg(p.lv[lf].rr + i);
     __syncthreads();
     int l = lf;
-    for (; !p.lv[l].coarsest; ++l) {
-        const RbTailLevel<M>& L = p.lv[l];
-        rb_down<B, KM, M, false>(L, view(l), (const M*)(sm + L.so.a), (const M*)(sm + L.so.lu),
-                                 (const int*)(sm + L.so.list), at_r(l), at_r(l), at_w(l), at_w(l), p.lv[l + 1].nb,
+    for (; !p.lv[l].coarsest; ++l)
+        rb_down<B, ND, M, false>(p.lv[l], matrix(l), at_r(l), at_r(l) + p.lv[l].g.nr * B, at_z(l), at_y(l),
                                  at_r(l + 1), tid, nth, sync);
-    }
-    rb_dense_rows<B, M, false>(p.lv[l].n, (const M*)(sm + p.lv[l].so.inv), at_r(l), up_of(l), tid, nth);
+    rb_dense_rows<B, M, false>(p.lv[l].g, (const M*)(sm + p.lv[l].so_a), at_r(l), up_of(l), tid, nth);
     __syncthreads();
-    for (--l; l >= lf; --l) {
-        const RbTailLevel<M>& L = p.lv[l];
-        rb_up<B, KM, M, false>(L, view(l), (const M*)(sm + L.so.a), (const M*)(sm + L.so.lu), at_r(l), at_r(l),
-                               at_w(l), at_w(l), up_of(l), tid, nth, sync);
-    }
+    for (--l; l >= lf; --l)
+        rb_up<B, ND, M, false>(p.lv[l], matrix(l), at_r(l), at_r(l) + p.lv[l].g.nr * B, at_z(l), at_y(l), up_of(l),
+                               tid, nth, sync);
 }
 
-template <int B, int KM, class M>
+template <int B, int ND, class M>
 __global__ void __launch_bounds__(kTailThreads)
     rb_tail_kernel(const __grid_constant__ RbTailParams<M> p, const KScal* sc, int skip_if_s)
 {
@@ -580,26 +984,24 @@ __global__ void __launch_bounds__(kTailThreads)
     if (trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0) trace[tk] = clock64();
     ++tk;
     auto sync = [&] { tail_step(trace, tk); };
-    // a warp (one slice of 32 rows) at a time, round robin over the blocks
+    // 32 rows (a warp) at a time, round robin over the blocks
     const int tid = (((int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x) << 5) | (int)(threadIdx.x & 31);
     const int nth = (int)(gridDim.x * blockDim.x);
+    auto matrix = [&](const RbTailLevel<M>& L) { return RbMatrix<const M>(L.a, ND, B * B, L.g.n, L.g.nr); };
     int l = 0;
     for (; l < lf && !p.lv[l].coarsest; ++l) {
         const RbTailLevel<M>& L = p.lv[l];
-        rb_down<B, KM, M, true>(L, L.m, L.a, L.lu, L.list, L.r, L.r_red, L.z, L.y, p.lv[l + 1].nb, p.lv[l + 1].rw,
-                                tid, nth, sync);
+        rb_down<B, ND, M, true>(L, matrix(L), L.rr, L.rb, L.z, L.y, p.lv[l + 1].r, tid, nth, sync);
     }
     if (l == lf) {
         // block 0 alone; the other blocks wait at the next cluster barrier
-        if constexpr (KM > 0) {
-            if (blockIdx.x == 0) rb_local_cycle<B, KM, M>(p, lf, tail_smem);
-        }
+        if (blockIdx.x == 0) rb_local_cycle<B, ND, M>(p, lf, tail_smem);
     } else {
-        rb_dense_rows<B, M, true>(p.lv[l].n, p.lv[l].inv, p.lv[l].r, p.lv[l].up, tid, nth);
+        rb_dense_rows<B, M, true>(p.lv[l].g, p.lv[l].a, p.lv[l].rr, p.lv[l].up, tid, nth);
     }
     sync();
     for (--l; l >= 0; --l) {
         const RbTailLevel<M>& L = p.lv[l];
-        rb_up<B, KM, M, true>(L, L.m, L.a, L.lu, L.r, L.r_red, L.z, L.y, L.up, tid, nth, sync);
+        rb_up<B, ND, M, true>(L, matrix(L), L.rr, L.rb, L.z, L.y, L.up, tid, nth, sync);
     }
 }

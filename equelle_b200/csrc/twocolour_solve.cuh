@@ -1,0 +1,439 @@
+// Host side of the two-colour form (twocolour.cuh): hierarchy, set-up, cycle
+// and BiCGStab.  Included by solver.cu, inside its anonymous namespace.
+
+#define WITH_ND(nd, ...)            \
+    if ((nd) == 4) {                \
+        constexpr int ND = 4;       \
+        __VA_ARGS__;                \
+    } else {                        \
+        constexpr int ND = 6;       \
+        __VA_ARGS__;                \
+    }
+#define WITH_RB(an, ...) WITH_BS((an).rb_bs, WITH_ND((an).rb_nd, __VA_ARGS__))
+
+template <class M>
+const M* rb_values(const RbLevel& L);
+template <>
+const double* rb_values<double>(const RbLevel& L) { return (L.coarsest ? L.inv64 : L.a64)->as<double>(); }
+template <>
+const float* rb_values<float>(const RbLevel& L) { return (L.coarsest ? L.inv32 : L.a32)->as<float>(); }
+
+template <class M>
+RbMatrix<const M> rb_matrix(const SolverAnalysis& an, const RbLevel& L)
+{
+    return RbMatrix<const M>(rb_values<M>(L), an.rb_nd, an.rb_bs * an.rb_bs, L.g.n, L.g.nr);
+}
+
+// Levels are coarsened only along the directions at least 1 / kSemiCoarsen
+// as strong as the strongest one: the point smoothers do not reduce error
+// that varies slowly along a strong direction and quickly along a weak one.
+// BiCGStab iterations of a two-phase solve on 48 x 48 x 32 cells of 10 x 10 x
+// 2 m (strengths 25 : 1 : 1): 38 with 2 x 2 x 2 aggregates on every level, 21
+// with one z-pairing level first, 17 with two (then 2 x 2 x 2 at 6.25 : 1),
+// 18 with three.  At 4 : 1 one z-pairing level and none are equal.
+constexpr double kSemiCoarsen = 6.5;
+
+// The aggregation of the next level from the direction strengths, which are
+// updated to that level's: a coarse cell has twice as many fine couplings for
+// every other direction that was paired.
+Aggregates choose_aggregates(const RbGrid& g, double (&strength)[3])
+{
+    const int dims[3] = {g.nx, g.ny, g.nz};
+    double top = 0.0;
+    for (int d = 0; d < 3; ++d)
+        if (dims[d] > 1) top = std::max(top, strength[d]);
+    int s[3], cut = 0;
+    for (int d = 0; d < 3; ++d) {
+        s[d] = dims[d] > 1 && !(strength[d] * kSemiCoarsen < top) ? 1 : 0;
+        cut += s[d];
+    }
+    for (int d = 0; d < 3; ++d) strength[d] *= std::ldexp(1.0, cut - s[d]);
+    Aggregates a;
+    a.sx = s[0];
+    a.sy = s[1];
+    a.sz = s[2];
+    a.g = cut > 0 ? 1 << (cut - 1) : 1;
+    a.fine = g;
+    a.coarse = RbGrid((g.nx + s[0]) >> s[0], (g.ny + s[1]) >> s[1], (g.nz + s[2]) >> s[2]);
+    return a;
+}
+
+void rb_gather(Core& c, const SolverAnalysis& an, const double* jval)
+{
+    const RbLevel& L = an.rb[0];
+    const int bb = an.rb_bs * an.rb_bs;
+    const int64_t tiles = (L.g.nr + 31) / 32 + (L.g.n - L.g.nr + 31) / 32;
+    const double vals = (double)L.g.n * (an.rb_nd + 1) * bb;
+    launch(c, "gather_values", [&] {
+        rb_gather_kernel<<<(int)std::min<int64_t>(tiles, 148 * 64), kThreads, 0, c.stream>>>(
+            L.g, bb, an.rb_nd, an.vmap->as<int>(), jval, L.a64->as<double>());
+    }, 12.0 * vals + 8.0 * an.nnz);
+}
+
+// The two-colour hierarchy of a system of `bs` unknowns per cell of the
+// Cartesian grid, built on the device; false when its pattern couples cells
+// that are no neighbours.
+bool rb_analyse(Core& c, SolverAnalysis& an, const Pattern& p, int bs, int coarsest, const double* jval)
+{
+    const int nd = c.nz > 1 ? 6 : 4, bb = bs * bs;
+    an.rb_bs = bs;
+    an.rb_nd = nd;
+    an.rb.emplace_back();
+    {
+        RbLevel& L = an.rb[0];
+        L.g = RbGrid(c.nx, c.ny, c.nz);
+        if ((double)L.g.n * (nd + 2) * bb >= (double)INT_MAX) fail(EQG_ERR_UNSUPPORTED, "linear system too large for 32-bit value offsets");
+        const size_t entries = (size_t)L.g.n * (nd + 1) * bb;
+        an.vmap = c.allocN<int>(entries);
+        Buf bad = c.allocN<int>(1);
+        EQG_CUDA(cudaMemsetAsync(an.vmap->ptr, 0xff, entries * sizeof(int), c.stream));
+        EQG_CUDA(cudaMemsetAsync(bad->ptr, 0, sizeof(int), c.stream));
+        launch(c, "rb_map", [&] {
+            rb_map_kernel<<<blocksFor((int64_t)L.g.n * bs), kThreads, 0, c.stream>>>(
+                L.g, bs, nd, p.rowptr->as<int>(), p.colind->as<int>(), an.vmap->as<int>(), bad->as<int>());
+        });
+        int flags = 0;
+        EQG_CUDA(cudaMemcpyAsync(c.pinned, bad->ptr, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+        c.sync();
+        std::memcpy(&flags, c.pinned, sizeof(int));
+        if (flags & 1) {
+            an.rb.clear();
+            an.vmap = nullptr;
+            return false;
+        }
+        if (bs == 1 && (flags & 2)) {  // a structurally missing diagonal entry
+            an.ok = false;
+            return true;
+        }
+    }
+    an.partials = c.allocN<double>((size_t)kRedBlocks * 3 + 3);
+    an.counter = c.allocN<unsigned int>(1);
+    EQG_CUDA(cudaMemsetAsync(an.counter->ptr, 0, sizeof(unsigned int), c.stream));
+    auto allocate = [&](RbLevel& L) {
+        L.n = L.g.n * bs;
+        L.vals = (int64_t)RbMatrix<double>::values(nd, bb, L.g.n, L.g.nr);
+        L.a64 = c.allocN<double>((size_t)L.vals);
+        L.v64 = c.allocN<double>((size_t)2 * L.n);
+    };
+    allocate(an.rb[0]);
+    double strength[3] = {1.0, 1.0, 1.0};
+    if ((c.nx > 1) + (c.ny > 1) + (c.nz > 1) > 1) {
+        rb_gather(c, an, jval);
+        double* out = an.partials->as<double>() + (size_t)kRedBlocks * 3;
+        launch(c, "mg_strength", [&] {
+            rb_strength_kernel<<<blocksFor(an.rb[0].g.n, kThreads, kRedBlocks), kThreads, 0, c.stream>>>(
+                an.rb[0].g, bs, nd, an.rb[0].a64->as<double>(), an.partials->as<double>(),
+                an.counter->as<unsigned int>(), out);
+        });
+        EQG_CUDA(cudaMemcpyAsync(c.pinned, out, 3 * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+        c.sync();
+        for (int d = 0; d < 3; ++d) strength[d] = c.pinned[d];
+    }
+    for (;;) {
+        RbLevel& F = an.rb.back();
+        F.agg = choose_aggregates(F.g, strength);
+        const int cut = F.agg.sx + F.agg.sy + F.agg.sz;
+        F.alpha = c.param_d("linsolver_mg_alpha", cut == 2 && c.nz == 1 ? kMgAlpha2d : kMgAlpha3d);
+        F.pre = cut > 1;
+        RbLevel C;
+        C.g = F.agg.coarse;
+        allocate(C);
+        const bool last = C.n <= coarsest || C.g.n == 1;
+        if (last) {
+            C.coarsest = true;
+            C.inv64 = c.allocN<double>((size_t)C.n * C.n);
+        }
+        an.rb.push_back(std::move(C));
+        if (last) break;
+    }
+    // levels of at most linsolver_mg_fuse_rows unknowns (0: none) run as one
+    // kernel, the last kMaxTail of them at most
+    const int fuse_rows = c.param_i("linsolver_mg_fuse_rows", 40000), nl = (int)an.rb.size();
+    for (int l = nl - 1; l >= 0 && nl - l <= kMaxTail && (an.rb[l].coarsest || an.rb[l].n <= fuse_rows); --l)
+        if (!an.rb[l].coarsest) an.tail_first = l;
+    // the right-hand side, and the BiCGStab vectors of the black half
+    const RbGrid& g = an.rb[0].g;
+    an.vec64 = c.allocN<double>(vec_stride(an.n) + 10 * vec_stride((g.n - g.nr) * bs));
+    an.multigrid = true;
+    if (c.verbose > 2) {
+        std::printf("        linear solver: %dx%d blocks, two colours, direction strengths %.3g %.3g %.3g, levels:", bs,
+                    bs, strength[0], strength[1], strength[2]);
+        for (auto& L : an.rb) std::printf(" %dx%dx%d", L.g.nx, L.g.ny, L.g.nz);
+        std::printf("\n");
+    }
+    return true;
+}
+
+// Matrices of every level and their factors from the Jacobian's values.
+void rb_setup(Core& c, SolverAnalysis& an, const double* jval, bool mixed)
+{
+    const int bs = an.rb_bs, bb = bs * bs, nd = an.rb_nd;
+    int* status = an.factor_status->as<int>();
+    rb_gather(c, an, jval);
+    for (size_t l = 0; l + 1 < an.rb.size(); ++l) {
+        const RbLevel &F = an.rb[l], &C = an.rb[l + 1];
+        launch(c, "mg_galerkin", [&] {
+            rb_galerkin_kernel<<<blocksFor((int64_t)C.g.n * bb), kThreads, 0, c.stream>>>(
+                F.agg, bb, nd, F.a64->as<double>(), C.a64->as<double>());
+        }, 8.0 * bb * (nd + 1) * ((double)F.g.n + C.g.n));
+    }
+    for (auto& L : an.rb) {
+        if (L.coarsest) {
+            EQG_CUDA(cudaMemsetAsync(L.inv64->ptr, 0, (size_t)L.n * L.n * sizeof(double), c.stream));
+            launch(c, "mg_dense_fill", [&] {
+                rb_dense_fill_kernel<<<blocksFor(L.g.n), kThreads, 0, c.stream>>>(L.g, bs, nd, L.a64->as<double>(),
+                                                                                  L.inv64->as<double>());
+            });
+            dense_inverse(c, L.n, L.inv64->as<double>(), status);
+        } else {
+            const RbMatrix<double> m(L.a64->as<double>(), nd, bb, L.g.n, L.g.nr);
+            const double nk = L.g.n - L.g.nr;
+            WITH_BS(bs, launch(c, "rb_factor_red", [&] {
+                        rb_factor_red_kernel<BS><<<blocksFor(L.g.nr), kThreads, 0, c.stream>>>(L.g, m.dr, status);
+                    }, 16.0 * bb * L.g.nr));
+            WITH_RB(an, launch(c, "rb_factor_black", [&] {
+                        rb_factor_black_kernel<BS, ND><<<blocksFor((int64_t)nk), kThreads, 0, c.stream>>>(L.g, m, status);
+                    }, 8.0 * bb * (nk * (2.0 * nd + 2.0) + L.g.nr * (nd + 1.0))));
+        }
+        if (mixed) {
+            if (L.coarsest) to_float(c, L.inv64, L.inv32, (int64_t)L.n * L.n);
+            else to_float(c, L.a64, L.a32, L.vals);
+        }
+    }
+}
+
+// ---- the cycle -------------------------------------------------------------------
+// The vectors of one level.  Level 0 works on the caller's black vectors, its
+// red right-hand side is zero.
+struct RbVectors {
+    const double *rr, *rb;
+    double *z, *y;
+    UpView up;
+    RbVectors(const SolverAnalysis& an, size_t l, const double* in, double* out)
+    {
+        const RbLevel& L = an.rb[l];
+        const size_t red = (size_t)L.g.nr * an.rb_bs;
+        double* v = L.v64->as<double>();
+        rr = l == 0 ? nullptr : v;
+        rb = l == 0 ? in : v + red;
+        y = v + L.n;
+        z = l == 0 ? out : y + red;
+        if (l > 0) {
+            const RbLevel& F = an.rb[l - 1];
+            up.agg = F.agg;
+            up.add = F.pre ? 1 : 0;
+            up.alpha = F.alpha;
+            up.w = l == 1 ? out : F.v64->as<double>() + F.n + (size_t)F.g.nr * an.rb_bs;
+        }
+    }
+};
+
+// The fused levels kept in block 0's shared memory: from the coarsest one
+// upward while they fit in kTailSmem bytes (the first fused level stays
+// cluster-wide).  Returns the first such level as an index into the fused
+// levels (their count: none) and its bytes; fills the layout and copies.
+template <class M>
+int plan_rb_local(Core& c, const SolverAnalysis& an, int& bytes, RbTailParams<M>* p)
+{
+    const int nlev = (int)an.rb.size() - an.tail_first;
+    bytes = 0;
+    if (an.tail_first < 0 || !c.param_i("linsolver_mg_local", 1)) return nlev;
+    int64_t off = 0;
+    auto place = [&](int64_t b) {
+        const int64_t o = off;
+        off += (b + 15) & ~(int64_t)15;
+        return (int)o;
+    };
+    int lf = nlev;
+    for (int i = nlev - 1; i >= 1; --i) {
+        const RbLevel& L = an.rb[an.tail_first + i];
+        const int64_t mat = (L.coarsest ? (int64_t)L.n * L.n : L.vals) * (int64_t)sizeof(M);
+        const int64_t before = off;
+        const int a = place(mat), r = place((int64_t)L.n * sizeof(double)),
+                  w = L.coarsest ? 0 : place((int64_t)L.n * sizeof(double));
+        if (off > kTailSmem) {
+            off = before;
+            break;
+        }
+        lf = i;
+        if (p) {
+            p->lv[i].so_a = a;
+            p->lv[i].so_r = r;
+            p->lv[i].so_w = w;
+            p->copies[p->ncopies++] = TailCopy{rb_values<M>(L), a, (int)mat};
+        }
+    }
+    if (lf == nlev) return nlev;
+    bytes = (int)off;
+    if (p) p->local_first = lf;
+    return lf;
+}
+
+template <class M>
+void launch_rb_tail(Core& c, const SolverAnalysis& an, const double* in, double* out, const KScal* sc, int skip)
+{
+    RbTailParams<M> p;
+    double bytes = 0.0;
+    for (size_t l = an.tail_first; l < an.rb.size(); ++l) {
+        const RbLevel& L = an.rb[l];
+        const RbVectors v(an, l, in, out);
+        RbTailLevel<M>& t = p.lv[p.nlev++];
+        t.g = L.g;
+        t.coarsest = L.coarsest ? 1 : 0;
+        t.pre = L.pre ? 1 : 0;
+        t.a = rb_values<M>(L);
+        t.rr = v.rr;
+        t.rb = v.rb;
+        t.r = const_cast<double*>(v.rr);
+        t.z = v.z;
+        t.y = v.y;
+        t.agg = L.agg;
+        t.up = v.up;
+        const int64_t mat = (L.coarsest ? (int64_t)L.n * L.n : L.vals) * (int64_t)sizeof(M);
+        p.reg[p.nregions++] = PrefetchRegion{t.a, (unsigned long long)mat};
+        bytes += mat + 4.0 * L.n * sizeof(double);
+    }
+    if (an.tail_trace) p.trace = an.tail_trace->as<long long>();
+    p.local_first = p.nlev;
+    int smem = 0;
+    const int mode = pc_mode<double, M>();
+    if (an.tail_local[mode] < p.nlev) plan_rb_local<M>(c, an, smem, &p);
+    TailLaunch cfg(c, an.tail_cluster[mode], smem);
+    WITH_RB(an, launch(c, "rb_tail", [&] {
+                EQG_CUDA(cudaLaunchKernelEx(&cfg.cfg, rb_tail_kernel<BS, ND, M>, p, sc, skip));
+            }, bytes));
+}
+
+// out = V-cycle(in) on the black rows, from level l down.
+template <class M>
+void rb_cycle(Core& c, const SolverAnalysis& an, size_t l, const double* in, double* out, const KScal* sc, int skip)
+{
+    if ((int)l == an.tail_first) {
+        launch_rb_tail<M>(c, an, in, out, sc, skip);
+        return;
+    }
+    const RbLevel& L = an.rb[l];
+    const RbVectors v(an, l, in, out);
+    if (L.coarsest) {
+        WITH_BS(an.rb_bs, launch(c, "rb_dense", [&] {
+                    launch_k(c, rb_dense_kernel<BS, M>, 1, 1024, L.g, rb_values<M>(L), v.rr, v.up, sc, skip);
+                }, (double)L.n * L.n * sizeof(M) + 2.0 * L.n * sizeof(double)));
+        return;
+    }
+    double* rc = an.rb[l + 1].v64->as<double>();
+    const RbMatrix<const M> m = rb_matrix<M>(an, L);
+    const int nr = L.g.nr, nk = L.g.n - nr, nt = L.threads;
+    // algorithmic bytes: the stored blocks of a half, the diagonal blocks, and
+    // every vector element read or written once
+    const double row = 8.0 * an.rb_bs, blk = (double)sizeof(M) * an.rb_bs * an.rb_bs, coarse = row * L.agg.coarse.n;
+    const double half_u = an.rb_nd * blk * nr, half_l = an.rb_nd * blk * nk, red = l == 0 ? 0.0 : row * nr;
+    auto y_rows = [&] {
+        WITH_RB(an, launch(c, "rb_y", [&] {
+                    launch_k(c, rb_y_kernel<BS, ND, M>, blocksFor(nr, nt), nt, L.g, m, v.rr, (const double*)v.z, v.y, sc,
+                             skip);
+                }, half_u + red + row * (nr + nk)));
+    };
+    if (L.pre) {
+        WITH_RB(an, launch(c, "rb_pre", [&] {
+                    launch_k(c, rb_pre_kernel<BS, ND, M>, blocksFor(nk, nt), nt, L.g, m, v.rr, v.rb, v.z, sc, skip);
+                }, (l == 0 ? 0.0 : half_l) + red + (blk + 2 * row) * nk));
+        y_rows();
+        WITH_RB(an, launch(c, "rb_res", [&] {
+                    launch_k(c, rb_res_kernel<BS, ND, M>, blocksFor((int64_t)L.agg.coarse.n * L.agg.g, nt), nt, L.agg, m,
+                             v.rb, (const double*)v.y, (const double*)v.z, rc, sc, skip);
+                }, half_l + (blk + 2 * row) * nk + row * nr + coarse));
+    } else {
+        WITH_BS(an.rb_bs, launch(c, "rb_restrict", [&] {
+                    launch_k(c, rb_restrict_kernel<BS>, blocksFor(L.agg.coarse.n, nt), nt, L.agg, v.rr, v.rb, rc, sc,
+                             skip);
+                }, row * nk + red + coarse));
+    }
+    rb_cycle<M>(c, an, l + 1, in, out, sc, skip);
+    y_rows();
+    const double to_fine = v.up.w ? row * v.up.agg.g * (v.up.add ? 2.0 : 1.0) : 0.0;
+    WITH_RB(an, launch(c, "rb_post", [&] {
+                launch_k(c, rb_post_kernel<BS, ND, M>, blocksFor(nk, nt), nt, L.g, m, v.rb, (const double*)v.y, v.z, v.up,
+                         sc, skip);
+            }, half_l + (2 * blk + 3 * row + to_fine) * nk + row * nr));
+    if (v.up.w == nullptr) return;
+    WITH_RB(an, launch(c, "rb_fin", [&] {
+                launch_k(c, rb_fin_kernel<BS, ND, M>, blocksFor(nr, nt), nt, L.g, m, v.rr, (const double*)v.z, v.up, sc,
+                         skip);
+            }, half_u + (blk + row + to_fine) * nr + row * nk));
+}
+
+// Chooses the cluster size of the fused levels; called before any capture.
+template <class M>
+void prepare_rb_tail(Core& c, SolverAnalysis& an)
+{
+    if (an.tail_first < 0) return;
+    const int mode = pc_mode<double, M>();
+    int& cl = an.tail_cluster[mode];
+    if (!cl) WITH_RB(an, cl = tail_cluster_size(c, rb_tail_kernel<BS, ND, M>));
+    int bytes = 0;
+    an.tail_local[mode] = plan_rb_local<M>(c, an, bytes, nullptr);
+    an.last_mode = mode;
+}
+
+// BiCGStab on the black half, M the type of the preconditioner's matrices:
+// the solution of A x = rhs, both in the natural order.
+template <class M>
+SolveResult bicgstab_rb(Core& c, SolverAnalysis& an, const double* rhs, double* xout, double tol, int max_iter,
+                        int check_every)
+{
+    const RbLevel& L0 = an.rb[0];
+    const RbGrid& g = L0.g;
+    const int bs = an.rb_bs, nr = g.nr, nk = g.n - nr, n = nk * bs;
+    double* b = an.vec64->as<double>();
+    const Vecs<double> v = vecs<double>(b + vec_stride(an.n), n);
+    KScal* sc = an.scal->as<KScal>();
+    double* part = an.partials->as<double>();
+    unsigned int* cnt = an.counter->as<unsigned int>();
+    const RbMatrix<const double> m = rb_matrix<double>(an, L0);
+    double* y = L0.v64->as<double>() + L0.n;
+    const int nbv = blocksFor(n, kThreads, kRedBlocks), nbk = blocksFor(nk, kThreads, kRedBlocks);
+    const double vb = 8.0 * n, yb = 8.0 * nr * bs, blk = 8.0 * bs * bs;
+    const double half_u = an.rb_nd * blk * nr, half_l = an.rb_nd * blk * nk;
+    WITH_BS(bs, launch(c, "permute", [&] {
+                rb_permute_kernel<BS><<<blocksFor(g.n), kThreads, 0, c.stream>>>(g, rhs, b);
+            }, 16.0 * an.n));
+    WITH_RB(an, launch(c, "rb_init", [&] {
+                rb_init_kernel<BS, ND><<<blocksFor(nr, kThreads, kRedBlocks), kThreads, 0, c.stream>>>(
+                    g, m, b, v.r, v.rhat, v.p, v.v, v.x, part, cnt, sc, tol * tol);
+            }, half_l + vb * 6.0 + yb));
+    auto product = [&](const double* z, const double* h, double* out, bool omega) {
+        WITH_RB(an, launch(c, "rb_spmv_y", [&] {
+                    launch_k(c, rb_y_kernel<BS, ND, double>, blocksFor(nr, L0.threads), L0.threads, g, m,
+                             (const double*)nullptr, z, y, (const KScal*)sc, (int)omega);
+                }, half_u + vb + yb));
+        WITH_RB(an, launch(c, omega ? "rb_spmv_omega" : "rb_spmv_alpha", [&] {
+                    launch_k(c, omega ? rb_spmv_kernel<BS, ND, true> : rb_spmv_kernel<BS, ND, false>, nbk, kThreads, g, m,
+                             z, (const double*)y, h, out, part, cnt, sc);
+                }, half_l + blk * nk + yb + 3.0 * vb));
+    };
+    auto iteration = [&] {
+        launch(c, "bicg_p", [&] {
+            launch_k(c, bicg_p_kernel<double>, blocksFor(n), kThreads, (const double*)v.r, (const double*)v.v, v.p, n,
+                     (const KScal*)sc);
+        }, 4.0 * vb);
+        rb_cycle<M>(c, an, 0, v.p, v.ph, sc, 0);
+        product(v.ph, v.rhat, v.v, false);
+        launch(c, "bicg_s", [&] {
+            launch_k(c, bicg_s_kernel<double>, nbv, kThreads, (const double*)v.r, (const double*)v.v, v.s, n, part, cnt,
+                     sc);
+        }, 3.0 * vb);
+        rb_cycle<M>(c, an, 0, v.s, v.sh, sc, 1);
+        product(v.sh, v.s, v.t, true);
+        launch(c, "bicg_xr", [&] {
+            launch_k(c, bicg_xr_kernel<double>, nbv, kThreads, (const double*)v.ph, (const double*)v.sh,
+                     (const double*)v.s, (const double*)v.t, (const double*)v.rhat, v.x, v.r, n, part, cnt, sc);
+        }, 8.0 * vb);
+    };
+    autotune<double, M>(c, an, [&] { rb_cycle<M>(c, an, 0, v.r, v.ph, sc, 0); });
+    const SolveResult res =
+        run_iterations(c, an, sizeof(M) == sizeof(double) ? 0 : 2, tol, max_iter, check_every, iteration);
+    WITH_RB(an, launch(c, "rb_solution", [&] {
+                rb_solution_kernel<BS, ND><<<blocksFor(nr), kThreads, 0, c.stream>>>(g, m, b, v.x, xout);
+            }, half_u + blk * nr + 3.0 * vb + 2.0 * yb));
+    return res;
+}
