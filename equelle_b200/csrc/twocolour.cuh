@@ -140,7 +140,10 @@ struct RbMatrix {
 };
 
 // acc += sum over the neighbours of A_d x_d, directions in order, row q of
-// `rows`; every load is issued before the first sum.
+// `rows`.  The loads are unconditional, so that all of them are issued before
+// the first sum (with a branch per neighbour the compiler waited for each one
+// in turn, in 34 registers): the block of a missing neighbour is stored as
+// zero, and the vector is then read at the row's own number, or the last one.
 template <int B, int ND, class M, bool CG>
 __device__ __forceinline__ void stencil_dot(const RbGrid& g, const Cell& e, int q, int rows, const M* __restrict__ a,
                                             const double* __restrict__ x, double (&acc)[B])
@@ -148,18 +151,13 @@ __device__ __forceinline__ void stencil_dot(const RbGrid& g, const Cell& e, int 
     constexpr int BB = B * B;
     M av[ND][BB];
     double xv[ND][B];
+    const int own = min(q, g.n - rows - 1);  // the other colour has n - rows cells
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
         int nq;
-        const bool has = neighbour(g, e, d, nq);
-#pragma unroll
-        for (int t = 0; t < BB; ++t) av[d][t] = (M)0;
-#pragma unroll
-        for (int t = 0; t < B; ++t) xv[d][t] = 0.0;
-        if (has) {
-            load_block<BB, M>(a + ((size_t)d * rows + q) * BB, av[d]);
-            load_bvec<B, double, CG>(x, nq, xv[d]);
-        }
+        if (!neighbour(g, e, d, nq)) nq = own;
+        load_block<BB, M>(a + ((size_t)d * rows + q) * BB, av[d]);
+        load_bvec<B, double, CG>(x, nq, xv[d]);
     }
 #pragma unroll
     for (int d = 0; d < ND; ++d)
@@ -171,10 +169,8 @@ __device__ __forceinline__ void stencil_dot(const RbGrid& g, const Cell& e, int 
 
 // y = D x of one block.
 template <int B, class M>
-__device__ __forceinline__ void block_mul(const M* __restrict__ a, const double (&x)[B], double (&y)[B])
+__device__ __forceinline__ void block_mul(const M (&av)[B * B], const double (&x)[B], double (&y)[B])
 {
-    M av[B * B];
-    load_block<B * B, M>(a, av);
 #pragma unroll
     for (int i = 0; i < B; ++i) {
         double s = 0.0;
@@ -227,16 +223,21 @@ template <int B, bool CG>
 __device__ __forceinline__ void scatter_up(const UpView& u, const Cell& e, const double (&z)[B])
 {
     if (u.w == nullptr) return;
-    for (int s = 0; s < u.agg.g; ++s) {
-        const int c = black_member(u.agg, e.i, e.j, e.k, s);
-        if (c < 0) continue;
-        double f[B];
+    // at most four members; all are read before the first is written
+    int c[4];
+    double f[4][B];
 #pragma unroll
-        for (int t = 0; t < B; ++t) f[t] = 0.0;
-        if (u.add) load_bvec<B, double, CG>(u.w, c >> 1, f);
+    for (int s = 0; s < 4; ++s) {
+        c[s] = s < u.agg.g ? black_member(u.agg, e.i, e.j, e.k, s) : -1;
 #pragma unroll
-        for (int t = 0; t < B; ++t) f[t] = __fma_rn(u.alpha, z[t], f[t]);
-        store_bvec<B, double>(u.w, c >> 1, f);
+        for (int t = 0; t < B; ++t) f[s][t] = 0.0;
+        if (u.add && c[s] >= 0) load_bvec<B, double, CG>(u.w, c[s] >> 1, f[s]);
+    }
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+#pragma unroll
+        for (int t = 0; t < B; ++t) f[s][t] = __fma_rn(u.alpha, z[t], f[s][t]);
+        if (c[s] >= 0) store_bvec<B, double>(u.w, c[s] >> 1, f[s]);
     }
 }
 
@@ -279,9 +280,11 @@ __device__ __forceinline__ void rb_fin_rows(const RbGrid& g, const RbMatrix<cons
 {
     for (int q = tid; q < g.nr; q += nth) {
         const Cell e = cell_of(g, 0, q);
+        M dv[B * B];
         double v[B], x[B];
+        load_block<B * B, M>(m.dr + (size_t)q * B * B, dv);
         red_row<B, ND, M, CG>(g, e, q, m.U, rr, z, v);
-        block_mul<B, M>(m.dr + (size_t)q * B * B, v, x);
+        block_mul<B, M>(dv, v, x);
         scatter_up<B, CG>(up, e, x);
     }
 }
@@ -293,14 +296,16 @@ __device__ __forceinline__ void rb_pre_rows(const RbGrid& g, const RbMatrix<cons
 {
     const int nk = g.n - g.nr;
     for (int q = tid; q < nk; q += nth) {
+        M dv[B * B];
         double acc[B], v[B], x[B];
 #pragma unroll
         for (int t = 0; t < B; ++t) acc[t] = 0.0;
-        if (rr) stencil_dot<B, ND, M, CG>(g, cell_of(g, 1, q), q, nk, m.L, rr, acc);
         load_bvec<B, double, CG>(rb, q, v);
+        load_block<B * B, M>(m.db + (size_t)q * B * B, dv);
+        if (rr) stencil_dot<B, ND, M, CG>(g, cell_of(g, 1, q), q, nk, m.L, rr, acc);
 #pragma unroll
         for (int t = 0; t < B; ++t) v[t] = __dsub_rn(v[t], acc[t]);
-        block_mul<B, M>(m.db + (size_t)q * B * B, v, x);
+        block_mul<B, M>(dv, v, x);
         store_bvec<B, double>(z, q, x);
     }
 }
@@ -310,12 +315,14 @@ template <int B, int ND, class M, bool CG>
 __device__ __forceinline__ void residual_row(const RbGrid& g, const Cell& e, int q, const RbMatrix<const M>& m,
                                              const double* rb, const double* y, const double (&z)[B], double (&t)[B])
 {
+    M av[B * B];
     double acc[B], az[B];
 #pragma unroll
     for (int c = 0; c < B; ++c) acc[c] = 0.0;
     load_bvec<B, double, CG>(rb, q, t);
-    block_mul<B, M>(m.abb + (size_t)q * B * B, z, az);
+    load_block<B * B, M>(m.abb + (size_t)q * B * B, av);
     stencil_dot<B, ND, M, CG>(g, e, q, g.n - g.nr, m.L, y, acc);
+    block_mul<B, M>(av, z, az);
 #pragma unroll
     for (int c = 0; c < B; ++c) t[c] = __dsub_rn(__dsub_rn(t[c], az[c]), acc[c]);
 }
@@ -383,10 +390,12 @@ __device__ __forceinline__ void rb_post_rows(const RbGrid& g, const RbMatrix<con
     const int nk = g.n - g.nr;
     for (int q = tid; q < nk; q += nth) {
         const Cell e = cell_of(g, 1, q);
+        M dv[B * B];
         double zv[B], t[B], x[B];
         load_bvec<B, double, CG>(z, q, zv);
+        load_block<B * B, M>(m.db + (size_t)q * B * B, dv);
         residual_row<B, ND, M, CG>(g, e, q, m, rb, y, zv, t);
-        block_mul<B, M>(m.db + (size_t)q * B * B, t, x);
+        block_mul<B, M>(dv, t, x);
 #pragma unroll
         for (int c = 0; c < B; ++c) zv[c] = __dadd_rn(zv[c], x[c]);
         store_bvec<B, double>(z, q, zv);
@@ -420,7 +429,7 @@ __device__ __forceinline__ void rb_dense_rows(const RbGrid& g, const M* __restri
 
 // ---- one step per launch ------------------------------------------------------
 template <int B, int ND, class M>
-__global__ void __launch_bounds__(512) rb_y_kernel(RbGrid g, RbMatrix<const M> m, const double* rr, const double* z,
+__global__ void __launch_bounds__(512, 1) rb_y_kernel(RbGrid g, RbMatrix<const M> m, const double* rr, const double* z,
                                                    double* y, const KScal* sc, int skip_if_s)
 {
     pdl_wait();
@@ -430,7 +439,7 @@ __global__ void __launch_bounds__(512) rb_y_kernel(RbGrid g, RbMatrix<const M> m
 }
 
 template <int B, int ND, class M>
-__global__ void __launch_bounds__(512) rb_fin_kernel(RbGrid g, RbMatrix<const M> m, const double* rr, const double* z,
+__global__ void __launch_bounds__(512, 1) rb_fin_kernel(RbGrid g, RbMatrix<const M> m, const double* rr, const double* z,
                                                      UpView up, const KScal* sc, int skip_if_s)
 {
     pdl_wait();
@@ -440,7 +449,7 @@ __global__ void __launch_bounds__(512) rb_fin_kernel(RbGrid g, RbMatrix<const M>
 }
 
 template <int B, int ND, class M>
-__global__ void __launch_bounds__(512) rb_pre_kernel(RbGrid g, RbMatrix<const M> m, const double* rr, const double* rb,
+__global__ void __launch_bounds__(512, 1) rb_pre_kernel(RbGrid g, RbMatrix<const M> m, const double* rr, const double* rb,
                                                      double* z, const KScal* sc, int skip_if_s)
 {
     pdl_wait();
@@ -450,7 +459,7 @@ __global__ void __launch_bounds__(512) rb_pre_kernel(RbGrid g, RbMatrix<const M>
 }
 
 template <int B, int ND, class M>
-__global__ void __launch_bounds__(512) rb_res_kernel(Aggregates a, RbMatrix<const M> m, const double* rb,
+__global__ void __launch_bounds__(512, 1) rb_res_kernel(Aggregates a, RbMatrix<const M> m, const double* rb,
                                                      const double* y, const double* z, double* rc, const KScal* sc,
                                                      int skip_if_s)
 {
@@ -461,7 +470,7 @@ __global__ void __launch_bounds__(512) rb_res_kernel(Aggregates a, RbMatrix<cons
 }
 
 template <int B>
-__global__ void __launch_bounds__(512) rb_restrict_kernel(Aggregates a, const double* rr, const double* rb, double* rc,
+__global__ void __launch_bounds__(512, 1) rb_restrict_kernel(Aggregates a, const double* rr, const double* rb, double* rc,
                                                           const KScal* sc, int skip_if_s)
 {
     pdl_wait();
@@ -471,7 +480,7 @@ __global__ void __launch_bounds__(512) rb_restrict_kernel(Aggregates a, const do
 }
 
 template <int B, int ND, class M>
-__global__ void __launch_bounds__(512) rb_post_kernel(RbGrid g, RbMatrix<const M> m, const double* rb, const double* y,
+__global__ void __launch_bounds__(512, 1) rb_post_kernel(RbGrid g, RbMatrix<const M> m, const double* rb, const double* y,
                                                       double* z, UpView up, const KScal* sc, int skip_if_s)
 {
     pdl_wait();
@@ -563,7 +572,7 @@ __global__ void __launch_bounds__(kThreads) rb_init_kernel(RbGrid g, RbMatrix<co
 // false: alpha = rho_new / (h . v), h the shadow residual) or
 // bicg_spmv_omega (omega = (v . h) / (v . v), h = s).
 template <int B, int ND, bool OMEGA>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 2)
     rb_spmv_kernel(RbGrid g, RbMatrix<const double> m, const double* __restrict__ z, const double* __restrict__ y,
                    const double* __restrict__ h, double* __restrict__ v, double* partials, unsigned int* counter,
                    KScal* sc)
@@ -581,10 +590,12 @@ __global__ void __launch_bounds__(kThreads)
         double acc[B], zv[B], az[B], hv[B];
 #pragma unroll
         for (int t = 0; t < B; ++t) acc[t] = 0.0;
+        double av[B * B];
         load_bvec<B, double>(z, q, zv);
         load_bvec<B, double>(h, q, hv);
-        block_mul<B, double>(m.abb + (size_t)q * B * B, zv, az);
+        load_block<B * B, double>(m.abb + (size_t)q * B * B, av);
         stencil_dot<B, ND, double, false>(g, cell_of(g, 1, q), q, nk, m.L, y, acc);
+        block_mul<B, double>(av, zv, az);
 #pragma unroll
         for (int t = 0; t < B; ++t) acc[t] += az[t];
         store_bvec<B, double>(v, q, acc);
@@ -621,8 +632,10 @@ __global__ void __launch_bounds__(kThreads) rb_solution_kernel(RbGrid g, RbMatri
         const int q = (int)q64;
         const Cell e = cell_of(g, 0, q);
         double v[B], z[B];
+        double dv[B * B];
+        load_block<B * B, double>(m.dr + (size_t)q * B * B, dv);
         red_row<B, ND, double, false>(g, e, q, m.U, b, x, v);
-        block_mul<B, double>(m.dr + (size_t)q * B * B, v, z);
+        block_mul<B, double>(dv, v, z);
 #pragma unroll
         for (int t = 0; t < B; ++t) out[(size_t)t * g.n + e.c] = z[t];
         if (q >= nk) continue;
@@ -966,7 +979,7 @@ __device__ void rb_local_cycle(const RbTailParams<M>& p, int lf, unsigned char* 
 }
 
 template <int B, int ND, class M>
-__global__ void __launch_bounds__(kTailThreads)
+__global__ void __launch_bounds__(kTailThreads, 1)
     rb_tail_kernel(const __grid_constant__ RbTailParams<M> p, const KScal* sc, int skip_if_s)
 {
     extern __shared__ __align__(16) unsigned char tail_smem[];
