@@ -1174,15 +1174,6 @@ __global__ void slot_sums_kernel(int64_t slots, int bb, const int* __restrict__ 
     }
 }
 
-// Inverse of the coarsest matrix (n <= kCoarsest unknowns, dense, row-major),
-// in place, by one thread block in shared memory: Gauss-Jordan elimination with partial pivoting
-// (Numerical Recipes, gaussj, row pivots only).  Per pivot k: a warp finds
-// the largest |a_rk|, r >= k (the lowest r among equals) while every thread
-// copies column k; rows k and p are swapped and row k is divided by the
-// pivot; every other row r takes a_rj - a_kj f_r with f_r its entry in
-// column k (column k itself becomes -f_r / pivot).  The row swaps show up
-// as column swaps of the result, undone in reverse order when the inverse
-// is written out.  A zero or non-finite pivot sets *status.
 constexpr int kCoarsest = 128;
 
 // The dense matrix of a level in the block sliced layout; `dense` is zero
@@ -1201,78 +1192,109 @@ __global__ void dense_fill_kernel(int nb, SellView m, const double* __restrict__
     }
 }
 
-__global__ void __launch_bounds__(1024) dense_inverse_kernel(int n, double* __restrict__ a, int* status)
+// Inverse of the coarsest matrix (n <= kCoarsest unknowns, dense, row-major),
+// in place, by one thread block: Gauss-Jordan elimination with partial
+// pivoting, rows left where they are.  Thread (t, j) keeps the entries of
+// column j in rows t, t + 4, ... in registers; per step k the threads of
+// column k publish it, every warp finds the largest entry among the rows that
+// have been no pivot yet (the lowest row among equals), the threads of that
+// row p publish it divided by the pivot (its entry in column k becomes
+// 1 / pivot), and every other row r takes a_rj - a_pj f_r with f_r its entry in
+// column k (column k itself becomes -f_r / pivot).  With p_k the pivot row of
+// step k, the inverse has a[p_k][j] in row k, column p_j.  A zero or
+// non-finite pivot sets *status.
+//
+// Bound: the chain of two barriers, a reduction and a division per step.
+// n = 128: 586 us with the matrix in shared memory and row swaps (three
+// barriers, a 2 x 128 KB sweep and an index division per entry and step),
+// 196 us from registers; n = 60: 91 us.
+constexpr int kInverseThreads = 512;
+
+__global__ void __launch_bounds__(kInverseThreads, 1) dense_inverse_kernel(int n, double* __restrict__ a, int* status)
 {
-    extern __shared__ __align__(16) double dsm[];
-    double* w = dsm;                  // n x n, row-major
-    double* colk = dsm + n * n;       // column k before the row swap
-    __shared__ int piv_row;
-    __shared__ int perm[kCoarsest];   // row swapped with k at step k
-    for (int i = threadIdx.x; i < n * n; i += blockDim.x) w[i] = a[i];
-    __syncthreads();
-    for (int k = 0; k < n; ++k) {
-        for (int r = threadIdx.x; r < n; r += blockDim.x) colk[r] = w[r * n + k];
-        if (threadIdx.x < 32) {
-            double best = -1.0;
-            int bi = n;
-            for (int r = k + (int)threadIdx.x; r < n; r += 32) {
-                const double v = fabs(w[r * n + k]);
-                if (v > best) {
-                    best = v;
-                    bi = r;
-                }
-            }
+    __shared__ double colk[2][kCoarsest], rowp[kCoarsest];
+    __shared__ int piv[kCoarsest], step_of[kCoarsest];  // pivot row of each step, and its inverse
+    constexpr int T = kInverseThreads / kCoarsest, M = kCoarsest / T;
+    const int j = threadIdx.x & (kCoarsest - 1), t = threadIdx.x / kCoarsest, lane = threadIdx.x & 31;
+    double w[M];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (ob > best || (ob == best && oi < bi)) {
-                    best = ob;
-                    bi = oi;
-                }
-            }
-            if (threadIdx.x == 0) {
-                piv_row = bi < n ? bi : k;
-                perm[k] = piv_row;
-                if (!(best > 0.0) || !isfinite(best)) *status = 1;
-            }
-        }
-        __syncthreads();
-        const int p = piv_row;
-        const double pv = colk[p];
-        for (int j = threadIdx.x; j < n; j += blockDim.x) {
-            const double tk = w[k * n + j], tp = w[p * n + j];
-            w[p * n + j] = tk;
-            w[k * n + j] = (j == k ? 1.0 : tp) / pv;
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < n * n; i += blockDim.x) {
-            const int r = i / n, j = i - r * n;
-            if (r == k) continue;
-            const double f = r == p ? colk[k] : colk[r];
-            w[i] = (j == k ? 0.0 : w[i]) - w[k * n + j] * f;
-        }
-        __syncthreads();
+    for (int m = 0; m < M; ++m) {
+        const int r = t + T * m;
+        w[m] = r < n && j < n ? a[r * n + j] : 0.0;
+        if (j == 0) colk[0][r] = w[m];
     }
-    // column j of the inverse is column src[j] of w: the swaps of steps
-    // n-1 .. 0 applied to the columns in turn
-    __shared__ int src[kCoarsest];
-    if (threadIdx.x == 0) {
-        for (int j = 0; j < n; ++j) src[j] = j;
-        for (int k = n - 1; k >= 0; --k) {
-            const int p = perm[k];
-            if (p != k) {
-                const int t = src[k];
-                src[k] = src[p];
-                src[p] = t;
+    unsigned used = 0;  // bit i: row lane + 32 i has been a pivot (or does not exist)
+#pragma unroll
+    for (int i = 0; i < kCoarsest / 32; ++i)
+        if (lane + 32 * i >= n) used |= 1u << i;
+    for (int k = 0; k < n; ++k) {
+        const double* col = colk[k & 1];
+        __syncthreads();
+        // the lane's best row, then the warp's: magnitudes compare as their bits
+        unsigned hi = 0, lo = 0;
+        int row = kCoarsest;
+#pragma unroll
+        for (int i = 0; i < kCoarsest / 32; ++i) {
+            if (used >> i & 1) continue;
+            const double v = col[lane + 32 * i];
+            const unsigned h = (unsigned)__double2hiint(v) & 0x7fffffffu, l = (unsigned)__double2loint(v);
+            if (row == kCoarsest || h > hi || (h == hi && l > lo)) {
+                hi = h;
+                lo = l;
+                row = lane + 32 * i;
             }
         }
+        const unsigned top = __reduce_max_sync(0xffffffffu, row < kCoarsest ? hi : 0u);
+        const bool in_hi = row < kCoarsest && hi == top;
+        const unsigned top_lo = __reduce_max_sync(0xffffffffu, in_hi ? lo : 0u);
+        const int p = (int)__reduce_min_sync(0xffffffffu, in_hi && lo == top_lo ? (unsigned)row : (unsigned)kCoarsest);
+        if ((p & 31) == lane) used |= 1u << (p >> 5);
+        const double pv = col[p];
+        const bool mine = t == p % T;
+        double x = 0.0;
+        if (mine) {
+            // the row's place, selected place by place: an index into w would
+            // put it in local memory (pl is opaque to the compiler)
+            int pl = p / T;
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                asm volatile("" : "+r"(pl));
+                x = pl == m ? w[m] : x;
+            }
+            x = (j == k ? 1.0 : x) / pv;
+            rowp[j] = x;
+        }
+        if (threadIdx.x == 0) {
+            piv[k] = p;
+            step_of[p] = k;
+            if (!(fabs(pv) > 0.0) || !isfinite(pv)) *status = 1;
+        }
+        __syncthreads();
+        const double g = rowp[j];
+        if (j == k)
+#pragma unroll
+            for (int m = 0; m < M; ++m) w[m] = 0.0;
+#pragma unroll
+        for (int m = 0; m < M; ++m) w[m] = __fma_rn(-g, col[t + T * m], w[m]);
+        if (mine) {
+            int pl = p / T;
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                asm volatile("" : "+r"(pl));
+                w[m] = pl == m ? x : w[m];
+            }
+        }
+        if (j == k + 1)
+#pragma unroll
+            for (int m = 0; m < M; ++m) colk[(k + 1) & 1][t + T * m] = w[m];
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < n * n; i += blockDim.x) {
-        const int r = i / n, j = i - r * n;
-        a[i] = w[r * n + src[j]];
-    }
+    if (j < n)
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            const int r = t + T * m;
+            if (r < n) a[step_of[r] * n + piv[j]] = w[m];
+        }
 }
 
 template <class T, class M>
@@ -3120,14 +3142,7 @@ void factor_level(Core& c, const Level& L, int* status)
 void dense_inverse(Core& c, int n, double* a, int* status)
 {
     launch(c, "mg_dense_inverse", [&] {
-        const size_t smem = ((size_t)n * n + n) * sizeof(double);
-        // one value for every call: runtimes on other host threads set the
-        // same attribute, and a smaller value set between this call's set and
-        // its launch would fail it
-        const size_t most = ((size_t)kCoarsest * kCoarsest + kCoarsest) * sizeof(double);
-        EQG_CUDA(cudaFuncSetAttribute(dense_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)std::max(smem, most)));
-        dense_inverse_kernel<<<1, 1024, smem, c.stream>>>(n, a, status);
+        dense_inverse_kernel<<<1, kInverseThreads, 0, c.stream>>>(n, a, status);
     }, 16.0 * n * n);
 }
 
