@@ -780,6 +780,7 @@ struct SweConst {
     // (x / 2^k and x * 2^-k round the same real number), else 0
     double inv_two, inv_dx, inv_dy;
     double s_dry, s_dummy, s_g, s_zero;  // the wave-speed maximum's slots
+    double zero_f_0, dummy_0;            // zero_f * 0 and dummy * 0
 };
 
 struct SweArrays {
@@ -821,33 +822,49 @@ struct SideFlux {
     double f0, f1, f2, speed;
 };
 
+// SEL of a program's constant b where the mask is set: a + b * 0, with b * 0
+// computed once (bz).
+__device__ __forceinline__ double SEL_WET(double a, double bz) { return ADD(a, bz); }
+
 // sideFlux of the program for a cell's values (as gathered to a face: 0.0 +
 // x) in both directions: toward x faces (normal (1, 0)) and y faces
-// (normal (0, 1)).  Height, pressure and sqrt(g h) belong to the cell.
-__device__ __forceinline__ void side_fluxes(const SweConst& k, double w, double hu, double hv, double bb, bool want_x,
-                                            bool want_y, SideFlux& fx, SideFlux& fy)
+// (normal (0, 1)).  Height, pressure and sqrt(g h) belong to the cell.  Every
+// lane of the warp calls it; a warp of wet cells (`all_wet`) takes the
+// selections with their one sum.
+template <bool ALL_WET>
+__device__ __forceinline__ void side_fluxes_of(const SweConst& k, bool wet, double raw, double hu, double hv,
+                                               SideFlux& fx, SideFlux& fy)
+{
+    auto sel = [&](double a) { return ALL_WET ? SEL_WET(a, k.zero_f_0) : SEL(wet, a, k.zero_f); };
+    const double h = ALL_WET ? SEL_WET(raw, k.dummy_0) : SEL(wet, raw, k.dummy);
+    const double p = MUL(k.half_g, MUL(h, h));
+    const double p0 = MUL(p, 0.0);
+    const double sgh = SQRT(MUL(k.g, h));
+    {
+        const double qn = ADD(MUL(hu, 1.0), MUL(hv, 0.0));
+        const double un = DIV(qn, h);
+        fx.f0 = sel(qn);
+        fx.f1 = sel(ADD(MUL(hu, un), MUL(p, 1.0)));
+        fx.f2 = sel(ADD(MUL(hv, un), p0));
+        fx.speed = sel(ADD(SQRT_OF_SQUARE(un), sgh));
+    }
+    {
+        const double qn = ADD(MUL(hu, 0.0), MUL(hv, 1.0));
+        const double un = DIV(qn, h);
+        fy.f0 = sel(qn);
+        fy.f1 = sel(ADD(MUL(hu, un), p0));
+        fy.f2 = sel(ADD(MUL(hv, un), MUL(p, 1.0)));
+        fy.speed = sel(ADD(SQRT_OF_SQUARE(un), sgh));
+    }
+}
+
+__device__ __forceinline__ void side_fluxes(const SweConst& k, double w, double hu, double hv, double bb, SideFlux& fx,
+                                            SideFlux& fy)
 {
     const double raw = SUB(w, bb);
     const bool wet = raw > k.dry;
-    const double h = SEL(wet, raw, k.dummy);
-    const double p = MUL(k.half_g, MUL(h, h));
-    const double sgh = SQRT(MUL(k.g, h));
-    if (want_x) {
-        const double qn = ADD(MUL(hu, 1.0), MUL(hv, 0.0));
-        const double un = DIV(qn, h);
-        fx.f0 = SEL(wet, qn, k.zero_f);
-        fx.f1 = SEL(wet, ADD(MUL(hu, un), MUL(p, 1.0)), k.zero_f);
-        fx.f2 = SEL(wet, ADD(MUL(hv, un), MUL(p, 0.0)), k.zero_f);
-        fx.speed = SEL(wet, ADD(SQRT_OF_SQUARE(un), sgh), k.zero_f);
-    }
-    if (want_y) {
-        const double qn = ADD(MUL(hu, 0.0), MUL(hv, 1.0));
-        const double un = DIV(qn, h);
-        fy.f0 = SEL(wet, qn, k.zero_f);
-        fy.f1 = SEL(wet, ADD(MUL(hu, un), MUL(p, 0.0)), k.zero_f);
-        fy.f2 = SEL(wet, ADD(MUL(hv, un), MUL(p, 1.0)), k.zero_f);
-        fy.speed = SEL(wet, ADD(SQRT_OF_SQUARE(un), sgh), k.zero_f);
-    }
+    if (__all_sync(0xffffffffu, wet)) side_fluxes_of<true>(k, wet, raw, hu, hv, fx, fy);
+    else side_fluxes_of<false>(k, wet, raw, hu, hv, fx, fy);
 }
 
 // All-face flux values (times the area) of an interior face between cells
@@ -907,119 +924,168 @@ __device__ __forceinline__ double block_max(double v, double* scratch)
     return v;
 }
 
-// Threads of a block: one per cell of a kBX x kBY window, the tile of
-// kTX x kTY cells it updates and a one-cell halo around it.
-constexpr int kBX = 32, kBY = 10;
-constexpr int kTX = kBX - 2, kTY = kBY - 2;
+// Cells that a warp updates per row (its outer lanes are the halo), warps of
+// a block, and the rows of a warp's strip (between the least and the most).
+constexpr int kLanes = 30, kStripWarps = 4, kStripMin = 8, kStripMax = 64;
 
-// One forward-Euler stage on a tile.  Each thread reads one cell of the
-// window and computes its side fluxes toward x and y faces; then threads
-// compute the flux of the x face west of their cell (window rows 1..kTY,
-// columns 1..kBX-1) and of the y face south of it (columns 1..kTX, rows
-// 1..kBY-1), each face once; each cell of the tile sums its four faces.
-// HEUN: the stage after the first, averaged with the step's start state,
-// and (WITH_MAX) the results' wave-speed maximum.
+// Arrays of a row in a warp's ring of rows in shared memory.
+enum SweRow { R_W, R_HU, R_HV, R_BM, R_BE, R_BW, R_BN, R_BS, R_W0, R_HU0, R_HV0 };
+constexpr int kRing = 3;  // the row being updated, the next one, one in flight
+__host__ __device__ constexpr int ring_arrays(bool heun) { return heun ? 11 : 8; }
+constexpr size_t ring_bytes(bool heun) { return (size_t)kStripWarps * kRing * ring_arrays(heun) * 32 * sizeof(double); }
+
+// One forward-Euler stage.  A warp takes a strip of kLanes columns and `rows`
+// rows and walks it row by row, one cell per lane: the side fluxes of a cell
+// are computed once, the flux of the face west of it from its own and the
+// left lane's side fluxes (the one east of it is the right lane's), the flux
+// of the face north of it from its own and the next row's, which is the next
+// row's south face.  Fluxes pass between lanes by shuffles and between rows in
+// registers; a lane's values come through a ring of rows in shared memory,
+// filled by asynchronous copies a row ahead of their use, which leaves the
+// registers to more warps (no barrier: a lane reads what it copied itself).
+// HEUN: the stage after the first, averaged with the step's start state, and
+// (WITH_MAX) the results' wave-speed maximum.
+//
+// Bound: HBM (88 B per cell, 112 with HEUN) and the FP64 pipe (some 170 and
+// 220 operations per cell) at about the same time.  Before: one thread per
+// cell of a 32 x 10 window in shared memory, three barriers per 30 x 8 tile,
+// a third more side fluxes than cells.  4096 x 4096, both stages and the
+// maximum: 1.32 ms; with the next row's values in registers (128, 16
+// warps per SM) 1.03 ms; this form 0.79 ms (five blocks of 96 registers per
+// SM; four: 0.81, six: 1.11).
 template <bool HEUN, bool WITH_MAX>
-__global__ void __launch_bounds__(kBX * kBY, 4) swe_stage_kernel(Grid2 g, SweConst k, SweArrays a)
+__global__ void __launch_bounds__(32 * kStripWarps, 5)
+    swe_stage_kernel(Grid2 g, SweConst k, SweArrays a, int strips_x, int rows)
 {
-    __shared__ double sw[kBY][kBX], shu[kBY][kBX], shv[kBY][kBX], sbm[kBY][kBX];  // as read
-    __shared__ double sfx[4][kBY][kBX], sfy[4][kBY][kBX];  // side fluxes toward x and y faces
-    __shared__ double fxs[3][kBY][kBX], fys[3][kBY][kBX];  // flux of the x face west of, y face south of a cell
+    constexpr int NA = ring_arrays(HEUN);
+    extern __shared__ double ring_all[];
     __shared__ double scratch[32];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int gi = blockIdx.x * kTX - 1 + tx, gj = blockIdx.y * kTY - 1 + ty;
-    const bool inside = gi >= 0 && gi < g.nx && gj >= 0 && gj < g.ny;
-    if (inside) {
-        const int64_t c = gi + (int64_t)g.nx * gj;
-        const double w = a.w[c], hu = a.hu[c], hv = a.hv[c], bm = a.bm[c];
-        sw[ty][tx] = w;
-        shu[ty][tx] = hu;
-        shv[ty][tx] = hv;
-        sbm[ty][tx] = bm;
-        SideFlux fx, fy;
-        side_fluxes(k, ROW(w), ROW(hu), ROW(hv), ROW(bm), true, true, fx, fy);
-        sfx[0][ty][tx] = fx.f0;
-        sfx[1][ty][tx] = fx.f1;
-        sfx[2][ty][tx] = fx.f2;
-        sfx[3][ty][tx] = fx.speed;
-        sfy[0][ty][tx] = fy.f0;
-        sfy[1][ty][tx] = fy.f1;
-        sfy[2][ty][tx] = fy.f2;
-        sfy[3][ty][tx] = fy.speed;
-    }
-    __syncthreads();
-    double F[3];
-    // x face gi (west of cell gi, east of cell gi - 1) in row gj
-    if (ty >= 1 && ty <= kTY && tx >= 1 && gj < g.ny && gi <= g.nx) {
-        if (gi == 0) {
-            wall_flux(k, sw[ty][tx], sbm[ty][tx], 1.0, 0.0, k.area_x, F);
-        } else if (gi == g.nx) {
-            wall_flux(k, sw[ty][tx - 1], sbm[ty][tx - 1], 1.0, 0.0, k.area_x, F);
-        } else {
-            const SideFlux fL{sfx[0][ty][tx - 1], sfx[1][ty][tx - 1], sfx[2][ty][tx - 1], sfx[3][ty][tx - 1]};
-            const SideFlux fR{sfx[0][ty][tx], sfx[1][ty][tx], sfx[2][ty][tx], sfx[3][ty][tx]};
-            interior_flux(k, ROW(sw[ty][tx - 1]), ROW(shu[ty][tx - 1]), ROW(shv[ty][tx - 1]), fL, ROW(sw[ty][tx]),
-                          ROW(shu[ty][tx]), ROW(shv[ty][tx]), fR, k.area_x, F);
-        }
-        fxs[0][ty][tx] = F[0];
-        fxs[1][ty][tx] = F[1];
-        fxs[2][ty][tx] = F[2];
-    }
-    // y face gj (south of cell gj, north of cell gj - 1) in column gi
-    if (tx >= 1 && tx <= kTX && ty >= 1 && gi < g.nx && gj <= g.ny) {
-        if (gj == 0) {
-            wall_flux(k, sw[ty][tx], sbm[ty][tx], 0.0, 1.0, k.area_y, F);
-        } else if (gj == g.ny) {
-            wall_flux(k, sw[ty - 1][tx], sbm[ty - 1][tx], 0.0, 1.0, k.area_y, F);
-        } else {
-            const SideFlux fL{sfy[0][ty - 1][tx], sfy[1][ty - 1][tx], sfy[2][ty - 1][tx], sfy[3][ty - 1][tx]};
-            const SideFlux fR{sfy[0][ty][tx], sfy[1][ty][tx], sfy[2][ty][tx], sfy[3][ty][tx]};
-            interior_flux(k, ROW(sw[ty - 1][tx]), ROW(shu[ty - 1][tx]), ROW(shv[ty - 1][tx]), fL, ROW(sw[ty][tx]),
-                          ROW(shu[ty][tx]), ROW(shv[ty][tx]), fR, k.area_y, F);
-        }
-        fys[0][ty][tx] = F[0];
-        fys[1][ty][tx] = F[1];
-        fys[2][ty][tx] = F[2];
-    }
-    __syncthreads();
+    const int lane = threadIdx.x & 31, strip = blockIdx.x * kStripWarps + (threadIdx.x >> 5);
+    double* const ring = ring_all + (size_t)(threadIdx.x >> 5) * kRing * NA * 32 + lane;
+    const int gi = (strip % strips_x) * kLanes - 1 + lane, j0 = (strip / strips_x) * rows;
+    const int j1 = min(j0 + rows, g.ny);
+    const int ci = min(max(gi, 0), g.nx - 1);  // lanes outside the grid read a cell whose results are not used
+    const bool owned = lane >= 1 && lane <= kLanes && gi < g.nx;
     double speed = -DBL_MAX;
-    if (tx >= 1 && tx <= kTX && ty >= 1 && ty <= kTY && inside) {
-        const int64_t c = gi + (int64_t)g.nx * gj;
-        const double w = sw[ty][tx], hu = shu[ty][tx], hv = shv[ty][tx], bm = sbm[ty][tx];
-        const double be = a.be[c], bw = a.bw[c], bn = a.bn[c], bs = a.bs[c];
-        double nd[3];
-        for (int m = 0; m < 3; ++m) {
-            double acc = 0.0;
-            acc = SUB(acc, fxs[m][ty][tx]);
-            acc = ADD(acc, fxs[m][ty][tx + 1]);
-            acc = SUB(acc, fys[m][ty][tx]);
-            acc = ADD(acc, fys[m][ty + 1][tx]);
-            nd[m] = SUB(0.0, acc);
+    if (j0 < g.ny) {  // the whole warp
+        auto at = [&](int slot, int arr) -> double& { return ring[(slot * NA + arr) * 32]; };
+        auto issue = [&](int j, int slot) {
+            const int64_t c = ci + (int64_t)g.nx * min(max(j, 0), g.ny - 1);
+            auto copy = [&](int arr, const double* p) {
+                const unsigned dst = (unsigned)__cvta_generic_to_shared(&at(slot, arr));
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(p + c) : "memory");
+            };
+            copy(R_W, a.w);
+            copy(R_HU, a.hu);
+            copy(R_HV, a.hv);
+            copy(R_BM, a.bm);
+            copy(R_BE, a.be);
+            copy(R_BW, a.bw);
+            copy(R_BN, a.bn);
+            copy(R_BS, a.bs);
+            if (HEUN) {
+                copy(R_W0, a.w0);
+                copy(R_HU0, a.hu0);
+                copy(R_HV0, a.hv0);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        int s0 = 1, s1 = 2, s2 = 0;  // slots of rows j, j + 1, j + 2
+        issue(j0 - 1, 0);
+        issue(j0, 1);
+        issue(j0 + 1, 2);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        double rw = ROW(at(1, R_W)), rhu = ROW(at(1, R_HU)), rhv = ROW(at(1, R_HV));  // as gathered to a face
+        SideFlux fx, fy;
+        double S[3];  // flux of the face south of the row
+        {
+            const double lw = ROW(at(0, R_W)), lhu = ROW(at(0, R_HU)), lhv = ROW(at(0, R_HV));
+            SideFlux lx, ly;
+            side_fluxes(k, lw, lhu, lhv, ROW(at(0, R_BM)), lx, ly);
+            side_fluxes(k, rw, rhu, rhv, ROW(at(1, R_BM)), fx, fy);
+            if (j0 > 0) interior_flux(k, lw, lhu, lhv, ly, rw, rhu, rhv, fy, k.area_y, S);
+            else wall_flux(k, at(1, R_W), at(1, R_BM), 0.0, 1.0, k.area_y, S);
         }
-        const double stx = DIVBY(ADD(SUB(w, be), SUB(w, bw)), k.two, k.inv_two);
-        const double sty = DIVBY(ADD(SUB(w, bn), SUB(w, bs)), k.two, k.inv_two);
-        const double dry_term = SEL(SUB(w, bm) > k.dry, k.one_c, k.zero_c);
-        const double bx = DIVBY(SUB(be, bw), k.dx, k.inv_dx), by = DIVBY(SUB(bn, bs), k.dy, k.inv_dy);
-        const double s0 = MUL(MUL(MUL(k.neg_g, bx), stx), dry_term);
-        const double s1 = MUL(MUL(MUL(k.neg_g, by), sty), dry_term);
-        double w1 = ADD(w, MUL(k.dt_vol, nd[0]));
-        double hu1 = ADD(hu, MUL(k.dt_vol, ADD(nd[1], MUL(k.vol, s0))));
-        double hv1 = ADD(hv, MUL(k.dt_vol, ADD(nd[2], MUL(k.vol, s1))));
-        if (HEUN) {
-            w1 = ADD(MUL(k.half, a.w0[c]), MUL(k.half, w1));
-            hu1 = ADD(MUL(k.half, a.hu0[c]), MUL(k.half, hu1));
-            hv1 = ADD(MUL(k.half, a.hv0[c]), MUL(k.half, hv1));
+        for (int j = j0; j < j1; ++j) {
+            issue(j + 2, s2);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            // the faces west and east of the cell
+            double nd[3], F[3];
+            {
+                auto left = [&](double x) { return __shfl_up_sync(0xffffffffu, x, 1); };
+                const SideFlux fl{left(fx.f0), left(fx.f1), left(fx.f2), left(fx.speed)};
+                const double lw = left(rw), lhu = left(rhu), lhv = left(rhv);
+                interior_flux(k, lw, lhu, lhv, fl, rw, rhu, rhv, fx, k.area_x, F);
+            }
+            double E[3];
+            for (int m = 0; m < 3; ++m) E[m] = __shfl_down_sync(0xffffffffu, F[m], 1);
+            if (gi == 0) wall_flux(k, at(s0, R_W), at(s0, R_BM), 1.0, 0.0, k.area_x, F);
+            if (gi == g.nx - 1) wall_flux(k, at(s0, R_W), at(s0, R_BM), 1.0, 0.0, k.area_x, E);
+            // the divergence: west, east, south, north faces from 0.0
+            for (int m = 0; m < 3; ++m) nd[m] = SUB(ADD(SUB(0.0, F[m]), E[m]), S[m]);
+            // the next row, and the face between it and this one
+            const double nw = ROW(at(s1, R_W)), nhu = ROW(at(s1, R_HU)), nhv = ROW(at(s1, R_HV));
+            SideFlux nfy;
+            side_fluxes(k, nw, nhu, nhv, ROW(at(s1, R_BM)), fx, nfy);
+            if (j + 1 < g.ny) interior_flux(k, rw, rhu, rhv, fy, nw, nhu, nhv, nfy, k.area_y, S);
+            else wall_flux(k, at(s0, R_W), at(s0, R_BM), 0.0, 1.0, k.area_y, S);
+            for (int m = 0; m < 3; ++m) nd[m] = SUB(0.0, ADD(nd[m], S[m]));
+            rw = nw;
+            rhu = nhu;
+            rhv = nhv;
+            fy = nfy;
+            // the update
+            const double w = at(s0, R_W), hu = at(s0, R_HU), hv = at(s0, R_HV), bm = at(s0, R_BM);
+            const double be = at(s0, R_BE), bw = at(s0, R_BW), bn = at(s0, R_BN), bs = at(s0, R_BS);
+            const double stx = DIVBY(ADD(SUB(w, be), SUB(w, bw)), k.two, k.inv_two);
+            const double sty = DIVBY(ADD(SUB(w, bn), SUB(w, bs)), k.two, k.inv_two);
+            const double dry_term = SEL(SUB(w, bm) > k.dry, k.one_c, k.zero_c);
+            const double bx = DIVBY(SUB(be, bw), k.dx, k.inv_dx), by = DIVBY(SUB(bn, bs), k.dy, k.inv_dy);
+            const double q0 = MUL(MUL(MUL(k.neg_g, bx), stx), dry_term);
+            const double q1 = MUL(MUL(MUL(k.neg_g, by), sty), dry_term);
+            double w1 = ADD(w, MUL(k.dt_vol, nd[0]));
+            double hu1 = ADD(hu, MUL(k.dt_vol, ADD(nd[1], MUL(k.vol, q0))));
+            double hv1 = ADD(hv, MUL(k.dt_vol, ADD(nd[2], MUL(k.vol, q1))));
+            if (HEUN) {
+                w1 = ADD(MUL(k.half, at(s0, R_W0)), MUL(k.half, w1));
+                hu1 = ADD(MUL(k.half, at(s0, R_HU0)), MUL(k.half, hu1));
+                hv1 = ADD(MUL(k.half, at(s0, R_HV0)), MUL(k.half, hv1));
+            }
+            if (owned) {
+                const int64_t c = ci + (int64_t)g.nx * j;
+                a.ow[c] = w1;
+                a.ohu[c] = hu1;
+                a.ohv[c] = hv1;
+                if (WITH_MAX) speed = fmax(speed, cell_speed(k, w1, hu1, hv1, bm));
+            }
+            const int s = s0;
+            s0 = s1;
+            s1 = s2;
+            s2 = s;
         }
-        a.ow[c] = w1;
-        a.ohu[c] = hu1;
-        a.ohv[c] = hv1;
-        if (WITH_MAX) speed = cell_speed(k, w1, hu1, hv1, bm);
+        asm volatile("cp.async.wait_all;" ::: "memory");
     }
     if (WITH_MAX) {
         speed = block_max(speed, scratch);
-        if (tx == 0 && ty == 0) a.partials[blockIdx.x + (int64_t)gridDim.x * blockIdx.y] = speed;
+        if (threadIdx.x == 0) a.partials[blockIdx.x] = speed;
     }
 }
+
+// The launch of a stage: strips of kLanes columns, of the most rows (a strip
+// costs the side fluxes of two more) that still give every SM four blocks of
+// warps: the walk of a strip is a chain, hidden by other warps only.
+struct StripGrid {
+    int strips_x, rows, blocks;
+    StripGrid(int nx, int ny)
+    {
+        strips_x = (nx + kLanes - 1) / kLanes;
+        const int64_t wanted = (int64_t)148 * 4 * kStripWarps;
+        rows = kStripMax;
+        while (rows > kStripMin && (int64_t)strips_x * ((ny + rows - 1) / rows) < wanted) rows /= 2;
+        const int64_t strips = (int64_t)strips_x * ((ny + rows - 1) / rows);
+        blocks = (int)((strips + kStripWarps - 1) / kStripWarps);
+    }
+};
 
 // The wave speed's maximum of a state, per block.
 __global__ void __launch_bounds__(256) swe_speed_kernel(int64_t n, SweConst k, const double* __restrict__ w,
@@ -1056,7 +1122,7 @@ double exact_inverse(double d)
 
 bool grid_fits(const Core& c)
 {
-    return c.cartesian && c.dim == 2 && c.nx >= 2 && c.ny >= 2 && (c.ny + kTY - 1) / kTY <= 65535;
+    return c.cartesian && c.dim == 2 && c.nx >= 2 && c.ny >= 2;
 }
 
 // Every variable a leaf (pending ones evaluated), every slot bound.
@@ -1141,6 +1207,8 @@ bool fused_materialize(Core& c, LazyNode* root)
     k.inv_two = exact_inverse(k.two);
     k.inv_dx = exact_inverse(k.dx);
     k.inv_dy = exact_inverse(k.dy);
+    k.zero_f_0 = k.zero_f * 0.0;
+    k.dummy_0 = k.dummy * 0.0;
 
     FuseState& st = state(c);
     const Buf& bmid = M.var[V_BMID]->leaf;
@@ -1153,8 +1221,9 @@ bool fused_materialize(Core& c, LazyNode* root)
         k.s_zero = st.speed_slots[T_ZERO];
     }
     const Grid2 g = grid2(c);
-    const dim3 block(kBX, kBY), grid((c.nx + kTX - 1) / kTX, (c.ny + kTY - 1) / kTY);
-    const int64_t nblocks = (int64_t)grid.x * grid.y;
+    const StripGrid sg(c.nx, c.ny);
+    const int block = 32 * kStripWarps, grid = sg.blocks;
+    const int64_t nblocks = grid;
     ensure_partials(c, st, nblocks);
     const size_t bytes = (size_t)c.nc * sizeof(double);
     Buf mid[3] = {c.alloc(bytes), c.alloc(bytes), c.alloc(bytes)};
@@ -1172,7 +1241,7 @@ bool fused_materialize(Core& c, LazyNode* root)
     a.ohu = mid[1]->as<double>();
     a.ohv = mid[2]->as<double>();
     // stage 1: state and five bottom arrays read, state written
-    launch(c, "swe_stage", [&] { swe_stage_kernel<false, false><<<grid, block, 0, c.stream>>>(g, k, a); },
+    launch(c, "swe_stage", [&] { swe_stage_kernel<false, false><<<grid, block, ring_bytes(false), c.stream>>>(g, k, a, sg.strips_x, sg.rows); },
            88.0 * c.nc);
     SweArrays b = a;
     b.w0 = a.w;
@@ -1187,7 +1256,7 @@ bool fused_materialize(Core& c, LazyNode* root)
     b.partials = st.partials->as<double>();
     // stage 2 and Heun's average: both states read as well
     if (with_max) {
-        launch(c, "swe_heun_stage", [&] { swe_stage_kernel<true, true><<<grid, block, 0, c.stream>>>(g, k, b); },
+        launch(c, "swe_heun_stage", [&] { swe_stage_kernel<true, true><<<grid, block, ring_bytes(true), c.stream>>>(g, k, b, sg.strips_x, sg.rows); },
                112.0 * c.nc);
         launch(c, "swe_max_final", [&] {
             max_final_kernel<<<1, 256, 0, c.stream>>>(st.partials->as<double>(), nblocks, st.result->as<double>());
@@ -1199,7 +1268,7 @@ bool fused_materialize(Core& c, LazyNode* root)
         st.cached.bmid = bmid;
         std::memcpy(st.cached.slots, st.speed_slots, sizeof(st.cached.slots));
     } else {
-        launch(c, "swe_heun_stage", [&] { swe_stage_kernel<true, false><<<grid, block, 0, c.stream>>>(g, k, b); },
+        launch(c, "swe_heun_stage", [&] { swe_stage_kernel<true, false><<<grid, block, ring_bytes(true), c.stream>>>(g, k, b, sg.strips_x, sg.rows); },
                112.0 * c.nc);
     }
     for (int m = 0; m < 3; ++m) lazy_make_leaf(roots[m], out[m]);
