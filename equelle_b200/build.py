@@ -1,7 +1,7 @@
 """Build recipe for libeqg.so (sm_100a) and the generated-style simulators.
 
-    python -m equelle_b200.build            # library + simulators
-    python -m equelle_b200.build --lib      # library only
+    python -m equelle_b200.build            # library, Python mirror, simulators
+    python -m equelle_b200.build --lib      # library and Python mirror only
 
 nvcc cross-compiles for sm_100a without a GPU; each .cu file is compiled in
 parallel and linked into equelle_b200/lib/libeqg.so.  The simulators in
@@ -13,6 +13,7 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 
 from . import INCLUDE_DIR, LIB_DIR, LIB_PATH, PKG_DIR
 
@@ -77,6 +78,20 @@ def build_library(force=False, verbose=False):
     return LIB_PATH
 
 
+def build_mirror(force=False):
+    """The native half of the Python mirror, as the extension module
+    equelle_b200._mirror of the running interpreter."""
+    src = os.path.join(CSRC, "mirror.cpp")
+    out = os.path.join(PKG_DIR, "_mirror" + sysconfig.get_config_var("EXT_SUFFIX"))
+    if force or _stale(out, [src, os.path.join(INCLUDE_DIR, "eqg.h")]):
+        # built beside its place and moved: another process may import it meanwhile
+        tmp = "%s.%d.tmp" % (out, os.getpid())
+        _run([CXX, "-std=c++17", "-O2", "-fPIC", "-shared", "-I" + INCLUDE_DIR,
+              "-I" + sysconfig.get_paths()["include"], "-o", tmp, src])
+        os.replace(tmp, out)
+    return out
+
+
 def build_simulators(force=False):
     """Each simulator becomes an executable and a shared library exposing
     `int eqg_sim_main(int argc, char** argv)` for in-process use."""
@@ -107,6 +122,7 @@ def main(argv=None):
     ap.add_argument("-v", action="store_true")
     a = ap.parse_args(argv)
     print(build_library(force=a.force, verbose=a.v))
+    print(build_mirror(force=a.force))
     if not a.lib:
         for p in build_simulators(force=a.force):
             print(p)

@@ -1,0 +1,707 @@
+// Native half of the Python runtime mirror (equelle_b200/runtime.py): the
+// handle types with their operators, and the runtime methods that a
+// program's time loop calls, as CPython types over the C ABI of
+// include/eqg.h.  An explicit program makes some 250 runtime calls a time
+// step; through ctypes a call cost 2.1 us of interpreter work (a Python
+// frame or two, an out-parameter object, argument conversion), of which the
+// library's part is 0.2 us: a shallow-water step on 64 x 48 cells took 0.79
+// ms, 0.19 ms with these.
+//
+// The entry points come as addresses from the ctypes library that the
+// runtime was given (the device library or the CPU oracle): nothing is
+// linked.  The interpreter lock is released around the library calls, as
+// ctypes does.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include "eqg.h"
+
+#include <cstddef>
+#include <cstring>
+#include <initializer_list>
+
+namespace {
+
+// ---- entry points of one library ----------------------------------------------
+struct Api {
+    decltype(&eqg_last_error) last_error;
+    decltype(&eqg_set_builtin) set_builtin;
+    decltype(&eqg_set_size) set_size;
+    decltype(&eqg_set_release) set_release;
+    decltype(&eqg_first_cell) first_cell;
+    decltype(&eqg_second_cell) second_cell;
+    decltype(&eqg_set_on) set_on;
+    decltype(&eqg_set_extend) set_extend;
+    decltype(&eqg_set_select) set_select;
+    decltype(&eqg_mask_release) mask_release;
+    decltype(&eqg_mask_logic) mask_logic;
+    decltype(&eqg_coll_constant) coll_constant;
+    decltype(&eqg_coll_release) coll_release;
+    decltype(&eqg_binary) binary;
+    decltype(&eqg_binary_scalar) binary_scalar;
+    decltype(&eqg_unary) unary;
+    decltype(&eqg_compare) compare;
+    decltype(&eqg_compare_scalar) compare_scalar;
+    decltype(&eqg_gradient) gradient;
+    decltype(&eqg_neg_gradient) neg_gradient;
+    decltype(&eqg_divergence) divergence;
+    decltype(&eqg_interior_divergence) interior_divergence;
+    decltype(&eqg_on) on;
+    decltype(&eqg_extend) extend;
+    decltype(&eqg_select) select;
+    decltype(&eqg_reduce) reduce;
+    decltype(&eqg_two_norm) two_norm;
+    decltype(&eqg_span_subset) span_subset;
+    decltype(&eqg_span_superset) span_superset;
+};
+
+struct Entry {
+    const char* name;
+    size_t offset;
+};
+#define E(name) {"eqg_" #name, offsetof(Api, name)}
+const Entry kEntries[] = {E(last_error), E(set_builtin), E(set_size), E(set_release), E(first_cell), E(second_cell),
+                          E(set_on), E(set_extend), E(set_select), E(mask_release), E(mask_logic), E(coll_constant),
+                          E(coll_release), E(binary), E(binary_scalar), E(unary), E(compare), E(compare_scalar),
+                          E(gradient), E(neg_gradient), E(divergence), E(interior_divergence), E(on), E(extend),
+                          E(select), E(reduce), E(two_norm), E(span_subset), E(span_superset)};
+#undef E
+
+// Classes of the Python module, set by register_classes().
+PyObject* g_coll_class = nullptr;
+PyObject* g_mask_class = nullptr;
+PyObject* g_set_class = nullptr;
+PyObject* g_error_class = nullptr;
+
+struct RuntimeObject {
+    PyObject_HEAD
+    Api api;
+    eqg_runtime* h;
+    bool bound;
+};
+
+struct HandleObject {
+    PyObject_HEAD
+    RuntimeObject* rt;  // owned
+    void* h;
+};
+
+extern PyTypeObject RuntimeBaseType, CollBaseType, MaskBaseType, SetBaseType;
+
+PyObject* raise_status(const Api& api, int status)
+{
+    const char* msg = api.last_error();
+    PyObject* e = PyObject_CallFunction(g_error_class, "is", status, msg ? msg : "");
+    if (e) {
+        PyErr_SetObject(g_error_class, e);
+        Py_DECREF(e);
+    }
+    return nullptr;
+}
+
+// Calls an entry point with the interpreter lock released.
+template <class F>
+int unlocked(F&& f)
+{
+    int st;
+    Py_BEGIN_ALLOW_THREADS
+    st = f();
+    Py_END_ALLOW_THREADS
+    return st;
+}
+
+PyObject* new_handle(PyObject* cls, RuntimeObject* rt, void* h)
+{
+    PyTypeObject* t = (PyTypeObject*)cls;
+    HandleObject* o = (HandleObject*)t->tp_alloc(t, 0);
+    if (!o) return nullptr;
+    Py_INCREF(rt);
+    o->rt = rt;
+    o->h = h;
+    return (PyObject*)o;
+}
+
+// A call that makes a handle: status and out-parameter to a Python object.
+template <class T, class F>
+PyObject* make(PyObject* cls, RuntimeObject* rt, F&& f)
+{
+    T* out = nullptr;
+    const int st = unlocked([&] { return f(&out); });
+    return st == EQG_OK ? new_handle(cls, rt, out) : raise_status(rt->api, st);
+}
+
+// The handle inside a Python object: a handle type's own, or the integer in
+// its attribute `h`.
+bool handle_of(PyObject* o, void** h)
+{
+    if (PyObject_TypeCheck(o, &CollBaseType) || PyObject_TypeCheck(o, &SetBaseType) ||
+        PyObject_TypeCheck(o, &MaskBaseType)) {
+        *h = ((HandleObject*)o)->h;
+        return true;
+    }
+    PyObject* v = PyObject_GetAttrString(o, "h");
+    if (!v) return false;
+    *h = v == Py_None ? nullptr : PyLong_AsVoidPtr(v);
+    Py_DECREF(v);
+    return !PyErr_Occurred();
+}
+
+bool double_of(PyObject* o, double* v)
+{
+    if (PyFloat_CheckExact(o)) {
+        *v = PyFloat_AS_DOUBLE(o);
+        return true;
+    }
+    PyObject* f = PyNumber_Float(o);  // as float(o)
+    if (!f) return false;
+    *v = PyFloat_AS_DOUBLE(f);
+    Py_DECREF(f);
+    return true;
+}
+
+// ---- handles ---------------------------------------------------------------------
+int handle_init(PyObject* self, PyObject* args, PyObject* kwargs)
+{
+    static const char* names[] = {"rt", "h", nullptr};
+    PyObject *rt, *h;
+    if (!PyArg_ParseTupleAndKeywords(args, kwargs, "O!O", (char**)names, &RuntimeBaseType, &rt, &h)) return -1;
+    void* p = nullptr;
+    if (h != Py_None) {
+        p = PyLong_AsVoidPtr(h);
+        if (!p && PyErr_Occurred()) return -1;
+    }
+    HandleObject* o = (HandleObject*)self;
+    Py_INCREF(rt);
+    Py_XSETREF(o->rt, (RuntimeObject*)rt);
+    o->h = p;
+    return 0;
+}
+
+// Gives the handle back to its library and lets go of the runtime.
+template <class Release>
+int handle_drop(PyObject* self, Release&& release)
+{
+    HandleObject* o = (HandleObject*)self;
+    if (o->h && o->rt && o->rt->bound) release(o->rt->api, o->h);
+    o->h = nullptr;
+    Py_CLEAR(o->rt);
+    return 0;
+}
+int coll_clear(PyObject* self)
+{
+    return handle_drop(self, [](const Api& a, void* h) { a.coll_release((eqg_coll*)h); });
+}
+int mask_clear(PyObject* self)
+{
+    return handle_drop(self, [](const Api& a, void* h) { a.mask_release((eqg_mask*)h); });
+}
+int set_clear(PyObject* self)
+{
+    return handle_drop(self, [](const Api& a, void* h) { a.set_release((eqg_set*)h); });
+}
+template <int (*Clear)(PyObject*)>
+void handle_dealloc(PyObject* self)
+{
+    PyObject_GC_UnTrack(self);
+    Clear(self);
+    Py_TYPE(self)->tp_free(self);
+}
+int handle_traverse(PyObject* self, visitproc visit, void* arg)
+{
+    Py_VISIT(((HandleObject*)self)->rt);
+    return 0;
+}
+
+PyObject* handle_get_rt(PyObject* self, void*)
+{
+    PyObject* rt = (PyObject*)((HandleObject*)self)->rt;
+    if (!rt) rt = Py_None;
+    return Py_NewRef(rt);
+}
+PyObject* handle_get_h(PyObject* self, void*)
+{
+    void* h = ((HandleObject*)self)->h;
+    if (!h) Py_RETURN_NONE;
+    return PyLong_FromVoidPtr(h);
+}
+int handle_set_h(PyObject* self, PyObject* v, void*)
+{
+    void* p = nullptr;
+    if (v && v != Py_None) {
+        p = PyLong_AsVoidPtr(v);
+        if (!p && PyErr_Occurred()) return -1;
+    }
+    ((HandleObject*)self)->h = p;
+    return 0;
+}
+PyGetSetDef handle_getset[] = {{"rt", handle_get_rt, nullptr, nullptr, nullptr},
+                               {"h", handle_get_h, handle_set_h, nullptr, nullptr},
+                               {nullptr, nullptr, nullptr, nullptr, nullptr}};
+
+Py_hash_t identity_hash(PyObject* self) { return (Py_hash_t)((uintptr_t)self >> 4); }
+
+// ---- scalar collections ------------------------------------------------------------
+// left op right where at least one is a collection.
+PyObject* coll_binary(int op, PyObject* left, PyObject* right)
+{
+    const bool l = PyObject_TypeCheck(left, &CollBaseType), r = PyObject_TypeCheck(right, &CollBaseType);
+    HandleObject* self = (HandleObject*)(l ? left : right);
+    RuntimeObject* rt = self->rt;
+    if (l && r) {
+        const eqg_coll *a = (eqg_coll*)((HandleObject*)left)->h, *b = (eqg_coll*)((HandleObject*)right)->h;
+        return make<eqg_coll>(g_coll_class, rt, [&](eqg_coll** o) { return rt->api.binary(rt->h, op, a, b, o); });
+    }
+    double s;
+    if (!double_of(l ? right : left, &s)) return nullptr;
+    const eqg_coll* a = (eqg_coll*)self->h;
+    return make<eqg_coll>(g_coll_class, rt,
+                          [&](eqg_coll** o) { return rt->api.binary_scalar(rt->h, op, a, s, l ? 0 : 1, o); });
+}
+PyObject* coll_add(PyObject* a, PyObject* b) { return coll_binary(EQG_ADD, a, b); }
+PyObject* coll_sub(PyObject* a, PyObject* b) { return coll_binary(EQG_SUB, a, b); }
+PyObject* coll_mul(PyObject* a, PyObject* b) { return coll_binary(EQG_MUL, a, b); }
+PyObject* coll_div(PyObject* a, PyObject* b) { return coll_binary(EQG_DIV, a, b); }
+
+PyObject* unary_of(RuntimeObject* rt, int op, const void* h)
+{
+    return make<eqg_coll>(g_coll_class, rt,
+                          [&](eqg_coll** o) { return rt->api.unary(rt->h, op, (const eqg_coll*)h, o); });
+}
+PyObject* coll_neg(PyObject* self)
+{
+    HandleObject* s = (HandleObject*)self;
+    return unary_of(s->rt, EQG_NEG, s->h);
+}
+
+PyObject* coll_compare_op(PyObject* self, int op, PyObject* other)
+{
+    HandleObject* s = (HandleObject*)self;
+    RuntimeObject* rt = s->rt;
+    const eqg_coll* a = (eqg_coll*)s->h;
+    if (PyObject_TypeCheck(other, &CollBaseType)) {
+        const eqg_coll* b = (eqg_coll*)((HandleObject*)other)->h;
+        return make<eqg_mask>(g_mask_class, rt, [&](eqg_mask** o) { return rt->api.compare(rt->h, op, a, b, o); });
+    }
+    double v;
+    if (!double_of(other, &v)) return nullptr;
+    return make<eqg_mask>(g_mask_class, rt,
+                          [&](eqg_mask** o) { return rt->api.compare_scalar(rt->h, op, a, v, 0, o); });
+}
+PyObject* coll_richcompare(PyObject* self, PyObject* other, int op)
+{
+    switch (op) {
+    case Py_LT: return coll_compare_op(self, EQG_LT, other);
+    case Py_LE: return coll_compare_op(self, EQG_LE, other);
+    case Py_GT: return coll_compare_op(self, EQG_GT, other);
+    case Py_GE: return coll_compare_op(self, EQG_GE, other);
+    default: Py_RETURN_NOTIMPLEMENTED;  // == and != compare identities
+    }
+}
+PyObject* coll_eq(PyObject* self, PyObject* other) { return coll_compare_op(self, EQG_EQ, other); }
+PyObject* coll_ne(PyObject* self, PyObject* other) { return coll_compare_op(self, EQG_NE, other); }
+
+PyMethodDef coll_methods[] = {{"eq", coll_eq, METH_O, nullptr}, {"ne", coll_ne, METH_O, nullptr},
+                              {nullptr, nullptr, 0, nullptr}};
+PyNumberMethods coll_number = {};
+
+// ---- masks ---------------------------------------------------------------------------
+PyObject* mask_logic_op(int op, PyObject* self, PyObject* other)
+{
+    if (!PyObject_TypeCheck(self, &MaskBaseType)) Py_RETURN_NOTIMPLEMENTED;
+    HandleObject* s = (HandleObject*)self;
+    RuntimeObject* rt = s->rt;
+    void* b = nullptr;
+    if (other && other != Py_None && !handle_of(other, &b)) return nullptr;
+    return make<eqg_mask>(g_mask_class, rt, [&](eqg_mask** o) {
+        return rt->api.mask_logic(rt->h, op, (eqg_mask*)s->h, (eqg_mask*)b, o);
+    });
+}
+PyObject* mask_and(PyObject* a, PyObject* b) { return mask_logic_op(EQG_AND, a, b); }
+PyObject* mask_or(PyObject* a, PyObject* b) { return mask_logic_op(EQG_OR, a, b); }
+PyObject* mask_invert(PyObject* a) { return mask_logic_op(EQG_NOT, a, nullptr); }
+PyNumberMethods mask_number = {};
+
+// ---- runtime ----------------------------------------------------------------------------
+// Positional and keyword arguments into v[0 .. n), of which the first `need`
+// are required.
+bool take(const char* fn, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames, const char* const* names, int n,
+          int need, PyObject** v)
+{
+    for (int i = 0; i < n; ++i) v[i] = nullptr;
+    if (nargs > n) {
+        PyErr_Format(PyExc_TypeError, "%s() takes at most %d arguments (%zd given)", fn, n, nargs);
+        return false;
+    }
+    for (Py_ssize_t i = 0; i < nargs; ++i) v[i] = args[i];
+    const Py_ssize_t nk = kwnames ? PyTuple_GET_SIZE(kwnames) : 0;
+    for (Py_ssize_t k = 0; k < nk; ++k) {
+        PyObject* name = PyTuple_GET_ITEM(kwnames, k);
+        int at = -1;
+        for (int i = 0; i < n; ++i)
+            if (PyUnicode_CompareWithASCIIString(name, names[i]) == 0) at = i;
+        if (at < 0 || v[at]) {
+            PyErr_Format(PyExc_TypeError, "%s() got an unexpected or repeated keyword argument '%U'", fn, name);
+            return false;
+        }
+        v[at] = args[nargs + k];
+    }
+    for (int i = 0; i < need; ++i)
+        if (!v[i]) {
+            PyErr_Format(PyExc_TypeError, "%s() missing required argument: '%s'", fn, names[i]);
+            return false;
+        }
+    return true;
+}
+
+#define METHOD_ARGS PyObject *self, PyObject *const *args, Py_ssize_t nargs, PyObject *kwnames
+RuntimeObject* rt_of(PyObject* self) { return (RuntimeObject*)self; }
+
+// Methods of one collection argument.
+template <class Get>
+PyObject* coll_method(METHOD_ARGS, const char* name, Get&& get)
+{
+    static const char* const names[] = {"x"};
+    PyObject* v[1];
+    void* h;
+    if (!take(name, args, nargs, kwnames, names, 1, 1, v) || !handle_of(v[0], &h)) return nullptr;
+    RuntimeObject* rt = rt_of(self);
+    return make<eqg_coll>(g_coll_class, rt,
+                          [&](eqg_coll** o) { return get(rt->api)(rt->h, (const eqg_coll*)h, o); });
+}
+PyObject* rt_gradient(METHOD_ARGS)
+{
+    return coll_method(self, args, nargs, kwnames, "gradient", [](const Api& a) { return a.gradient; });
+}
+PyObject* rt_neg_gradient(METHOD_ARGS)
+{
+    return coll_method(self, args, nargs, kwnames, "negGradient", [](const Api& a) { return a.neg_gradient; });
+}
+PyObject* rt_divergence(METHOD_ARGS)
+{
+    return coll_method(self, args, nargs, kwnames, "divergence", [](const Api& a) { return a.divergence; });
+}
+PyObject* rt_interior_divergence(METHOD_ARGS)
+{
+    return coll_method(self, args, nargs, kwnames, "interiorDivergence",
+                       [](const Api& a) { return a.interior_divergence; });
+}
+PyObject* rt_sqrt(METHOD_ARGS)
+{
+    static const char* const names[] = {"x"};
+    PyObject* v[1];
+    void* h;
+    if (!take("sqrt", args, nargs, kwnames, names, 1, 1, v) || !handle_of(v[0], &h)) return nullptr;
+    return unary_of(rt_of(self), EQG_SQRT, h);
+}
+
+PyObject* builtin_set(PyObject* self, int which)
+{
+    RuntimeObject* rt = rt_of(self);
+    return make<eqg_set>(g_set_class, rt, [&](eqg_set** o) { return rt->api.set_builtin(rt->h, which, o); });
+}
+PyObject* rt_all_cells(PyObject* self, PyObject*) { return builtin_set(self, EQG_ALL_CELLS); }
+PyObject* rt_boundary_cells(PyObject* self, PyObject*) { return builtin_set(self, EQG_BOUNDARY_CELLS); }
+PyObject* rt_interior_cells(PyObject* self, PyObject*) { return builtin_set(self, EQG_INTERIOR_CELLS); }
+PyObject* rt_all_faces(PyObject* self, PyObject*) { return builtin_set(self, EQG_ALL_FACES); }
+PyObject* rt_boundary_faces(PyObject* self, PyObject*) { return builtin_set(self, EQG_BOUNDARY_FACES); }
+PyObject* rt_interior_faces(PyObject* self, PyObject*) { return builtin_set(self, EQG_INTERIOR_FACES); }
+
+template <class Get>
+PyObject* set_method(METHOD_ARGS, const char* name, Get&& get)
+{
+    static const char* const names[] = {"faces"};
+    PyObject* v[1];
+    void* h;
+    if (!take(name, args, nargs, kwnames, names, 1, 1, v) || !handle_of(v[0], &h)) return nullptr;
+    RuntimeObject* rt = rt_of(self);
+    return make<eqg_set>(g_set_class, rt, [&](eqg_set** o) { return get(rt->api)(rt->h, (const eqg_set*)h, o); });
+}
+PyObject* rt_first_cell(METHOD_ARGS)
+{
+    return set_method(self, args, nargs, kwnames, "firstCell", [](const Api& a) { return a.first_cell; });
+}
+PyObject* rt_second_cell(METHOD_ARGS)
+{
+    return set_method(self, args, nargs, kwnames, "secondCell", [](const Api& a) { return a.second_cell; });
+}
+
+PyObject* constant_of(RuntimeObject* rt, PyObject* value, int64_t n)
+{
+    double s;
+    if (!double_of(value, &s)) return nullptr;
+    return make<eqg_coll>(g_coll_class, rt, [&](eqg_coll** o) { return rt->api.coll_constant(rt->h, s, n, o); });
+}
+
+// operatorExtend(data, a, b=None): a constant over a, or data from a to b.
+PyObject* rt_extend(METHOD_ARGS)
+{
+    static const char* const names[] = {"data", "a", "b"};
+    PyObject* v[3];
+    if (!take("operatorExtend", args, nargs, kwnames, names, 3, 2, v)) return nullptr;
+    RuntimeObject* rt = rt_of(self);
+    if (!v[2] || v[2] == Py_None) {
+        int64_t n = 0;
+        if (PyObject_TypeCheck(v[1], &SetBaseType)) {
+            HandleObject* s = (HandleObject*)v[1];
+            const int st = s->rt->api.set_size((eqg_set*)s->h, &n);
+            if (st != EQG_OK) return raise_status(s->rt->api, st);
+        } else {
+            n = PyObject_Size(v[1]);
+            if (n < 0) return nullptr;
+        }
+        return constant_of(rt, v[0], n);
+    }
+    void *d, *a, *b;
+    if (!handle_of(v[0], &d) || !handle_of(v[1], &a) || !handle_of(v[2], &b)) return nullptr;
+    const eqg_set *from = (eqg_set*)a, *to = (eqg_set*)b;
+    if (PyObject_TypeCheck(v[0], &SetBaseType))
+        return make<eqg_set>(g_set_class, rt,
+                             [&](eqg_set** o) { return rt->api.set_extend(rt->h, (eqg_set*)d, from, to, o); });
+    return make<eqg_coll>(g_coll_class, rt,
+                          [&](eqg_coll** o) { return rt->api.extend(rt->h, (eqg_coll*)d, from, to, o); });
+}
+
+PyObject* rt_on(METHOD_ARGS)
+{
+    static const char* const names[] = {"data", "from_set", "to_set"};
+    PyObject* v[3];
+    void *d, *a, *b;
+    if (!take("operatorOn", args, nargs, kwnames, names, 3, 3, v) || !handle_of(v[0], &d) || !handle_of(v[1], &a) ||
+        !handle_of(v[2], &b))
+        return nullptr;
+    RuntimeObject* rt = rt_of(self);
+    const eqg_set *from = (eqg_set*)a, *to = (eqg_set*)b;
+    if (PyObject_TypeCheck(v[0], &SetBaseType))
+        return make<eqg_set>(g_set_class, rt,
+                             [&](eqg_set** o) { return rt->api.set_on(rt->h, (eqg_set*)d, from, to, o); });
+    return make<eqg_coll>(g_coll_class, rt,
+                          [&](eqg_coll** o) { return rt->api.on(rt->h, (eqg_coll*)d, from, to, o); });
+}
+
+PyObject* rt_trinary_if(METHOD_ARGS)
+{
+    static const char* const names[] = {"pred", "a", "b"};
+    PyObject* v[3];
+    void *m, *a, *b;
+    if (!take("trinaryIf", args, nargs, kwnames, names, 3, 3, v) || !handle_of(v[0], &m) || !handle_of(v[1], &a) ||
+        !handle_of(v[2], &b))
+        return nullptr;
+    RuntimeObject* rt = rt_of(self);
+    const eqg_mask* p = (eqg_mask*)m;
+    if (PyObject_TypeCheck(v[1], &SetBaseType))
+        return make<eqg_set>(g_set_class, rt, [&](eqg_set** o) {
+            return rt->api.set_select(rt->h, p, (eqg_set*)a, (eqg_set*)b, o);
+        });
+    return make<eqg_coll>(g_coll_class, rt, [&](eqg_coll** o) {
+        return rt->api.select(rt->h, p, (eqg_coll*)a, (eqg_coll*)b, o);
+    });
+}
+
+PyObject* reduce_of(METHOD_ARGS, const char* name, int op)
+{
+    static const char* const names[] = {"x"};
+    PyObject* v[1];
+    void* h;
+    if (!take(name, args, nargs, kwnames, names, 1, 1, v) || !handle_of(v[0], &h)) return nullptr;
+    RuntimeObject* rt = rt_of(self);
+    double r = 0.0;
+    const int st = unlocked([&] {
+        return op < 0 ? rt->api.two_norm(rt->h, (eqg_coll*)h, &r) : rt->api.reduce(rt->h, op, (eqg_coll*)h, &r);
+    });
+    return st == EQG_OK ? PyFloat_FromDouble(r) : raise_status(rt->api, st);
+}
+PyObject* rt_min(METHOD_ARGS) { return reduce_of(self, args, nargs, kwnames, "minReduce", EQG_MIN); }
+PyObject* rt_max(METHOD_ARGS) { return reduce_of(self, args, nargs, kwnames, "maxReduce", EQG_MAX); }
+PyObject* rt_sum(METHOD_ARGS) { return reduce_of(self, args, nargs, kwnames, "sumReduce", EQG_SUM); }
+PyObject* rt_prod(METHOD_ARGS) { return reduce_of(self, args, nargs, kwnames, "prodReduce", EQG_PROD); }
+PyObject* rt_two_norm(METHOD_ARGS) { return reduce_of(self, args, nargs, kwnames, "twoNorm", -1); }
+
+// spanSubset(u, start, num), spanSuperset(u, start, total)
+PyObject* span_of(METHOD_ARGS, bool subset)
+{
+    static const char* const names[2][3] = {{"u", "start", "total"}, {"u", "start", "num"}};
+    PyObject* v[3];
+    void* h;
+    if (!take(subset ? "spanSubset" : "spanSuperset", args, nargs, kwnames, names[subset ? 1 : 0], 3, 3, v) ||
+        !handle_of(v[0], &h))
+        return nullptr;
+    int64_t n[2];
+    for (int i = 0; i < 2; ++i) {
+        PyObject* l = PyNumber_Long(v[i + 1]);  // as int(...)
+        if (!l) return nullptr;
+        n[i] = PyLong_AsLongLong(l);
+        Py_DECREF(l);
+        if (n[i] == -1 && PyErr_Occurred()) return nullptr;
+    }
+    RuntimeObject* rt = rt_of(self);
+    return make<eqg_coll>(g_coll_class, rt, [&](eqg_coll** o) {
+        return (subset ? rt->api.span_subset : rt->api.span_superset)(rt->h, (eqg_coll*)h, n[0], n[1], o);
+    });
+}
+PyObject* rt_span_subset(METHOD_ARGS) { return span_of(self, args, nargs, kwnames, true); }
+PyObject* rt_span_superset(METHOD_ARGS) { return span_of(self, args, nargs, kwnames, false); }
+
+// _bind({name: address}): the entry points of the runtime's library.
+PyObject* rt_bind(PyObject* self, PyObject* table)
+{
+    RuntimeObject* rt = rt_of(self);
+    for (const Entry& e : kEntries) {
+        PyObject* a = PyMapping_GetItemString(table, e.name);
+        if (!a) return nullptr;
+        void* p = PyLong_AsVoidPtr(a);
+        Py_DECREF(a);
+        if (!p) {
+            if (!PyErr_Occurred()) PyErr_Format(PyExc_ValueError, "no address of %s", e.name);
+            return nullptr;
+        }
+        std::memcpy((char*)&rt->api + e.offset, &p, sizeof(p));
+    }
+    rt->bound = true;
+    Py_RETURN_NONE;
+}
+
+PyObject* rt_get_h(PyObject* self, void*)
+{
+    eqg_runtime* h = rt_of(self)->h;
+    if (!h) Py_RETURN_NONE;
+    return PyLong_FromVoidPtr(h);
+}
+int rt_set_h(PyObject* self, PyObject* v, void*)
+{
+    void* p = nullptr;
+    if (v && v != Py_None) {
+        p = PyLong_AsVoidPtr(v);
+        if (!p && PyErr_Occurred()) return -1;
+    }
+    rt_of(self)->h = (eqg_runtime*)p;
+    return 0;
+}
+PyGetSetDef rt_getset[] = {{"h", rt_get_h, rt_set_h, nullptr, nullptr}, {nullptr, nullptr, nullptr, nullptr, nullptr}};
+
+#define FAST(f) (PyCFunction)(void (*)(void))(f), METH_FASTCALL | METH_KEYWORDS, nullptr
+PyMethodDef rt_methods[] = {{"_bind", rt_bind, METH_O, nullptr},
+                            {"gradient", FAST(rt_gradient)},
+                            {"negGradient", FAST(rt_neg_gradient)},
+                            {"divergence", FAST(rt_divergence)},
+                            {"interiorDivergence", FAST(rt_interior_divergence)},
+                            {"sqrt", FAST(rt_sqrt)},
+                            {"allCells", rt_all_cells, METH_NOARGS, nullptr},
+                            {"boundaryCells", rt_boundary_cells, METH_NOARGS, nullptr},
+                            {"interiorCells", rt_interior_cells, METH_NOARGS, nullptr},
+                            {"allFaces", rt_all_faces, METH_NOARGS, nullptr},
+                            {"boundaryFaces", rt_boundary_faces, METH_NOARGS, nullptr},
+                            {"interiorFaces", rt_interior_faces, METH_NOARGS, nullptr},
+                            {"firstCell", FAST(rt_first_cell)},
+                            {"secondCell", FAST(rt_second_cell)},
+                            {"operatorExtend", FAST(rt_extend)},
+                            {"operatorOn", FAST(rt_on)},
+                            {"trinaryIf", FAST(rt_trinary_if)},
+                            {"minReduce", FAST(rt_min)},
+                            {"maxReduce", FAST(rt_max)},
+                            {"sumReduce", FAST(rt_sum)},
+                            {"prodReduce", FAST(rt_prod)},
+                            {"twoNorm", FAST(rt_two_norm)},
+                            {"spanSubset", FAST(rt_span_subset)},
+                            {"spanSuperset", FAST(rt_span_superset)},
+                            {nullptr, nullptr, 0, nullptr}};
+
+PyTypeObject make_type(const char* name, size_t size)
+{
+    PyTypeObject t = {PyVarObject_HEAD_INIT(nullptr, 0)};
+    t.tp_name = name;
+    t.tp_basicsize = (Py_ssize_t)size;
+    t.tp_flags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_BASETYPE;
+    t.tp_new = PyType_GenericNew;
+    return t;
+}
+PyTypeObject RuntimeBaseType = make_type("equelle_b200._mirror.RuntimeBase", sizeof(RuntimeObject));
+PyTypeObject CollBaseType = make_type("equelle_b200._mirror.CollBase", sizeof(HandleObject));
+PyTypeObject MaskBaseType = make_type("equelle_b200._mirror.MaskBase", sizeof(HandleObject));
+PyTypeObject SetBaseType = make_type("equelle_b200._mirror.SetBase", sizeof(HandleObject));
+
+// register_classes(CollOfScalar, CollOfBool, EntitySet, EqgError)
+PyObject* register_classes(PyObject*, PyObject* args)
+{
+    PyObject *c, *m, *s, *e;
+    if (!PyArg_ParseTuple(args, "OOOO", &c, &m, &s, &e)) return nullptr;
+    if (!PyType_Check(c) || !PyType_IsSubtype((PyTypeObject*)c, &CollBaseType) || !PyType_Check(m) ||
+        !PyType_IsSubtype((PyTypeObject*)m, &MaskBaseType) || !PyType_Check(s) ||
+        !PyType_IsSubtype((PyTypeObject*)s, &SetBaseType)) {
+        PyErr_SetString(PyExc_TypeError, "the classes must derive from CollBase, MaskBase and SetBase");
+        return nullptr;
+    }
+    Py_XSETREF(g_coll_class, Py_NewRef(c));
+    Py_XSETREF(g_mask_class, Py_NewRef(m));
+    Py_XSETREF(g_set_class, Py_NewRef(s));
+    Py_XSETREF(g_error_class, Py_NewRef(e));
+    Py_RETURN_NONE;
+}
+
+// entry_points(): the names that RuntimeBase._bind needs addresses of.
+PyObject* entry_points(PyObject*, PyObject*)
+{
+    const Py_ssize_t n = sizeof(kEntries) / sizeof(kEntries[0]);
+    PyObject* t = PyTuple_New(n);
+    for (Py_ssize_t i = 0; t && i < n; ++i) {
+        PyObject* s = PyUnicode_FromString(kEntries[i].name);
+        if (!s) {
+            Py_DECREF(t);
+            return nullptr;
+        }
+        PyTuple_SET_ITEM(t, i, s);
+    }
+    return t;
+}
+
+PyMethodDef module_methods[] = {{"register_classes", register_classes, METH_VARARGS, nullptr},
+                                {"entry_points", entry_points, METH_NOARGS, nullptr},
+                                {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_mirror", nullptr, -1, module_methods,
+                          nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__mirror(void)
+{
+    RuntimeBaseType.tp_methods = rt_methods;
+    RuntimeBaseType.tp_getset = rt_getset;
+    coll_number.nb_add = coll_add;
+    coll_number.nb_subtract = coll_sub;
+    coll_number.nb_multiply = coll_mul;
+    coll_number.nb_true_divide = coll_div;
+    coll_number.nb_negative = coll_neg;
+    CollBaseType.tp_as_number = &coll_number;
+    CollBaseType.tp_richcompare = coll_richcompare;
+    CollBaseType.tp_hash = identity_hash;
+    CollBaseType.tp_methods = coll_methods;
+    CollBaseType.tp_dealloc = handle_dealloc<coll_clear>;
+    CollBaseType.tp_clear = coll_clear;
+    mask_number.nb_and = mask_and;
+    mask_number.nb_or = mask_or;
+    mask_number.nb_invert = mask_invert;
+    MaskBaseType.tp_as_number = &mask_number;
+    MaskBaseType.tp_dealloc = handle_dealloc<mask_clear>;
+    MaskBaseType.tp_clear = mask_clear;
+    SetBaseType.tp_dealloc = handle_dealloc<set_clear>;
+    SetBaseType.tp_clear = set_clear;
+    for (PyTypeObject* t : {&CollBaseType, &MaskBaseType, &SetBaseType}) {
+        t->tp_flags |= Py_TPFLAGS_HAVE_GC;
+        t->tp_traverse = handle_traverse;
+        t->tp_getset = handle_getset;
+        t->tp_init = handle_init;
+    }
+    PyObject* m = PyModule_Create(&module_def);
+    if (!m) return nullptr;
+    const struct {
+        const char* name;
+        PyTypeObject* type;
+    } types[] = {{"RuntimeBase", &RuntimeBaseType}, {"CollBase", &CollBaseType}, {"MaskBase", &MaskBaseType},
+                 {"SetBase", &SetBaseType}};
+    for (const auto& t : types) {
+        if (PyType_Ready(t.type) < 0 || PyModule_AddObjectRef(m, t.name, (PyObject*)t.type) < 0) {
+            Py_DECREF(m);
+            return nullptr;
+        }
+    }
+    return m;
+}

@@ -6,6 +6,10 @@ EquelleRuntimeCPU.hpp:35-134), so simulators and tests can be written in
 the generated style from Python.  Works with any library that exports the
 ABI of include/eqg.h: the device runtime (equelle_b200.load_library()) or
 the CPU oracle used by the tests.
+
+The handles' operators and the runtime methods of a program's time loop are
+native (csrc/mirror.cpp, built into the package as _mirror); what is here
+reads results back, makes collections from host arrays and runs the solves.
 """
 import ctypes as C
 
@@ -13,23 +17,17 @@ import numpy as np
 
 from . import capi
 
-
-class _Handle:
-    _release = None
-
-    def __init__(self, rt, h):
-        self.rt = rt
-        self.h = h
-
-    def __del__(self):
-        h, self.h = getattr(self, "h", None), None
-        if h:
-            getattr(self.rt.lib, self._release)(h)
+try:
+    from . import _mirror
+except ImportError:  # not built yet: a few seconds of the system compiler
+    from . import build
+    build.build_mirror()
+    from . import _mirror
 
 
-class EntitySet(_Handle):
+class EntitySet(_mirror.SetBase):
     """CollOfCell / CollOfFace."""
-    _release = "eqg_set_release"
+    __slots__ = ()
 
     def __len__(self):
         n = C.c_int64()
@@ -52,8 +50,9 @@ class EntitySet(_Handle):
         return out
 
 
-class CollOfBool(_Handle):
-    _release = "eqg_mask_release"
+class CollOfBool(_mirror.MaskBase):
+    """Masks; & | ~ are native."""
+    __slots__ = ()
 
     def __len__(self):
         n = C.c_int64()
@@ -66,22 +65,11 @@ class CollOfBool(_Handle):
             self.rt._ok(self.rt.lib.eqg_mask_to_host(self.h, out.ctypes.data_as(capi.c_u8_p)))
         return out.astype(bool)
 
-    def _logic(self, op, other):
-        return self.rt._mask(self.rt.lib.eqg_mask_logic, op, self.h, other.h if other is not None else None)
 
-    def __and__(self, o):
-        return self._logic(capi.AND, o)
-
-    def __or__(self, o):
-        return self._logic(capi.OR, o)
-
-    def __invert__(self):
-        return self._logic(capi.NOT, None)
-
-
-class CollOfScalar(_Handle):
-    """Value plus optional Jacobian (AutoDiffBlock<double>)."""
-    _release = "eqg_coll_release"
+class CollOfScalar(_mirror.CollBase):
+    """Value plus optional Jacobian (AutoDiffBlock<double>).  Arithmetic
+    (equelleTypes.hpp:86-211), negation, < <= > >= and eq(), ne() are native."""
+    __slots__ = ()
 
     def __len__(self):
         n = C.c_int64()
@@ -111,64 +99,8 @@ class CollOfScalar(_Handle):
             val.ctypes.data_as(capi.c_dbl_p)))
         return r.value, c.value, ptr, col[:nnz.value], val[:nnz.value]
 
-    # arithmetic (equelleTypes.hpp:86-211)
-    def _bin(self, op, other, reflected=False):
-        rt = self.rt
-        if isinstance(other, CollOfScalar):
-            a, b = (other, self) if reflected else (self, other)
-            return rt._coll(rt.lib.eqg_binary, op, a.h, b.h)
-        return rt._coll(rt.lib.eqg_binary_scalar, op, self.h, float(other), 1 if reflected else 0)
 
-    def __add__(self, o):
-        return self._bin(capi.ADD, o)
-
-    def __radd__(self, o):
-        return self._bin(capi.ADD, o, True)
-
-    def __sub__(self, o):
-        return self._bin(capi.SUB, o)
-
-    def __rsub__(self, o):
-        return self._bin(capi.SUB, o, True)
-
-    def __mul__(self, o):
-        return self._bin(capi.MUL, o)
-
-    def __rmul__(self, o):
-        return self._bin(capi.MUL, o, True)
-
-    def __truediv__(self, o):
-        return self._bin(capi.DIV, o)
-
-    def __rtruediv__(self, o):
-        return self._bin(capi.DIV, o, True)
-
-    def __neg__(self):
-        return self.rt._coll(self.rt.lib.eqg_unary, capi.NEG, self.h)
-
-    def _cmp(self, op, other):
-        rt = self.rt
-        if isinstance(other, CollOfScalar):
-            return rt._mask(rt.lib.eqg_compare, op, self.h, other.h)
-        return rt._mask(rt.lib.eqg_compare_scalar, op, self.h, float(other), 0)
-
-    def __lt__(self, o):
-        return self._cmp(capi.LT, o)
-
-    def __le__(self, o):
-        return self._cmp(capi.LE, o)
-
-    def __gt__(self, o):
-        return self._cmp(capi.GT, o)
-
-    def __ge__(self, o):
-        return self._cmp(capi.GE, o)
-
-    def eq(self, o):
-        return self._cmp(capi.EQ, o)
-
-    def ne(self, o):
-        return self._cmp(capi.NE, o)
+_mirror.register_classes(CollOfScalar, CollOfBool, EntitySet, capi.EqgError)
 
 
 class CollOfVector:
@@ -202,11 +134,21 @@ class CollOfVector:
         return CollOfVector(a / s for a in self.cols)
 
 
-class Runtime:
+def _addresses(lib):
+    """Entry point addresses of a bound library, looked up once per library."""
+    table = getattr(lib, "_eqg_addresses", None)
+    if table is None:
+        table = {n: C.cast(getattr(lib, n), C.c_void_p).value for n in _mirror.entry_points()}
+        lib._eqg_addresses = table
+    return table
+
+
+class Runtime(_mirror.RuntimeBase):
     """equelle::EquelleRuntimeCPU over a library exporting include/eqg.h."""
 
     def __init__(self, lib, params):
         self.lib = lib
+        self._bind(_addresses(lib))
         keys = [str(k).encode() for k in params]
         vals = [str(v).lower() if isinstance(v, bool) else str(v) for v in params.values()]
         vals = [v.encode() for v in vals]
@@ -221,7 +163,7 @@ class Runtime:
         self.dimensions = info.dimensions
 
     def __del__(self):
-        h, self.h = getattr(self, "h", None), None
+        h, self.h = self.h, None
         if h:
             self.lib.eqg_runtime_destroy(h)
 
@@ -262,31 +204,7 @@ class Runtime:
     def variable(self, init):
         return self._coll(self.lib.eqg_variable, init.h)
 
-    # -- topology --------------------------------------------------------
-    def allCells(self):
-        return self._set(self.lib.eqg_set_builtin, capi.ALL_CELLS)
-
-    def boundaryCells(self):
-        return self._set(self.lib.eqg_set_builtin, capi.BOUNDARY_CELLS)
-
-    def interiorCells(self):
-        return self._set(self.lib.eqg_set_builtin, capi.INTERIOR_CELLS)
-
-    def allFaces(self):
-        return self._set(self.lib.eqg_set_builtin, capi.ALL_FACES)
-
-    def boundaryFaces(self):
-        return self._set(self.lib.eqg_set_builtin, capi.BOUNDARY_FACES)
-
-    def interiorFaces(self):
-        return self._set(self.lib.eqg_set_builtin, capi.INTERIOR_FACES)
-
-    def firstCell(self, faces):
-        return self._set(self.lib.eqg_first_cell, faces.h)
-
-    def secondCell(self, faces):
-        return self._set(self.lib.eqg_second_cell, faces.h)
-
+    # -- topology (index sets, firstCell and secondCell are native) ----------
     def norm(self, x):
         if isinstance(x, EntitySet):
             return self._coll(self.lib.eqg_measure, x.h)
@@ -303,70 +221,16 @@ class Runtime:
     def normal(self, faces):
         return CollOfVector(self._coll(self.lib.eqg_normal, faces.h, d) for d in range(self.dimensions))
 
-    # -- math ------------------------------------------------------------
-    def sqrt(self, x):
-        return self._coll(self.lib.eqg_unary, capi.SQRT, x.h)
-
+    # -- math (gradient, divergence, On, Extend, trinaryIf, sqrt and the
+    # reductions are native) ----------------------------------------------
     def dot(self, v1, v2):
         r = v1.col(0) * v2.col(0)
         for d in range(1, self.dimensions):
             r = r + v1.col(d) * v2.col(d)
         return r
 
-    def gradient(self, x):
-        return self._coll(self.lib.eqg_gradient, x.h)
-
-    def negGradient(self, x):
-        return self._coll(self.lib.eqg_neg_gradient, x.h)
-
-    def divergence(self, x):
-        return self._coll(self.lib.eqg_divergence, x.h)
-
-    def interiorDivergence(self, x):
-        return self._coll(self.lib.eqg_interior_divergence, x.h)
-
     def isEmpty(self, s):
         return self._mask(self.lib.eqg_set_is_empty, s.h)
-
-    def operatorExtend(self, data, a, b=None):
-        if b is None:
-            return self.constant(data, len(a))
-        if isinstance(data, EntitySet):
-            return self._set(self.lib.eqg_set_extend, data.h, a.h, b.h)
-        return self._coll(self.lib.eqg_extend, data.h, a.h, b.h)
-
-    def operatorOn(self, data, from_set, to_set):
-        if isinstance(data, EntitySet):
-            return self._set(self.lib.eqg_set_on, data.h, from_set.h, to_set.h)
-        return self._coll(self.lib.eqg_on, data.h, from_set.h, to_set.h)
-
-    def trinaryIf(self, pred, a, b):
-        if isinstance(a, EntitySet):
-            return self._set(self.lib.eqg_set_select, pred.h, a.h, b.h)
-        return self._coll(self.lib.eqg_select, pred.h, a.h, b.h)
-
-    # -- reductions ------------------------------------------------------
-    def _reduce(self, op, x):
-        r = C.c_double()
-        self._ok(self.lib.eqg_reduce(self.h, op, x.h, C.byref(r)))
-        return r.value
-
-    def minReduce(self, x):
-        return self._reduce(capi.MIN, x)
-
-    def maxReduce(self, x):
-        return self._reduce(capi.MAX, x)
-
-    def sumReduce(self, x):
-        return self._reduce(capi.SUM, x)
-
-    def prodReduce(self, x):
-        return self._reduce(capi.PROD, x)
-
-    def twoNorm(self, x):
-        r = C.c_double()
-        self._ok(self.lib.eqg_two_norm(self.h, x.h, C.byref(r)))
-        return r.value
 
     # -- solvers ---------------------------------------------------------
     def newtonSolve(self, rescomp, u0):
@@ -397,11 +261,14 @@ class Runtime:
         start = np.concatenate([[0], np.cumsum(num)[:-1]]).astype(int)
         total = int(sum(num))
 
+        start = [int(v) for v in start]
+
+        # Opm::subset(u, ESpan(num, 1, start)) and its inverse, native
         def sub(u, i):
-            return self._coll(self.lib.eqg_span_subset, u.h, int(start[i]), int(num[i]))
+            return self.spanSubset(u, start[i], num[i])
 
         def sup(x, i):
-            return self._coll(self.lib.eqg_span_superset, x.h, int(start[i]), total)
+            return self.spanSuperset(x, start[i], total)
 
         def combined(u):
             parts = [sub(u, i) for i in range(len(num))]
@@ -416,14 +283,6 @@ class Runtime:
             u0 = u0 + sup(u0s[i], i)
         u = self.newtonSolve(combined, u0)
         return tuple(sub(u, i) for i in range(len(num)))
-
-    def spanSubset(self, u, start, num):
-        """Opm::subset(u, ESpan(num, 1, start))."""
-        return self._coll(self.lib.eqg_span_subset, u.h, int(start), int(num))
-
-    def spanSuperset(self, u, start, total):
-        """Opm::superset(u, ESpan(len(u), 1, start), total)."""
-        return self._coll(self.lib.eqg_span_superset, u.h, int(start), int(total))
 
     def solveForUpdate(self, residual):
         return self._coll(self.lib.eqg_solve_for_update, residual.h)
