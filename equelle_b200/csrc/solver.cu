@@ -2380,17 +2380,17 @@ constexpr int pc_mode()
 // (default 16, at most 16), reduced until the device reports that it can
 // schedule one cluster of that size.
 template <class Kernel>
-int tail_cluster_size(Core& c, Kernel kern)
+int tail_cluster_size(Core& c, Kernel kern, int smem)
 {
     int want = std::min(16, std::max(1, c.param_i("linsolver_mg_cluster", 16)));
     if (want > 8) EQG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    EQG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem));
+    EQG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     for (; want > 1; want /= 2) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
         cfg.gridDim = dim3(want);
         cfg.blockDim = dim3(kTailThreads);
-        cfg.dynamicSmemBytes = kTailSmem;
+        cfg.dynamicSmemBytes = smem;
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = want;
         attr[0].val.clusterDim.y = 1;
@@ -2533,7 +2533,7 @@ void prepare_tail(Core& c, SolverAnalysis& an)
     int& cl = an.tail_cluster[mode];
     const int bs = an.levels[an.tail_first].bs;
     int bytes = 0;
-    if (!cl) WITH_BS(bs, WITH_KMAX(an.tail_kmax, cl = tail_cluster_size(c, mg_tail_kernel<BS, KK, T, M>)));
+    if (!cl) WITH_BS(bs, WITH_KMAX(an.tail_kmax, cl = tail_cluster_size(c, mg_tail_kernel<BS, KK, T, M>, kTailSmem)));
     an.tail_local[mode] = plan_local<T, M>(c, an, bytes, nullptr);
     an.last_mode = mode;
 }
@@ -2648,14 +2648,21 @@ void report_tail_trace(Core& c, const SolverAnalysis& an)
     int l = an.tail_first;
     if (!an.rb.empty()) {
         auto name = [&](int k, const char* what) { names.push_back("L" + std::to_string(k) + "." + what); };
-        for (; l < lf && l < last; ++l) {
+        const int local = c.param_i("linsolver_mg_local", 1) ? kRbSoloCells : 0;
+        int solo = last;
+        while (solo > an.tail_first && an.rb[solo - 1].g.n <= local) --solo;
+        name(l, "load");
+        for (; l < solo; ++l) {
             if (an.rb[l].pre) {
                 name(l, "pre");
                 name(l, "y");
+                name(l, "residual");
             }
-            name(l, an.rb[l].pre ? "residual" : "restrict");
+            name(l, "restrict");
         }
-        name(l, l == lf ? "shared" : "dense");
+        if (solo < last) name(solo, "solo down");
+        name(last, "dense");
+        if (solo < last && solo > an.tail_first) name(solo, "solo up");
         for (--l; l >= an.tail_first; --l) {
             name(l, "y");
             if (l == 0) break;
@@ -2919,7 +2926,7 @@ void autotune(Core& c, SolverAnalysis& an, Apply&& apply)
     if (an.rb.empty()) collect(an.levels);
     else collect(an.rb);
     key << "; fused from " << an.tail_first << "; precision " << mode;
-    if (!an.rb.empty()) key << "; two colours";
+    if (!an.rb.empty()) key << "; two colours, resident";
     std::string file = c.param_s("linsolver_tune_file", "");
     if (file.empty() && std::getenv("EQG_TUNE_FILE")) file = std::getenv("EQG_TUNE_FILE");
     {
@@ -2931,7 +2938,8 @@ void autotune(Core& c, SolverAnalysis& an, Apply&& apply)
         auto it = g_tune_cache.find(key.str());
         if (it != g_tune_cache.end() && it->second.threads.size() == lv.size()) {
             for (size_t i = 0; i < lv.size(); ++i) *lv[i] = it->second.threads[i];
-            if (an.tail_first >= 0 && it->second.cluster > 0 && it->second.cluster <= an.tail_cluster[mode])
+            if (an.rb.empty() && an.tail_first >= 0 && it->second.cluster > 0 &&
+                it->second.cluster <= an.tail_cluster[mode])
                 an.tail_cluster[mode] = it->second.cluster;
             return;
         }
@@ -2972,7 +2980,7 @@ void autotune(Core& c, SolverAnalysis& an, Apply&& apply)
         *threads = best_t;
     }
     int& cl = an.tail_cluster[mode];
-    if (an.tail_first >= 0 && cl > 1) {
+    if (an.rb.empty() && an.tail_first >= 0 && cl > 1) {
         const int top = cl;
         int best_c = cl;
         for (int cand : {top / 2, top / 4}) {

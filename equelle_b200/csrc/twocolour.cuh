@@ -22,7 +22,7 @@
 // is one sweep from any z_b: the red part of the iterate is never needed
 // before the last line, the residual of the down-leg is summed straight into
 // the coarse right-hand side (rb_res_rows), and the coarse level's last two
-// steps add alpha times their rows to the fine black cells (scatter_up).  A
+// steps add alpha times their rows to the fine black cells (UpRow).  A
 // level with pre-smoothing (Level::pre) takes six half products of its
 // factors, one without three; level 0 needs no red rows at all.
 //
@@ -144,7 +144,7 @@ struct RbMatrix {
 // the first sum (with a branch per neighbour the compiler waited for each one
 // in turn, in 34 registers): the block of a missing neighbour is stored as
 // zero, and the vector is then read at the row's own number, or the last one.
-template <int B, int ND, class M, bool CG>
+template <int B, int ND, class M>
 __device__ __forceinline__ void stencil_dot(const RbGrid& g, const Cell& e, int q, int rows, const M* __restrict__ a,
                                             const double* __restrict__ x, double (&acc)[B])
 {
@@ -157,7 +157,7 @@ __device__ __forceinline__ void stencil_dot(const RbGrid& g, const Cell& e, int 
         int nq;
         if (!neighbour(g, e, d, nq)) nq = own;
         load_block<BB, M>(a + ((size_t)d * rows + q) * BB, av[d]);
-        load_bvec<B, double, CG>(x, nq, xv[d]);
+        load_bvec<B, double>(x, nq, xv[d]);
     }
 #pragma unroll
     for (int d = 0; d < ND; ++d)
@@ -219,62 +219,67 @@ struct UpView {
     double* w = nullptr;  // null: no finer level
 };
 
-template <int B, bool CG>
-__device__ __forceinline__ void scatter_up(const UpView& u, const Cell& e, const double (&z)[B])
-{
-    if (u.w == nullptr) return;
-    // at most four members; all are read before the first is written
+// The fine members of one row (at most four) and their values, read before
+// the row is computed.
+template <int B>
+struct UpRow {
     int c[4];
     double f[4][B];
+    template <bool CG>
+    __device__ __forceinline__ void load(const UpView& u, const Cell& e)
+    {
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-        c[s] = s < u.agg.g ? black_member(u.agg, e.i, e.j, e.k, s) : -1;
+        for (int s = 0; s < 4; ++s) {
+            c[s] = u.w != nullptr && s < u.agg.g ? black_member(u.agg, e.i, e.j, e.k, s) : -1;
 #pragma unroll
-        for (int t = 0; t < B; ++t) f[s][t] = 0.0;
-        if (u.add && c[s] >= 0) load_bvec<B, double, CG>(u.w, c[s] >> 1, f[s]);
+            for (int t = 0; t < B; ++t) f[s][t] = 0.0;
+            if (u.add && c[s] >= 0) load_bvec<B, double, CG>(u.w, c[s] >> 1, f[s]);
+        }
     }
+    __device__ __forceinline__ void store(const UpView& u, const double (&z)[B])
+    {
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
+        for (int s = 0; s < 4; ++s) {
 #pragma unroll
-        for (int t = 0; t < B; ++t) f[s][t] = __fma_rn(u.alpha, z[t], f[s][t]);
-        if (c[s] >= 0) store_bvec<B, double>(u.w, c[s] >> 1, f[s]);
+            for (int t = 0; t < B; ++t) f[s][t] = __fma_rn(u.alpha, z[t], f[s][t]);
+            if (c[s] >= 0) store_bvec<B, double>(u.w, c[s] >> 1, f[s]);
+        }
     }
-}
+};
 
 // ---- the steps ------------------------------------------------------------------
-// Loops over the rows of a colour for thread `tid` of `nth`, shared by the
-// one-step kernels and the fused coarse cycle (see mg_tail_kernel), so that
-// both compute every element alike (operations written out: the compiler
-// contracted products and sums differently in the shared-memory cycle).  rr, y: red vectors (rr null: zero), rb,
+// Loops over the rows of a colour for thread `tid` of `nth`.  The resident
+// coarse cycle below computes every element alike (operations written out:
+// the compiler contracted products and sums differently there).  rr, y: red vectors (rr null: zero), rb,
 // z: black ones.
 
-template <int B, int ND, class M, bool CG>
+template <int B, int ND, class M>
 __device__ __forceinline__ void red_row(const RbGrid& g, const Cell& e, int q, const M* U, const double* rr,
                                         const double* z, double (&v)[B])
 {
     double acc[B];
 #pragma unroll
     for (int t = 0; t < B; ++t) acc[t] = v[t] = 0.0;
-    if (rr) load_bvec<B, double, CG>(rr, q, v);
-    stencil_dot<B, ND, M, CG>(g, e, q, g.nr, U, z, acc);
+    if (rr) load_bvec<B, double>(rr, q, v);
+    stencil_dot<B, ND, M>(g, e, q, g.nr, U, z, acc);
 #pragma unroll
     for (int t = 0; t < B; ++t) v[t] = __dsub_rn(v[t], acc[t]);
 }
 
 // y = rr - U z
-template <int B, int ND, class M, bool CG>
+template <int B, int ND, class M>
 __device__ __forceinline__ void rb_y_rows(const RbGrid& g, const RbMatrix<const M>& m, const double* rr,
                                           const double* z, double* y, int tid, int nth)
 {
     for (int q = tid; q < g.nr; q += nth) {
         double v[B];
-        red_row<B, ND, M, CG>(g, cell_of(g, 0, q), q, m.U, rr, z, v);
+        red_row<B, ND, M>(g, cell_of(g, 0, q), q, m.U, rr, z, v);
         store_bvec<B, double>(y, q, v);
     }
 }
 
 // D_r^-1 (rr - U z), handed to the finer level (nothing else reads it).
-template <int B, int ND, class M, bool CG>
+template <int B, int ND, class M>
 __device__ __forceinline__ void rb_fin_rows(const RbGrid& g, const RbMatrix<const M>& m, const double* rr,
                                             const double* z, const UpView& up, int tid, int nth)
 {
@@ -282,15 +287,17 @@ __device__ __forceinline__ void rb_fin_rows(const RbGrid& g, const RbMatrix<cons
         const Cell e = cell_of(g, 0, q);
         M dv[B * B];
         double v[B], x[B];
+        UpRow<B> fine;
+        fine.template load<false>(up, e);
         load_block<B * B, M>(m.dr + (size_t)q * B * B, dv);
-        red_row<B, ND, M, CG>(g, e, q, m.U, rr, z, v);
+        red_row<B, ND, M>(g, e, q, m.U, rr, z, v);
         block_mul<B, M>(dv, v, x);
-        scatter_up<B, CG>(up, e, x);
+        fine.store(up, x);
     }
 }
 
 // z = D_b^-1 (rb - L rr): the sweep from z = 0.
-template <int B, int ND, class M, bool CG>
+template <int B, int ND, class M>
 __device__ __forceinline__ void rb_pre_rows(const RbGrid& g, const RbMatrix<const M>& m, const double* rr,
                                             const double* rb, double* z, int tid, int nth)
 {
@@ -300,9 +307,9 @@ __device__ __forceinline__ void rb_pre_rows(const RbGrid& g, const RbMatrix<cons
         double acc[B], v[B], x[B];
 #pragma unroll
         for (int t = 0; t < B; ++t) acc[t] = 0.0;
-        load_bvec<B, double, CG>(rb, q, v);
+        load_bvec<B, double>(rb, q, v);
         load_block<B * B, M>(m.db + (size_t)q * B * B, dv);
-        if (rr) stencil_dot<B, ND, M, CG>(g, cell_of(g, 1, q), q, nk, m.L, rr, acc);
+        if (rr) stencil_dot<B, ND, M>(g, cell_of(g, 1, q), q, nk, m.L, rr, acc);
 #pragma unroll
         for (int t = 0; t < B; ++t) v[t] = __dsub_rn(v[t], acc[t]);
         block_mul<B, M>(dv, v, x);
@@ -311,7 +318,7 @@ __device__ __forceinline__ void rb_pre_rows(const RbGrid& g, const RbMatrix<cons
 }
 
 // t = rb - A_bb z - L y of one black row.
-template <int B, int ND, class M, bool CG>
+template <int B, int ND, class M>
 __device__ __forceinline__ void residual_row(const RbGrid& g, const Cell& e, int q, const RbMatrix<const M>& m,
                                              const double* rb, const double* y, const double (&z)[B], double (&t)[B])
 {
@@ -319,9 +326,9 @@ __device__ __forceinline__ void residual_row(const RbGrid& g, const Cell& e, int
     double acc[B], az[B];
 #pragma unroll
     for (int c = 0; c < B; ++c) acc[c] = 0.0;
-    load_bvec<B, double, CG>(rb, q, t);
+    load_bvec<B, double>(rb, q, t);
     load_block<B * B, M>(m.abb + (size_t)q * B * B, av);
-    stencil_dot<B, ND, M, CG>(g, e, q, g.n - g.nr, m.L, y, acc);
+    stencil_dot<B, ND, M>(g, e, q, g.n - g.nr, m.L, y, acc);
     block_mul<B, M>(av, z, az);
 #pragma unroll
     for (int c = 0; c < B; ++c) t[c] = __dsub_rn(__dsub_rn(t[c], az[c]), acc[c]);
@@ -331,7 +338,7 @@ __device__ __forceinline__ void residual_row(const RbGrid& g, const Cell& e, int
 // aggregate, g lanes per aggregate in the order of the coarse cells (a
 // member's row follows its neighbour's: whole segments), summed by a
 // butterfly over the g lanes.  rc: red coarse cells, then black ones.
-template <int B, int ND, class M, bool CG>
+template <int B, int ND, class M>
 __device__ __forceinline__ void rb_res_rows(const Aggregates& a, const RbMatrix<const M>& m, const double* rb,
                                             const double* y, const double* z, double* rc, int tid, int nth)
 {
@@ -345,8 +352,8 @@ __device__ __forceinline__ void rb_res_rows(const Aggregates& a, const RbMatrix<
         if (c >= 0) {
             const int q = c >> 1;
             double zv[B];
-            load_bvec<B, double, CG>(z, q, zv);
-            residual_row<B, ND, M, CG>(a.fine, cell_at(a.fine, c), q, m, rb, y, zv, t);
+            load_bvec<B, double>(z, q, zv);
+            residual_row<B, ND, M>(a.fine, cell_at(a.fine, c), q, m, rb, y, zv, t);
         }
         for (int o = 1; o < a.g; o <<= 1)
 #pragma unroll
@@ -358,7 +365,7 @@ __device__ __forceinline__ void rb_res_rows(const Aggregates& a, const RbMatrix<
 
 // The same of the right-hand side itself (rr null: zero), for a level
 // without pre-smoothing: pairs, a black member and the red one beside it.
-template <int B, bool CG>
+template <int B>
 __device__ __forceinline__ void rb_restrict_rows(const Aggregates& a, const double* rr, const double* rb, double* rc,
                                                  int tid, int nth)
 {
@@ -374,7 +381,7 @@ __device__ __forceinline__ void rb_restrict_rows(const Aggregates& a, const doub
             const double* r = ((i + j + k) & 1) ? rb : rr;
             if (!r) continue;
             double v[B];
-            load_bvec<B, double, CG>(r, (i + a.fine.nx * (j + a.fine.ny * k)) >> 1, v);
+            load_bvec<B, double>(r, (i + a.fine.nx * (j + a.fine.ny * k)) >> 1, v);
 #pragma unroll
             for (int t = 0; t < B; ++t) s[t] += v[t];
         }
@@ -383,7 +390,7 @@ __device__ __forceinline__ void rb_restrict_rows(const Aggregates& a, const doub
 }
 
 // z += D_b^-1 (rb - A_bb z - L y), handed to the finer level.
-template <int B, int ND, class M, bool CG>
+template <int B, int ND, class M>
 __device__ __forceinline__ void rb_post_rows(const RbGrid& g, const RbMatrix<const M>& m, const double* rb,
                                              const double* y, double* z, const UpView& up, int tid, int nth)
 {
@@ -392,27 +399,29 @@ __device__ __forceinline__ void rb_post_rows(const RbGrid& g, const RbMatrix<con
         const Cell e = cell_of(g, 1, q);
         M dv[B * B];
         double zv[B], t[B], x[B];
-        load_bvec<B, double, CG>(z, q, zv);
+        UpRow<B> fine;
+        fine.template load<false>(up, e);
+        load_bvec<B, double>(z, q, zv);
         load_block<B * B, M>(m.db + (size_t)q * B * B, dv);
-        residual_row<B, ND, M, CG>(g, e, q, m, rb, y, zv, t);
+        residual_row<B, ND, M>(g, e, q, m, rb, y, zv, t);
         block_mul<B, M>(dv, t, x);
 #pragma unroll
         for (int c = 0; c < B; ++c) zv[c] = __dadd_rn(zv[c], x[c]);
         store_bvec<B, double>(z, q, zv);
-        scatter_up<B, CG>(up, e, zv);
+        fine.store(up, zv);
     }
 }
 
 // The coarsest level: inv r, a warp per unknown (see dense_rows; red cells,
 // then black ones), handed to the finer level.
-template <int B, class M, bool CG>
+template <int B, class M>
 __device__ __forceinline__ void rb_dense_rows(const RbGrid& g, const M* __restrict__ inv, const double* r,
                                               const UpView& up, int tid, int nth)
 {
     const int lane = tid & 31, n = g.n * B;
     for (int i = tid >> 5; i < n; i += nth >> 5) {
         double s = 0.0;
-        for (int j = lane; j < n; j += 32) s = __fma_rn((double)inv[i * n + j], CG ? __ldcg(r + j) : r[j], s);
+        for (int j = lane; j < n; j += 32) s = __fma_rn((double)inv[i * n + j], r[j], s);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         const int P = i / B, c = i - P * B;
@@ -421,7 +430,7 @@ __device__ __forceinline__ void rb_dense_rows(const RbGrid& g, const M* __restri
             const int f = black_member(up.agg, e.i, e.j, e.k, lane);
             if (f >= 0) {
                 double* w = up.w + (size_t)(f >> 1) * B + c;
-                *w = __fma_rn(up.alpha, s, up.add ? (CG ? __ldcg(w) : *w) : 0.0);
+                *w = __fma_rn(up.alpha, s, up.add ? *w : 0.0);
             }
         }
     }
@@ -435,7 +444,7 @@ __global__ void __launch_bounds__(512, 1) rb_y_kernel(RbGrid g, RbMatrix<const M
     pdl_wait();
     if (mg_skip(sc, skip_if_s)) return;
     THREAD_RANGE;
-    rb_y_rows<B, ND, M, false>(g, m, rr, z, y, tid, nth);
+    rb_y_rows<B, ND, M>(g, m, rr, z, y, tid, nth);
 }
 
 template <int B, int ND, class M>
@@ -445,7 +454,7 @@ __global__ void __launch_bounds__(512, 1) rb_fin_kernel(RbGrid g, RbMatrix<const
     pdl_wait();
     if (mg_skip(sc, skip_if_s)) return;
     THREAD_RANGE;
-    rb_fin_rows<B, ND, M, false>(g, m, rr, z, up, tid, nth);
+    rb_fin_rows<B, ND, M>(g, m, rr, z, up, tid, nth);
 }
 
 template <int B, int ND, class M>
@@ -455,7 +464,7 @@ __global__ void __launch_bounds__(512, 1) rb_pre_kernel(RbGrid g, RbMatrix<const
     pdl_wait();
     if (mg_skip(sc, skip_if_s)) return;
     THREAD_RANGE;
-    rb_pre_rows<B, ND, M, false>(g, m, rr, rb, z, tid, nth);
+    rb_pre_rows<B, ND, M>(g, m, rr, rb, z, tid, nth);
 }
 
 template <int B, int ND, class M>
@@ -466,7 +475,7 @@ __global__ void __launch_bounds__(512, 1) rb_res_kernel(Aggregates a, RbMatrix<c
     pdl_wait();
     if (mg_skip(sc, skip_if_s)) return;
     THREAD_RANGE;
-    rb_res_rows<B, ND, M, false>(a, m, rb, y, z, rc, tid, nth);
+    rb_res_rows<B, ND, M>(a, m, rb, y, z, rc, tid, nth);
 }
 
 template <int B>
@@ -476,7 +485,7 @@ __global__ void __launch_bounds__(512, 1) rb_restrict_kernel(Aggregates a, const
     pdl_wait();
     if (mg_skip(sc, skip_if_s)) return;
     THREAD_RANGE;
-    rb_restrict_rows<B, false>(a, rr, rb, rc, tid, nth);
+    rb_restrict_rows<B>(a, rr, rb, rc, tid, nth);
 }
 
 template <int B, int ND, class M>
@@ -486,7 +495,7 @@ __global__ void __launch_bounds__(512, 1) rb_post_kernel(RbGrid g, RbMatrix<cons
     pdl_wait();
     if (mg_skip(sc, skip_if_s)) return;
     THREAD_RANGE;
-    rb_post_rows<B, ND, M, false>(g, m, rb, y, z, up, tid, nth);
+    rb_post_rows<B, ND, M>(g, m, rb, y, z, up, tid, nth);
 }
 
 template <int B, class M>
@@ -495,7 +504,7 @@ __global__ void __launch_bounds__(1024) rb_dense_kernel(RbGrid g, const M* __res
 {
     pdl_wait();
     if (mg_skip(sc, skip_if_s)) return;
-    rb_dense_rows<B, M, false>(g, inv, r, up, (int)threadIdx.x, (int)blockDim.x);
+    rb_dense_rows<B, M>(g, inv, r, up, (int)threadIdx.x, (int)blockDim.x);
 }
 
 // ---- BiCGStab on the black half ------------------------------------------------
@@ -538,7 +547,7 @@ __global__ void __launch_bounds__(kThreads) rb_init_kernel(RbGrid g, RbMatrix<co
         double acc[B];
 #pragma unroll
         for (int t = 0; t < B; ++t) acc[t] = 0.0;
-        stencil_dot<B, ND, double, false>(g, cell_of(g, 1, q), q, nk, m.L, b, acc);
+        stencil_dot<B, ND, double>(g, cell_of(g, 1, q), q, nk, m.L, b, acc);
         load_bvec<B, double>(bb, q, w);
 #pragma unroll
         for (int t = 0; t < B; ++t) {
@@ -594,7 +603,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         load_bvec<B, double>(z, q, zv);
         load_bvec<B, double>(h, q, hv);
         load_block<B * B, double>(m.abb + (size_t)q * B * B, av);
-        stencil_dot<B, ND, double, false>(g, cell_of(g, 1, q), q, nk, m.L, y, acc);
+        stencil_dot<B, ND, double>(g, cell_of(g, 1, q), q, nk, m.L, y, acc);
         block_mul<B, double>(av, zv, az);
 #pragma unroll
         for (int t = 0; t < B; ++t) acc[t] += az[t];
@@ -634,7 +643,7 @@ __global__ void __launch_bounds__(kThreads) rb_solution_kernel(RbGrid g, RbMatri
         double v[B], z[B];
         double dv[B * B];
         load_block<B * B, double>(m.dr + (size_t)q * B * B, dv);
-        red_row<B, ND, double, false>(g, e, q, m.U, b, x, v);
+        red_row<B, ND, double>(g, e, q, m.U, b, x, v);
         block_mul<B, double>(dv, v, z);
 #pragma unroll
         for (int t = 0; t < B; ++t) out[(size_t)t * g.n + e.c] = z[t];
@@ -883,99 +892,385 @@ __global__ void rb_dense_fill_kernel(RbGrid g, int B, int nd, const double* __re
 }
 
 // ---- the coarse end of the cycle in one kernel ----------------------------------
-// As mg_tail_kernel: one thread-block cluster, a cluster barrier between the
-// steps, the coarsest levels in block 0's shared memory.
+// The levels from one down to the dense solve and back, resident in the shared
+// memory of one thread-block cluster: every block holds the matrix rows and
+// the vector entries of its share of each level's cells, neighbours' values are
+// read from the other blocks' shared memory, and a cluster barrier ends a step.
+// A step through global memory was two or three round trips to L2 of some
+// 1000 cycles each and a barrier that waits for the stores to reach it: 2.4k
+// to 9k cycles; from distributed shared memory 1.2k to 2.5k, most of it index
+// arithmetic and FP64 latency.  (Every step has one call site: inlined once more
+// for the first level, its code was fetched anew and took 8k to 10k.)  The cycle
+// from the 32x32x4 level of two-phase 128x128x64: 33 -> 19 us, from the 64x64
+// level of 512x512 22 us.  The smallest levels
+// are block 0's alone (solo), with block barriers; the dense solve's rows are
+// shared out again.  The matrices are copied in at every launch, before the
+// wait for the previous kernel.  Products and sums are those of the one-step
+// kernels, in their order; where those add alpha zc to the finer level's z
+// (UpRow), the finer level here reads both (z0_at): the same bits.
+constexpr int kRbTailSmem = 220 * 1024;
+constexpr int kRbSoloCells = 256;  // a level of at most these cells is block 0's
+
 template <class M>
 struct RbTailLevel {
     RbGrid g;
     int coarsest = 0, pre = 1;
-    const M* a = nullptr;           // matrix (RbMatrix), or the dense inverse of the coarsest level
-    const double* rr = nullptr;     // right-hand side, red (null: zero) and black
-    const double* rb = nullptr;
-    double* r = nullptr;            // where the finer level's restriction writes it
-    double* z = nullptr;            // black iterate
-    double* y = nullptr;            // red work vector
-    Aggregates agg;                 // to the next level
-    UpView up;                      // where its rows go
-    int so_a = 0, so_r = 0, so_w = 0;  // offsets in block 0's shared memory
+    int rows = 0;     // rows of a colour that a block holds
+    FastDiv by_rows;  // the block of a row
+    double alpha = 1.0;
+    const M* a = nullptr;  // matrix (RbMatrix), or the dense inverse of the coarsest level
+    Aggregates agg;        // to the next level
+    int so_m = 0, so_v = 0, vec = 0;  // shared memory: matrix, vectors and a vector's bytes
+    int so_r = 0;                     // coarsest level: a copy of its right-hand side
 };
 
 template <class M>
 struct RbTailParams {
     RbTailLevel<M> lv[kMaxTail];
     int nlev = 0;
-    int local_first = kMaxTail;
-    int nregions = 0;
-    int ncopies = 0;
-    PrefetchRegion reg[kMaxTail];
-    TailCopy copies[kMaxTail];
+    int solo_first = 0;                    // first level that is block 0's (nlev - 1: none)
+    const double *rr = nullptr, *rb = nullptr;  // the first level's right-hand side
+    double* z = nullptr;                   // where its black rows go when it is level 0
+    UpView up;                             // where its rows go otherwise
     long long* trace = nullptr;
 };
 static_assert(sizeof(RbTailParams<double>) <= 4096, "fused cycle parameters exceed 4 KB");
 
-// One level's steps down to the coarse right-hand side rc; sync() ends a step.
-template <int B, int ND, class M, bool CG, class Sync>
-__device__ __forceinline__ void rb_down(const RbTailLevel<M>& L, const RbMatrix<const M>& m, const double* rr,
-                                        const double* rb, double* z, double* y, double* rc, int tid, int nth,
-                                        Sync&& sync)
+// A vector over the rows of a colour, spread over the cluster's blocks.
+struct RbVec {
+    unsigned base;  // shared memory address in every block
+    int rows;
+    FastDiv by;
+};
+
+__device__ __forceinline__ unsigned remote(const RbVec& v, int q, int bytes)
 {
-    if (L.pre) {
-        rb_pre_rows<B, ND, M, CG>(L.g, m, rr, rb, z, tid, nth);
-        sync();
-        rb_y_rows<B, ND, M, CG>(L.g, m, rr, z, y, tid, nth);
-        sync();
-        rb_res_rows<B, ND, M, CG>(L.agg, m, rb, y, z, rc, tid, nth);
+    const int owner = v.by(q);
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(v.base + (unsigned)((q - owner * v.rows) * bytes)), "r"(owner));
+    return a;
+}
+
+template <int B>
+__device__ __forceinline__ void load_vec(const RbVec& v, int q, double (&x)[B])
+{
+    const unsigned a = remote(v, q, 8 * B);
+    if constexpr (B == 2) {
+        asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(x[0]), "=d"(x[1]) : "r"(a) : "memory");
     } else {
-        rb_restrict_rows<B, CG>(L.agg, rr, rb, rc, tid, nth);
+#pragma unroll
+        for (int t = 0; t < B; ++t)
+            asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(x[t]) : "r"(a + 8 * t) : "memory");
+    }
+}
+
+template <int B>
+__device__ __forceinline__ void store_vec(const RbVec& v, int q, const double (&x)[B])
+{
+    const unsigned a = remote(v, q, 8 * B);
+#pragma unroll
+    for (int t = 0; t < B; ++t)
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a + 8 * t), "d"(x[t]) : "memory");
+}
+
+// A level as a block sees it.
+template <int B, int ND, class M>
+struct RbTailView {
+    static constexpr int BB = B * B;
+    const RbTailLevel<M>& L;
+    const M *U, *Lo, *dr, *abb, *db;  // this block's rows
+    RbVec rr, rb, y, z, t;
+    int lo;  // this block's first row of a colour
+    __device__ __forceinline__ RbTailView(const RbTailLevel<M>& level, unsigned char* sm, int rank) : L(level)
+    {
+        U = reinterpret_cast<const M*>(sm + L.so_m);
+        Lo = U + (size_t)ND * L.rows * BB;
+        dr = Lo + (size_t)ND * L.rows * BB;
+        abb = dr + (size_t)L.rows * BB;
+        db = abb + (size_t)L.rows * BB;
+        const unsigned v = (unsigned)__cvta_generic_to_shared(sm + L.so_v);
+        rr = RbVec{v, L.rows, L.by_rows};
+        rb = RbVec{v + L.vec, L.rows, L.by_rows};
+        y = RbVec{v + 2 * L.vec, L.rows, L.by_rows};
+        z = RbVec{v + 3 * L.vec, L.rows, L.by_rows};
+        t = RbVec{v + 4 * L.vec, L.rows, L.by_rows};
+        lo = rank * L.rows;
+    }
+    __device__ __forceinline__ int hi(int colour) const
+    {
+        return min(lo + L.rows, colour ? L.g.n - L.g.nr : L.g.nr);
+    }
+};
+
+// stencil_dot over a block's rows, the neighbours' values from get(neighbour's
+// cell, its number, value).
+template <int B, int ND, class M, class Get>
+__device__ __forceinline__ void tail_dot(const RbGrid& g, const Cell& e, int q, int others, const M* a, int rows, int ql,
+                                         Get&& get, double (&acc)[B])
+{
+    constexpr int BB = B * B;
+    M av[ND][BB];
+    double xv[ND][B];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+        int nq;
+        Cell f = e;
+        if (neighbour(g, e, d, nq)) {
+            const int s = d & 1 ? 1 : -1;
+            if (d < 2) f.i += s;
+            else if (d < 4) f.j += s;
+            else f.k += s;
+        } else {
+            nq = min(q, others - 1);  // a zero block
+        }
+        load_block<BB, M>(a + ((size_t)d * rows + ql) * BB, av[d]);
+        get(f, nq, xv[d]);
+    }
+#pragma unroll
+    for (int d = 0; d < ND; ++d)
+#pragma unroll
+        for (int i = 0; i < B; ++i)
+#pragma unroll
+            for (int j = 0; j < B; ++j) acc[i] = __fma_rn((double)av[d][i * B + j], xv[d][j], acc[i]);
+}
+
+// z + alpha zc of a black cell (z taken as zero without pre-smoothing): the
+// iterate after the coarse correction.
+template <int B, int ND, class M>
+__device__ __forceinline__ void z0_at(const RbTailView<B, ND, M>& V, const RbTailView<B, ND, M>& C, const Cell& f, int q,
+                                      double (&x)[B])
+{
+    const Aggregates& a = V.L.agg;
+    const int ci = f.i >> a.sx, cj = f.j >> a.sy, ck = f.k >> a.sz;
+    const int P = ci + a.coarse.nx * (cj + a.coarse.ny * ck);
+    double zc[B];
+    load_vec<B>(((ci + cj + ck) & 1) ? C.z : C.y, P >> 1, zc);
+#pragma unroll
+    for (int t = 0; t < B; ++t) x[t] = 0.0;
+    if (V.L.pre) load_vec<B>(V.z, q, x);
+#pragma unroll
+    for (int t = 0; t < B; ++t) x[t] = __fma_rn(V.L.alpha, zc[t], x[t]);
+}
+
+// One level's steps down to the coarse right-hand side; sync() ends a step.
+template <int B, int ND, class M, class Sync>
+__device__ __forceinline__ void tail_down(const RbTailView<B, ND, M>& V, const RbTailView<B, ND, M>& C, bool has_red,
+                                          int tid, int nth, Sync&& sync)
+{
+    constexpr int BB = B * B;
+    const RbTailLevel<M>& L = V.L;
+    const RbGrid& g = L.g;
+    const int nk = g.n - g.nr;
+    if (L.pre) {
+        for (int q = V.lo + tid; q < V.hi(1); q += nth) {  // rb_pre_rows
+            const int ql = q - V.lo;
+            M dv[BB];
+            double acc[B], v[B], x[B];
+#pragma unroll
+            for (int t = 0; t < B; ++t) acc[t] = 0.0;
+            load_vec<B>(V.rb, q, v);
+            load_block<BB, M>(V.db + (size_t)ql * BB, dv);
+            if (has_red)
+                tail_dot<B, ND, M>(g, cell_of(g, 1, q), q, g.nr, V.Lo, L.rows, ql,
+                                   [&](const Cell&, int nq, double (&w)[B]) { load_vec<B>(V.rr, nq, w); }, acc);
+#pragma unroll
+            for (int t = 0; t < B; ++t) v[t] = __dsub_rn(v[t], acc[t]);
+            block_mul<B, M>(dv, v, x);
+            store_vec<B>(V.z, q, x);
+        }
+        sync();
+        for (int q = V.lo + tid; q < V.hi(0); q += nth) {  // rb_y_rows
+            double acc[B], v[B];
+#pragma unroll
+            for (int t = 0; t < B; ++t) acc[t] = v[t] = 0.0;
+            if (has_red) load_vec<B>(V.rr, q, v);
+            tail_dot<B, ND, M>(g, cell_of(g, 0, q), q, nk, V.U, L.rows, q - V.lo,
+                               [&](const Cell&, int nq, double (&w)[B]) { load_vec<B>(V.z, nq, w); }, acc);
+#pragma unroll
+            for (int t = 0; t < B; ++t) v[t] = __dsub_rn(v[t], acc[t]);
+            store_vec<B>(V.y, q, v);
+        }
+        sync();
+        for (int q = V.lo + tid; q < V.hi(1); q += nth) {  // the residual of rb_res_rows
+            const int ql = q - V.lo;
+            M av[BB];
+            double acc[B], az[B], z[B], t[B];
+#pragma unroll
+            for (int c = 0; c < B; ++c) acc[c] = 0.0;
+            load_vec<B>(V.rb, q, t);
+            load_vec<B>(V.z, q, z);
+            load_block<BB, M>(V.abb + (size_t)ql * BB, av);
+            tail_dot<B, ND, M>(g, cell_of(g, 1, q), q, g.nr, V.Lo, L.rows, ql,
+                               [&](const Cell&, int nq, double (&w)[B]) { load_vec<B>(V.y, nq, w); }, acc);
+            block_mul<B, M>(av, z, az);
+#pragma unroll
+            for (int c = 0; c < B; ++c) t[c] = __dsub_rn(__dsub_rn(t[c], az[c]), acc[c]);
+            store_vec<B>(V.t, q, t);
+        }
+        sync();
+    }
+    // the coarse rows that this block holds
+    const RbGrid& G = C.L.g;
+    for (int i = tid; i < 2 * C.L.rows; i += nth) {
+        const int colour = i < C.L.rows ? 0 : 1, q = C.lo + i - (colour ? C.L.rows : 0);
+        if (q >= C.hi(colour)) continue;
+        const Cell e = cell_of(G, colour, q);
+        double s[B];
+        if (L.pre) {  // the butterfly sum of rb_res_rows
+            double w[4][B];
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                const int c = m < L.agg.g ? black_member(L.agg, e.i, e.j, e.k, m) : -1;
+#pragma unroll
+                for (int t = 0; t < B; ++t) w[m][t] = 0.0;
+                if (c >= 0) load_vec<B>(V.t, c >> 1, w[m]);
+            }
+#pragma unroll
+            for (int t = 0; t < B; ++t)
+                s[t] = L.agg.g == 1 ? w[0][t]
+                                    : L.agg.g == 2 ? __dadd_rn(w[0][t], w[1][t])
+                                                   : __dadd_rn(__dadd_rn(w[0][t], w[1][t]), __dadd_rn(w[2][t], w[3][t]));
+        } else {  // rb_restrict_rows
+            const Aggregates& a = L.agg;
+#pragma unroll
+            for (int t = 0; t < B; ++t) s[t] = 0.0;
+            for (int o = 0; o < (1 << (a.sx + a.sy + a.sz)); ++o) {
+                const int x = (e.i << a.sx) + (a.sx ? o & 1 : 0), y = (e.j << a.sy) + (a.sy ? (o >> a.sx) & 1 : 0),
+                          z = (e.k << a.sz) + (a.sz ? o >> (a.sx + a.sy) : 0);
+                if (x >= g.nx || y >= g.ny || z >= g.nz) continue;
+                const bool black = (x + y + z) & 1;
+                if (!black && !has_red) continue;
+                double w[B];
+                load_vec<B>(black ? V.rb : V.rr, (x + g.nx * (y + g.ny * z)) >> 1, w);
+#pragma unroll
+                for (int t = 0; t < B; ++t) s[t] = __dadd_rn(s[t], w[t]);
+            }
+        }
+        store_vec<B>(colour ? C.rb : C.rr, q, s);
     }
     sync();
 }
 
-template <int B, int ND, class M, bool CG, class Sync>
-__device__ __forceinline__ void rb_up(const RbTailLevel<M>& L, const RbMatrix<const M>& m, const double* rr,
-                                      const double* rb, double* z, double* y, const UpView& up, int tid, int nth,
-                                      Sync&& sync)
+// The steps after the coarse correction: y, the black rows, and the red ones
+// unless the level is level 0.  The first level's rows leave the cluster: to
+// p.z (level 0) or up the finer level.
+template <int B, int ND, class M, class Sync>
+__device__ __forceinline__ void tail_up(const RbTailParams<M>& p, const RbTailView<B, ND, M>& V,
+                                        const RbTailView<B, ND, M>& C, bool has_red, bool first, int tid, int nth,
+                                        Sync&& sync)
 {
-    rb_y_rows<B, ND, M, CG>(L.g, m, rr, z, y, tid, nth);
+    const bool need_red = !first || p.z == nullptr;
+    const UpView up = first ? p.up : UpView();
+    constexpr int BB = B * B;
+    const RbTailLevel<M>& L = V.L;
+    const RbGrid& g = L.g;
+    const int nk = g.n - g.nr;
+    for (int q = V.lo + tid; q < V.hi(0); q += nth) {  // rb_y_rows
+        double acc[B], v[B];
+#pragma unroll
+        for (int t = 0; t < B; ++t) acc[t] = v[t] = 0.0;
+        if (has_red) load_vec<B>(V.rr, q, v);
+        tail_dot<B, ND, M>(g, cell_of(g, 0, q), q, nk, V.U, L.rows, q - V.lo,
+                           [&](const Cell& f, int nq, double (&w)[B]) { z0_at<B, ND, M>(V, C, f, nq, w); }, acc);
+#pragma unroll
+        for (int t = 0; t < B; ++t) v[t] = __dsub_rn(v[t], acc[t]);
+        store_vec<B>(V.y, q, v);
+    }
     sync();
-    rb_post_rows<B, ND, M, CG>(L.g, m, rb, y, z, up, tid, nth);
-    if (up.w == nullptr) return;
+    for (int q = V.lo + tid; q < V.hi(1); q += nth) {  // rb_post_rows
+        const int ql = q - V.lo;
+        const Cell e = cell_of(g, 1, q);
+        M av[BB], dv[BB];
+        double acc[B], az[B], z[B], t[B], x[B];
+        UpRow<B> fine;
+        if (up.w) fine.template load<true>(up, e);
+#pragma unroll
+        for (int c = 0; c < B; ++c) acc[c] = 0.0;
+        z0_at<B, ND, M>(V, C, e, q, z);
+        load_vec<B>(V.rb, q, t);
+        load_block<BB, M>(V.abb + (size_t)ql * BB, av);
+        load_block<BB, M>(V.db + (size_t)ql * BB, dv);
+        tail_dot<B, ND, M>(g, e, q, g.nr, V.Lo, L.rows, ql,
+                           [&](const Cell&, int nq, double (&w)[B]) { load_vec<B>(V.y, nq, w); }, acc);
+        block_mul<B, M>(av, z, az);
+#pragma unroll
+        for (int c = 0; c < B; ++c) t[c] = __dsub_rn(__dsub_rn(t[c], az[c]), acc[c]);
+        block_mul<B, M>(dv, t, x);
+#pragma unroll
+        for (int c = 0; c < B; ++c) z[c] = __dadd_rn(z[c], x[c]);
+        if (need_red) store_vec<B>(V.z, q, z);
+        else store_bvec<B, double>(p.z, q, z);
+        if (up.w) fine.store(up, z);
+    }
+    if (!need_red) return;
     sync();
-    rb_fin_rows<B, ND, M, CG>(L.g, m, rr, z, up, tid, nth);
+    for (int q = V.lo + tid; q < V.hi(0); q += nth) {  // rb_fin_rows
+        const int ql = q - V.lo;
+        const Cell e = cell_of(g, 0, q);
+        M dv[BB];
+        double acc[B], v[B], x[B];
+        UpRow<B> fine;
+        if (up.w) fine.template load<true>(up, e);
+#pragma unroll
+        for (int t = 0; t < B; ++t) acc[t] = v[t] = 0.0;
+        load_block<BB, M>(V.dr + (size_t)ql * BB, dv);
+        if (has_red) load_vec<B>(V.rr, q, v);
+        tail_dot<B, ND, M>(g, e, q, nk, V.U, L.rows, ql,
+                           [&](const Cell&, int nq, double (&w)[B]) { load_vec<B>(V.z, nq, w); }, acc);
+#pragma unroll
+        for (int t = 0; t < B; ++t) v[t] = __dsub_rn(v[t], acc[t]);
+        block_mul<B, M>(dv, v, x);
+        store_vec<B>(V.y, q, x);  // its right-hand side was read by the rows before the last barrier
+        if (up.w) fine.store(up, x);
+    }
     sync();
 }
 
-// The levels from lf on, on block 0 alone, in its shared memory; the
-// correction goes to level lf - 1's z in global memory.
-template <int B, int ND, class M>
-__device__ void rb_local_cycle(const RbTailParams<M>& p, int lf, unsigned char* sm)
+// Starts the copy of `bytes` from global to shared memory, both on a boundary
+// of PIECE bytes.
+template <int PIECE>
+__device__ __forceinline__ void copy_in(unsigned dst, const void* src, int bytes, int tid, int nth)
 {
+    for (int i = tid * PIECE; i < bytes; i += nth * PIECE) {
+        if constexpr (PIECE == 16)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i), "l"((const char*)src + i) : "memory");
+        else
+            asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst + i), "l"((const char*)src + i), "n"(PIECE)
+                         : "memory");
+    }
+}
+
+// Starts the copies of this block's rows of every level.
+template <int B, int ND, class M>
+__device__ __forceinline__ void tail_copies(const RbTailParams<M>& p, unsigned char* sm, int rank, int nblocks)
+{
+    constexpr int BB = B * B, BLK = BB * (int)sizeof(M);
+    constexpr int PIECE = BLK % 16 == 0 ? 16 : BLK % 8 == 0 ? 8 : 4;
     const int tid = (int)threadIdx.x, nth = (int)blockDim.x;
-    auto sync = [] { __syncthreads(); };
-    auto at_r = [&](int l) { return (double*)(sm + p.lv[l].so_r); };
-    auto at_y = [&](int l) { return (double*)(sm + p.lv[l].so_w); };
-    auto at_z = [&](int l) { return at_y(l) + p.lv[l].g.nr * B; };
-    auto matrix = [&](int l) {
-        const RbGrid& g = p.lv[l].g;
-        return RbMatrix<const M>((const M*)(sm + p.lv[l].so_a), ND, B * B, g.n, g.nr);
-    };
-    auto up_of = [&](int l) {
-        UpView u = p.lv[l].up;
-        if (l > lf) u.w = at_z(l - 1);
-        return u;
-    };
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    for (int i = tid; i < p.lv[lf].g.n * B; i += nth) at_r(lf)[i] = __ldcg(p.lv[lf].rr + i);
-    __syncthreads();
-    int l = lf;
-    for (; !p.lv[l].coarsest; ++l)
-        rb_down<B, ND, M, false>(p.lv[l], matrix(l), at_r(l), at_r(l) + p.lv[l].g.nr * B, at_z(l), at_y(l),
-                                 at_r(l + 1), tid, nth, sync);
-    rb_dense_rows<B, M, false>(p.lv[l].g, (const M*)(sm + p.lv[l].so_a), at_r(l), up_of(l), tid, nth);
-    __syncthreads();
-    for (--l; l >= lf; --l)
-        rb_up<B, ND, M, false>(p.lv[l], matrix(l), at_r(l), at_r(l) + p.lv[l].g.nr * B, at_z(l), at_y(l), up_of(l),
-                               tid, nth, sync);
+    for (int l = 0; l < p.nlev; ++l) {
+        const RbTailLevel<M>& L = p.lv[l];
+        unsigned dst = (unsigned)__cvta_generic_to_shared(sm + L.so_m);
+        if (L.coarsest) {
+            const int n = L.g.n * B, rows = (n + nblocks - 1) / nblocks, r0 = rank * rows;
+            if (r0 < n)
+                copy_in<(int)sizeof(M)>(dst, L.a + (size_t)r0 * n, min(rows, n - r0) * n * (int)sizeof(M), tid, nth);
+            continue;
+        }
+        const RbMatrix<const M> m(L.a, ND, BB, L.g.n, L.g.nr);
+        const int nk = L.g.n - L.g.nr, lo = rank * L.rows;
+        const int red = min(L.rows, L.g.nr - lo) * BLK, black = min(L.rows, nk - lo) * BLK;
+        const size_t at = (size_t)lo * BB;
+        auto part = [&](const M* src, int bytes) {
+            if (bytes > 0) copy_in<PIECE>(dst, src, bytes, tid, nth);
+            dst += L.rows * BLK;
+        };
+        for (int d = 0; d < ND; ++d) part(m.U + (size_t)d * L.g.nr * BB + at, red);
+        for (int d = 0; d < ND; ++d) part(m.L + (size_t)d * nk * BB + at, black);
+        part(m.dr + at, red);
+        part(m.abb + at, black);
+        part(m.db + at, black);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
 template <int B, int ND, class M>
@@ -983,38 +1278,77 @@ __global__ void __launch_bounds__(kTailThreads, 1)
     rb_tail_kernel(const __grid_constant__ RbTailParams<M> p, const KScal* sc, int skip_if_s)
 {
     extern __shared__ __align__(16) unsigned char tail_smem[];
-    // constant during a solve: fetched before the wait for the previous kernel
-    const int lf = p.local_first < p.nlev ? p.local_first : p.nlev;
-    if (lf < p.nlev && blockIdx.x == 0) start_local_copies(p.copies, p.ncopies, tail_smem);
-    prefetch_regions(p.reg, p.nregions);
+    const int rank = (int)blockIdx.x, nblocks = (int)gridDim.x;  // one cluster
+    const int tid = (int)threadIdx.x, nth = (int)blockDim.x;
+    // the matrices do not change during a solve: copied before the wait for
+    // the previous kernel
+    tail_copies<B, ND, M>(p, tail_smem, rank, nblocks);
     pdl_wait();
-    if (mg_skip(sc, skip_if_s)) {
+    if (mg_skip(sc, skip_if_s)) {  // the same in every block
         asm volatile("cp.async.wait_all;" ::: "memory");
         return;
     }
     long long* const trace = p.trace;
     int tk = 0;
-    if (trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0) trace[tk] = clock64();
+    if (trace != nullptr && rank == 0 && tid == 0) trace[tk] = clock64();
     ++tk;
+    // ends a step: of the cluster, or of block 0 alone (one call site per step,
+    // whatever the level: the steps' code is fetched once)
+    auto sync_of = [&](bool alone) {
+        if (alone) __syncthreads();
+        else tail_step(trace, tk);
+    };
     auto sync = [&] { tail_step(trace, tk); };
-    // 32 rows (a warp) at a time, round robin over the blocks
-    const int tid = (((int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x) << 5) | (int)(threadIdx.x & 31);
-    const int nth = (int)(gridDim.x * blockDim.x);
-    auto matrix = [&](const RbTailLevel<M>& L) { return RbMatrix<const M>(L.a, ND, B * B, L.g.n, L.g.nr); };
-    int l = 0;
-    for (; l < lf && !p.lv[l].coarsest; ++l) {
-        const RbTailLevel<M>& L = p.lv[l];
-        rb_down<B, ND, M, true>(L, matrix(L), L.rr, L.rb, L.z, L.y, p.lv[l + 1].r, tid, nth, sync);
+    using View = RbTailView<B, ND, M>;
+    auto view = [&](int l) { return View(p.lv[l], tail_smem, rank); };
+    const int last = p.nlev - 1, solo = p.solo_first;
+    const bool red0 = p.rr != nullptr;
+    {
+        const View V = view(0);
+        double w[B];
+        for (int q = V.lo + tid; red0 && q < V.hi(0); q += nth) {
+            load_bvec<B, double>(p.rr, q, w);
+            store_vec<B>(V.rr, q, w);
+        }
+        for (int q = V.lo + tid; q < V.hi(1); q += nth) {
+            load_bvec<B, double>(p.rb, q, w);
+            store_vec<B>(V.rb, q, w);
+        }
     }
-    if (l == lf) {
-        // block 0 alone; the other blocks wait at the next cluster barrier
-        if (blockIdx.x == 0) rb_local_cycle<B, ND, M>(p, lf, tail_smem);
-    } else {
-        rb_dense_rows<B, M, true>(p.lv[l].g, p.lv[l].a, p.lv[l].rr, p.lv[l].up, tid, nth);
-    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     sync();
-    for (--l; l >= 0; --l) {
-        const RbTailLevel<M>& L = p.lv[l];
-        rb_up<B, ND, M, true>(L, matrix(L), L.rr, L.rb, L.z, L.y, L.up, tid, nth, sync);
+    for (int l = 0; l < last; ++l)
+        if (l < solo || rank == 0)
+            tail_down<B, ND, M>(view(l), view(l + 1), l > 0 || red0, tid, nth, [&] { sync_of(l >= solo); });
+    if (solo < last) sync();
+    {  // rb_dense_rows, the right-hand side copied to every block first
+        const View V = view(last);
+        const int n = V.L.g.n * B, nr = V.L.g.nr, rows = (n + nblocks - 1) / nblocks, lane = tid & 31;
+        const M* inv = reinterpret_cast<const M*>(tail_smem + V.L.so_m);
+        double* r = reinterpret_cast<double*>(tail_smem + V.L.so_r);
+        if (tid < V.L.g.n) {
+            double w[B];
+            load_vec<B>(tid < nr ? V.rr : V.rb, tid < nr ? tid : tid - nr, w);
+            store_bvec<B, double>(r, tid, w);
+        }
+        __syncthreads();
+        for (int k = tid >> 5; k < rows && rank * rows + k < n; k += nth >> 5) {
+            double s = 0.0;
+            for (int j = lane; j < n; j += 32) s = __fma_rn((double)inv[k * n + j], r[j], s);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) {
+                const int i = rank * rows + k, P = i / B, c = i - P * B;
+                const unsigned a = remote(P < nr ? V.y : V.z, P < nr ? P : P - nr, 8 * B) + 8 * c;
+                asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(s) : "memory");
+            }
+        }
+        sync();
     }
+    for (int l = last - 1; l >= 0; --l) {
+        if (l == solo - 1 && solo < last) sync();  // block 0's levels are done
+        if (l < solo || rank == 0)
+            tail_up<B, ND, M>(p, view(l), view(l + 1), l > 0 || red0, l == 0, tid, nth, [&] { sync_of(l >= solo); });
+    }
+    cluster_barrier();  // no block leaves while another may read its shared memory
 }

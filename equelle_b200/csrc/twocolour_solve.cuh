@@ -146,11 +146,6 @@ bool rb_analyse(Core& c, SolverAnalysis& an, const Pattern& p, int bs, int coars
         an.rb.push_back(std::move(C));
         if (last) break;
     }
-    // levels of at most linsolver_mg_fuse_rows unknowns (0: none) run as one
-    // kernel, the last kMaxTail of them at most
-    const int fuse_rows = c.param_i("linsolver_mg_fuse_rows", 40000), nl = (int)an.rb.size();
-    for (int l = nl - 1; l >= 0 && nl - l <= kMaxTail && (an.rb[l].coarsest || an.rb[l].n <= fuse_rows); --l)
-        if (!an.rb[l].coarsest) an.tail_first = l;
     // the right-hand side, and the BiCGStab vectors of the black half
     const RbGrid& g = an.rb[0].g;
     an.vec64 = c.allocN<double>(vec_stride(an.n) + 10 * vec_stride((g.n - g.nr) * bs));
@@ -228,77 +223,82 @@ struct RbVectors {
     }
 };
 
-// The fused levels kept in block 0's shared memory: from the coarsest one
-// upward while they fit in kTailSmem bytes (the first fused level stays
-// cluster-wide).  Returns the first such level as an index into the fused
-// levels (their count: none) and its bytes; fills the layout and copies.
+// The levels that a cluster of `cl` blocks holds in shared memory: from the
+// coarsest one upward, of at most linsolver_mg_fuse_rows unknowns (0: none),
+// while every block's share fits in kRbTailSmem bytes.  Returns the first one
+// (-1: none) and the bytes of a block; fills the layout.  The levels of at
+// most kRbSoloCells cells are block 0's (linsolver_mg_local=0: none).
 template <class M>
-int plan_rb_local(Core& c, const SolverAnalysis& an, int& bytes, RbTailParams<M>* p)
+int plan_rb_tail(Core& c, const SolverAnalysis& an, int cl, int& bytes, RbTailParams<M>* p)
 {
-    const int nlev = (int)an.rb.size() - an.tail_first;
-    bytes = 0;
-    if (an.tail_first < 0 || !c.param_i("linsolver_mg_local", 1)) return nlev;
+    const int nl = (int)an.rb.size(), fuse_rows = c.param_i("linsolver_mg_fuse_rows", 40000);
+    const int solo_cells = c.param_i("linsolver_mg_local", 1) ? kRbSoloCells : 0, bs = an.rb_bs;
+    auto al = [](int64_t b) { return (b + 15) & ~(int64_t)15; };
     int64_t off = 0;
-    auto place = [&](int64_t b) {
-        const int64_t o = off;
-        off += (b + 15) & ~(int64_t)15;
-        return (int)o;
-    };
-    int lf = nlev;
-    for (int i = nlev - 1; i >= 1; --i) {
-        const RbLevel& L = an.rb[an.tail_first + i];
-        const int64_t mat = (L.coarsest ? (int64_t)L.n * L.n : L.vals) * (int64_t)sizeof(M);
-        const int64_t before = off;
-        const int a = place(mat), r = place((int64_t)L.n * sizeof(double)),
-                  w = L.coarsest ? 0 : place((int64_t)L.n * sizeof(double));
-        if (off > kTailSmem) {
-            off = before;
-            break;
-        }
-        lf = i;
-        if (p) {
-            p->lv[i].so_a = a;
-            p->lv[i].so_r = r;
-            p->lv[i].so_w = w;
-            p->copies[p->ncopies++] = TailCopy{rb_values<M>(L), a, (int)mat};
-        }
+    int first = -1;
+    RbTailParams<M> q;
+    int solo = nl - 1;
+    for (int l = nl - 1; l >= 0 && nl - l <= kMaxTail; --l) {
+        const RbLevel& L = an.rb[l];
+        if (!L.coarsest && L.n > fuse_rows) break;
+        const bool alone = !L.coarsest && L.g.n <= solo_cells;
+        // the coarsest level's vectors are where the level above restricts to
+        const bool vectors_alone = alone || (L.coarsest && l > 0 && an.rb[l - 1].g.n <= solo_cells);
+        RbTailLevel<M>& t = q.lv[l - std::max(0, nl - kMaxTail)];
+        t.g = L.g;
+        t.coarsest = L.coarsest ? 1 : 0;
+        t.pre = L.pre ? 1 : 0;
+        t.alpha = L.alpha;
+        t.a = rb_values<M>(L);
+        t.agg = L.agg;
+        t.rows = vectors_alone ? L.g.nr : (L.g.nr + cl - 1) / cl;
+        t.by_rows = FastDiv((unsigned)t.rows);
+        t.vec = (int)al((int64_t)t.rows * bs * sizeof(double));
+        const int64_t mat = L.coarsest ? (int64_t)((L.n + cl - 1) / cl) * L.n
+                                       : (int64_t)(2 * an.rb_nd + 3) * t.rows * bs * bs;
+        const int64_t need = al(mat * (int64_t)sizeof(M)) + 5 * (int64_t)t.vec +
+                             (L.coarsest ? al((int64_t)L.n * sizeof(double)) : 0);
+        // more rows than half the threads of a block are better spread over the
+        // whole GPU, one launch per step (two-phase 255x257 mixed, whose
+        // 128x129 level would be 516 rows a block: 6.6 against 6.4 ms a step)
+        if (!alone && !L.coarsest && t.rows > kTailThreads / 2 && cl > 1) break;
+        if (off + need > kRbTailSmem) break;
+        t.so_m = (int)off;
+        t.so_v = (int)(off + al(mat * (int64_t)sizeof(M)));
+        t.so_r = t.so_v + 5 * t.vec;
+        off += need;
+        if (alone) solo = l;
+        if (!L.coarsest) first = l;
     }
-    if (lf == nlev) return nlev;
+    if (first < 0) return -1;
     bytes = (int)off;
-    if (p) p->local_first = lf;
-    return lf;
+    if (p) {
+        p->nlev = nl - first;
+        p->solo_first = solo - first;
+        for (int i = 0; i < p->nlev; ++i) p->lv[i] = q.lv[first + i - std::max(0, nl - kMaxTail)];
+    }
+    return first;
 }
 
 template <class M>
 void launch_rb_tail(Core& c, const SolverAnalysis& an, const double* in, double* out, const KScal* sc, int skip)
 {
+    const int cl = an.tail_cluster[pc_mode<double, M>()];
     RbTailParams<M> p;
+    int smem = 0;
+    if (plan_rb_tail<M>(c, an, cl, smem, &p) != an.tail_first) fail(EQG_ERR_DEVICE, "fused coarse cycle: another plan");
+    const RbVectors v(an, an.tail_first, in, out);
+    p.rr = v.rr;
+    p.rb = v.rb;
+    p.up = v.up;
+    if (an.tail_first == 0) p.z = v.z;
     double bytes = 0.0;
     for (size_t l = an.tail_first; l < an.rb.size(); ++l) {
         const RbLevel& L = an.rb[l];
-        const RbVectors v(an, l, in, out);
-        RbTailLevel<M>& t = p.lv[p.nlev++];
-        t.g = L.g;
-        t.coarsest = L.coarsest ? 1 : 0;
-        t.pre = L.pre ? 1 : 0;
-        t.a = rb_values<M>(L);
-        t.rr = v.rr;
-        t.rb = v.rb;
-        t.r = const_cast<double*>(v.rr);
-        t.z = v.z;
-        t.y = v.y;
-        t.agg = L.agg;
-        t.up = v.up;
-        const int64_t mat = (L.coarsest ? (int64_t)L.n * L.n : L.vals) * (int64_t)sizeof(M);
-        p.reg[p.nregions++] = PrefetchRegion{t.a, (unsigned long long)mat};
-        bytes += mat + 4.0 * L.n * sizeof(double);
+        bytes += (double)(L.coarsest ? (int64_t)L.n * L.n : L.vals) * sizeof(M) + 4.0 * L.n * sizeof(double);
     }
     if (an.tail_trace) p.trace = an.tail_trace->as<long long>();
-    p.local_first = p.nlev;
-    int smem = 0;
-    const int mode = pc_mode<double, M>();
-    if (an.tail_local[mode] < p.nlev) plan_rb_local<M>(c, an, smem, &p);
-    TailLaunch cfg(c, an.tail_cluster[mode], smem);
+    TailLaunch cfg(c, cl, smem);
     WITH_RB(an, launch(c, "rb_tail", [&] {
                 EQG_CUDA(cudaLaunchKernelEx(&cfg.cfg, rb_tail_kernel<BS, ND, M>, p, sc, skip));
             }, bytes));
@@ -362,16 +362,16 @@ void rb_cycle(Core& c, const SolverAnalysis& an, size_t l, const double* in, dou
             }, half_u + (blk + row + to_fine) * nr + row * nk));
 }
 
-// Chooses the cluster size of the fused levels; called before any capture.
+// Chooses the cluster size and the levels of the fused cycle; called before
+// any capture.
 template <class M>
 void prepare_rb_tail(Core& c, SolverAnalysis& an)
 {
-    if (an.tail_first < 0) return;
     const int mode = pc_mode<double, M>();
     int& cl = an.tail_cluster[mode];
-    if (!cl) WITH_RB(an, cl = tail_cluster_size(c, rb_tail_kernel<BS, ND, M>));
+    if (!cl) WITH_RB(an, cl = tail_cluster_size(c, rb_tail_kernel<BS, ND, M>, kRbTailSmem));
     int bytes = 0;
-    an.tail_local[mode] = plan_rb_local<M>(c, an, bytes, nullptr);
+    an.tail_first = plan_rb_tail<M>(c, an, cl, bytes, nullptr);
     an.last_mode = mode;
 }
 
