@@ -634,6 +634,7 @@ OpMatrixP new_opmatrix(Core& c, int n_out, int n_src, int max_row, int64_t nnz)
     m->n_src = n_src;
     m->max_row = max_row;
     m->nnz = nnz;
+    m->unit = true;  // the operators of the Cartesian grid: differences and sums
     m->ptr = c.allocN<int32_t>((size_t)n_out + 1);
     m->src = c.allocN<int32_t>(nnz > 0 ? nnz : 1);
     m->w = c.allocN<double>(nnz > 0 ? nnz : 1);
@@ -724,6 +725,7 @@ void build_grid(Core& c, eqg_set** builtin)
         m->n_out = c.nc;
         m->n_src = c.nif;
         m->max_row = 2 * c.dim;
+        m->unit = true;
         Buf cnt = c.allocN<int64_t>(nc64);
         launch(c, "div_interior_count", [&] { div_interior_kernel<false><<<blocksFor(nc64), kThreads, 0, c.stream>>>(d, ipos->as<int32_t>(),
                                                                                cnt->as<int64_t>(), nullptr, nullptr,

@@ -74,8 +74,9 @@ struct Pattern {
     std::map<std::pair<uint64_t, uint64_t>, Buf> merge_maps;
     // for a pattern made as M J (gradient, divergence, On, Extend, spans):
     // per entry, the positions of J's entries that add into it (see
-    // spgemm_plan_kernel), int32[nnz+1] bounds and int32 packed positions
-    Buf plan_start, plan_contrib;
+    // spgemm_plan_kernel), int32[nnz+1] bounds, int32 signed positions and
+    // int32 rows of J
+    Buf plan_start, plan_contrib, plan_jrow;
     int64_t plan_entries = 0;
     // for a union pattern whose operands have entries in disjoint row
     // ranges, the one with the lower rows first: the union's entries are
@@ -95,6 +96,7 @@ struct OpMatrix {
     int n_out = 0, n_src = 0;
     int max_row = 0;
     int64_t nnz = 0;
+    bool unit = false;  // every weight is 1 or -1
     // a helper operator of the Cartesian grid that the stencil kernels apply
     // to values by face and cell index arithmetic (STENCIL_*; 0: none)
     int stencil = 0;

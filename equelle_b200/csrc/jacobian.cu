@@ -16,6 +16,7 @@
 
 #include <cub/cub.cuh>
 
+#include <algorithm>
 #include <climits>
 #include <cstring>
 
@@ -97,6 +98,115 @@ __device__ __forceinline__ double apply_deferred(const Deferred& d, int64_t row,
     return x;
 }
 
+
+// Entries of a Jacobian that a thread of the elementwise and planned product
+// kernels takes at once.  An entry is a chain of dependent loads (its row and
+// positions, then the operands' values and the rules' row values); with one
+// entry per thread these kernels ran at 1.6 to 2.5 TB/s and waited for that
+// chain in 22 to 33 of the 27 to 38 cycles between two instructions of a warp,
+// so the loads of each link are issued for all of a thread's entries before
+// the next link.  Two-phase, 128x128x64 (12.5 M entries on faces): elementwise
+// 153 -> 105 us, product 79 -> 39 us, all residuals of a step 15.9 -> 11.9 ms
+// (two entries: 12.6 ms).
+constexpr int kEntries = 4;
+
+// rule_weights of kEntries rows: the rule is looked at once, the row values
+// of all entries are loaded before they are used.
+template <int E>
+__device__ __forceinline__ void rule_weights_of(const Rule& r, const int (&i)[E], double (&wa)[E], double (&wb)[E],
+                                                double (&post)[E])
+{
+    double a[E], b[E];
+    auto load = [&](const double* p, double (&v)[E], double s) {
+#pragma unroll
+        for (int u = 0; u < E; ++u) v[u] = p ? p[i[u]] : s;
+    };
+#pragma unroll
+    for (int u = 0; u < E; ++u) wa[u] = wb[u] = post[u] = 1.0;
+    switch (r.rule) {
+    case JR_ADD: break;
+    case JR_SUB:
+#pragma unroll
+        for (int u = 0; u < E; ++u) wb[u] = -1.0;
+        break;
+    case JR_MUL:
+        load(r.va, a, r.s);
+        load(r.vb, b, r.s);
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            wa[u] = b[u];
+            wb[u] = a[u];
+        }
+        break;
+    case JR_DIV:
+        load(r.va, a, r.s);
+        load(r.vb, b, r.s);
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            wa[u] = b[u];
+            wb[u] = -a[u];
+            post[u] = 1.0 / (b[u] * b[u]);
+        }
+        break;
+    case JR_SCALE_CONST:
+#pragma unroll
+        for (int u = 0; u < E; ++u) wa[u] = r.s;
+        break;
+    case JR_DIV_BY_CONST:
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            wa[u] = r.s;
+            post[u] = 1.0 / (r.s * r.s);
+        }
+        break;
+    case JR_SQRT:
+        load(r.vout, a, 0.0);
+#pragma unroll
+        for (int u = 0; u < E; ++u) wa[u] = 0.5 / a[u];
+        break;
+    case JR_SIGN:
+        load(r.va, a, 0.0);
+#pragma unroll
+        for (int u = 0; u < E; ++u) wa[u] = a[u] >= 0.0 ? 1.0 : -1.0;
+        break;
+    case JR_NEG:
+#pragma unroll
+        for (int u = 0; u < E; ++u) wa[u] = -1.0;
+        break;
+    case JR_SELECT: {
+        uint8_t m[E];
+#pragma unroll
+        for (int u = 0; u < E; ++u) m[u] = r.mask[i[u]];
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            wa[u] = m[u] ? 1.0 : 0.0;
+            wb[u] = m[u] ? 0.0 : 1.0;
+        }
+        break;
+    }
+    }
+}
+
+// apply_deferred for E entries, with its arithmetic.
+template <int E>
+__device__ __forceinline__ void apply_deferred_of(const Deferred& d, const int (&row)[E], double (&x)[E])
+{
+    for (int k = 0; k < d.n; ++k) {
+        const DeferredRule& q = d.r[k];
+        double wa[E], wb[E], post[E];
+        rule_weights_of<E>(Rule{q.rule, q.va, q.vb, q.vout, q.mask, q.s}, row, wa, wb, post);
+#pragma unroll
+        for (int u = 0; u < E; ++u) x[u] = post[u] * __fma_rn(q.side == 0 ? wa[u] : wb[u], x[u], 0.0);
+    }
+}
+
+// This thread's entries: e + u blockDim for u < kEntries, e from the loop;
+// past the end the last entry (its result is not stored).
+#define ENTRY_STRIDE(e, n)                                                                                  \
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x * kEntries + threadIdx.x; e < (n);                    \
+         e += (int64_t)gridDim.x * blockDim.x * kEntries)
+
+inline int entry_blocks(int64_t n) { return blocksFor((n + kEntries - 1) / kEntries); }
 
 // ---------------------------------------------------------------------------
 // Conservative product M*J by K-way merge of the selected rows of J.
@@ -208,25 +318,27 @@ __global__ void spgemm_numeric_kernel(int n_out, const int* __restrict__ mptr, c
 
 // Position plan of M*J for one output pattern: for every output entry, the
 // entries of J that the K-way merge adds into it, in the merge's order
-// (stream t of M's row ascending), packed as t << kPlanShift | position in
-// J.  Built once with the output pattern; the numeric product then runs one
-// thread per output entry, with the same operations in the same order as
-// spgemm_numeric_kernel.
-constexpr int kPlanShift = 27;
-constexpr int kPlanMask = (1 << kPlanShift) - 1;
+// (ascending stream of M's row).  Built once with the output pattern; the
+// numeric product then runs over output entries, with the operations of
+// spgemm_numeric_kernel in its order.  For operators with weights 1 and -1 (all
+// that the runtime makes: differences, divergence, On, Extend, spans): a
+// contribution is its position in J, the weight's sign in the top bit (a
+// product with 1 or -1 is exact), and J's row, so the product reads nothing
+// of M.
+constexpr int kPlanMask = 0x7fffffff;
 
 template <int KMAX, bool COUNT>
 __global__ void spgemm_plan_kernel(int n_out, const int* __restrict__ mptr, const int* __restrict__ msrc,
-                                   const int* __restrict__ jptr, const int* __restrict__ jcol,
-                                   const int* __restrict__ optr, const int* __restrict__ ocol,
-                                   int64_t* __restrict__ cnt, const int* __restrict__ start,
-                                   int* __restrict__ contrib)
+                                   const double* __restrict__ mw, const int* __restrict__ jptr,
+                                   const int* __restrict__ jcol, const int* __restrict__ optr,
+                                   const int* __restrict__ ocol, int64_t* __restrict__ cnt,
+                                   const int* __restrict__ start, int* __restrict__ contrib, int* __restrict__ jrow)
 {
     GRID_STRIDE(i, n_out)
     {
         Streams<KMAX> s;
-        s.load((int)i, mptr, msrc, nullptr, jptr);
-        const int p1 = optr[i + 1];
+        s.load((int)i, mptr, msrc, mw, jptr);
+        const int m0 = mptr[i], p1 = optr[i + 1];
         for (int p = optr[i]; p < p1; ++p) {
             const int c = ocol[p];
             int n = 0;
@@ -234,7 +346,10 @@ __global__ void spgemm_plan_kernel(int n_out, const int* __restrict__ mptr, cons
 #pragma unroll
             for (int t = 0; t < KMAX; ++t) {
                 if (s.pos[t] < s.end[t] && jcol[s.pos[t]] == c) {
-                    if (!COUNT) contrib[o + n] = (t << kPlanShift) | s.pos[t];
+                    if (!COUNT) {
+                        contrib[o + n] = s.pos[t] | (s.w[t] < 0.0 ? (int)0x80000000 : 0);
+                        jrow[o + n] = msrc[m0 + t];
+                    }
                     ++n;
                     ++s.pos[t];
                 }
@@ -244,24 +359,48 @@ __global__ void spgemm_plan_kernel(int n_out, const int* __restrict__ mptr, cons
     }
 }
 
-__global__ void spgemm_planned_kernel(int64_t nnz, const int* __restrict__ rowidx, const int* __restrict__ mptr,
-                                      const double* __restrict__ mw, const int* __restrict__ start,
-                                      const int* __restrict__ contrib, const double* __restrict__ jval,
-                                      double* __restrict__ oval, const int* __restrict__ msrc, const Deferred dj)
+__global__ void __launch_bounds__(kThreads) spgemm_planned_kernel(int64_t nnz, const int* __restrict__ start,
+                                                                  const int* __restrict__ contrib,
+                                                                  const int* __restrict__ jrow,
+                                                                  const double* __restrict__ jval,
+                                                                  double* __restrict__ oval, const Deferred dj)
 {
-    GRID_STRIDE(e, nnz)
+    ENTRY_STRIDE(e0, nnz)
     {
-        const int m0 = mptr[rowidx[e]];
-        const int k1 = start[e + 1];
-        double acc = 0.0;
-        for (int k = start[e]; k < k1; ++k) {
-            const int q = contrib[k];
-            const int t = q >> kPlanShift;
-            // J's value with its deferred rules, in J's row (M's source)
-            const double jv = dj.n ? apply_deferred(dj, msrc[m0 + t], jval[q & kPlanMask]) : jval[q & kPlanMask];
-            acc += mw[m0 + t] * jv;
+        int k[kEntries], k1[kEntries];
+        double acc[kEntries];
+        bool more = false;
+#pragma unroll
+        for (int u = 0; u < kEntries; ++u) {
+            const int64_t e = min(e0 + (int64_t)u * blockDim.x, nnz - 1);
+            k[u] = start[e];
+            k1[u] = start[e + 1];
+            acc[u] = 0.0;
         }
-        oval[e] = acc;
+        do {  // the next contribution of every entry (each has at least one)
+            int q[kEntries], row[kEntries];
+            double x[kEntries];
+#pragma unroll
+            for (int u = 0; u < kEntries; ++u) {
+                const int at = max(min(k[u], k1[u] - 1), 0);
+                q[u] = contrib[at];
+                row[u] = dj.n ? jrow[at] : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < kEntries; ++u) x[u] = jval[q[u] & kPlanMask];
+            if (dj.n) apply_deferred_of<kEntries>(dj, row, x);
+            more = false;
+#pragma unroll
+            for (int u = 0; u < kEntries; ++u) {
+                if (k[u] < k1[u]) acc[u] += q[u] < 0 ? -x[u] : x[u];
+                more |= ++k[u] < k1[u];
+            }
+        } while (more);
+#pragma unroll
+        for (int u = 0; u < kEntries; ++u) {
+            const int64_t e = e0 + (int64_t)u * blockDim.x;
+            if (e < nnz) oval[e] = acc[u];
+        }
     }
 }
 
@@ -335,28 +474,59 @@ __global__ void i64_to_rowptr_kernel(const int64_t* incl, int n, int* rowptr)
 // Elementwise Jacobian rules over patterns (operands read through their
 // deferred rules da, db).
 // ---------------------------------------------------------------------------
-// Operands share the output pattern: one thread per nonzero.
-__global__ void ew_flat_kernel(Rule r, const int* __restrict__ rowidx, const double* __restrict__ ja,
-                               const double* __restrict__ jb, double* __restrict__ out, int64_t nnz,
-                               const Deferred da, const Deferred db)
+// Operands share the output pattern.
+__global__ void __launch_bounds__(kThreads) ew_flat_kernel(Rule r, const int* __restrict__ rowidx,
+                                                           const double* __restrict__ ja,
+                                                           const double* __restrict__ jb, double* __restrict__ out,
+                                                           int64_t nnz, const Deferred da, const Deferred db)
 {
-    GRID_STRIDE(e, nnz)
+    ENTRY_STRIDE(e0, nnz)
     {
-        const int i = rowidx[e];
-        double wa, wb, post;
-        rule_weights(r, i, wa, wb, post);
-        double acc = 0.0;
-        if (ja) acc += wa * apply_deferred(da, i, ja[e]);
-        if (jb) acc += wb * apply_deferred(db, i, jb[e]);
-        out[e] = post * acc;
+        int i[kEntries];
+        double a[kEntries], b[kEntries], wa[kEntries], wb[kEntries], post[kEntries];
+#pragma unroll
+        for (int u = 0; u < kEntries; ++u) {
+            const int64_t e = min(e0 + (int64_t)u * blockDim.x, nnz - 1);
+            i[u] = rowidx[e];
+            a[u] = ja ? ja[e] : 0.0;
+            b[u] = jb ? jb[e] : 0.0;
+        }
+        rule_weights_of<kEntries>(r, i, wa, wb, post);
+        if (ja) apply_deferred_of<kEntries>(da, i, a);
+        if (jb) apply_deferred_of<kEntries>(db, i, b);
+#pragma unroll
+        for (int u = 0; u < kEntries; ++u) {
+            const int64_t e = e0 + (int64_t)u * blockDim.x;
+            double acc = 0.0;
+            if (ja) acc = __fma_rn(wa[u], a[u], acc);
+            if (jb) acc = __fma_rn(wb[u], b[u], acc);
+            if (e < nnz) out[e] = post[u] * acc;
+        }
     }
 }
 
 // out = the stored values with their deferred rules applied.
-__global__ void apply_deferred_kernel(const Deferred d, const int* __restrict__ rowidx, const double* __restrict__ j,
-                                      double* __restrict__ out, int64_t nnz)
+__global__ void __launch_bounds__(kThreads) apply_deferred_kernel(const Deferred d, const int* __restrict__ rowidx,
+                                                                  const double* __restrict__ j,
+                                                                  double* __restrict__ out, int64_t nnz)
 {
-    GRID_STRIDE(e, nnz) out[e] = apply_deferred(d, rowidx[e], j[e]);
+    ENTRY_STRIDE(e0, nnz)
+    {
+        int i[kEntries];
+        double x[kEntries];
+#pragma unroll
+        for (int u = 0; u < kEntries; ++u) {
+            const int64_t e = min(e0 + (int64_t)u * blockDim.x, nnz - 1);
+            i[u] = rowidx[e];
+            x[u] = j[e];
+        }
+        apply_deferred_of<kEntries>(d, i, x);
+#pragma unroll
+        for (int u = 0; u < kEntries; ++u) {
+            const int64_t e = e0 + (int64_t)u * blockDim.x;
+            if (e < nnz) out[e] = x[u];
+        }
+    }
 }
 
 // Operands on different patterns: merge each row into the union pattern.
@@ -417,23 +587,41 @@ __global__ void merge_map_kernel(int rows, const int* __restrict__ aptr, const i
     }
 }
 
-// ew_merge_kernel through the position maps: one thread per nonzero, the
-// same operations in the same order.
-__global__ void ew_mapped_kernel(Rule r, const int* __restrict__ rowidx, const int* __restrict__ ia,
-                                 const int* __restrict__ ib, const double* __restrict__ ja,
-                                 const double* __restrict__ jb, double* __restrict__ out, int64_t nnz,
-                                 const Deferred da, const Deferred db)
+// ew_merge_kernel through the position maps: the same operations in the same
+// order.
+__global__ void __launch_bounds__(kThreads) ew_mapped_kernel(Rule r, const int* __restrict__ rowidx,
+                                                             const int* __restrict__ ia, const int* __restrict__ ib,
+                                                             const double* __restrict__ ja,
+                                                             const double* __restrict__ jb, double* __restrict__ out,
+                                                             int64_t nnz, const Deferred da, const Deferred db)
 {
-    GRID_STRIDE(e, nnz)
+    ENTRY_STRIDE(e0, nnz)
     {
-        const int i = rowidx[e];
-        double wa, wb, post;
-        rule_weights(r, i, wa, wb, post);
-        const int xa = ia[e], xb = ib[e];
-        double acc = 0.0;
-        if (xa >= 0) acc += wa * apply_deferred(da, i, ja[xa]);
-        if (xb >= 0) acc += wb * apply_deferred(db, i, jb[xb]);
-        out[e] = post * acc;
+        int i[kEntries], xa[kEntries], xb[kEntries];
+        double a[kEntries], b[kEntries], wa[kEntries], wb[kEntries], post[kEntries];
+#pragma unroll
+        for (int u = 0; u < kEntries; ++u) {
+            const int64_t e = min(e0 + (int64_t)u * blockDim.x, nnz - 1);
+            i[u] = rowidx[e];
+            xa[u] = ia[e];
+            xb[u] = ib[e];
+        }
+#pragma unroll
+        for (int u = 0; u < kEntries; ++u) {
+            a[u] = xa[u] >= 0 ? ja[xa[u]] : 0.0;
+            b[u] = xb[u] >= 0 ? jb[xb[u]] : 0.0;
+        }
+        rule_weights_of<kEntries>(r, i, wa, wb, post);
+        apply_deferred_of<kEntries>(da, i, a);
+        apply_deferred_of<kEntries>(db, i, b);
+#pragma unroll
+        for (int u = 0; u < kEntries; ++u) {
+            const int64_t e = e0 + (int64_t)u * blockDim.x;
+            double acc = 0.0;
+            if (xa[u] >= 0) acc = __fma_rn(wa[u], a[u], acc);
+            if (xb[u] >= 0) acc = __fma_rn(wb[u], b[u], acc);
+            if (e < nnz) out[e] = post[u] * acc;
+        }
     }
 }
 
@@ -520,19 +708,19 @@ void spgemm_build_plan(Core& c, const OpMatrix& m, const Pattern& j, Pattern& ou
     const int nb = blocksFor(m.n_out);
     launch(c, "spgemm_plan_count", [&] {
         spgemm_plan_kernel<KMAX, true><<<nb, kThreads, 0, c.stream>>>(
-            m.n_out, m.ptr->as<int>(), m.src->as<int>(), j.rowptr->as<int>(), j.colind->as<int>(),
-            out.rowptr->as<int>(), out.colind->as<int>(), cnt->as<int64_t>(), nullptr, nullptr);
+            m.n_out, m.ptr->as<int>(), m.src->as<int>(), m.w->as<double>(), j.rowptr->as<int>(), j.colind->as<int>(),
+            out.rowptr->as<int>(), out.colind->as<int>(), cnt->as<int64_t>(), nullptr, nullptr, nullptr);
     });
     const int64_t total = counts_to_rowptr(c, cnt, (int)out.nnz, out.plan_start);
     out.plan_entries = total;
     out.plan_contrib = c.allocN<int>(total > 0 ? total : 1);
+    out.plan_jrow = c.allocN<int>(total > 0 ? total : 1);
     launch(c, "spgemm_plan_fill", [&] {
         spgemm_plan_kernel<KMAX, false><<<nb, kThreads, 0, c.stream>>>(
-            m.n_out, m.ptr->as<int>(), m.src->as<int>(), j.rowptr->as<int>(), j.colind->as<int>(),
+            m.n_out, m.ptr->as<int>(), m.src->as<int>(), m.w->as<double>(), j.rowptr->as<int>(), j.colind->as<int>(),
             out.rowptr->as<int>(), out.colind->as<int>(), nullptr, out.plan_start->as<int>(),
-            out.plan_contrib->as<int>());
+            out.plan_contrib->as<int>(), out.plan_jrow->as<int>());
     });
-    pattern_build_rowidx(c, out);
 }
 
 template <int KMAX>
@@ -542,15 +730,15 @@ void spgemm_numeric(Core& c, const OpMatrix& m, const Pattern& jp, const double*
     if (m.n_out <= 0) return;
     if (jd.n && !op.plan_start) fail(EQG_ERR_DEVICE, "operator product of deferred Jacobian values without a plan");
     if (op.plan_start) {
-        // algorithmic bytes: the output's row indices and plan, the
-        // contributing Jacobian values and M's row pointers and weights, the
-        // output values
-        const double bytes = 16.0 * op.nnz + 12.0 * op.plan_entries + 4.0 * (m.n_out + 1) + 8.0 * m.nnz;
+        // algorithmic bytes: the output's values and plan bounds, the
+        // contributions and the Jacobian values they add (their rows and the
+        // rules' row values where rules are deferred)
+        const double bytes =
+            12.0 * op.nnz + (jd.n ? 16.0 : 12.0) * op.plan_entries + 16.0 * jd.n * jp.rows;
         launch(c, "spgemm_planned", [&] {
-            spgemm_planned_kernel<<<blocksFor(op.nnz), kThreads, 0, c.stream>>>(
-                op.nnz, op.rowidx->as<int>(), m.ptr->as<int>(), m.w->as<double>(), op.plan_start->as<int>(),
-                op.plan_contrib->as<int>(), jv, ov, m.src->as<int>(), jd);
-        }, bytes + 16.0 * jd.n * jp.rows);
+            spgemm_planned_kernel<<<entry_blocks(op.nnz), kThreads, 0, c.stream>>>(
+                op.nnz, op.plan_start->as<int>(), op.plan_contrib->as<int>(), op.plan_jrow->as<int>(), jv, ov, jd);
+        }, bytes);
         return;
     }
     // algorithmic bytes: M (row pointers, sources, weights), the Jacobian
@@ -583,6 +771,7 @@ OpMatrixP opmat_from_host(Core& c, int n_out, int n_src, const std::vector<int32
     m->n_out = n_out;
     m->n_src = n_src;
     for (int i = 0; i < n_out; ++i) m->max_row = std::max(m->max_row, ptr[i + 1] - ptr[i]);
+    m->unit = std::all_of(w.begin(), w.end(), [](double x) { return x == 1.0 || x == -1.0; });
     m->nnz = (int64_t)src.size();
     m->ptr = c.allocN<int32_t>(ptr.size());
     m->src = c.allocN<int32_t>(src.empty() ? 1 : src.size());
@@ -603,6 +792,7 @@ OpMatrixP opmat_from_map(Core& c, const int32_t* map_dev, int n_out, int n_src, 
     m->n_out = n_out;
     m->n_src = n_src;
     m->max_row = 1;
+    m->unit = true;
     Buf cnt = c.allocN<int64_t>(n_out > 0 ? n_out : 1);
     Buf err = c.allocN<int32_t>(1);
     EQG_CUDA(cudaMemsetAsync(err->ptr, 0, 4, c.stream));
@@ -686,8 +876,8 @@ PatternP pattern_spgemm(Core& c, const OpMatrix& m, const PatternP& j, bool with
     case 8: spgemm_symbolic<8>(c, m, *j, *p); break;
     default: spgemm_symbolic<16>(c, m, *j, *p); break;
     }
-    // the position plan, when positions and streams fit its packing
-    if (with_plan && c.param_i("spgemm_plan", 1) != 0 && j->nnz <= kPlanMask && p->nnz < (int64_t)INT_MAX / 2) {
+    // the position plan, for weights of 1 and -1
+    if (with_plan && m.unit && c.param_i("spgemm_plan", 1) != 0 && p->nnz < (int64_t)INT_MAX / 2) {
         switch (kmax_for(m.max_row)) {
         case 1: spgemm_build_plan<1>(c, m, *j, *p); break;
         case 2: spgemm_build_plan<2>(c, m, *j, *p); break;
@@ -722,7 +912,7 @@ void jacobian_apply_deferred(Core& c, const Deferred& d, Pattern& p, const doubl
     if (p.nnz <= 0) return;
     pattern_build_rowidx(c, p);
     launch(c, "jac_deferred", [&] {
-        apply_deferred_kernel<<<blocksFor(p.nnz), kThreads, 0, c.stream>>>(d, p.rowidx->as<int>(), j, out, p.nnz);
+        apply_deferred_kernel<<<entry_blocks(p.nnz), kThreads, 0, c.stream>>>(d, p.rowidx->as<int>(), j, out, p.nnz);
     }, 20.0 * p.nnz + 4.0 * p.nnz + 16.0 * d.n * p.rows);
 }
 
@@ -826,7 +1016,7 @@ void jacobian_elementwise(Core& c, const JacArgs& a, const Pattern& out, double*
     if (flat) {
         pattern_build_rowidx(c, const_cast<Pattern&>(out));
         launch(c, "jac_flat", [&] {
-            ew_flat_kernel<<<blocksFor(out.nnz), kThreads, 0, c.stream>>>(
+            ew_flat_kernel<<<entry_blocks(out.nnz), kThreads, 0, c.stream>>>(
                 r, out.rowidx->as<int>(), a.pa ? a.ja : nullptr, a.pb ? a.jb : nullptr, jout, out.nnz, a.da, a.db);
         }, bytes);
     } else if (out.nnz < (int64_t)INT_MAX / 2) {
@@ -845,7 +1035,7 @@ void jacobian_elementwise(Core& c, const JacArgs& a, const Pattern& out, double*
             });
         }
         launch(c, "jac_merge", [&] {
-            ew_mapped_kernel<<<blocksFor(out.nnz), kThreads, 0, c.stream>>>(
+            ew_mapped_kernel<<<entry_blocks(out.nnz), kThreads, 0, c.stream>>>(
                 r, out.rowidx->as<int>(), maps->as<int>(), maps->as<int>() + out.nnz, a.pa ? a.ja : nullptr,
                 a.pb ? a.jb : nullptr, jout, out.nnz, a.da, a.db);
         }, bytes);
