@@ -87,13 +87,18 @@ enum { ST_RUN = 0, ST_CONV = 1, ST_BREAK = 2 };
 __device__ __forceinline__ bool stopped(const KScal* sc) { return sc->status != ST_RUN; }
 
 // Every kernel of a BiCGStab iteration calls this before it reads anything
-// that an earlier kernel wrote (first thing, except for the fused coarse
-// cycle's prefetches of constant data): those kernels are launched as
+// that an earlier kernel of the iterations wrote (first thing, except for
+// reads of the matrices, which the iterations do not write): those kernels are launched as
 // programmatic dependent launches (launch_k), so their blocks may be
 // scheduled while the kernel before them on the stream still runs; this
 // waits until that kernel has completed and its writes are visible (at once
 // when the kernel was launched normally).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// The kernel after this one may be scheduled from here on (once every block
+// of this one has come here): it finds SMs that this one leaves idle or has
+// left, and waits in its own pdl_wait.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 
 // Block-wide sum of NV values; returns sums to thread 0.
 template <int NV>
@@ -836,6 +841,7 @@ template <class T>
 __global__ void bicg_p_kernel(const T* __restrict__ r, const T* __restrict__ v, T* __restrict__ p, int n,
                               const KScal* sc)
 {
+    pdl_trigger();
     pdl_wait();
     if (stopped(sc)) return;
     const double beta = (sc->rho_new / sc->rho) * (sc->alpha / sc->omega);
@@ -903,6 +909,7 @@ template <class T>
 __global__ void bicg_s_kernel(const T* __restrict__ r, const T* __restrict__ v, T* __restrict__ s, int n,
                               double* partials, unsigned int* counter, KScal* sc)
 {
+    pdl_trigger();
     pdl_wait();
     if (stopped(sc)) return;
     const double alpha = sc->alpha;
@@ -975,6 +982,7 @@ __global__ void bicg_xr_kernel(const T* __restrict__ ph, const T* __restrict__ s
                                const T* __restrict__ t, const T* __restrict__ rhat, T* __restrict__ x,
                                T* __restrict__ r, int n, double* partials, unsigned int* counter, KScal* sc)
 {
+    pdl_trigger();
     pdl_wait();
     if (stopped(sc)) return;
     const double alpha = sc->alpha;

@@ -139,33 +139,60 @@ struct RbMatrix {
     static size_t values(int nd, int bb, int n, int nr) { return ((size_t)(nd + 1) * n + (n - nr)) * bb; }
 };
 
-// acc += sum over the neighbours of A_d x_d, directions in order, row q of
-// `rows`.  The loads are unconditional, so that all of them are issued before
+// One block of a level's matrix, which no kernel of a solve writes: read past
+// L1 (every block is used once per kernel), and where it stands relative to
+// pdl_wait (the assembly statements keep their order).
+template <int BB, class M>
+__device__ __forceinline__ void load_matrix(const M* p, M (&v)[BB])
+{
+    if constexpr (BB == 4 && sizeof(M) == 8) {
+        asm volatile("ld.global.nc.L1::no_allocate.v4.f64 {%0, %1, %2, %3}, [%4];"
+                     : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+    } else if constexpr (BB == 4) {
+        asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p));
+    } else if constexpr (sizeof(M) == 8) {
+#pragma unroll
+        for (int e = 0; e < BB; ++e) asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v[e]) : "l"(p + e));
+    } else {
+#pragma unroll
+        for (int e = 0; e < BB; ++e) asm volatile("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v[e]) : "l"(p + e));
+    }
+}
+
+// A row's off-diagonal blocks and its neighbours' numbers.  load() reads
+// nothing that a solve writes; dot() adds sum A_d x_d to acc, directions in
+// order.  The loads are unconditional, so that all of them are issued before
 // the first sum (with a branch per neighbour the compiler waited for each one
 // in turn, in 34 registers): the block of a missing neighbour is stored as
 // zero, and the vector is then read at the row's own number, or the last one.
 template <int B, int ND, class M>
-__device__ __forceinline__ void stencil_dot(const RbGrid& g, const Cell& e, int q, int rows, const M* __restrict__ a,
-                                            const double* __restrict__ x, double (&acc)[B])
-{
-    constexpr int BB = B * B;
-    M av[ND][BB];
-    double xv[ND][B];
-    const int own = min(q, g.n - rows - 1);  // the other colour has n - rows cells
+struct StencilRow {
+    M av[ND][B * B];
+    int nq[ND];
+    // row q of `rows`, cell e
+    __device__ __forceinline__ void load(const RbGrid& g, const Cell& e, int q, int rows, const M* a)
+    {
+        const int own = max(min(q, g.n - rows - 1), 0);  // the other colour has n - rows cells
 #pragma unroll
-    for (int d = 0; d < ND; ++d) {
-        int nq;
-        if (!neighbour(g, e, d, nq)) nq = own;
-        load_block<BB, M>(a + ((size_t)d * rows + q) * BB, av[d]);
-        load_bvec<B, double>(x, nq, xv[d]);
+        for (int d = 0; d < ND; ++d) {
+            if (!neighbour(g, e, d, nq[d])) nq[d] = own;
+            load_matrix<B * B, M>(a + ((size_t)d * rows + q) * (B * B), av[d]);
+        }
     }
+    __device__ __forceinline__ void dot(const double* x, double (&acc)[B]) const
+    {
+        double xv[ND][B];
 #pragma unroll
-    for (int d = 0; d < ND; ++d)
+        for (int d = 0; d < ND; ++d) load_bvec<B, double>(x, nq[d], xv[d]);
 #pragma unroll
-        for (int i = 0; i < B; ++i)
+        for (int d = 0; d < ND; ++d)
 #pragma unroll
-            for (int j = 0; j < B; ++j) acc[i] = __fma_rn((double)av[d][i * B + j], xv[d][j], acc[i]);
-}
+            for (int i = 0; i < B; ++i)
+#pragma unroll
+                for (int j = 0; j < B; ++j) acc[i] = __fma_rn((double)av[d][i * B + j], xv[d][j], acc[i]);
+    }
+};
 
 // y = D x of one block.
 template <int B, class M>
@@ -225,12 +252,17 @@ template <int B>
 struct UpRow {
     int c[4];
     double f[4][B];
-    template <bool CG>
-    __device__ __forceinline__ void load(const UpView& u, const Cell& e)
+    __device__ __forceinline__ void members(const UpView& u, const Cell& e)
+    {
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+            c[s] = u.w != nullptr && s < u.agg.g ? black_member(u.agg, e.i, e.j, e.k, s) : -1;
+    }
+    template <bool CG = false>
+    __device__ __forceinline__ void load(const UpView& u)
     {
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
-            c[s] = u.w != nullptr && s < u.agg.g ? black_member(u.agg, e.i, e.j, e.k, s) : -1;
 #pragma unroll
             for (int t = 0; t < B; ++t) f[s][t] = 0.0;
             if (u.add && c[s] >= 0) load_bvec<B, double, CG>(u.w, c[s] >> 1, f[s]);
@@ -248,90 +280,131 @@ struct UpRow {
 };
 
 // ---- the steps ------------------------------------------------------------------
-// Loops over the rows of a colour for thread `tid` of `nth`.  The resident
-// coarse cycle below computes every element alike (operations written out:
-// the compiler contracted products and sums differently there).  rr, y: red vectors (rr null: zero), rb,
-// z: black ones.
+// One kernel per step.  The resident coarse cycle below computes every
+// element alike (operations written out: the compiler contracted products and
+// sums differently there).  rr, y: red vectors (rr null: zero), rb, z: black
+// ones.
 
+// Rows tid, tid + nth, ... of `rows`: load(q) reads what no kernel of the
+// solve writes (matrix blocks, neighbours' numbers), run(q) the rest.  The
+// kernel after this one may start as soon as every block here has, and the
+// first row's load comes before the wait for the kernel ahead: a step's
+// matrix, most of its bytes, comes in while the step before it ends, on SMs
+// that this one does not need or has left.  The matrices were complete before
+// the solve's first kernel, which is launched without that liberty.  Krylov
+// iterations of a step, without and with it: two-phase 48x40 2.77 -> 2.49 ms,
+// 255x257 mixed 6.4 -> 5.8, 512x512 10.4 -> 8.9, 33x31x17 7.0 -> 6.2,
+// 128x128x64 45.2 -> 43.8 (its finest level takes seven waves of blocks, of
+// which only the first gains).  False: nothing ran.
+template <class Load, class Run>
+__device__ __forceinline__ bool for_rows(int rows, const KScal* sc, int skip_if_s, Load&& load, Run&& run)
+{
+    pdl_trigger();
+    const int tid = (int)(blockIdx.x * blockDim.x + threadIdx.x), nth = (int)(gridDim.x * blockDim.x);
+    if (tid < rows) load(tid);
+    pdl_wait();
+    if (mg_skip(sc, skip_if_s)) return false;
+    for (int q = tid; q < rows; q += nth) {
+        if (q != tid) load(q);
+        run(q);
+    }
+    return true;
+}
+
+// v = rr - U z of red row q.
 template <int B, int ND, class M>
-__device__ __forceinline__ void red_row(const RbGrid& g, const Cell& e, int q, const M* U, const double* rr,
-                                        const double* z, double (&v)[B])
+__device__ __forceinline__ void red_row(const StencilRow<B, ND, M>& row, int q, const double* rr, const double* z,
+                                        double (&v)[B])
 {
     double acc[B];
 #pragma unroll
     for (int t = 0; t < B; ++t) acc[t] = v[t] = 0.0;
     if (rr) load_bvec<B, double>(rr, q, v);
-    stencil_dot<B, ND, M>(g, e, q, g.nr, U, z, acc);
+    row.dot(z, acc);
 #pragma unroll
     for (int t = 0; t < B; ++t) v[t] = __dsub_rn(v[t], acc[t]);
 }
 
-// y = rr - U z
+// t = rb - A_bb z - L y of one black row: the blocks of L in row, A_bb in av.
 template <int B, int ND, class M>
-__device__ __forceinline__ void rb_y_rows(const RbGrid& g, const RbMatrix<const M>& m, const double* rr,
-                                          const double* z, double* y, int tid, int nth)
-{
-    for (int q = tid; q < g.nr; q += nth) {
-        double v[B];
-        red_row<B, ND, M>(g, cell_of(g, 0, q), q, m.U, rr, z, v);
-        store_bvec<B, double>(y, q, v);
-    }
-}
-
-// D_r^-1 (rr - U z), handed to the finer level (nothing else reads it).
-template <int B, int ND, class M>
-__device__ __forceinline__ void rb_fin_rows(const RbGrid& g, const RbMatrix<const M>& m, const double* rr,
-                                            const double* z, const UpView& up, int tid, int nth)
-{
-    for (int q = tid; q < g.nr; q += nth) {
-        const Cell e = cell_of(g, 0, q);
-        M dv[B * B];
-        double v[B], x[B];
-        UpRow<B> fine;
-        fine.template load<false>(up, e);
-        load_block<B * B, M>(m.dr + (size_t)q * B * B, dv);
-        red_row<B, ND, M>(g, e, q, m.U, rr, z, v);
-        block_mul<B, M>(dv, v, x);
-        fine.store(up, x);
-    }
-}
-
-// z = D_b^-1 (rb - L rr): the sweep from z = 0.
-template <int B, int ND, class M>
-__device__ __forceinline__ void rb_pre_rows(const RbGrid& g, const RbMatrix<const M>& m, const double* rr,
-                                            const double* rb, double* z, int tid, int nth)
-{
-    const int nk = g.n - g.nr;
-    for (int q = tid; q < nk; q += nth) {
-        M dv[B * B];
-        double acc[B], v[B], x[B];
-#pragma unroll
-        for (int t = 0; t < B; ++t) acc[t] = 0.0;
-        load_bvec<B, double>(rb, q, v);
-        load_block<B * B, M>(m.db + (size_t)q * B * B, dv);
-        if (rr) stencil_dot<B, ND, M>(g, cell_of(g, 1, q), q, nk, m.L, rr, acc);
-#pragma unroll
-        for (int t = 0; t < B; ++t) v[t] = __dsub_rn(v[t], acc[t]);
-        block_mul<B, M>(dv, v, x);
-        store_bvec<B, double>(z, q, x);
-    }
-}
-
-// t = rb - A_bb z - L y of one black row.
-template <int B, int ND, class M>
-__device__ __forceinline__ void residual_row(const RbGrid& g, const Cell& e, int q, const RbMatrix<const M>& m,
+__device__ __forceinline__ void residual_row(const StencilRow<B, ND, M>& row, const M (&av)[B * B], int q,
                                              const double* rb, const double* y, const double (&z)[B], double (&t)[B])
 {
-    M av[B * B];
     double acc[B], az[B];
 #pragma unroll
     for (int c = 0; c < B; ++c) acc[c] = 0.0;
     load_bvec<B, double>(rb, q, t);
-    load_block<B * B, M>(m.abb + (size_t)q * B * B, av);
-    stencil_dot<B, ND, M>(g, e, q, g.n - g.nr, m.L, y, acc);
+    row.dot(y, acc);
     block_mul<B, M>(av, z, az);
 #pragma unroll
     for (int c = 0; c < B; ++c) t[c] = __dsub_rn(__dsub_rn(t[c], az[c]), acc[c]);
+}
+
+// y = rr - U z
+template <int B, int ND, class M>
+__global__ void __launch_bounds__(512, 1) rb_y_kernel(RbGrid g, RbMatrix<const M> m, const double* rr, const double* z,
+                                                   double* y, const KScal* sc, int skip_if_s)
+{
+    StencilRow<B, ND, M> row;
+    for_rows(
+        g.nr, sc, skip_if_s, [&](int q) { row.load(g, cell_of(g, 0, q), q, g.nr, m.U); },
+        [&](int q) {
+            double v[B];
+            red_row<B, ND, M>(row, q, rr, z, v);
+            store_bvec<B, double>(y, q, v);
+        });
+}
+
+// D_r^-1 (rr - U z), handed to the finer level (nothing else reads it).
+template <int B, int ND, class M>
+__global__ void __launch_bounds__(512, 1) rb_fin_kernel(RbGrid g, RbMatrix<const M> m, const double* rr, const double* z,
+                                                     UpView up, const KScal* sc, int skip_if_s)
+{
+    StencilRow<B, ND, M> row;
+    UpRow<B> fine;
+    M dv[B * B];
+    for_rows(
+        g.nr, sc, skip_if_s,
+        [&](int q) {
+            const Cell e = cell_of(g, 0, q);
+            row.load(g, e, q, g.nr, m.U);
+            load_matrix<B * B, M>(m.dr + (size_t)q * B * B, dv);
+            fine.members(up, e);
+        },
+        [&](int q) {
+            double v[B], x[B];
+            fine.load(up);
+            red_row<B, ND, M>(row, q, rr, z, v);
+            block_mul<B, M>(dv, v, x);
+            fine.store(up, x);
+        });
+}
+
+// z = D_b^-1 (rb - L rr): the sweep from z = 0.
+template <int B, int ND, class M>
+__global__ void __launch_bounds__(512, 1) rb_pre_kernel(RbGrid g, RbMatrix<const M> m, const double* rr, const double* rb,
+                                                     double* z, const KScal* sc, int skip_if_s)
+{
+    const int nk = g.n - g.nr;
+    StencilRow<B, ND, M> row;
+    M dv[B * B];
+    for_rows(
+        nk, sc, skip_if_s,
+        [&](int q) {
+            if (rr) row.load(g, cell_of(g, 1, q), q, nk, m.L);
+            load_matrix<B * B, M>(m.db + (size_t)q * B * B, dv);
+        },
+        [&](int q) {
+            double acc[B], v[B], x[B];
+#pragma unroll
+            for (int t = 0; t < B; ++t) acc[t] = 0.0;
+            load_bvec<B, double>(rb, q, v);
+            if (rr) row.dot(rr, acc);
+#pragma unroll
+            for (int t = 0; t < B; ++t) v[t] = __dsub_rn(v[t], acc[t]);
+            block_mul<B, M>(dv, v, x);
+            store_bvec<B, double>(z, q, x);
+        });
 }
 
 // Coarse right-hand side: the sum of t over the black members of each
@@ -339,77 +412,100 @@ __device__ __forceinline__ void residual_row(const RbGrid& g, const Cell& e, int
 // member's row follows its neighbour's: whole segments), summed by a
 // butterfly over the g lanes.  rc: red coarse cells, then black ones.
 template <int B, int ND, class M>
-__device__ __forceinline__ void rb_res_rows(const Aggregates& a, const RbMatrix<const M>& m, const double* rb,
-                                            const double* y, const double* z, double* rc, int tid, int nth)
+__global__ void __launch_bounds__(512, 1) rb_res_kernel(Aggregates a, RbMatrix<const M> m, const double* rb,
+                                                     const double* y, const double* z, double* rc, const KScal* sc,
+                                                     int skip_if_s)
 {
     const int items = a.coarse.n * a.g, padded = (items + 31) & ~31, lg = a.g == 4 ? 2 : a.g - 1;
-    for (int it = tid; it < padded; it += nth) {
-        const Cell C = cell_at(a.coarse, it < items ? it >> lg : 0);
-        const int c = it < items ? black_member(a, C.i, C.j, C.k, it & (a.g - 1)) : -1;
-        double t[B];
+    const int nk = a.fine.n - a.fine.nr;
+    StencilRow<B, ND, M> row;
+    M av[B * B];
+    Cell C;
+    int c = -1;
+    for_rows(
+        padded, sc, skip_if_s,
+        [&](int it) {
+            C = cell_at(a.coarse, it < items ? it >> lg : 0);
+            c = it < items ? black_member(a, C.i, C.j, C.k, it & (a.g - 1)) : -1;
+            if (c < 0) return;
+            row.load(a.fine, cell_at(a.fine, c), c >> 1, nk, m.L);
+            load_matrix<B * B, M>(m.abb + (size_t)(c >> 1) * B * B, av);
+        },
+        [&](int it) {
+            double t[B];
 #pragma unroll
-        for (int v = 0; v < B; ++v) t[v] = 0.0;
-        if (c >= 0) {
-            const int q = c >> 1;
-            double zv[B];
-            load_bvec<B, double>(z, q, zv);
-            residual_row<B, ND, M>(a.fine, cell_at(a.fine, c), q, m, rb, y, zv, t);
-        }
-        for (int o = 1; o < a.g; o <<= 1)
+            for (int v = 0; v < B; ++v) t[v] = 0.0;
+            if (c >= 0) {
+                double zv[B];
+                load_bvec<B, double>(z, c >> 1, zv);
+                residual_row<B, ND, M>(row, av, c >> 1, rb, y, zv, t);
+            }
+            for (int o = 1; o < a.g; o <<= 1)
 #pragma unroll
-            for (int v = 0; v < B; ++v) t[v] += __shfl_xor_sync(0xffffffffu, t[v], o);
-        if (it < items && (it & (a.g - 1)) == 0)
-            store_bvec<B, double>(rc, (C.c >> 1) + (((C.i + C.j + C.k) & 1) ? a.coarse.nr : 0), t);
-    }
+                for (int v = 0; v < B; ++v) t[v] += __shfl_xor_sync(0xffffffffu, t[v], o);
+            if (it < items && (it & (a.g - 1)) == 0)
+                store_bvec<B, double>(rc, (C.c >> 1) + (((C.i + C.j + C.k) & 1) ? a.coarse.nr : 0), t);
+        });
 }
 
 // The same of the right-hand side itself (rr null: zero), for a level
 // without pre-smoothing: pairs, a black member and the red one beside it.
 template <int B>
-__device__ __forceinline__ void rb_restrict_rows(const Aggregates& a, const double* rr, const double* rb, double* rc,
-                                                 int tid, int nth)
+__global__ void __launch_bounds__(512, 1) rb_restrict_kernel(Aggregates a, const double* rr, const double* rb, double* rc,
+                                                          const KScal* sc, int skip_if_s)
 {
-    for (int p = tid; p < a.coarse.n; p += nth) {
-        const Cell C = cell_at(a.coarse, p);
-        double s[B];
+    for_rows(
+        a.coarse.n, sc, skip_if_s, [](int) {},
+        [&](int p) {
+            const Cell C = cell_at(a.coarse, p);
+            double s[B];
 #pragma unroll
-        for (int t = 0; t < B; ++t) s[t] = 0.0;
-        const int i0 = C.i << a.sx, j0 = C.j << a.sy, k0 = C.k << a.sz;
-        for (int o = 0; o < (1 << (a.sx + a.sy + a.sz)); ++o) {
-            const int i = i0 + (a.sx ? o & 1 : 0), j = j0 + (a.sy ? (o >> a.sx) & 1 : 0), k = k0 + (a.sz ? o >> (a.sx + a.sy) : 0);
-            if (i >= a.fine.nx || j >= a.fine.ny || k >= a.fine.nz) continue;
-            const double* r = ((i + j + k) & 1) ? rb : rr;
-            if (!r) continue;
-            double v[B];
-            load_bvec<B, double>(r, (i + a.fine.nx * (j + a.fine.ny * k)) >> 1, v);
+            for (int t = 0; t < B; ++t) s[t] = 0.0;
+            const int i0 = C.i << a.sx, j0 = C.j << a.sy, k0 = C.k << a.sz;
+            for (int o = 0; o < (1 << (a.sx + a.sy + a.sz)); ++o) {
+                const int i = i0 + (a.sx ? o & 1 : 0), j = j0 + (a.sy ? (o >> a.sx) & 1 : 0),
+                          k = k0 + (a.sz ? o >> (a.sx + a.sy) : 0);
+                if (i >= a.fine.nx || j >= a.fine.ny || k >= a.fine.nz) continue;
+                const double* r = ((i + j + k) & 1) ? rb : rr;
+                if (!r) continue;
+                double v[B];
+                load_bvec<B, double>(r, (i + a.fine.nx * (j + a.fine.ny * k)) >> 1, v);
 #pragma unroll
-            for (int t = 0; t < B; ++t) s[t] += v[t];
-        }
-        store_bvec<B, double>(rc, (p >> 1) + (((C.i + C.j + C.k) & 1) ? a.coarse.nr : 0), s);
-    }
+                for (int t = 0; t < B; ++t) s[t] += v[t];
+            }
+            store_bvec<B, double>(rc, (p >> 1) + (((C.i + C.j + C.k) & 1) ? a.coarse.nr : 0), s);
+        });
 }
 
 // z += D_b^-1 (rb - A_bb z - L y), handed to the finer level.
 template <int B, int ND, class M>
-__device__ __forceinline__ void rb_post_rows(const RbGrid& g, const RbMatrix<const M>& m, const double* rb,
-                                             const double* y, double* z, const UpView& up, int tid, int nth)
+__global__ void __launch_bounds__(512, 1) rb_post_kernel(RbGrid g, RbMatrix<const M> m, const double* rb, const double* y,
+                                                      double* z, UpView up, const KScal* sc, int skip_if_s)
 {
     const int nk = g.n - g.nr;
-    for (int q = tid; q < nk; q += nth) {
-        const Cell e = cell_of(g, 1, q);
-        M dv[B * B];
-        double zv[B], t[B], x[B];
-        UpRow<B> fine;
-        fine.template load<false>(up, e);
-        load_bvec<B, double>(z, q, zv);
-        load_block<B * B, M>(m.db + (size_t)q * B * B, dv);
-        residual_row<B, ND, M>(g, e, q, m, rb, y, zv, t);
-        block_mul<B, M>(dv, t, x);
+    StencilRow<B, ND, M> row;
+    UpRow<B> fine;
+    M av[B * B], dv[B * B];
+    for_rows(
+        nk, sc, skip_if_s,
+        [&](int q) {
+            const Cell e = cell_of(g, 1, q);
+            row.load(g, e, q, nk, m.L);
+            load_matrix<B * B, M>(m.abb + (size_t)q * B * B, av);
+            load_matrix<B * B, M>(m.db + (size_t)q * B * B, dv);
+            fine.members(up, e);
+        },
+        [&](int q) {
+            double zv[B], t[B], x[B];
+            fine.load(up);
+            load_bvec<B, double>(z, q, zv);
+            residual_row<B, ND, M>(row, av, q, rb, y, zv, t);
+            block_mul<B, M>(dv, t, x);
 #pragma unroll
-        for (int c = 0; c < B; ++c) zv[c] = __dadd_rn(zv[c], x[c]);
-        store_bvec<B, double>(z, q, zv);
-        fine.store(up, zv);
-    }
+            for (int c = 0; c < B; ++c) zv[c] = __dadd_rn(zv[c], x[c]);
+            store_bvec<B, double>(z, q, zv);
+            fine.store(up, zv);
+        });
 }
 
 // The coarsest level: inv r, a warp per unknown (see dense_rows; red cells,
@@ -436,72 +532,11 @@ __device__ __forceinline__ void rb_dense_rows(const RbGrid& g, const M* __restri
     }
 }
 
-// ---- one step per launch ------------------------------------------------------
-template <int B, int ND, class M>
-__global__ void __launch_bounds__(512, 1) rb_y_kernel(RbGrid g, RbMatrix<const M> m, const double* rr, const double* z,
-                                                   double* y, const KScal* sc, int skip_if_s)
-{
-    pdl_wait();
-    if (mg_skip(sc, skip_if_s)) return;
-    THREAD_RANGE;
-    rb_y_rows<B, ND, M>(g, m, rr, z, y, tid, nth);
-}
-
-template <int B, int ND, class M>
-__global__ void __launch_bounds__(512, 1) rb_fin_kernel(RbGrid g, RbMatrix<const M> m, const double* rr, const double* z,
-                                                     UpView up, const KScal* sc, int skip_if_s)
-{
-    pdl_wait();
-    if (mg_skip(sc, skip_if_s)) return;
-    THREAD_RANGE;
-    rb_fin_rows<B, ND, M>(g, m, rr, z, up, tid, nth);
-}
-
-template <int B, int ND, class M>
-__global__ void __launch_bounds__(512, 1) rb_pre_kernel(RbGrid g, RbMatrix<const M> m, const double* rr, const double* rb,
-                                                     double* z, const KScal* sc, int skip_if_s)
-{
-    pdl_wait();
-    if (mg_skip(sc, skip_if_s)) return;
-    THREAD_RANGE;
-    rb_pre_rows<B, ND, M>(g, m, rr, rb, z, tid, nth);
-}
-
-template <int B, int ND, class M>
-__global__ void __launch_bounds__(512, 1) rb_res_kernel(Aggregates a, RbMatrix<const M> m, const double* rb,
-                                                     const double* y, const double* z, double* rc, const KScal* sc,
-                                                     int skip_if_s)
-{
-    pdl_wait();
-    if (mg_skip(sc, skip_if_s)) return;
-    THREAD_RANGE;
-    rb_res_rows<B, ND, M>(a, m, rb, y, z, rc, tid, nth);
-}
-
-template <int B>
-__global__ void __launch_bounds__(512, 1) rb_restrict_kernel(Aggregates a, const double* rr, const double* rb, double* rc,
-                                                          const KScal* sc, int skip_if_s)
-{
-    pdl_wait();
-    if (mg_skip(sc, skip_if_s)) return;
-    THREAD_RANGE;
-    rb_restrict_rows<B>(a, rr, rb, rc, tid, nth);
-}
-
-template <int B, int ND, class M>
-__global__ void __launch_bounds__(512, 1) rb_post_kernel(RbGrid g, RbMatrix<const M> m, const double* rb, const double* y,
-                                                      double* z, UpView up, const KScal* sc, int skip_if_s)
-{
-    pdl_wait();
-    if (mg_skip(sc, skip_if_s)) return;
-    THREAD_RANGE;
-    rb_post_rows<B, ND, M>(g, m, rb, y, z, up, tid, nth);
-}
-
 template <int B, class M>
 __global__ void __launch_bounds__(1024) rb_dense_kernel(RbGrid g, const M* __restrict__ inv, const double* r, UpView up,
                                                         const KScal* sc, int skip_if_s)
 {
+    pdl_trigger();
     pdl_wait();
     if (mg_skip(sc, skip_if_s)) return;
     rb_dense_rows<B, M>(g, inv, r, up, (int)threadIdx.x, (int)blockDim.x);
@@ -547,7 +582,9 @@ __global__ void __launch_bounds__(kThreads) rb_init_kernel(RbGrid g, RbMatrix<co
         double acc[B];
 #pragma unroll
         for (int t = 0; t < B; ++t) acc[t] = 0.0;
-        stencil_dot<B, ND, double>(g, cell_of(g, 1, q), q, nk, m.L, b, acc);
+        StencilRow<B, ND, double> row;
+        row.load(g, cell_of(g, 1, q), q, nk, m.L);
+        row.dot(b, acc);
         load_bvec<B, double>(bb, q, w);
 #pragma unroll
         for (int t = 0; t < B; ++t) {
@@ -582,38 +619,41 @@ __global__ void __launch_bounds__(kThreads) rb_init_kernel(RbGrid g, RbMatrix<co
 // bicg_spmv_omega (omega = (v . h) / (v . v), h = s).
 template <int B, int ND, bool OMEGA>
 __global__ void __launch_bounds__(kThreads, 2)
-    rb_spmv_kernel(RbGrid g, RbMatrix<const double> m, const double* __restrict__ z, const double* __restrict__ y,
-                   const double* __restrict__ h, double* __restrict__ v, double* partials, unsigned int* counter,
+    rb_spmv_kernel(RbGrid g, RbMatrix<const double> m, const double* z, const double* y, const double* h, double* v,
+                   double* partials, unsigned int* counter,
                    KScal* sc)
 {
-    pdl_wait();
-    if (stopped(sc) || (OMEGA && sc->s_conv)) return;
     constexpr int ND_ = OMEGA ? 2 : 1;
     const int nk = g.n - g.nr;
     double d[ND_];
 #pragma unroll
     for (int k = 0; k < ND_; ++k) d[k] = 0.0;
-    GRID_STRIDE(q64, nk)
-    {
-        const int q = (int)q64;
-        double acc[B], zv[B], az[B], hv[B];
+    StencilRow<B, ND, double> row;
+    double av[B * B];
+    const bool ran = for_rows(
+        nk, sc, OMEGA,
+        [&](int q) {
+            row.load(g, cell_of(g, 1, q), q, nk, m.L);
+            load_matrix<B * B, double>(m.abb + (size_t)q * B * B, av);
+        },
+        [&](int q) {
+            double acc[B], zv[B], az[B], hv[B];
 #pragma unroll
-        for (int t = 0; t < B; ++t) acc[t] = 0.0;
-        double av[B * B];
-        load_bvec<B, double>(z, q, zv);
-        load_bvec<B, double>(h, q, hv);
-        load_block<B * B, double>(m.abb + (size_t)q * B * B, av);
-        stencil_dot<B, ND, double>(g, cell_of(g, 1, q), q, nk, m.L, y, acc);
-        block_mul<B, double>(av, zv, az);
+            for (int t = 0; t < B; ++t) acc[t] = 0.0;
+            load_bvec<B, double>(z, q, zv);
+            load_bvec<B, double>(h, q, hv);
+            row.dot(y, acc);
+            block_mul<B, double>(av, zv, az);
 #pragma unroll
-        for (int t = 0; t < B; ++t) acc[t] += az[t];
-        store_bvec<B, double>(v, q, acc);
+            for (int t = 0; t < B; ++t) acc[t] += az[t];
+            store_bvec<B, double>(v, q, acc);
 #pragma unroll
-        for (int t = 0; t < B; ++t) {
-            d[0] += hv[t] * acc[t];
-            if (OMEGA) d[ND_ - 1] += acc[t] * acc[t];
-        }
-    }
+            for (int t = 0; t < B; ++t) {
+                d[0] += hv[t] * acc[t];
+                if (OMEGA) d[ND_ - 1] += acc[t] * acc[t];
+            }
+        });
+    if (!ran) return;  // the same in every block
     double s[ND_];
     if (grid_sum<ND_>(d, partials, counter, s)) {
         if (OMEGA) {
@@ -642,8 +682,10 @@ __global__ void __launch_bounds__(kThreads) rb_solution_kernel(RbGrid g, RbMatri
         const Cell e = cell_of(g, 0, q);
         double v[B], z[B];
         double dv[B * B];
-        load_block<B * B, double>(m.dr + (size_t)q * B * B, dv);
-        red_row<B, ND, double>(g, e, q, m.U, b, x, v);
+        StencilRow<B, ND, double> row;
+        row.load(g, e, q, g.nr, m.U);
+        load_matrix<B * B, double>(m.dr + (size_t)q * B * B, dv);
+        red_row<B, ND, double>(row, q, b, x, v);
         block_mul<B, double>(dv, v, z);
 #pragma unroll
         for (int t = 0; t < B; ++t) out[(size_t)t * g.n + e.c] = z[t];
@@ -1183,7 +1225,10 @@ __device__ __forceinline__ void tail_up(const RbTailParams<M>& p, const RbTailVi
         M av[BB], dv[BB];
         double acc[B], az[B], z[B], t[B], x[B];
         UpRow<B> fine;
-        if (up.w) fine.template load<true>(up, e);
+        if (up.w) {
+            fine.members(up, e);
+            fine.template load<true>(up);
+        }
 #pragma unroll
         for (int c = 0; c < B; ++c) acc[c] = 0.0;
         z0_at<B, ND, M>(V, C, e, q, z);
@@ -1210,7 +1255,10 @@ __device__ __forceinline__ void tail_up(const RbTailParams<M>& p, const RbTailVi
         M dv[BB];
         double acc[B], v[B], x[B];
         UpRow<B> fine;
-        if (up.w) fine.template load<true>(up, e);
+        if (up.w) {
+            fine.members(up, e);
+            fine.template load<true>(up);
+        }
 #pragma unroll
         for (int t = 0; t < B; ++t) acc[t] = v[t] = 0.0;
         load_block<BB, M>(V.dr + (size_t)ql * BB, dv);
@@ -1282,6 +1330,7 @@ __global__ void __launch_bounds__(kTailThreads, 1)
     const int tid = (int)threadIdx.x, nth = (int)blockDim.x;
     // the matrices do not change during a solve: copied before the wait for
     // the previous kernel
+    pdl_trigger();
     tail_copies<B, ND, M>(p, tail_smem, rank, nblocks);
     pdl_wait();
     if (mg_skip(sc, skip_if_s)) {  // the same in every block
