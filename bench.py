@@ -59,7 +59,8 @@ KRYLOV_KERNELS = {"bicg_p", "bicg_spmv_alpha", "bicg_s", "bicg_spmv_omega", "bic
                   "rb_spmv_y", "rb_spmv_alpha", "rb_spmv_omega",
                   "residual", "add_float", "sumsq"}
 SETUP_KERNELS = {"bicg_init", "gather_values", "mg_galerkin", "mg_ap_values", "bilu_factor", "mg_dense_inverse",
-                 "to_float", "permute", "unpermute", "mg_strength", "rb_init", "rb_solution"}
+                 "to_float", "permute", "unpermute", "mg_strength", "rb_init", "rb_solution", "rb_map", "rb_factor_red",
+                 "rb_factor_black"}
 
 
 def parse():

@@ -1200,10 +1200,25 @@ __global__ void dense_fill_kernel(int nb, SellView m, const double* __restrict__
     }
 }
 
+// v[i] of a register array by a run-time index, five selections deep (an index
+// into the array would put it in local memory).
+template <int N>
+__device__ __forceinline__ double select_of(const double (&v)[N], int i)
+{
+    if constexpr (N == 1) {
+        return v[0];
+    } else {
+        double h[N / 2];
+#pragma unroll
+        for (int m = 0; m < N / 2; ++m) h[m] = i & N / 2 ? v[m + N / 2] : v[m];
+        return select_of<N / 2>(h, i);
+    }
+}
+
 // Inverse of the coarsest matrix (n <= kCoarsest unknowns, dense, row-major),
 // in place, by one thread block: Gauss-Jordan elimination with partial
 // pivoting, rows left where they are.  Thread (t, j) keeps the entries of
-// column j in rows t, t + 4, ... in registers; per step k the threads of
+// column j in rows M t ... M t + M - 1 in registers; per step k the threads of
 // column k publish it, every warp finds the largest entry among the rows that
 // have been no pivot yet (the lowest row among equals), the threads of that
 // row p publish it divided by the pivot (its entry in column k becomes
@@ -1215,19 +1230,25 @@ __global__ void dense_fill_kernel(int nb, SellView m, const double* __restrict__
 // Bound: the chain of two barriers, a reduction and a division per step.
 // n = 128: 586 us with the matrix in shared memory and row swaps (three
 // barriers, a 2 x 128 KB sweep and an index division per entry and step),
-// 196 us from registers; n = 60: 91 us.
+// 196 us from registers with rows t, t + 4, ... a thread, which read the
+// column in single values and picked the pivot's row in 32 dependent
+// selections, 183 us so (with the two-colour form's dense fill, 6 us); n = 60:
+// 91 and 67 us (warps without a row or column of the matrix only take part in
+// the barriers).
 constexpr int kInverseThreads = 512;
 
-__global__ void __launch_bounds__(kInverseThreads, 1) dense_inverse_kernel(int n, double* __restrict__ a, int* status)
+__device__ __forceinline__ void dense_inverse_block(int n, double* __restrict__ a, int* status)
 {
-    __shared__ double colk[2][kCoarsest], rowp[kCoarsest];
+    __shared__ __align__(16) double colk[2][kCoarsest];
+    __shared__ double rowp[kCoarsest];
     __shared__ int piv[kCoarsest], step_of[kCoarsest];  // pivot row of each step, and its inverse
     constexpr int T = kInverseThreads / kCoarsest, M = kCoarsest / T;
     const int j = threadIdx.x & (kCoarsest - 1), t = threadIdx.x / kCoarsest, lane = threadIdx.x & 31;
+    const bool active = (j & ~31) < n && t * M < n;  // the same in a warp
     double w[M];
 #pragma unroll
     for (int m = 0; m < M; ++m) {
-        const int r = t + T * m;
+        const int r = t * M + m;
         w[m] = r < n && j < n ? a[r * n + j] : 0.0;
         if (j == 0) colk[0][r] = w[m];
     }
@@ -1238,54 +1259,55 @@ __global__ void __launch_bounds__(kInverseThreads, 1) dense_inverse_kernel(int n
     for (int k = 0; k < n; ++k) {
         const double* col = colk[k & 1];
         __syncthreads();
-        // the lane's best row, then the warp's: magnitudes compare as their bits
-        unsigned hi = 0, lo = 0;
-        int row = kCoarsest;
-#pragma unroll
-        for (int i = 0; i < kCoarsest / 32; ++i) {
-            if (used >> i & 1) continue;
-            const double v = col[lane + 32 * i];
-            const unsigned h = (unsigned)__double2hiint(v) & 0x7fffffffu, l = (unsigned)__double2loint(v);
-            if (row == kCoarsest || h > hi || (h == hi && l > lo)) {
-                hi = h;
-                lo = l;
-                row = lane + 32 * i;
-            }
-        }
-        const unsigned top = __reduce_max_sync(0xffffffffu, row < kCoarsest ? hi : 0u);
-        const bool in_hi = row < kCoarsest && hi == top;
-        const unsigned top_lo = __reduce_max_sync(0xffffffffu, in_hi ? lo : 0u);
-        const int p = (int)__reduce_min_sync(0xffffffffu, in_hi && lo == top_lo ? (unsigned)row : (unsigned)kCoarsest);
-        if ((p & 31) == lane) used |= 1u << (p >> 5);
-        const double pv = col[p];
-        const bool mine = t == p % T;
+        int p = 0;
         double x = 0.0;
-        if (mine) {
-            // the row's place, selected place by place: an index into w would
-            // put it in local memory (pl is opaque to the compiler)
-            int pl = p / T;
+        if (active) {
+            // the lane's best row, then the warp's: magnitudes compare as their bits
+            unsigned hi = 0, lo = 0;
+            int row = kCoarsest;
 #pragma unroll
-            for (int m = 0; m < M; ++m) {
-                asm volatile("" : "+r"(pl));
-                x = pl == m ? w[m] : x;
+            for (int i = 0; i < kCoarsest / 32; ++i) {
+                if (used >> i & 1) continue;
+                const double v = col[lane + 32 * i];
+                const unsigned h = (unsigned)__double2hiint(v) & 0x7fffffffu, l = (unsigned)__double2loint(v);
+                if (row == kCoarsest || h > hi || (h == hi && l > lo)) {
+                    hi = h;
+                    lo = l;
+                    row = lane + 32 * i;
+                }
             }
-            x = (j == k ? 1.0 : x) / pv;
-            rowp[j] = x;
-        }
-        if (threadIdx.x == 0) {
-            piv[k] = p;
-            step_of[p] = k;
-            if (!(fabs(pv) > 0.0) || !isfinite(pv)) *status = 1;
+            const unsigned top = __reduce_max_sync(0xffffffffu, row < kCoarsest ? hi : 0u);
+            const bool in_hi = row < kCoarsest && hi == top;
+            const unsigned top_lo = __reduce_max_sync(0xffffffffu, in_hi ? lo : 0u);
+            p = (int)__reduce_min_sync(0xffffffffu, in_hi && lo == top_lo ? (unsigned)row : (unsigned)kCoarsest);
+            if ((p & 31) == lane) used |= 1u << (p >> 5);
+            const double pv = col[p];
+            if (t == p / M) {
+                x = (j == k ? 1.0 : select_of<M>(w, p % M)) / pv;
+                rowp[j] = x;
+            }
+            if (threadIdx.x == 0) {
+                piv[k] = p;
+                step_of[p] = k;
+                if (!(fabs(pv) > 0.0) || !isfinite(pv)) *status = 1;
+            }
         }
         __syncthreads();
+        if (!active) continue;
         const double g = rowp[j];
         if (j == k)
 #pragma unroll
             for (int m = 0; m < M; ++m) w[m] = 0.0;
 #pragma unroll
-        for (int m = 0; m < M; ++m) w[m] = __fma_rn(-g, col[t + T * m], w[m]);
-        if (mine) {
-            int pl = p / T;
+        for (int m = 0; m < M; m += 2) {
+            const double2 f = *reinterpret_cast<const double2*>(col + t * M + m);
+            w[m] = __fma_rn(-g, f.x, w[m]);
+            w[m + 1] = __fma_rn(-g, f.y, w[m + 1]);
+        }
+        if (t == p / M) {
+            // place by place; pl is opaque to the compiler, which made a jump
+            // per place of it
+            int pl = p % M;
 #pragma unroll
             for (int m = 0; m < M; ++m) {
                 asm volatile("" : "+r"(pl));
@@ -1294,15 +1316,21 @@ __global__ void __launch_bounds__(kInverseThreads, 1) dense_inverse_kernel(int n
         }
         if (j == k + 1)
 #pragma unroll
-            for (int m = 0; m < M; ++m) colk[(k + 1) & 1][t + T * m] = w[m];
+            for (int m = 0; m < M; m += 2)
+                *reinterpret_cast<double2*>(&colk[(k + 1) & 1][t * M + m]) = make_double2(w[m], w[m + 1]);
     }
     __syncthreads();
     if (j < n)
 #pragma unroll
         for (int m = 0; m < M; ++m) {
-            const int r = t + T * m;
+            const int r = t * M + m;
             if (r < n) a[step_of[r] * n + piv[j]] = w[m];
         }
+}
+
+__global__ void __launch_bounds__(kInverseThreads, 1) dense_inverse_kernel(int n, double* __restrict__ a, int* status)
+{
+    dense_inverse_block(n, a, status);
 }
 
 template <class T, class M>

@@ -809,31 +809,43 @@ __global__ void __launch_bounds__(kThreads) rb_galerkin_kernel(Aggregates a, int
         const bool red = ((C.i + C.j + C.k) & 1) == 0;
         const int q = c >> 1, rows = red ? g.nr : g.n - g.nr;
         double diag = 0.0, off[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        for (int o = 0; o < 8; ++o) {
-            const int dx = o & 1, dy = (o >> 1) & 1, dz = o >> 2;
-            if ((dx && !a.sx) || (dy && !a.sy) || (dz && !a.sz)) continue;
-            Cell m;
-            m.i = (C.i << a.sx) + dx;
-            m.j = (C.j << a.sy) + dy;
-            m.k = (C.k << a.sz) + dz;
-            if (m.i >= f.nx || m.j >= f.ny || m.k >= f.nz) continue;
-            m.c = m.i + f.nx * (m.j + f.ny * m.k);
-            const bool mr = ((m.i + m.j + m.k) & 1) == 0;
-            const int mq = m.c >> 1, mrows = mr ? f.nr : f.n - f.nr;
-            diag += (mr ? F.dr : F.abb)[(size_t)mq * bb + e];
+        const int nx = 1 << a.sx, ny = 1 << a.sy, nz = 1 << a.sz;
+        for (int dz = 0; dz < nz; ++dz)
+            for (int dy = 0; dy < ny; ++dy) {
+                // a member and the one beside it, or only it: their loads
+                // before the first sum (a missing neighbour's block is zero).
+                // A level of a few blocks waits for little else: 13 -> 5.3 us
+                double v[2][6], dd[2];
+                bool in[2];
 #pragma unroll
-            for (int d = 0; d < 6; ++d) {
-                if (d >= nd) break;
-                int nq;
-                if (!neighbour(f, m, d, nq)) continue;
-                const double v = (mr ? F.U : F.L)[((size_t)d * mrows + mq) * bb + e];
-                // inside the aggregate: the direction is paired and leads to
-                // the other half
-                const bool inner = d < 2 ? a.sx && dx != (d & 1) : d < 4 ? a.sy && dy != (d & 1) : a.sz && dz != (d & 1);
-                if (inner) diag += v;
-                else off[d] += v;
+                for (int dx = 0; dx < 2; ++dx) {
+                    Cell m;
+                    m.i = (C.i << a.sx) + dx;
+                    m.j = (C.j << a.sy) + dy;
+                    m.k = (C.k << a.sz) + dz;
+                    in[dx] = dx < nx && m.i < f.nx && m.j < f.ny && m.k < f.nz;
+                    m.c = in[dx] ? m.i + f.nx * (m.j + f.ny * m.k) : 0;
+                    const bool mr = ((m.i + m.j + m.k) & 1) == 0 || !in[dx];
+                    const int mq = m.c >> 1, mrows = mr ? f.nr : f.n - f.nr;
+                    dd[dx] = (mr ? F.dr : F.abb)[(size_t)mq * bb + e];
+#pragma unroll
+                    for (int d = 0; d < 6; ++d)
+                        v[dx][d] = d < nd ? (mr ? F.U : F.L)[((size_t)d * mrows + mq) * bb + e] : 0.0;
+                }
+#pragma unroll
+                for (int dx = 0; dx < 2; ++dx) {
+                    if (!in[dx]) continue;
+                    diag += dd[dx];
+#pragma unroll
+                    for (int d = 0; d < 6; ++d) {
+                        // inside the aggregate: the direction is paired and
+                        // leads to the other half
+                        const bool inner = d < 2 ? a.sx && dx != (d & 1) : d < 4 ? a.sy && dy != (d & 1) : a.sz && dz != (d & 1);
+                        if (inner) diag += v[dx][d];
+                        else off[d] += v[dx][d];
+                    }
+                }
             }
-        }
         (red ? G.dr : G.abb)[(size_t)q * bb + e] = diag;
 #pragma unroll
         for (int d = 0; d < 6; ++d)
@@ -841,13 +853,70 @@ __global__ void __launch_bounds__(kThreads) rb_galerkin_kernel(Aggregates a, int
     }
 }
 
-// D_r^-1 over the red cells.
+// The factors need no order between levels, so one launch does all of them:
+// blocks [first, first + blocks) take the rows of a level (a launch per level
+// and colour was 3.5 to 6.7 us each for the small ones).
+struct RbFactorLevel {
+    RbGrid g;
+    double* a = nullptr;
+    int first = 0, blocks = 0;
+};
+
+constexpr int kMaxRbLevels = 32;  // every one has at most half the cells of the one before
+
+struct RbFactorParams {
+    int nlev = 0;
+    RbFactorLevel lv[kMaxRbLevels];
+    RbGrid dense;                     // the coarsest level
+    const double* dense_a = nullptr;
+    double* inverse = nullptr;
+    __device__ __forceinline__ const RbFactorLevel& of(int block) const
+    {
+        int l = 0;
+        while (l + 1 < nlev && block >= lv[l + 1].first) ++l;
+        return lv[l];
+    }
+};
+
+// The coarsest matrix, dense and row-major (red cells, then black ones), by
+// one block, for dense_inverse_block.
 template <int B>
-__global__ void __launch_bounds__(kThreads) rb_factor_red_kernel(RbGrid g, double* __restrict__ dr, int* status)
+__device__ __forceinline__ void dense_fill(const RbGrid& g, int nd, const double* a, double* dense)
 {
     constexpr int BB = B * B;
-    GRID_STRIDE(q, g.nr)
-    {
+    const int n = g.n * B, tid = (int)threadIdx.x, nth = (int)blockDim.x;
+    const RbMatrix<const double> m(a, nd, BB, g.n, g.nr);
+    for (int x = tid; x < n * n; x += nth) dense[x] = 0.0;
+    __syncthreads();
+    for (int x = tid; x < g.n * (nd + 1); x += nth) {
+        const int P = x / (nd + 1), d = x - P * (nd + 1);
+        const bool red = P < g.nr;
+        const int rows = red ? g.nr : g.n - g.nr, q = red ? P : P - g.nr;
+        const Cell e = cell_of(g, red ? 0 : 1, q);
+        int nq, Q = P;
+        const double* v = (red ? m.dr : m.abb) + (size_t)q * BB;
+        if (d < nd) {
+            if (!neighbour(g, e, d, nq)) continue;
+            Q = red ? g.nr + nq : nq;
+            v = (red ? m.U : m.L) + ((size_t)d * rows + q) * BB;
+        }
+#pragma unroll
+        for (int t = 0; t < BB; ++t) dense[(size_t)(P * B + t / B) * n + Q * B + t % B] = v[t];
+    }
+    __syncthreads();
+}
+
+// D_r^-1 over the red cells of all levels.
+template <int B>
+__global__ void __launch_bounds__(kThreads) rb_factor_red_kernel(const __grid_constant__ RbFactorParams p, int nd,
+                                                                int* status)
+{
+    constexpr int BB = B * B;
+    const RbFactorLevel& L = p.of((int)blockIdx.x);
+    const RbGrid& g = L.g;
+    double* const dr = RbMatrix<double>(L.a, nd, BB, g.n, g.nr).dr;
+    for (int64_t q = (int64_t)(blockIdx.x - L.first) * blockDim.x + threadIdx.x; q < g.nr;
+         q += (int64_t)L.blocks * blockDim.x) {
         double d[BB];
 #pragma unroll
         for (int e = 0; e < BB; ++e) d[e] = dr[q * BB + e];
@@ -860,12 +929,21 @@ __global__ void __launch_bounds__(kThreads) rb_factor_red_kernel(RbGrid g, doubl
 // L = A_br D_r^-1 and D_b^-1 = (A_bb - sum L U)^-1 over the black cells: of
 // L U only the diagonal block is in the pattern (block ILU(0)).
 template <int B, int ND>
-__global__ void __launch_bounds__(kThreads) rb_factor_black_kernel(RbGrid g, RbMatrix<double> m, int* status)
+__global__ void __launch_bounds__(kInverseThreads, 1)
+    rb_factor_black_kernel(const __grid_constant__ RbFactorParams p, int* status)
 {
     constexpr int BB = B * B;
+    if (blockIdx.x == 0) {
+        dense_fill<B>(p.dense, ND, p.dense_a, p.inverse);
+        dense_inverse_block(p.dense.n * B, p.inverse, status);
+        return;
+    }
+    const RbFactorLevel& L = p.of((int)blockIdx.x);
+    const RbGrid& g = L.g;
+    const RbMatrix<double> m(L.a, ND, BB, g.n, g.nr);
     const int nk = g.n - g.nr;
-    GRID_STRIDE(q64, nk)
-    {
+    for (int64_t q64 = (int64_t)(blockIdx.x - L.first) * blockDim.x + threadIdx.x; q64 < nk;
+         q64 += (int64_t)L.blocks * blockDim.x) {
         const int q = (int)q64;
         const Cell e = cell_of(g, 1, q);
         double D[BB];
@@ -906,30 +984,6 @@ __global__ void __launch_bounds__(kThreads) rb_factor_black_kernel(RbGrid g, RbM
         if (!invert_block<B>(D)) *status = 1;
 #pragma unroll
         for (int t = 0; t < BB; ++t) m.db[(size_t)q * BB + t] = D[t];
-    }
-}
-
-// The coarsest matrix, dense and row-major (red cells, then black ones), for
-// dense_inverse_kernel; `dense` is zero beforehand.
-__global__ void rb_dense_fill_kernel(RbGrid g, int B, int nd, const double* __restrict__ a, double* __restrict__ dense)
-{
-    const int bb = B * B, n = g.n * B;
-    const RbMatrix<const double> m(a, nd, bb, g.n, g.nr);
-    GRID_STRIDE(P64, g.n)
-    {
-        const int P = (int)P64;
-        const bool red = P < g.nr;
-        const int rows = red ? g.nr : g.n - g.nr, q = red ? P : P - g.nr;
-        const Cell e = cell_of(g, red ? 0 : 1, q);
-        for (int t = 0; t < bb; ++t)
-            dense[(size_t)(P * B + t / B) * n + P * B + t % B] = (red ? m.dr : m.abb)[(size_t)q * bb + t];
-        for (int d = 0; d < nd; ++d) {
-            int nq;
-            if (!neighbour(g, e, d, nq)) continue;
-            const int Q = red ? g.nr + nq : nq;
-            for (int t = 0; t < bb; ++t)
-                dense[(size_t)(P * B + t / B) * n + Q * B + t % B] = (red ? m.U : m.L)[((size_t)d * rows + q) * bb + t];
-        }
     }
 }
 
