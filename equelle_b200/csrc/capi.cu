@@ -280,14 +280,20 @@ eqg_coll* apply_operator(const CoreP& cp, const OpMatrixP& mp, const eqg_coll* x
     if (x->n != m.n_src) fail(EQG_ERR_ARG, "operator applied to a collection of the wrong size");
     if (c.fuse && lazy_ok(c, x)) return lazy_coll(cp, m.n_out, lazy_opmat(mp, lazy_node(x)));
     Buf val = c.allocN<double>(m.n_out > 0 ? m.n_out : 1);
-    opmat_apply_values(c, m, coll_values(c, x), val->as<double>());
-    if (!x->pat) return new_coll(cp, m.n_out, val);
+    const double* xv = coll_values(c, x);
+    if (!x->pat) {
+        opmat_apply_values(c, m, xv, val->as<double>());
+        return new_coll(cp, m.n_out, val);
+    }
     PatternP p = pattern_spgemm(c, m, x->pat);
+    const bool joint = spgemm_joins_values(c, m, *p);
+    if (!joint) opmat_apply_values(c, m, xv, val->as<double>());
     // deferred rules on x's values go into the planned product; without a
     // plan, x is materialized first
     if (x->jdef.n > 0 && !spgemm_has_plan(*p)) materialized_jacobian(c, x);
     Buf jv = c.allocN<double>(p->nnz > 0 ? p->nnz : 1);
-    spgemm_values(c, m, *x->pat, x->jval->as<double>(), *p, jv->as<double>(), &x->jdef);
+    spgemm_values(c, m, *x->pat, x->jval->as<double>(), *p, jv->as<double>(), &x->jdef, xv,
+                  joint ? val->as<double>() : nullptr);
     return new_coll(cp, m.n_out, val, p, jv);
 }
 
@@ -1084,7 +1090,15 @@ int eqg_binary(eqg_runtime* rt, int op, const eqg_coll* a, const eqg_coll* b, eq
             return;
         }
         Buf val = c.allocN<double>(a->n > 0 ? a->n : 1);
-        k_binary(c, op, coll_values(c, a), coll_values(c, b), val->as<double>(), a->n);
+        JacArgs ja;
+        ja.xa = coll_values(c, a);
+        ja.xb = coll_values(c, b);
+        if (a->pat && b->pat) {  // computed with the Jacobian
+            ja.value = val->as<double>();
+            ja.n = a->n;
+        } else {
+            k_binary(c, op, ja.xa, ja.xb, val->as<double>(), a->n);
+        }
         // A sum with one Jacobian shares that Jacobian unchanged (Zero + J).
         if (op == EQG_ADD && (!a->pat || !b->pat)) {
             const eqg_coll* j = a->pat ? a : b;
@@ -1095,7 +1109,6 @@ int eqg_binary(eqg_runtime* rt, int op, const eqg_coll* a, const eqg_coll* b, eq
             *out = sharing_jacobian(new_coll(rt->core, a->n, val), a);
             return;
         }
-        JacArgs ja;
         ja.rule = op == EQG_ADD ? JR_ADD : op == EQG_SUB ? JR_SUB : op == EQG_MUL ? JR_MUL : JR_DIV;
         ja.va = a->val->as<double>();
         ja.vb = b->val->as<double>();
@@ -1306,10 +1319,17 @@ int eqg_select(eqg_runtime* rt, const eqg_mask* pred, const eqg_coll* a, const e
         }
         Buf val = c.allocN<double>(pred->n > 0 ? pred->n : 1);
         const uint8_t* mv = mask_values(c, pred);
-        k_select_value(c, mv, coll_values(c, a), coll_values(c, b), val->as<double>(), pred->n);
         JacArgs ja;
         ja.rule = JR_SELECT;
         ja.mask = mv;
+        ja.xa = coll_values(c, a);
+        ja.xb = coll_values(c, b);
+        if (a->pat && b->pat) {  // computed with the Jacobian
+            ja.value = val->as<double>();
+            ja.n = pred->n;
+        } else {
+            k_select_value(c, mv, ja.xa, ja.xb, val->as<double>(), pred->n);
+        }
         *out = jac_rule(rt->core, pred->n, val, ja, a, b, pred->v);
     });
 }

@@ -445,10 +445,14 @@ Buf ones(Core& c, int64_t n);
 // with_plan: also build the output's position plan (spgemm_plan_kernel)
 PatternP pattern_spgemm(Core& c, const OpMatrix& m, const PatternP& j, bool with_plan = true);
 // ov = M jv; with deferred rules on jv only through the output's position
-// plan (spgemm_has_plan), whose kernel applies them per source row.
+// plan (spgemm_has_plan), whose kernel applies them per source row.  With y
+// (only with a plan) also y = M x, in the same launch.
 void spgemm_values(Core& c, const OpMatrix& m, const Pattern& jp, const double* jv, const Pattern& op,
-                   double* ov, const Deferred* jd = nullptr);
+                   double* ov, const Deferred* jd = nullptr, const double* x = nullptr, double* y = nullptr);
 inline bool spgemm_has_plan(const Pattern& op) { return (bool)op.plan_start; }
+// Whether the product should take the values along: not for the grid's own
+// stencils, whose values need no operator, nor for many rows.
+bool spgemm_joins_values(const Core& c, const OpMatrix& m, const Pattern& op);
 PatternP pattern_union(Core& c, const PatternP& a, const PatternP& b);
 // Elementwise Jacobian rule: out_row(i) = post_i * (wa_i * A_row(i) (+) wb_i * B_row(i)).
 // Weights come from the operand values per op (see jacobian.cu).
@@ -473,6 +477,12 @@ struct JacArgs {
     const Pattern* pb = nullptr;
     const double* jb = nullptr;
     Deferred da, db;  // rules deferred on the operands' stored values
+    // the operation's value on n rows (JR_ADD to JR_DIV, JR_SELECT), to be
+    // computed with its Jacobian; null: it has been
+    double* value = nullptr;
+    const double* xa = nullptr;
+    const double* xb = nullptr;
+    int64_t n = 0;
 };
 void jacobian_elementwise(Core& c, const JacArgs& args, const Pattern& out, double* jout);
 // Stored values with the deferred rules applied (one pass), into out.

@@ -99,6 +99,16 @@ __device__ __forceinline__ double apply_deferred(const Deferred& d, int64_t row,
 }
 
 
+// Row i of M x, accumulated from 0.0 over ascending source entries.
+__device__ __forceinline__ double opmat_row(int64_t i, const int* __restrict__ mptr, const int* __restrict__ msrc,
+                                            const double* __restrict__ mw, const double* __restrict__ x)
+{
+    double acc = 0.0;
+    const int e1 = mptr[i + 1];
+    for (int e = mptr[i]; e < e1; ++e) acc += mw[e] * x[msrc[e]];
+    return acc;
+}
+
 // Entries of a Jacobian that a thread of the elementwise and planned product
 // kernels takes at once.  An entry is a chain of dependent loads (its row and
 // positions, then the operands' values and the rules' row values); with one
@@ -201,12 +211,73 @@ __device__ __forceinline__ void apply_deferred_of(const Deferred& d, const int (
 }
 
 // This thread's entries: e + u blockDim for u < kEntries, e from the loop;
-// past the end the last entry (its result is not stored).
+// past the end the last entry (its result is not stored).  vp: the launch's
+// ValuePart.
 #define ENTRY_STRIDE(e, n)                                                                                  \
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x * kEntries + threadIdx.x; e < (n);                    \
-         e += (int64_t)gridDim.x * blockDim.x * kEntries)
+         e += (int64_t)(gridDim.x - vp.blocks) * blockDim.x * kEntries)
 
 inline int entry_blocks(int64_t n) { return blocksFor((n + kEntries - 1) / kEntries); }
+
+// The values that go with a Jacobian, by the blocks from `first` on of the
+// launch that computes it: small systems wait for launches, not for their
+// kernels.  Residuals of a step, apart and joint: two-phase 48x40 1.96 -> 1.60
+// ms (982 -> 847 launches), 33x31x17 2.09 -> 1.65, 512x512 (524k faces) 3.70 ->
+// 3.56; but heat 1000x701 (1.4 M faces) 0.57 -> 0.62 and two-phase 128x128x64
+// (3.1 M) 12.1 -> 13.1: there the values' kernels, which fill an SM with four
+// times as many warps as fit beside the Jacobian's registers, are worth their
+// launch.  Hence the line between them.
+constexpr int64_t kJointRows = 1 << 19;
+
+struct ValuePart {
+    int64_t n = 0;
+    const double* a = nullptr;
+    const double* b = nullptr;
+    const uint8_t* mask = nullptr;
+    double* out = nullptr;
+    unsigned first = 0;  // 0: no value blocks
+    int blocks = 0;
+    // The launch's grid with the value blocks behind `entries` blocks.
+    int grid(int entries)
+    {
+        if (!out || n <= 0) return entries;
+        first = (unsigned)entries;
+        blocks = entry_blocks(n);
+        return entries + blocks;
+    }
+};
+
+// f(row) for this block's share of the values' rows; false: a block of the
+// Jacobian's entries.
+template <class F>
+__device__ __forceinline__ bool value_blocks(const ValuePart& v, F&& f)
+{
+    if (!v.first || blockIdx.x < v.first) return false;
+    for (int64_t i0 = (int64_t)(blockIdx.x - v.first) * blockDim.x * kEntries + threadIdx.x; i0 < v.n;
+         i0 += (int64_t)v.blocks * blockDim.x * kEntries) {
+#pragma unroll
+        for (int u = 0; u < kEntries; ++u) {
+            const int64_t i = i0 + (int64_t)u * blockDim.x;
+            if (i < v.n) f(i);
+        }
+    }
+    return true;
+}
+
+// The value of an elementwise operation (binary_kernel, select_kernel).
+__device__ __forceinline__ bool ew_values(const ValuePart& v, int rule)
+{
+    return value_blocks(v, [&](int64_t i) {
+        const double a = v.a[i], b = v.b[i];
+        double x;
+        if (rule == JR_ADD) x = a + b;
+        else if (rule == JR_SUB) x = a - b;
+        else if (rule == JR_MUL) x = a * b;
+        else if (rule == JR_DIV) x = a / b;
+        else x = a * (v.mask[i] ? 1.0 : 0.0) + b * (v.mask[i] ? 0.0 : 1.0);
+        v.out[i] = x;
+    });
+}
 
 // ---------------------------------------------------------------------------
 // Conservative product M*J by K-way merge of the selected rows of J.
@@ -363,8 +434,12 @@ __global__ void __launch_bounds__(kThreads) spgemm_planned_kernel(int64_t nnz, c
                                                                   const int* __restrict__ contrib,
                                                                   const int* __restrict__ jrow,
                                                                   const double* __restrict__ jval,
-                                                                  double* __restrict__ oval, const Deferred dj)
+                                                                  double* __restrict__ oval, const Deferred dj,
+                                                                  const int* __restrict__ mptr,
+                                                                  const int* __restrict__ msrc,
+                                                                  const double* __restrict__ mw, const ValuePart vp)
 {
+    if (value_blocks(vp, [&](int64_t i) { vp.out[i] = opmat_row(i, mptr, msrc, mw, vp.a); })) return;
     ENTRY_STRIDE(e0, nnz)
     {
         int k[kEntries], k1[kEntries];
@@ -404,18 +479,12 @@ __global__ void __launch_bounds__(kThreads) spgemm_planned_kernel(int64_t nnz, c
     }
 }
 
-// y = M x, each row accumulated from 0.0 over ascending source entries.
+// y = M x
 __global__ void opmat_apply_kernel(int n_out, const int* __restrict__ mptr, const int* __restrict__ msrc,
                                    const double* __restrict__ mw, const double* __restrict__ x,
                                    double* __restrict__ y)
 {
-    GRID_STRIDE(i, n_out)
-    {
-        double acc = 0.0;
-        const int e1 = mptr[i + 1];
-        for (int e = mptr[i]; e < e1; ++e) acc += mw[e] * x[msrc[e]];
-        y[i] = acc;
-    }
+    GRID_STRIDE(i, n_out) y[i] = opmat_row(i, mptr, msrc, mw, x);
 }
 
 __global__ void map_count_kernel(const int32_t* map, int64_t n, int64_t* cnt, int n_src, int32_t* err)
@@ -478,8 +547,10 @@ __global__ void i64_to_rowptr_kernel(const int64_t* incl, int n, int* rowptr)
 __global__ void __launch_bounds__(kThreads) ew_flat_kernel(Rule r, const int* __restrict__ rowidx,
                                                            const double* __restrict__ ja,
                                                            const double* __restrict__ jb, double* __restrict__ out,
-                                                           int64_t nnz, const Deferred da, const Deferred db)
+                                                           int64_t nnz, const Deferred da, const Deferred db,
+                                                             const ValuePart vp)
 {
+    if (ew_values(vp, r.rule)) return;
     ENTRY_STRIDE(e0, nnz)
     {
         int i[kEntries];
@@ -510,6 +581,7 @@ __global__ void __launch_bounds__(kThreads) apply_deferred_kernel(const Deferred
                                                                   const double* __restrict__ j,
                                                                   double* __restrict__ out, int64_t nnz)
 {
+    const ValuePart vp;
     ENTRY_STRIDE(e0, nnz)
     {
         int i[kEntries];
@@ -593,8 +665,10 @@ __global__ void __launch_bounds__(kThreads) ew_mapped_kernel(Rule r, const int* 
                                                              const int* __restrict__ ia, const int* __restrict__ ib,
                                                              const double* __restrict__ ja,
                                                              const double* __restrict__ jb, double* __restrict__ out,
-                                                             int64_t nnz, const Deferred da, const Deferred db)
+                                                             int64_t nnz, const Deferred da, const Deferred db,
+                                                             const ValuePart vp)
 {
+    if (ew_values(vp, r.rule)) return;
     ENTRY_STRIDE(e0, nnz)
     {
         int i[kEntries], xa[kEntries], xb[kEntries];
@@ -725,7 +799,7 @@ void spgemm_build_plan(Core& c, const OpMatrix& m, const Pattern& j, Pattern& ou
 
 template <int KMAX>
 void spgemm_numeric(Core& c, const OpMatrix& m, const Pattern& jp, const double* jv, const Pattern& op, double* ov,
-                    const Deferred& jd)
+                    const Deferred& jd, const double* x, double* y)
 {
     if (m.n_out <= 0) return;
     if (jd.n && !op.plan_start) fail(EQG_ERR_DEVICE, "operator product of deferred Jacobian values without a plan");
@@ -735,10 +809,16 @@ void spgemm_numeric(Core& c, const OpMatrix& m, const Pattern& jp, const double*
         // rules' row values where rules are deferred)
         const double bytes =
             12.0 * op.nnz + (jd.n ? 16.0 : 12.0) * op.plan_entries + 16.0 * jd.n * jp.rows;
+        ValuePart vp;
+        vp.n = m.n_out;
+        vp.a = x;
+        vp.out = y;
         launch(c, "spgemm_planned", [&] {
-            spgemm_planned_kernel<<<entry_blocks(op.nnz), kThreads, 0, c.stream>>>(
-                op.nnz, op.plan_start->as<int>(), op.plan_contrib->as<int>(), op.plan_jrow->as<int>(), jv, ov, jd);
-        }, bytes);
+            const int grid = vp.grid(entry_blocks(op.nnz));
+            spgemm_planned_kernel<<<grid, kThreads, 0, c.stream>>>(
+                op.nnz, op.plan_start->as<int>(), op.plan_contrib->as<int>(), op.plan_jrow->as<int>(), jv, ov, jd,
+                m.ptr->as<int>(), m.src->as<int>(), m.w->as<double>(), vp);
+        }, bytes + (y ? 4.0 * (m.n_out + 1) + 12.0 * m.nnz + 8.0 * m.n_src + 8.0 * m.n_out : 0.0));
         return;
     }
     // algorithmic bytes: M (row pointers, sources, weights), the Jacobian
@@ -893,17 +973,18 @@ PatternP pattern_spgemm(Core& c, const OpMatrix& m, const PatternP& j, bool with
 }
 
 void spgemm_values(Core& c, const OpMatrix& m, const Pattern& jp, const double* jv, const Pattern& op, double* ov,
-                   const Deferred* jd)
+                   const Deferred* jd, const double* x, double* y)
 {
+    if (y && !op.plan_start) fail(EQG_ERR_DEVICE, "values beside an operator product without a plan");
     const Deferred none;
     const Deferred& d = jd ? *jd : none;
     switch (kmax_for(m.max_row)) {
-    case 1: spgemm_numeric<1>(c, m, jp, jv, op, ov, d); break;
-    case 2: spgemm_numeric<2>(c, m, jp, jv, op, ov, d); break;
-    case 4: spgemm_numeric<4>(c, m, jp, jv, op, ov, d); break;
-    case 6: spgemm_numeric<6>(c, m, jp, jv, op, ov, d); break;
-    case 8: spgemm_numeric<8>(c, m, jp, jv, op, ov, d); break;
-    default: spgemm_numeric<16>(c, m, jp, jv, op, ov, d); break;
+    case 1: spgemm_numeric<1>(c, m, jp, jv, op, ov, d, x, y); break;
+    case 2: spgemm_numeric<2>(c, m, jp, jv, op, ov, d, x, y); break;
+    case 4: spgemm_numeric<4>(c, m, jp, jv, op, ov, d, x, y); break;
+    case 6: spgemm_numeric<6>(c, m, jp, jv, op, ov, d, x, y); break;
+    case 8: spgemm_numeric<8>(c, m, jp, jv, op, ov, d, x, y); break;
+    default: spgemm_numeric<16>(c, m, jp, jv, op, ov, d, x, y); break;
     }
 }
 
@@ -914,6 +995,11 @@ void jacobian_apply_deferred(Core& c, const Deferred& d, Pattern& p, const doubl
     launch(c, "jac_deferred", [&] {
         apply_deferred_kernel<<<entry_blocks(p.nnz), kThreads, 0, c.stream>>>(d, p.rowidx->as<int>(), j, out, p.nnz);
     }, 20.0 * p.nnz + 4.0 * p.nnz + 16.0 * d.n * p.rows);
+}
+
+bool spgemm_joins_values(const Core& c, const OpMatrix& m, const Pattern& op)
+{
+    return spgemm_has_plan(op) && m.n_out <= kJointRows && !(m.stencil && c.stencil_ops);
 }
 
 PatternP pattern_union(Core& c, const PatternP& a, const PatternP& b)
@@ -989,7 +1075,28 @@ void jacobian_elementwise(Core& c, const JacArgs& a, const Pattern& out, double*
 {
     Rule r{a.rule, a.va, a.vb, a.vout, a.mask, a.s};
     const bool flat = (!a.pa || a.pa->id == out.id) && (!a.pb || a.pb->id == out.id);
-    if (out.nnz <= 0) return;
+    // the value of the operation, where it is asked for and no kernel below
+    // computes it beside the Jacobian
+    auto value_alone = [&] {
+        if (!a.value) return;
+        if (a.rule == JR_SELECT) k_select_value(c, a.mask, a.xa, a.xb, a.value, a.n);
+        else k_binary(c, a.rule - JR_ADD + EW_ADD, a.xa, a.xb, a.value, a.n);
+    };
+    if (out.nnz <= 0) {
+        value_alone();
+        return;
+    }
+    ValuePart vp;
+    if (a.n <= kJointRows) {
+        vp.n = a.n;
+        vp.a = a.xa;
+        vp.b = a.xb;
+        vp.mask = a.mask;
+        vp.out = a.value;
+    } else {
+        value_alone();
+    }
+    const double value_bytes = vp.out ? (a.rule == JR_SELECT ? 25.0 : 24.0) * a.n : 0.0;
     // algorithmic bytes: the operand Jacobians' values and the output's once,
     // the output's row pointers, the per-row operand values the rule uses;
     // operands on other patterns add their column indices and the output's
@@ -1007,6 +1114,7 @@ void jacobian_elementwise(Core& c, const JacArgs& a, const Pattern& out, double*
         const Deferred& dx = a_first ? a.da : a.db;
         const Deferred& dy = a_first ? a.db : a.da;
         if (dx.n || dy.n) pattern_build_rowidx(c, const_cast<Pattern&>(out));
+        if (vp.out) value_alone();
         launch(c, "jac_concat", [&] {
             concat_kernel<<<blocksFor(out.nnz), kThreads, 0, c.stream>>>(
                 x, n1, y, n2, jout, (dx.n || dy.n) ? out.rowidx->as<int>() : nullptr, dx, dy);
@@ -1016,9 +1124,10 @@ void jacobian_elementwise(Core& c, const JacArgs& a, const Pattern& out, double*
     if (flat) {
         pattern_build_rowidx(c, const_cast<Pattern&>(out));
         launch(c, "jac_flat", [&] {
-            ew_flat_kernel<<<entry_blocks(out.nnz), kThreads, 0, c.stream>>>(
-                r, out.rowidx->as<int>(), a.pa ? a.ja : nullptr, a.pb ? a.jb : nullptr, jout, out.nnz, a.da, a.db);
-        }, bytes);
+            const int grid = vp.grid(entry_blocks(out.nnz));
+            ew_flat_kernel<<<grid, kThreads, 0, c.stream>>>(
+                r, out.rowidx->as<int>(), a.pa ? a.ja : nullptr, a.pb ? a.jb : nullptr, jout, out.nnz, a.da, a.db, vp);
+        }, bytes + value_bytes);
     } else if (out.nnz < (int64_t)INT_MAX / 2) {
         // through position maps kept with the output pattern
         Pattern& o = const_cast<Pattern&>(out);
@@ -1035,11 +1144,13 @@ void jacobian_elementwise(Core& c, const JacArgs& a, const Pattern& out, double*
             });
         }
         launch(c, "jac_merge", [&] {
-            ew_mapped_kernel<<<entry_blocks(out.nnz), kThreads, 0, c.stream>>>(
+            const int grid = vp.grid(entry_blocks(out.nnz));
+            ew_mapped_kernel<<<grid, kThreads, 0, c.stream>>>(
                 r, out.rowidx->as<int>(), maps->as<int>(), maps->as<int>() + out.nnz, a.pa ? a.ja : nullptr,
-                a.pb ? a.jb : nullptr, jout, out.nnz, a.da, a.db);
-        }, bytes);
+                a.pb ? a.jb : nullptr, jout, out.nnz, a.da, a.db, vp);
+        }, bytes + value_bytes);
     } else {
+        if (vp.out) value_alone();
         launch(c, "jac_merge", [&] { ew_merge_kernel<<<blocksFor(out.rows), kThreads, 0, c.stream>>>(
             r, out.rows, a.pa ? a.pa->rowptr->as<int>() : nullptr, a.pa ? a.pa->colind->as<int>() : nullptr,
             a.pa ? a.ja : nullptr, a.pb ? a.pb->rowptr->as<int>() : nullptr, a.pb ? a.pb->colind->as<int>() : nullptr,
