@@ -123,7 +123,9 @@ const char* eqg_backend_name(void);
  * linsolver_max_sweeps (60) for refine, linsolver_check_every (4),
  * linsolver_block (1: ncomp x ncomp block ILU(0) for 2 or 3 unknowns per
  * cell; 0: scalar ILU(0)), linsolver_mg_fuse_rows (40000: the V-cycle
- * levels up to this size run as one kernel; 0: none), linsolver_mg_cluster
+ * levels up to this size run as one kernel, as far as they fit in its
+ * cluster's shared memory, or with refine or scalar blocks through global
+ * memory; 0: none), linsolver_mg_cluster
  * (16: thread blocks of that kernel's cluster, at most 16),
  * linsolver_mg_alpha (factor of the coarse-grid correction z += alpha P zc;
  * 1.9 for 2 x 2 aggregates of 2D grids, else 1.4), linsolver_mg_ap_rows
@@ -132,8 +134,9 @@ const char* eqg_backend_name(void);
  * stages), linsolver_mg_coarsest (128: coarsening stops at
  * this many unknowns, at most 128; that level is solved with a dense
  * inverse), linsolver_pdl (1: the BiCGStab iteration's kernels
- * as programmatic dependent launches; 0: plain launches), linsolver_mg_local (1: that kernel keeps its coarsest levels in one thread
- * block's shared memory while they fit in 200 KB; 0: off),
+ * as programmatic dependent launches; 0: plain launches),
+ * linsolver_mg_local (1: that kernel keeps its coarsest levels in one thread
+ * block's shared memory; 0: off),
  * linsolver_tail_trace (0; 1: print the SM clock cycles of every step of the
  * last fused cycle after each linear solve), lazy (0; 1:
  * defer value-only elementwise operations and evaluate them in batches),
@@ -145,8 +148,9 @@ const char* eqg_backend_name(void);
  * linsolver_fallback (1: a solve that the multigrid preconditioner does not
  * converge is repeated once with block ILU(0) alone; 0: reported as a
  * failure), linsolver_autotune (1: choose threads per block of the launch-per-step
- * V-cycle levels and the fused cycle's cluster size by timing, once per
- * Jacobian pattern and precision; 0: 256 and the largest cluster),
+ * V-cycle levels, with refine or scalar blocks of systems also the fused
+ * cycle's cluster size, by timing, once per Jacobian pattern and precision; 0: the defaults and the
+ * largest cluster),
  * linsolver_tune_file (a JSON file caching those choices; default
  * $EQG_TUNE_FILE, else none), spgemm_plan / span_share / jac_concat /
  * jac_defer / stencil_ops (1; 0 switches off an assembly fast path, for
