@@ -77,7 +77,7 @@ struct RuntimeObject {
     PyObject_HEAD
     Api api;
     eqg_runtime* h;
-    bool bound;
+    bool bound, created;  // has its library's entry points; has been given a handle
 };
 
 struct HandleObject {
@@ -87,6 +87,30 @@ struct HandleObject {
 };
 
 extern PyTypeObject RuntimeBaseType, CollBaseType, MaskBaseType, SetBaseType;
+
+// An object whose __init__ has not run (or not got that far) lacks what it
+// sets: an error, as for any Python attribute.
+void* lacks(PyObject* o, const char* name)
+{
+    PyErr_Format(PyExc_AttributeError, "'%s' object has no attribute '%s'", Py_TYPE(o)->tp_name, name);
+    return nullptr;
+}
+
+// The runtime that a method is called on; null (an error) before its __init__.
+RuntimeObject* rt_of(PyObject* self)
+{
+    RuntimeObject* rt = (RuntimeObject*)self;
+    if (!rt->bound) return (RuntimeObject*)lacks(self, "lib");
+    if (!rt->created) return (RuntimeObject*)lacks(self, "h");
+    return rt;
+}
+
+// The runtime of a handle; null (an error) before the handle's __init__.
+RuntimeObject* rt_of_handle(PyObject* handle)
+{
+    RuntimeObject* rt = ((HandleObject*)handle)->rt;
+    return rt ? rt_of((PyObject*)rt) : (RuntimeObject*)lacks(handle, "rt");
+}
 
 PyObject* raise_status(const Api& api, int status)
 {
@@ -136,6 +160,10 @@ bool handle_of(PyObject* o, void** h)
 {
     if (PyObject_TypeCheck(o, &CollBaseType) || PyObject_TypeCheck(o, &SetBaseType) ||
         PyObject_TypeCheck(o, &MaskBaseType)) {
+        if (!((HandleObject*)o)->rt) {
+            lacks(o, "h");
+            return false;
+        }
         *h = ((HandleObject*)o)->h;
         return true;
     }
@@ -215,12 +243,12 @@ int handle_traverse(PyObject* self, visitproc visit, void* arg)
 PyObject* handle_get_rt(PyObject* self, void*)
 {
     PyObject* rt = (PyObject*)((HandleObject*)self)->rt;
-    if (!rt) rt = Py_None;
-    return Py_NewRef(rt);
+    return rt ? Py_NewRef(rt) : (PyObject*)lacks(self, "rt");
 }
 PyObject* handle_get_h(PyObject* self, void*)
 {
     void* h = ((HandleObject*)self)->h;
+    if (!((HandleObject*)self)->rt) return (PyObject*)lacks(self, "h");
     if (!h) Py_RETURN_NONE;
     return PyLong_FromVoidPtr(h);
 }
@@ -246,9 +274,12 @@ PyObject* coll_binary(int op, PyObject* left, PyObject* right)
 {
     const bool l = PyObject_TypeCheck(left, &CollBaseType), r = PyObject_TypeCheck(right, &CollBaseType);
     HandleObject* self = (HandleObject*)(l ? left : right);
-    RuntimeObject* rt = self->rt;
+    RuntimeObject* rt = rt_of_handle((PyObject*)self);
+    if (!rt) return nullptr;
     if (l && r) {
-        const eqg_coll *a = (eqg_coll*)((HandleObject*)left)->h, *b = (eqg_coll*)((HandleObject*)right)->h;
+        void *a0, *b0;
+        if (!handle_of(left, &a0) || !handle_of(right, &b0)) return nullptr;
+        const eqg_coll *a = (eqg_coll*)a0, *b = (eqg_coll*)b0;
         return make<eqg_coll>(g_coll_class, rt, [&](eqg_coll** o) { return rt->api.binary(rt->h, op, a, b, o); });
     }
     double s;
@@ -269,17 +300,19 @@ PyObject* unary_of(RuntimeObject* rt, int op, const void* h)
 }
 PyObject* coll_neg(PyObject* self)
 {
-    HandleObject* s = (HandleObject*)self;
-    return unary_of(s->rt, EQG_NEG, s->h);
+    RuntimeObject* rt = rt_of_handle(self);
+    return rt ? unary_of(rt, EQG_NEG, ((HandleObject*)self)->h) : nullptr;
 }
 
 PyObject* coll_compare_op(PyObject* self, int op, PyObject* other)
 {
-    HandleObject* s = (HandleObject*)self;
-    RuntimeObject* rt = s->rt;
-    const eqg_coll* a = (eqg_coll*)s->h;
+    RuntimeObject* rt = rt_of_handle(self);
+    if (!rt) return nullptr;
+    const eqg_coll* a = (eqg_coll*)((HandleObject*)self)->h;
     if (PyObject_TypeCheck(other, &CollBaseType)) {
-        const eqg_coll* b = (eqg_coll*)((HandleObject*)other)->h;
+        void* b0;
+        if (!handle_of(other, &b0)) return nullptr;
+        const eqg_coll* b = (eqg_coll*)b0;
         return make<eqg_mask>(g_mask_class, rt, [&](eqg_mask** o) { return rt->api.compare(rt->h, op, a, b, o); });
     }
     double v;
@@ -309,7 +342,8 @@ PyObject* mask_logic_op(int op, PyObject* self, PyObject* other)
 {
     if (!PyObject_TypeCheck(self, &MaskBaseType)) Py_RETURN_NOTIMPLEMENTED;
     HandleObject* s = (HandleObject*)self;
-    RuntimeObject* rt = s->rt;
+    RuntimeObject* rt = rt_of_handle(self);
+    if (!rt) return nullptr;
     void* b = nullptr;
     if (other && other != Py_None && !handle_of(other, &b)) return nullptr;
     return make<eqg_mask>(g_mask_class, rt, [&](eqg_mask** o) {
@@ -354,7 +388,6 @@ bool take(const char* fn, PyObject* const* args, Py_ssize_t nargs, PyObject* kwn
 }
 
 #define METHOD_ARGS PyObject *self, PyObject *const *args, Py_ssize_t nargs, PyObject *kwnames
-RuntimeObject* rt_of(PyObject* self) { return (RuntimeObject*)self; }
 
 // Methods of one collection argument.
 template <class Get>
@@ -365,6 +398,7 @@ PyObject* coll_method(METHOD_ARGS, const char* name, Get&& get)
     void* h;
     if (!take(name, args, nargs, kwnames, names, 1, 1, v) || !handle_of(v[0], &h)) return nullptr;
     RuntimeObject* rt = rt_of(self);
+    if (!rt) return nullptr;
     return make<eqg_coll>(g_coll_class, rt,
                           [&](eqg_coll** o) { return get(rt->api)(rt->h, (const eqg_coll*)h, o); });
 }
@@ -391,12 +425,14 @@ PyObject* rt_sqrt(METHOD_ARGS)
     PyObject* v[1];
     void* h;
     if (!take("sqrt", args, nargs, kwnames, names, 1, 1, v) || !handle_of(v[0], &h)) return nullptr;
-    return unary_of(rt_of(self), EQG_SQRT, h);
+    RuntimeObject* rt = rt_of(self);
+    return rt ? unary_of(rt, EQG_SQRT, h) : nullptr;
 }
 
 PyObject* builtin_set(PyObject* self, int which)
 {
     RuntimeObject* rt = rt_of(self);
+    if (!rt) return nullptr;
     return make<eqg_set>(g_set_class, rt, [&](eqg_set** o) { return rt->api.set_builtin(rt->h, which, o); });
 }
 PyObject* rt_all_cells(PyObject* self, PyObject*) { return builtin_set(self, EQG_ALL_CELLS); }
@@ -414,6 +450,7 @@ PyObject* set_method(METHOD_ARGS, const char* name, Get&& get)
     void* h;
     if (!take(name, args, nargs, kwnames, names, 1, 1, v) || !handle_of(v[0], &h)) return nullptr;
     RuntimeObject* rt = rt_of(self);
+    if (!rt) return nullptr;
     return make<eqg_set>(g_set_class, rt, [&](eqg_set** o) { return get(rt->api)(rt->h, (const eqg_set*)h, o); });
 }
 PyObject* rt_first_cell(METHOD_ARGS)
@@ -439,12 +476,14 @@ PyObject* rt_extend(METHOD_ARGS)
     PyObject* v[3];
     if (!take("operatorExtend", args, nargs, kwnames, names, 3, 2, v)) return nullptr;
     RuntimeObject* rt = rt_of(self);
+    if (!rt) return nullptr;
     if (!v[2] || v[2] == Py_None) {
         int64_t n = 0;
         if (PyObject_TypeCheck(v[1], &SetBaseType)) {
-            HandleObject* s = (HandleObject*)v[1];
-            const int st = s->rt->api.set_size((eqg_set*)s->h, &n);
-            if (st != EQG_OK) return raise_status(s->rt->api, st);
+            RuntimeObject* owner = rt_of_handle(v[1]);
+            if (!owner) return nullptr;
+            const int st = owner->api.set_size((eqg_set*)((HandleObject*)v[1])->h, &n);
+            if (st != EQG_OK) return raise_status(owner->api, st);
         } else {
             n = PyObject_Size(v[1]);
             if (n < 0) return nullptr;
@@ -470,6 +509,7 @@ PyObject* rt_on(METHOD_ARGS)
         !handle_of(v[2], &b))
         return nullptr;
     RuntimeObject* rt = rt_of(self);
+    if (!rt) return nullptr;
     const eqg_set *from = (eqg_set*)a, *to = (eqg_set*)b;
     if (PyObject_TypeCheck(v[0], &SetBaseType))
         return make<eqg_set>(g_set_class, rt,
@@ -487,6 +527,7 @@ PyObject* rt_trinary_if(METHOD_ARGS)
         !handle_of(v[2], &b))
         return nullptr;
     RuntimeObject* rt = rt_of(self);
+    if (!rt) return nullptr;
     const eqg_mask* p = (eqg_mask*)m;
     if (PyObject_TypeCheck(v[1], &SetBaseType))
         return make<eqg_set>(g_set_class, rt, [&](eqg_set** o) {
@@ -504,6 +545,7 @@ PyObject* reduce_of(METHOD_ARGS, const char* name, int op)
     void* h;
     if (!take(name, args, nargs, kwnames, names, 1, 1, v) || !handle_of(v[0], &h)) return nullptr;
     RuntimeObject* rt = rt_of(self);
+    if (!rt) return nullptr;
     double r = 0.0;
     const int st = unlocked([&] {
         return op < 0 ? rt->api.two_norm(rt->h, (eqg_coll*)h, &r) : rt->api.reduce(rt->h, op, (eqg_coll*)h, &r);
@@ -534,6 +576,7 @@ PyObject* span_of(METHOD_ARGS, bool subset)
         if (n[i] == -1 && PyErr_Occurred()) return nullptr;
     }
     RuntimeObject* rt = rt_of(self);
+    if (!rt) return nullptr;
     return make<eqg_coll>(g_coll_class, rt, [&](eqg_coll** o) {
         return (subset ? rt->api.span_subset : rt->api.span_superset)(rt->h, (eqg_coll*)h, n[0], n[1], o);
     });
@@ -544,7 +587,7 @@ PyObject* rt_span_superset(METHOD_ARGS) { return span_of(self, args, nargs, kwna
 // _bind({name: address}): the entry points of the runtime's library.
 PyObject* rt_bind(PyObject* self, PyObject* table)
 {
-    RuntimeObject* rt = rt_of(self);
+    RuntimeObject* rt = (RuntimeObject*)self;
     for (const Entry& e : kEntries) {
         PyObject* a = PyMapping_GetItemString(table, e.name);
         if (!a) return nullptr;
@@ -562,7 +605,8 @@ PyObject* rt_bind(PyObject* self, PyObject* table)
 
 PyObject* rt_get_h(PyObject* self, void*)
 {
-    eqg_runtime* h = rt_of(self)->h;
+    eqg_runtime* h = ((RuntimeObject*)self)->h;
+    if (!((RuntimeObject*)self)->created) return (PyObject*)lacks(self, "h");
     if (!h) Py_RETURN_NONE;
     return PyLong_FromVoidPtr(h);
 }
@@ -573,7 +617,8 @@ int rt_set_h(PyObject* self, PyObject* v, void*)
         p = PyLong_AsVoidPtr(v);
         if (!p && PyErr_Occurred()) return -1;
     }
-    rt_of(self)->h = (eqg_runtime*)p;
+    ((RuntimeObject*)self)->h = (eqg_runtime*)p;
+    ((RuntimeObject*)self)->created = true;
     return 0;
 }
 PyGetSetDef rt_getset[] = {{"h", rt_get_h, rt_set_h, nullptr, nullptr}, {nullptr, nullptr, nullptr, nullptr, nullptr}};

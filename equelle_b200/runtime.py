@@ -163,7 +163,7 @@ class Runtime(_mirror.RuntimeBase):
         self.dimensions = info.dimensions
 
     def __del__(self):
-        h, self.h = self.h, None
+        h, self.h = getattr(self, "h", None), None
         if h:
             self.lib.eqg_runtime_destroy(h)
 

@@ -1,0 +1,42 @@
+"""Objects of the Python mirror as a program may meet them besides its plain
+runtime calls: before their __init__ has run.  Over the CPU oracle."""
+import subprocess
+import sys
+
+from conftest import ORACLE_LIB, ROOT
+
+
+# every route to a member that __init__ sets, each in a process of its own
+# (a crash there is this test's failure, not the end of the run)
+BEFORE_INIT = {
+    "operand": "x + 1.0", "operand_right": "1.0 - x", "operands": "y + x", "neg": "-x", "compare": "x < 2.0",
+    "compare_right": "y < x", "eq": "x.eq(y)", "mask": "~m", "masks": "(y < 2.0) & m", "rt": "x.rt", "h": "x.h",
+    "argument": "er.gradient(x)", "extend_over": "er.operatorExtend(1.0, s)", "on": "er.operatorOn(x, s, s)",
+    "select": "er.trinaryIf(m, x, x)", "first_cell": "er.firstCell(s)", "reduce": "er.maxReduce(x)",
+    "builtin": "early.allCells()", "method": "early.gradient(y)", "sqrt": "early.sqrt(y)",
+    "extend": "early.operatorExtend(1.0, er.allCells())", "norm2": "early.twoNorm(y)",
+    "span": "early.spanSubset(y, 0, 1)", "runtime_h": "early.h", "bound": "half.allFaces()"}
+
+
+def test_members_before_init_are_attribute_errors(oracle_lib):
+    code = """
+import ctypes, sys
+import numpy as np
+from equelle_b200 import capi
+from equelle_b200.runtime import CollOfBool, CollOfScalar, EntitySet, Runtime, _addresses
+lib = capi.bind(ctypes.CDLL(sys.argv[1], mode=ctypes.RTLD_LOCAL))
+er = Runtime(lib, dict(grid_dim=2, nx=8, ny=6))
+y = er.collection(np.arange(48.0))
+x, m, s = CollOfScalar.__new__(CollOfScalar), CollOfBool.__new__(CollOfBool), EntitySet.__new__(EntitySet)
+early, half = Runtime.__new__(Runtime), Runtime.__new__(Runtime)
+half.lib = lib
+half._bind(_addresses(lib))
+try:
+    eval(sys.argv[2])
+except AttributeError:
+    print("attribute error")
+"""
+    runs = {k: subprocess.Popen([sys.executable, "-c", code, ORACLE_LIB, e], cwd=ROOT, text=True,
+                                stdout=subprocess.PIPE, stderr=subprocess.PIPE) for k, e in BEFORE_INIT.items()}
+    out = {k: p.communicate() + (p.returncode,) for k, p in runs.items()}
+    assert {k: o for k, o in out.items() if o != ("attribute error\n", "", 0)} == {}
