@@ -27,7 +27,6 @@ except ImportError:  # not built yet: a few seconds of the system compiler
 
 class EntitySet(_mirror.SetBase):
     """CollOfCell / CollOfFace."""
-    __slots__ = ()
 
     def __len__(self):
         n = C.c_int64()
@@ -52,7 +51,6 @@ class EntitySet(_mirror.SetBase):
 
 class CollOfBool(_mirror.MaskBase):
     """Masks; & | ~ are native."""
-    __slots__ = ()
 
     def __len__(self):
         n = C.c_int64()
@@ -69,7 +67,6 @@ class CollOfBool(_mirror.MaskBase):
 class CollOfScalar(_mirror.CollBase):
     """Value plus optional Jacobian (AutoDiffBlock<double>).  Arithmetic
     (equelleTypes.hpp:86-211), negation, < <= > >= and eq(), ne() are native."""
-    __slots__ = ()
 
     def __len__(self):
         n = C.c_int64()

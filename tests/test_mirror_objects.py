@@ -1,9 +1,22 @@
 """Objects of the Python mirror as a program may meet them besides its plain
-runtime calls: before their __init__ has run.  Over the CPU oracle."""
+runtime calls: before their __init__ has run, with weak references and
+attributes.  Over the CPU oracle."""
+import gc
 import subprocess
 import sys
+import weakref
+
+import numpy as np
+import pytest
 
 from conftest import ORACLE_LIB, ROOT
+from equelle_b200.runtime import Runtime
+
+
+@pytest.fixture()
+def er(oracle_lib):
+    return Runtime(oracle_lib, dict(grid_dim=2, nx=8, ny=6))
+
 
 
 # every route to a member that __init__ sets, each in a process of its own
@@ -40,3 +53,24 @@ except AttributeError:
                                 stdout=subprocess.PIPE, stderr=subprocess.PIPE) for k, e in BEFORE_INIT.items()}
     out = {k: p.communicate() + (p.returncode,) for k, p in runs.items()}
     assert {k: o for k, o in out.items() if o != ("attribute error\n", "", 0)} == {}
+
+
+def test_handles_take_weak_references_and_attributes(er):
+    """As objects of ordinary classes: a weak reference that dies with the
+    handle, attributes, and cycles through them."""
+    for make in (lambda: er.collection(np.arange(48.0)), lambda: er.mask(np.ones(48)), er.allCells):
+        h = make()
+        gone = weakref.ref(h)
+        h.name = "pressure"
+        h.itself = h
+        assert h.name == "pressure" and gone() is h
+        with pytest.raises(AttributeError):
+            h.other
+        del h
+        gc.collect()
+        assert gone() is None
+    x = er.collection(np.arange(48.0))
+    kept = weakref.WeakValueDictionary(x=x)
+    assert np.array_equal((kept["x"] + 1.0).value(), np.arange(48.0) + 1.0)
+    del x
+    assert "x" not in kept
