@@ -67,10 +67,25 @@ const Entry kEntries[] = {E(last_error), E(set_builtin), E(set_size), E(set_rele
                           E(select), E(reduce), E(two_norm), E(span_subset), E(span_superset)};
 #undef E
 
-// Classes of the Python module, set by register_classes().
-PyObject* g_coll_class = nullptr;
-PyObject* g_mask_class = nullptr;
-PyObject* g_set_class = nullptr;
+// Classes of the Python module, set by register_classes(), and the runtime's
+// methods that make their objects.
+template <class T>
+struct Made;
+template <>
+struct Made<eqg_coll> {
+    static inline PyObject* cls = nullptr;
+    static constexpr const char* hook = "_coll";
+};
+template <>
+struct Made<eqg_mask> {
+    static inline PyObject* cls = nullptr;
+    static constexpr const char* hook = "_mask";
+};
+template <>
+struct Made<eqg_set> {
+    static inline PyObject* cls = nullptr;
+    static constexpr const char* hook = "_set";
+};
 PyObject* g_error_class = nullptr;
 
 struct RuntimeObject {
@@ -78,6 +93,7 @@ struct RuntimeObject {
     Api api;
     eqg_runtime* h;
     bool bound, created;  // has its library's entry points; has been given a handle
+    bool hooked;          // its class overrides a method that handles are made through
 };
 
 struct HandleObject {
@@ -145,14 +161,40 @@ PyObject* new_handle(PyObject* cls, RuntimeObject* rt, void* h)
     return (PyObject*)o;
 }
 
-// A call that makes a handle: status and out-parameter to a Python object.
-template <class T, class F>
-PyObject* make(PyObject* cls, RuntimeObject* rt, F&& f)
+PyObject* as_object(int v) { return PyLong_FromLong(v); }
+PyObject* as_object(int64_t v) { return PyLong_FromLongLong(v); }
+PyObject* as_object(double v) { return PyFloat_FromDouble(v); }
+PyObject* as_object(const void* v) { return v ? PyLong_FromVoidPtr((void*)v) : Py_NewRef(Py_None); }
+
+// runtime.<hook>(runtime.lib.<name>, args...)
+template <class... A>
+PyObject* call_hook(RuntimeObject* rt, const char* hook, const char* name, A... args)
 {
-    T* out = nullptr;
-    const int st = unlocked([&] { return f(&out); });
-    return st == EQG_OK ? new_handle(cls, rt, out) : raise_status(rt->api, st);
+    constexpr Py_ssize_t N = 1 + sizeof...(A);
+    PyObject* lib = PyObject_GetAttrString((PyObject*)rt, "lib");
+    PyObject* v[N] = {lib ? PyObject_GetAttrString(lib, name) : nullptr, as_object(args)...};
+    Py_XDECREF(lib);
+    PyObject* m = PyObject_GetAttrString((PyObject*)rt, hook);
+    bool ok = m != nullptr;
+    for (PyObject* o : v) ok = ok && o;
+    PyObject* r = ok ? PyObject_Vectorcall(m, v, N, nullptr) : nullptr;
+    for (PyObject* o : v) Py_XDECREF(o);
+    Py_XDECREF(m);
+    return r;
 }
+
+// Calls an entry point that makes a handle, and makes its Python object; a
+// runtime class with methods of its own for that (_coll and the like) makes it
+// through them.
+template <class T, class F, class... A>
+PyObject* make(RuntimeObject* rt, F Api::*fn, const char* name, A... args)
+{
+    if (rt->hooked) return call_hook(rt, Made<T>::hook, name, args...);
+    T* out = nullptr;
+    const int st = unlocked([&] { return (rt->api.*fn)(rt->h, args..., &out); });
+    return st == EQG_OK ? new_handle(Made<T>::cls, rt, out) : raise_status(rt->api, st);
+}
+#define ENTRY(name) &Api::name, "eqg_" #name
 
 // The handle inside a Python object: a handle type's own, or the integer in
 // its attribute `h`.
@@ -280,13 +322,12 @@ PyObject* coll_binary(int op, PyObject* left, PyObject* right)
         void *a0, *b0;
         if (!handle_of(left, &a0) || !handle_of(right, &b0)) return nullptr;
         const eqg_coll *a = (eqg_coll*)a0, *b = (eqg_coll*)b0;
-        return make<eqg_coll>(g_coll_class, rt, [&](eqg_coll** o) { return rt->api.binary(rt->h, op, a, b, o); });
+        return make<eqg_coll>(rt, ENTRY(binary), op, a, b);
     }
     double s;
     if (!double_of(l ? right : left, &s)) return nullptr;
     const eqg_coll* a = (eqg_coll*)self->h;
-    return make<eqg_coll>(g_coll_class, rt,
-                          [&](eqg_coll** o) { return rt->api.binary_scalar(rt->h, op, a, s, l ? 0 : 1, o); });
+    return make<eqg_coll>(rt, ENTRY(binary_scalar), op, a, s, l ? 0 : 1);
 }
 PyObject* coll_add(PyObject* a, PyObject* b) { return coll_binary(EQG_ADD, a, b); }
 PyObject* coll_sub(PyObject* a, PyObject* b) { return coll_binary(EQG_SUB, a, b); }
@@ -295,8 +336,7 @@ PyObject* coll_div(PyObject* a, PyObject* b) { return coll_binary(EQG_DIV, a, b)
 
 PyObject* unary_of(RuntimeObject* rt, int op, const void* h)
 {
-    return make<eqg_coll>(g_coll_class, rt,
-                          [&](eqg_coll** o) { return rt->api.unary(rt->h, op, (const eqg_coll*)h, o); });
+    return make<eqg_coll>(rt, ENTRY(unary), op, (const eqg_coll*)h);
 }
 PyObject* coll_neg(PyObject* self)
 {
@@ -313,12 +353,11 @@ PyObject* coll_compare_op(PyObject* self, int op, PyObject* other)
         void* b0;
         if (!handle_of(other, &b0)) return nullptr;
         const eqg_coll* b = (eqg_coll*)b0;
-        return make<eqg_mask>(g_mask_class, rt, [&](eqg_mask** o) { return rt->api.compare(rt->h, op, a, b, o); });
+        return make<eqg_mask>(rt, ENTRY(compare), op, a, b);
     }
     double v;
     if (!double_of(other, &v)) return nullptr;
-    return make<eqg_mask>(g_mask_class, rt,
-                          [&](eqg_mask** o) { return rt->api.compare_scalar(rt->h, op, a, v, 0, o); });
+    return make<eqg_mask>(rt, ENTRY(compare_scalar), op, a, v, 0);
 }
 PyObject* coll_richcompare(PyObject* self, PyObject* other, int op)
 {
@@ -346,9 +385,7 @@ PyObject* mask_logic_op(int op, PyObject* self, PyObject* other)
     if (!rt) return nullptr;
     void* b = nullptr;
     if (other && other != Py_None && !handle_of(other, &b)) return nullptr;
-    return make<eqg_mask>(g_mask_class, rt, [&](eqg_mask** o) {
-        return rt->api.mask_logic(rt->h, op, (eqg_mask*)s->h, (eqg_mask*)b, o);
-    });
+    return make<eqg_mask>(rt, ENTRY(mask_logic), op, (const eqg_mask*)s->h, (const eqg_mask*)b);
 }
 PyObject* mask_and(PyObject* a, PyObject* b) { return mask_logic_op(EQG_AND, a, b); }
 PyObject* mask_or(PyObject* a, PyObject* b) { return mask_logic_op(EQG_OR, a, b); }
@@ -390,8 +427,8 @@ bool take(const char* fn, PyObject* const* args, Py_ssize_t nargs, PyObject* kwn
 #define METHOD_ARGS PyObject *self, PyObject *const *args, Py_ssize_t nargs, PyObject *kwnames
 
 // Methods of one collection argument.
-template <class Get>
-PyObject* coll_method(METHOD_ARGS, const char* name, Get&& get)
+template <class F>
+PyObject* coll_method(METHOD_ARGS, const char* name, F Api::*fn, const char* entry)
 {
     static const char* const names[] = {"x"};
     PyObject* v[1];
@@ -399,25 +436,23 @@ PyObject* coll_method(METHOD_ARGS, const char* name, Get&& get)
     if (!take(name, args, nargs, kwnames, names, 1, 1, v) || !handle_of(v[0], &h)) return nullptr;
     RuntimeObject* rt = rt_of(self);
     if (!rt) return nullptr;
-    return make<eqg_coll>(g_coll_class, rt,
-                          [&](eqg_coll** o) { return get(rt->api)(rt->h, (const eqg_coll*)h, o); });
+    return make<eqg_coll>(rt, fn, entry, (const eqg_coll*)h);
 }
 PyObject* rt_gradient(METHOD_ARGS)
 {
-    return coll_method(self, args, nargs, kwnames, "gradient", [](const Api& a) { return a.gradient; });
+    return coll_method(self, args, nargs, kwnames, "gradient", ENTRY(gradient));
 }
 PyObject* rt_neg_gradient(METHOD_ARGS)
 {
-    return coll_method(self, args, nargs, kwnames, "negGradient", [](const Api& a) { return a.neg_gradient; });
+    return coll_method(self, args, nargs, kwnames, "negGradient", ENTRY(neg_gradient));
 }
 PyObject* rt_divergence(METHOD_ARGS)
 {
-    return coll_method(self, args, nargs, kwnames, "divergence", [](const Api& a) { return a.divergence; });
+    return coll_method(self, args, nargs, kwnames, "divergence", ENTRY(divergence));
 }
 PyObject* rt_interior_divergence(METHOD_ARGS)
 {
-    return coll_method(self, args, nargs, kwnames, "interiorDivergence",
-                       [](const Api& a) { return a.interior_divergence; });
+    return coll_method(self, args, nargs, kwnames, "interiorDivergence", ENTRY(interior_divergence));
 }
 PyObject* rt_sqrt(METHOD_ARGS)
 {
@@ -433,7 +468,7 @@ PyObject* builtin_set(PyObject* self, int which)
 {
     RuntimeObject* rt = rt_of(self);
     if (!rt) return nullptr;
-    return make<eqg_set>(g_set_class, rt, [&](eqg_set** o) { return rt->api.set_builtin(rt->h, which, o); });
+    return make<eqg_set>(rt, ENTRY(set_builtin), which);
 }
 PyObject* rt_all_cells(PyObject* self, PyObject*) { return builtin_set(self, EQG_ALL_CELLS); }
 PyObject* rt_boundary_cells(PyObject* self, PyObject*) { return builtin_set(self, EQG_BOUNDARY_CELLS); }
@@ -442,8 +477,8 @@ PyObject* rt_all_faces(PyObject* self, PyObject*) { return builtin_set(self, EQG
 PyObject* rt_boundary_faces(PyObject* self, PyObject*) { return builtin_set(self, EQG_BOUNDARY_FACES); }
 PyObject* rt_interior_faces(PyObject* self, PyObject*) { return builtin_set(self, EQG_INTERIOR_FACES); }
 
-template <class Get>
-PyObject* set_method(METHOD_ARGS, const char* name, Get&& get)
+template <class F>
+PyObject* set_method(METHOD_ARGS, const char* name, F Api::*fn, const char* entry)
 {
     static const char* const names[] = {"faces"};
     PyObject* v[1];
@@ -451,22 +486,23 @@ PyObject* set_method(METHOD_ARGS, const char* name, Get&& get)
     if (!take(name, args, nargs, kwnames, names, 1, 1, v) || !handle_of(v[0], &h)) return nullptr;
     RuntimeObject* rt = rt_of(self);
     if (!rt) return nullptr;
-    return make<eqg_set>(g_set_class, rt, [&](eqg_set** o) { return get(rt->api)(rt->h, (const eqg_set*)h, o); });
+    return make<eqg_set>(rt, fn, entry, (const eqg_set*)h);
 }
 PyObject* rt_first_cell(METHOD_ARGS)
 {
-    return set_method(self, args, nargs, kwnames, "firstCell", [](const Api& a) { return a.first_cell; });
+    return set_method(self, args, nargs, kwnames, "firstCell", ENTRY(first_cell));
 }
 PyObject* rt_second_cell(METHOD_ARGS)
 {
-    return set_method(self, args, nargs, kwnames, "secondCell", [](const Api& a) { return a.second_cell; });
+    return set_method(self, args, nargs, kwnames, "secondCell", ENTRY(second_cell));
 }
 
 PyObject* constant_of(RuntimeObject* rt, PyObject* value, int64_t n)
 {
+    if (rt->hooked) return PyObject_CallMethod((PyObject*)rt, "constant", "OL", value, (long long)n);
     double s;
     if (!double_of(value, &s)) return nullptr;
-    return make<eqg_coll>(g_coll_class, rt, [&](eqg_coll** o) { return rt->api.coll_constant(rt->h, s, n, o); });
+    return make<eqg_coll>(rt, ENTRY(coll_constant), s, n);
 }
 
 // operatorExtend(data, a, b=None): a constant over a, or data from a to b.
@@ -494,10 +530,8 @@ PyObject* rt_extend(METHOD_ARGS)
     if (!handle_of(v[0], &d) || !handle_of(v[1], &a) || !handle_of(v[2], &b)) return nullptr;
     const eqg_set *from = (eqg_set*)a, *to = (eqg_set*)b;
     if (PyObject_TypeCheck(v[0], &SetBaseType))
-        return make<eqg_set>(g_set_class, rt,
-                             [&](eqg_set** o) { return rt->api.set_extend(rt->h, (eqg_set*)d, from, to, o); });
-    return make<eqg_coll>(g_coll_class, rt,
-                          [&](eqg_coll** o) { return rt->api.extend(rt->h, (eqg_coll*)d, from, to, o); });
+        return make<eqg_set>(rt, ENTRY(set_extend), (const eqg_set*)d, from, to);
+    return make<eqg_coll>(rt, ENTRY(extend), (const eqg_coll*)d, from, to);
 }
 
 PyObject* rt_on(METHOD_ARGS)
@@ -512,10 +546,8 @@ PyObject* rt_on(METHOD_ARGS)
     if (!rt) return nullptr;
     const eqg_set *from = (eqg_set*)a, *to = (eqg_set*)b;
     if (PyObject_TypeCheck(v[0], &SetBaseType))
-        return make<eqg_set>(g_set_class, rt,
-                             [&](eqg_set** o) { return rt->api.set_on(rt->h, (eqg_set*)d, from, to, o); });
-    return make<eqg_coll>(g_coll_class, rt,
-                          [&](eqg_coll** o) { return rt->api.on(rt->h, (eqg_coll*)d, from, to, o); });
+        return make<eqg_set>(rt, ENTRY(set_on), (const eqg_set*)d, from, to);
+    return make<eqg_coll>(rt, ENTRY(on), (const eqg_coll*)d, from, to);
 }
 
 PyObject* rt_trinary_if(METHOD_ARGS)
@@ -530,12 +562,8 @@ PyObject* rt_trinary_if(METHOD_ARGS)
     if (!rt) return nullptr;
     const eqg_mask* p = (eqg_mask*)m;
     if (PyObject_TypeCheck(v[1], &SetBaseType))
-        return make<eqg_set>(g_set_class, rt, [&](eqg_set** o) {
-            return rt->api.set_select(rt->h, p, (eqg_set*)a, (eqg_set*)b, o);
-        });
-    return make<eqg_coll>(g_coll_class, rt, [&](eqg_coll** o) {
-        return rt->api.select(rt->h, p, (eqg_coll*)a, (eqg_coll*)b, o);
-    });
+        return make<eqg_set>(rt, ENTRY(set_select), p, (const eqg_set*)a, (const eqg_set*)b);
+    return make<eqg_coll>(rt, ENTRY(select), p, (const eqg_coll*)a, (const eqg_coll*)b);
 }
 
 PyObject* reduce_of(METHOD_ARGS, const char* name, int op)
@@ -550,6 +578,12 @@ PyObject* reduce_of(METHOD_ARGS, const char* name, int op)
     const int st = unlocked([&] {
         return op < 0 ? rt->api.two_norm(rt->h, (eqg_coll*)h, &r) : rt->api.reduce(rt->h, op, (eqg_coll*)h, &r);
     });
+    if (rt->hooked) {
+        PyObject* checked = PyObject_CallMethod((PyObject*)rt, "_ok", "i", st);
+        if (!checked) return nullptr;
+        Py_DECREF(checked);
+        return PyFloat_FromDouble(r);
+    }
     return st == EQG_OK ? PyFloat_FromDouble(r) : raise_status(rt->api, st);
 }
 PyObject* rt_min(METHOD_ARGS) { return reduce_of(self, args, nargs, kwnames, "minReduce", EQG_MIN); }
@@ -577,17 +611,21 @@ PyObject* span_of(METHOD_ARGS, bool subset)
     }
     RuntimeObject* rt = rt_of(self);
     if (!rt) return nullptr;
-    return make<eqg_coll>(g_coll_class, rt, [&](eqg_coll** o) {
-        return (subset ? rt->api.span_subset : rt->api.span_superset)(rt->h, (eqg_coll*)h, n[0], n[1], o);
-    });
+    const eqg_coll* x = (const eqg_coll*)h;
+    return subset ? make<eqg_coll>(rt, ENTRY(span_subset), x, n[0], n[1])
+                  : make<eqg_coll>(rt, ENTRY(span_superset), x, n[0], n[1]);
 }
 PyObject* rt_span_subset(METHOD_ARGS) { return span_of(self, args, nargs, kwnames, true); }
 PyObject* rt_span_superset(METHOD_ARGS) { return span_of(self, args, nargs, kwnames, false); }
 
-// _bind({name: address}): the entry points of the runtime's library.
-PyObject* rt_bind(PyObject* self, PyObject* table)
+// _bind({name: address}, hooked=False): the entry points of the runtime's
+// library, and whether handles go through methods that its class overrides.
+PyObject* rt_bind(PyObject* self, PyObject* args)
 {
     RuntimeObject* rt = (RuntimeObject*)self;
+    PyObject* table;
+    int hooked = 0;
+    if (!PyArg_ParseTuple(args, "O|p", &table, &hooked)) return nullptr;
     for (const Entry& e : kEntries) {
         PyObject* a = PyMapping_GetItemString(table, e.name);
         if (!a) return nullptr;
@@ -600,6 +638,7 @@ PyObject* rt_bind(PyObject* self, PyObject* table)
         std::memcpy((char*)&rt->api + e.offset, &p, sizeof(p));
     }
     rt->bound = true;
+    rt->hooked = hooked != 0;
     Py_RETURN_NONE;
 }
 
@@ -624,7 +663,7 @@ int rt_set_h(PyObject* self, PyObject* v, void*)
 PyGetSetDef rt_getset[] = {{"h", rt_get_h, rt_set_h, nullptr, nullptr}, {nullptr, nullptr, nullptr, nullptr, nullptr}};
 
 #define FAST(f) (PyCFunction)(void (*)(void))(f), METH_FASTCALL | METH_KEYWORDS, nullptr
-PyMethodDef rt_methods[] = {{"_bind", rt_bind, METH_O, nullptr},
+PyMethodDef rt_methods[] = {{"_bind", rt_bind, METH_VARARGS, nullptr},
                             {"gradient", FAST(rt_gradient)},
                             {"negGradient", FAST(rt_neg_gradient)},
                             {"divergence", FAST(rt_divergence)},
@@ -675,9 +714,9 @@ PyObject* register_classes(PyObject*, PyObject* args)
         PyErr_SetString(PyExc_TypeError, "the classes must derive from CollBase, MaskBase and SetBase");
         return nullptr;
     }
-    Py_XSETREF(g_coll_class, Py_NewRef(c));
-    Py_XSETREF(g_mask_class, Py_NewRef(m));
-    Py_XSETREF(g_set_class, Py_NewRef(s));
+    Py_XSETREF(Made<eqg_coll>::cls, Py_NewRef(c));
+    Py_XSETREF(Made<eqg_mask>::cls, Py_NewRef(m));
+    Py_XSETREF(Made<eqg_set>::cls, Py_NewRef(s));
     Py_XSETREF(g_error_class, Py_NewRef(e));
     Py_RETURN_NONE;
 }

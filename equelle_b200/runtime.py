@@ -145,7 +145,9 @@ class Runtime(_mirror.RuntimeBase):
 
     def __init__(self, lib, params):
         self.lib = lib
-        self._bind(_addresses(lib))
+        # a class that overrides the methods handles are made through gets them
+        # called, by the native methods too
+        self._bind(_addresses(lib), any(getattr(type(self), n) is not f for n, f in _PLAIN.items()))
         keys = [str(k).encode() for k in params]
         vals = [str(v).lower() if isinstance(v, bool) else str(v) for v in params.values()]
         vals = [v.encode() for v in vals]
@@ -310,3 +312,6 @@ class Runtime(_mirror.RuntimeBase):
 
     def synchronize(self):
         self._ok(self.lib.eqg_runtime_synchronize(self.h))
+
+
+_PLAIN = {n: vars(Runtime)[n] for n in ("_ok", "_out", "_coll", "_mask", "_set", "constant")}

@@ -1,6 +1,7 @@
 """Objects of the Python mirror as a program may meet them besides its plain
 runtime calls: before their __init__ has run, with weak references and
-attributes.  Over the CPU oracle."""
+attributes, and of classes that override the methods handles are made
+through.  Over the CPU oracle."""
 import gc
 import subprocess
 import sys
@@ -74,3 +75,65 @@ def test_handles_take_weak_references_and_attributes(er):
     assert np.array_equal((kept["x"] + 1.0).value(), np.arange(48.0) + 1.0)
     del x
     assert "x" not in kept
+
+
+def test_overridden_plumbing_is_called(oracle_lib):
+    """A Runtime subclass that overrides the methods every handle is made
+    through sees each call, with the entry point and its arguments; the
+    results are those of the plain class."""
+    class Traced(Runtime):
+        def __init__(self, *args):
+            self.calls = []
+            super().__init__(*args)
+
+        def _coll(self, fn, *args):
+            self.calls.append((fn.__name__, len(args)))
+            return super()._coll(fn, *args)
+
+        def _mask(self, fn, *args):
+            self.calls.append((fn.__name__, len(args)))
+            return super()._mask(fn, *args)
+
+        def _set(self, fn, *args):
+            self.calls.append((fn.__name__, len(args)))
+            return super()._set(fn, *args)
+
+        def constant(self, value, n):
+            self.calls.append(("constant", value, n))
+            return super().constant(value, n)
+
+    class Checked(Runtime):
+        statuses = []
+
+        def _ok(self, status):
+            self.statuses.append(status)
+            super()._ok(status)
+
+    grid = dict(grid_dim=2, nx=8, ny=6)
+
+    def stream(er):
+        x, cells = er.collection(np.linspace(0.5, 2.0, 48)), er.allCells()
+        faces = er.interiorFaces()
+        f = er.firstCell(faces)
+        m = ~((x < 1.0) & (x < x)) | x.eq(2.0)
+        y = er.trinaryIf(m, x + x, 2.0 / x)
+        z = er.operatorOn(y, cells, f) * er.sqrt(er.operatorExtend(4.0, faces)) - er.gradient(-y)
+        return [m.values(), er.divergence(z).value(), er.spanSuperset(er.spanSubset(y, 3, 4), 1, 9).value(),
+                np.array([er.maxReduce(y), er.twoNorm(z)]), er.trinaryIf(m, cells, cells).indices()]
+
+    traced = Traced(oracle_lib, grid)
+    got = stream(traced)
+    assert traced.calls == [
+        ("eqg_coll_from_host", 2), ("eqg_set_builtin", 1), ("eqg_set_builtin", 1), ("eqg_first_cell", 1),
+        ("eqg_compare_scalar", 4), ("eqg_compare", 3), ("eqg_mask_logic", 3), ("eqg_mask_logic", 3),
+        ("eqg_compare_scalar", 4), ("eqg_mask_logic", 3), ("eqg_binary", 3), ("eqg_binary_scalar", 4),
+        ("eqg_select", 3), ("eqg_on", 3), ("constant", 4.0, 7 * 6 + 8 * 5), ("eqg_coll_constant", 2), ("eqg_unary", 2),
+        ("eqg_binary", 3), ("eqg_unary", 2), ("eqg_gradient", 1), ("eqg_binary", 3), ("eqg_divergence", 1),
+        ("eqg_span_subset", 3), ("eqg_span_superset", 3), ("eqg_set_select", 3)]
+    want = stream(Runtime(oracle_lib, grid))
+    checked = Checked(oracle_lib, grid)
+    for g, c, w in zip(got, stream(checked), want):
+        assert np.array_equal(g, w) and np.array_equal(c, w)
+    n = len(checked.statuses)
+    checked.minReduce(checked.constant(1.0, 3))
+    assert checked.statuses[n:] == [0, 0]
