@@ -247,14 +247,37 @@ int handle_init(PyObject* self, PyObject* args, PyObject* kwargs)
     return 0;
 }
 
-// Gives the handle back to its library and lets go of the runtime.
+// Whether there are other threads of the interpreter.  (Thread states are
+// deleted with the interpreter lock held, which the caller has.)
+bool other_threads()
+{
+    PyThreadState* head = PyInterpreterState_ThreadHead(PyInterpreterState_Get());
+    return head && PyThreadState_Next(head);
+}
+
+// Gives the handle back to its library and lets go of the runtime.  Without
+// the interpreter lock where another thread may want it: the release of a
+// destroyed runtime's last handle waits for its stream.  (Letting the lock go
+// takes 65 ns, a fifth of an operation on small collections.)  The object
+// holds nothing any more when other threads may run.
 template <class Release>
 int handle_drop(PyObject* self, Release&& release)
 {
     HandleObject* o = (HandleObject*)self;
-    if (o->h && o->rt && o->rt->bound) release(o->rt->api, o->h);
+    void* h = o->h;
+    RuntimeObject* rt = o->rt;
     o->h = nullptr;
-    Py_CLEAR(o->rt);
+    o->rt = nullptr;
+    if (h && rt && rt->bound) {
+        if (other_threads()) {
+            Py_BEGIN_ALLOW_THREADS
+            release(rt->api, h);
+            Py_END_ALLOW_THREADS
+        } else {
+            release(rt->api, h);
+        }
+    }
+    Py_XDECREF(rt);
     return 0;
 }
 int coll_clear(PyObject* self)

@@ -1,17 +1,20 @@
 """Objects of the Python mirror as a program may meet them besides its plain
 runtime calls: before their __init__ has run, with weak references and
-attributes, and of classes that override the methods handles are made
-through.  Over the CPU oracle."""
+attributes, of classes that override the methods handles are made through,
+and while other threads run.  Over the CPU oracle."""
+import ctypes
 import gc
 import subprocess
 import sys
+import threading
+import time
 import weakref
 
 import numpy as np
 import pytest
 
 from conftest import ORACLE_LIB, ROOT
-from equelle_b200.runtime import Runtime
+from equelle_b200.runtime import CollOfBool, CollOfScalar, EntitySet, Runtime, _mirror
 
 
 @pytest.fixture()
@@ -137,3 +140,32 @@ def test_overridden_plumbing_is_called(oracle_lib):
     n = len(checked.statuses)
     checked.minReduce(checked.constant(1.0, 3))
     assert checked.statuses[n:] == [0, 0]
+
+
+@pytest.mark.parametrize("kind", ["coll", "mask", "set"])
+def test_handles_are_released_without_the_interpreter_lock(kind):
+    """A library's release may take long (the last handle of a destroyed
+    runtime waits for its stream): other threads run meanwhile.  The release
+    is libc's usleep here, its argument the handle."""
+    classes = dict(coll=CollOfScalar, mask=CollOfBool, set=EntitySet)
+    usleep = ctypes.cast(ctypes.CDLL(None).usleep, ctypes.c_void_p).value
+    er = Runtime.__new__(Runtime)
+    er._bind({n: usleep for n in _mirror.entry_points()})
+    er.h = None
+    started = threading.Event()
+
+    def drop():
+        x = classes[kind](er, 900000)
+        started.set()
+        del x
+
+    t = threading.Thread(target=drop)
+    longest, last = 0.0, time.perf_counter()
+    t.start()
+    started.wait()
+    while t.is_alive():
+        now = time.perf_counter()
+        longest, last = max(longest, now - last), now
+        time.sleep(0.001)
+    t.join()
+    assert longest < 0.45
