@@ -20,9 +20,16 @@ from . import capi
 try:
     from . import _mirror
 except ImportError:  # not built yet: a few seconds of the system compiler
-    from . import build
-    build.build_mirror()
-    from . import _mirror
+    try:
+        from . import build
+        build.build_mirror()
+        from . import _mirror
+    except (ImportError, OSError, RuntimeError) as e:
+        import warnings
+        warnings.warn("the native module equelle_b200._mirror is not built and cannot be built here (%s); runtime "
+                      "calls go through ctypes, some ten times the host time each" % str(e).splitlines()[0],
+                      RuntimeWarning, stacklevel=2)
+        from . import _mirror_py as _mirror
 
 
 class EntitySet(_mirror.SetBase):
