@@ -48,6 +48,7 @@
 // returns at once after convergence or breakdown, so the host enqueues
 // several iterations between convergence checks without a round trip.
 #include "eqg_internal.cuh"
+#include "size_limits.cuh"
 
 #include <algorithm>
 #include <chrono>

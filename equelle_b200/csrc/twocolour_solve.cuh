@@ -72,17 +72,17 @@ void rb_gather(Core& c, const SolverAnalysis& an, const double* jval)
 
 // The two-colour hierarchy of a system of `bs` unknowns per cell of the
 // Cartesian grid, built on the device; false when its pattern couples cells
-// that are no neighbours.
+// that are no neighbours, or the form has no room for it.
 bool rb_analyse(Core& c, SolverAnalysis& an, const Pattern& p, int bs, int coarsest, const double* jval)
 {
     const int nd = c.nz > 1 ? 6 : 4, bb = bs * bs;
+    if (!two_colour_fits((int64_t)c.nx * c.ny * c.nz, nd, bb)) return false;
     an.rb_bs = bs;
     an.rb_nd = nd;
     an.rb.emplace_back();
     {
         RbLevel& L = an.rb[0];
         L.g = RbGrid(c.nx, c.ny, c.nz);
-        if ((double)L.g.n * (nd + 2) * bb >= (double)INT_MAX) fail(EQG_ERR_UNSUPPORTED, "linear system too large for 32-bit value offsets");
         const size_t entries = (size_t)L.g.n * (nd + 1) * bb;
         an.vmap = c.allocN<int>(entries);
         Buf bad = c.allocN<int>(1);
