@@ -13,6 +13,7 @@
 // the input patterns (and operator), so each Newton iteration after the
 // first only runs the numeric kernels.
 #include "eqg_internal.cuh"
+#include "size_limits.cuh"
 
 #include <cub/cub.cuh>
 
@@ -957,7 +958,7 @@ PatternP pattern_spgemm(Core& c, const OpMatrix& m, const PatternP& j, bool with
     default: spgemm_symbolic<16>(c, m, *j, *p); break;
     }
     // the position plan, for weights of 1 and -1
-    if (with_plan && m.unit && c.param_i("spgemm_plan", 1) != 0 && p->nnz < (int64_t)INT_MAX / 2) {
+    if (with_plan && m.unit && c.param_i("spgemm_plan", 1) != 0 && plan_fits(j->nnz, p->nnz)) {
         switch (kmax_for(m.max_row)) {
         case 1: spgemm_build_plan<1>(c, m, *j, *p); break;
         case 2: spgemm_build_plan<2>(c, m, *j, *p); break;
