@@ -84,6 +84,9 @@ struct Pattern {
     // a union)
     uint64_t concat_first = 0, concat_second = 0;
     std::shared_ptr<SolverAnalysis> analysis;  // linear-solver analysis, built on demand
+    // the one that a system of this pattern with other strong directions had
+    // (two-colour form)
+    std::shared_ptr<SolverAnalysis> analysis_other;
     // the analysis without multigrid, for a solve that the multigrid
     // preconditioner did not converge (linsolver_fallback)
     std::shared_ptr<SolverAnalysis> analysis_fallback;

@@ -1728,6 +1728,14 @@ struct RbLevel {
     Buf a64, a32;            // matrix, then its factors
     Buf inv64, inv32;        // coarsest level
     Buf v64;                 // right-hand side; red work vector and black iterate
+
+    void allocate(Core& c, int bs, int nd)
+    {
+        n = g.n * bs;
+        vals = (int64_t)RbMatrix<double>::values(nd, bs * bs, g.n, g.nr);
+        a64 = c.allocN<double>((size_t)vals);
+        v64 = c.allocN<double>((size_t)2 * n);
+    }
 };
 
 struct SolverAnalysis {
@@ -1740,6 +1748,10 @@ struct SolverAnalysis {
     // its block size and number of directions
     std::vector<RbLevel> rb;
     int rb_bs = 1, rb_nd = 4;
+    // directions of more than one cell, the most unknowns of its coarsest
+    // level, and the directions that each level pairs (choose_hierarchy)
+    int rb_directions = 1, rb_coarsest = 1;
+    std::vector<int> rb_pairs;
     std::vector<Level> levels;
     Buf vmap;        // level-0 value <- Jacobian entry (-1: zero)
     Buf vec64, vec32, scal, partials, counter, factor_status;
@@ -2135,7 +2147,7 @@ std::shared_ptr<SolverAnalysis> analyse(Core& c, const Pattern& p, bool natural,
     an->nnz = p.nnz;
     an->natural = natural;
     an->scal = c.alloc(sizeof(KScal));
-    an->factor_status = c.allocN<int>(1);
+    an->factor_status = c.allocN<double>(4);  // a flag (int); in the two-colour form also the strengths, from [1] on
     HostCsr A;
     A.n = n;
     auto read_pattern = [&] {
@@ -3220,23 +3232,35 @@ namespace {
 
 #include "twocolour_solve.cuh"
 
-// One solve in the two-colour form.
-SolveResult solve_rb(Core& c, SolverAnalysis& an, const double* jval, const double* rhs, double* xout, bool mixed,
-                     double tol, int max_iter, int check_every)
+// One solve in the two-colour form, with the hierarchy that the system's own
+// strengths choose: results do not depend on the systems solved before.
+// `slot` is the analysis of the pattern's last solve; where this system needs
+// other pairs, the analysis of the solve before that (`other`) is used or
+// replaced, so that systems that alternate find theirs again.
+SolveResult solve_rb(Core& c, std::shared_ptr<SolverAnalysis>& slot, std::shared_ptr<SolverAnalysis>& other,
+                     const double* jval, const double* rhs, double* xout, bool mixed, double tol, int max_iter,
+                     int check_every)
 {
-    c.factor_clock.start(c.stream);
-    EQG_CUDA(cudaMemsetAsync(an.factor_status->ptr, 0, sizeof(int), c.stream));
-    rb_setup(c, an, jval, mixed);
-    prepare_tail_trace(c, an);
-    if (mixed) prepare_rb_tail<float>(c, an);
-    else prepare_rb_tail<double>(c, an);
-    c.factor_clock.stop(c.stream);
-    int fstat = 0;
-    EQG_CUDA(cudaMemcpyAsync(c.pinned, an.factor_status->ptr, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    c.sync();
-    std::memcpy(&fstat, c.pinned, sizeof(int));
+    bool zero_pivot = false;
+    for (int pass = 0; pass < 2; ++pass) {
+        SolverAnalysis& an = *slot;
+        c.factor_clock.start(c.stream);
+        EQG_CUDA(cudaMemsetAsync(an.factor_status->ptr, 0, sizeof(int), c.stream));
+        rb_setup(c, an, jval, mixed);
+        prepare_tail_trace(c, an);
+        if (mixed) prepare_rb_tail<float>(c, an);
+        else prepare_rb_tail<double>(c, an);
+        c.factor_clock.stop(c.stream);
+        zero_pivot = rb_report(c, an);
+        if (an.rb_directions < 2 || pass) break;
+        std::vector<int> pairs = choose_hierarchy(an.rb[0].g, an.rb_bs, an.rb_coarsest, c.pinned + 1);
+        if (pairs == an.rb_pairs) break;
+        if (!other || other->rb_pairs != pairs) other = rb_repaired(c, an, std::move(pairs));
+        std::swap(slot, other);
+    }
+    SolverAnalysis& an = *slot;
     SolveResult res;
-    if (fstat) return res;  // zero pivot
+    if (zero_pivot) return res;
     c.krylov_clock.start(c.stream);
     res = mixed ? bicgstab_rb<float>(c, an, rhs, xout, tol, max_iter, check_every)
                 : bicgstab_rb<double>(c, an, rhs, xout, tol, max_iter, check_every);
@@ -3280,7 +3304,7 @@ SolveResult solve_with(Core& c, const PatternP& p, std::shared_ptr<SolverAnalysi
         res.converged = true;
         return res;
     }
-    if (!an.rb.empty()) return solve_rb(c, an, jval, rhs, xout, mixed, tol, max_iter, check_every);
+    if (!an.rb.empty()) return solve_rb(c, slot, p->analysis_other, jval, rhs, xout, mixed, tol, max_iter, check_every);
     // level matrices and their factorizations (FP64)
     c.factor_clock.start(c.stream);
     const Level& L0 = an.levels[0];

@@ -33,10 +33,10 @@ RbMatrix<const M> rb_matrix(const SolverAnalysis& an, const RbLevel& L)
 // 18 with three.  At 4 : 1 one z-pairing level and none are equal.
 constexpr double kSemiCoarsen = 6.5;
 
-// The aggregation of the next level from the direction strengths, which are
-// updated to that level's: a coarse cell has twice as many fine couplings for
-// every other direction that was paired.
-Aggregates choose_aggregates(const RbGrid& g, double (&strength)[3])
+// The directions that the next level pairs, bit d for direction d, from the
+// direction strengths, which are updated to that level's: a coarse cell has
+// twice as many fine couplings for every other direction that was paired.
+int choose_pairs(const RbGrid& g, double (&strength)[3])
 {
     const int dims[3] = {g.nx, g.ny, g.nz};
     double top = 0.0;
@@ -48,14 +48,33 @@ Aggregates choose_aggregates(const RbGrid& g, double (&strength)[3])
         cut += s[d];
     }
     for (int d = 0; d < 3; ++d) strength[d] *= std::ldexp(1.0, cut - s[d]);
+    return s[0] | s[1] << 1 | s[2] << 2;
+}
+
+Aggregates aggregates_of(const RbGrid& g, int pairs)
+{
     Aggregates a;
-    a.sx = s[0];
-    a.sy = s[1];
-    a.sz = s[2];
+    a.sx = pairs & 1;
+    a.sy = pairs >> 1 & 1;
+    a.sz = pairs >> 2;
+    const int cut = a.sx + a.sy + a.sz;
     a.g = cut > 0 ? 1 << (cut - 1) : 1;
     a.fine = g;
-    a.coarse = RbGrid((g.nx + s[0]) >> s[0], (g.ny + s[1]) >> s[1], (g.nz + s[2]) >> s[2]);
+    a.coarse = RbGrid((g.nx + a.sx) >> a.sx, (g.ny + a.sy) >> a.sy, (g.nz + a.sz) >> a.sz);
     return a;
+}
+
+// The pairs of every level of a hierarchy whose coarsest level has at most
+// `coarsest` unknowns, `bs` per cell.
+std::vector<int> choose_hierarchy(RbGrid g, int bs, int coarsest, const double* strength)
+{
+    double s[3] = {strength[0], strength[1], strength[2]};
+    std::vector<int> pairs;
+    do {
+        pairs.push_back(choose_pairs(g, s));
+        g = aggregates_of(g, pairs.back()).coarse;
+    } while (g.n * bs > coarsest && g.n > 1);
+    return pairs;
 }
 
 void rb_gather(Core& c, const SolverAnalysis& an, const double* jval)
@@ -70,6 +89,57 @@ void rb_gather(Core& c, const SolverAnalysis& an, const double* jval)
     }, 12.0 * vals + 8.0 * an.nnz);
 }
 
+// The strengths of the gathered matrix's directions (rb_strength_kernel).
+void rb_strengths(Core& c, const SolverAnalysis& an)
+{
+    const RbGrid& g = an.rb[0].g;
+    double* out = an.factor_status->as<double>() + 1;
+    WITH_BS(an.rb_bs, launch(c, "mg_strength", [&] {
+                rb_strength_kernel<BS><<<blocksFor(g.n, kThreads, kRedBlocks), kThreads, 0, c.stream>>>(
+                    g, an.rb_nd, an.rb[0].a64->as<double>(), an.partials->as<double>(),
+                    an.counter->as<unsigned int>(), out);
+            }, 8.0 * an.rb_bs * (an.rb_nd + 1) * g.n));
+}
+
+// Waits for what a set-up reports: whether a pivot was zero, and the
+// strengths, to c.pinned[1..3] (grids of more than one direction).
+bool rb_report(Core& c, const SolverAnalysis& an)
+{
+    EQG_CUDA(cudaMemcpyAsync(c.pinned, an.factor_status->ptr, 4 * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    c.sync();
+    int fstat = 0;
+    std::memcpy(&fstat, c.pinned, sizeof(int));
+    return fstat != 0;
+}
+
+// The levels below level 0, as an.rb_pairs says.
+void rb_levels(Core& c, SolverAnalysis& an)
+{
+    const int bs = an.rb_bs, nd = an.rb_nd;
+    for (size_t l = 0; l < an.rb_pairs.size(); ++l) {
+        RbLevel C;
+        {
+            RbLevel& F = an.rb[l];
+            F.agg = aggregates_of(F.g, an.rb_pairs[l]);
+            const int cut = F.agg.sx + F.agg.sy + F.agg.sz;
+            F.alpha = c.param_d("linsolver_mg_alpha", cut == 2 && c.nz == 1 ? kMgAlpha2d : kMgAlpha3d);
+            F.pre = cut > 1;
+            C.g = F.agg.coarse;
+        }
+        C.allocate(c, bs, nd);
+        if (l + 1 == an.rb_pairs.size()) {
+            C.coarsest = true;
+            C.inv64 = c.allocN<double>((size_t)C.n * C.n);
+        }
+        an.rb.push_back(std::move(C));
+    }
+    if (c.verbose > 2) {
+        std::printf("        linear solver: %dx%d blocks, two colours, levels:", bs, bs);
+        for (auto& L : an.rb) std::printf(" %dx%dx%d", L.g.nx, L.g.ny, L.g.nz);
+        std::printf("\n");
+    }
+}
+
 // The two-colour hierarchy of a system of `bs` unknowns per cell of the
 // Cartesian grid, built on the device; false when its pattern couples cells
 // that are no neighbours, or the form has no room for it.
@@ -79,6 +149,7 @@ bool rb_analyse(Core& c, SolverAnalysis& an, const Pattern& p, int bs, int coars
     if (!two_colour_fits((int64_t)c.nx * c.ny * c.nz, nd, bb)) return false;
     an.rb_bs = bs;
     an.rb_nd = nd;
+    an.rb_coarsest = coarsest;
     an.rb.emplace_back();
     {
         RbLevel& L = an.rb[0];
@@ -106,57 +177,51 @@ bool rb_analyse(Core& c, SolverAnalysis& an, const Pattern& p, int bs, int coars
             return true;
         }
     }
-    an.partials = c.allocN<double>((size_t)kRedBlocks * 3 + 3);
+    an.partials = c.allocN<double>((size_t)kRedBlocks * 9);
     an.counter = c.allocN<unsigned int>(1);
     EQG_CUDA(cudaMemsetAsync(an.counter->ptr, 0, sizeof(unsigned int), c.stream));
-    auto allocate = [&](RbLevel& L) {
-        L.n = L.g.n * bs;
-        L.vals = (int64_t)RbMatrix<double>::values(nd, bb, L.g.n, L.g.nr);
-        L.a64 = c.allocN<double>((size_t)L.vals);
-        L.v64 = c.allocN<double>((size_t)2 * L.n);
-    };
-    allocate(an.rb[0]);
-    double strength[3] = {1.0, 1.0, 1.0};
-    if ((c.nx > 1) + (c.ny > 1) + (c.nz > 1) > 1) {
-        rb_gather(c, an, jval);
-        double* out = an.partials->as<double>() + (size_t)kRedBlocks * 3;
-        launch(c, "mg_strength", [&] {
-            rb_strength_kernel<<<blocksFor(an.rb[0].g.n, kThreads, kRedBlocks), kThreads, 0, c.stream>>>(
-                an.rb[0].g, bs, nd, an.rb[0].a64->as<double>(), an.partials->as<double>(),
-                an.counter->as<unsigned int>(), out);
-        });
-        EQG_CUDA(cudaMemcpyAsync(c.pinned, out, 3 * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-        c.sync();
-        for (int d = 0; d < 3; ++d) strength[d] = c.pinned[d];
-    }
-    for (;;) {
-        RbLevel& F = an.rb.back();
-        F.agg = choose_aggregates(F.g, strength);
-        const int cut = F.agg.sx + F.agg.sy + F.agg.sz;
-        F.alpha = c.param_d("linsolver_mg_alpha", cut == 2 && c.nz == 1 ? kMgAlpha2d : kMgAlpha3d);
-        F.pre = cut > 1;
-        RbLevel C;
-        C.g = F.agg.coarse;
-        allocate(C);
-        const bool last = C.n <= coarsest || C.g.n == 1;
-        if (last) {
-            C.coarsest = true;
-            C.inv64 = c.allocN<double>((size_t)C.n * C.n);
-        }
-        an.rb.push_back(std::move(C));
-        if (last) break;
-    }
-    // the right-hand side, and the BiCGStab vectors of the black half
+    an.rb[0].allocate(c, bs, nd);
     const RbGrid& g = an.rb[0].g;
+    an.rb_directions = (c.nx > 1) + (c.ny > 1) + (c.nz > 1);
+    double strength[3] = {1.0, 1.0, 1.0};
+    if (an.rb_directions > 1) {
+        rb_gather(c, an, jval);
+        rb_strengths(c, an);
+        rb_report(c, an);
+        for (int d = 0; d < 3; ++d) strength[d] = c.pinned[1 + d];
+    }
+    an.rb_pairs = choose_hierarchy(g, bs, coarsest, strength);
+    // the right-hand side, and the BiCGStab vectors of the black half
     an.vec64 = c.allocN<double>(vec_stride(an.n) + 10 * vec_stride((g.n - g.nr) * bs));
     an.multigrid = true;
-    if (c.verbose > 2) {
-        std::printf("        linear solver: %dx%d blocks, two colours, direction strengths %.3g %.3g %.3g, levels:", bs,
-                    bs, strength[0], strength[1], strength[2]);
-        for (auto& L : an.rb) std::printf(" %dx%dx%d", L.g.nx, L.g.ny, L.g.nz);
-        std::printf("\n");
-    }
+    rb_levels(c, an);
     return true;
+}
+
+// The analysis of the same pattern for other pairs: level 0 and the vectors
+// are those of `an`.
+std::shared_ptr<SolverAnalysis> rb_repaired(Core& c, const SolverAnalysis& an, std::vector<int> pairs)
+{
+    auto b = std::make_shared<SolverAnalysis>();
+    b->n = an.n;
+    b->nnz = an.nnz;
+    b->natural = an.natural;
+    b->multigrid = true;
+    b->rb_bs = an.rb_bs;
+    b->rb_nd = an.rb_nd;
+    b->rb_coarsest = an.rb_coarsest;
+    b->rb_directions = an.rb_directions;
+    b->rb_pairs = std::move(pairs);
+    b->vmap = an.vmap;
+    b->vec64 = an.vec64;
+    b->scal = an.scal;
+    b->partials = an.partials;
+    b->counter = an.counter;
+    b->factor_status = an.factor_status;
+    b->rb.push_back(an.rb[0]);
+    b->rb[0].threads = kThreads;
+    rb_levels(c, *b);
+    return b;
 }
 
 // Matrices of every level and their factors from the Jacobian's values.
@@ -165,6 +230,7 @@ void rb_setup(Core& c, SolverAnalysis& an, const double* jval, bool mixed)
     const int bs = an.rb_bs, bb = bs * bs, nd = an.rb_nd;
     int* status = an.factor_status->as<int>();
     rb_gather(c, an, jval);
+    if (an.rb_directions > 1) rb_strengths(c, an);
     for (size_t l = 0; l + 1 < an.rb.size(); ++l) {
         const RbLevel &F = an.rb[l], &C = an.rb[l + 1];
         launch(c, "mg_galerkin", [&] {
