@@ -93,7 +93,10 @@ __device__ __forceinline__ bool stopped(const KScal* sc) { return sc->status != 
 // programmatic dependent launches (launch_k), so their blocks may be
 // scheduled while the kernel before them on the stream still runs; this
 // waits until that kernel has completed and its writes are visible (at once
-// when the kernel was launched normally).
+// when the kernel was launched normally).  Vectors that the kernel before may
+// still be writing when this one starts are not `const __restrict__`: that
+// would promise that nothing writes them in this kernel's lifetime, and the
+// compiler could read them through the non-coherent path.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // The kernel after this one may be scheduled from here on (once every block
@@ -716,8 +719,8 @@ __device__ __forceinline__ void dense_rows(int n, const M* __restrict__ inv, con
 
 template <int B, int KM, class T, class M>
 __global__ void bilu_lower_kernel(int r0, int r1, int r_first, int last, SellView m, const M* __restrict__ lu,
-                                  const T* __restrict__ b, T* __restrict__ out, T* __restrict__ zadd,
-                                  const KScal* sc, int skip_if_s)
+                                  const T* b, T* __restrict__ out, T* __restrict__ zadd, const KScal* sc,
+                                  int skip_if_s)
 {
     pdl_wait();
     if (mg_skip(sc, skip_if_s)) return;
@@ -727,8 +730,8 @@ __global__ void bilu_lower_kernel(int r0, int r1, int r_first, int last, SellVie
 
 template <int B, int KM, class T, class M>
 __global__ void bilu_upper_kernel(int r0, int r1, int first, SellView m, const M* __restrict__ lu,
-                                  const T* __restrict__ b, T* __restrict__ out, T* __restrict__ zadd,
-                                  const KScal* sc, int skip_if_s)
+                                  const T* b, T* __restrict__ out, T* __restrict__ zadd, const KScal* sc,
+                                  int skip_if_s)
 {
     pdl_wait();
     if (mg_skip(sc, skip_if_s)) return;
@@ -839,7 +842,7 @@ inline size_t vec_stride(int n) { return ((size_t)(n > 0 ? n : 1) + 3) & ~(size_
          i += (int64_t)gridDim.x * blockDim.x)
 
 template <class T>
-__global__ void bicg_p_kernel(const T* __restrict__ r, const T* __restrict__ v, T* __restrict__ p, int n,
+__global__ void bicg_p_kernel(const T* r, const T* v, T* __restrict__ p, int n,
                               const KScal* sc)
 {
     pdl_trigger();
@@ -907,7 +910,7 @@ __global__ void __launch_bounds__(kThreads, spmv_min_blocks<B, KM, T>(8)) bicg_s
 
 // s = r - alpha v ; ss = s . s
 template <class T>
-__global__ void bicg_s_kernel(const T* __restrict__ r, const T* __restrict__ v, T* __restrict__ s, int n,
+__global__ void bicg_s_kernel(const T* r, const T* v, T* __restrict__ s, int n,
                               double* partials, unsigned int* counter, KScal* sc)
 {
     pdl_trigger();
@@ -979,8 +982,7 @@ __global__ void __launch_bounds__(kThreads, spmv_min_blocks<B, KM, T>(6)) bicg_s
 
 // x += alpha ph + omega sh ; r = s - omega t ; rr = r.r ; rho_new = rhat.r
 template <class T>
-__global__ void bicg_xr_kernel(const T* __restrict__ ph, const T* __restrict__ sh, const T* __restrict__ s,
-                               const T* __restrict__ t, const T* __restrict__ rhat, T* __restrict__ x,
+__global__ void bicg_xr_kernel(const T* ph, const T* sh, const T* s, const T* t, const T* rhat, T* __restrict__ x,
                                T* __restrict__ r, int n, double* partials, unsigned int* counter, KScal* sc)
 {
     pdl_trigger();
