@@ -126,19 +126,27 @@ __device__ __forceinline__ void block_sum(double (&v)[NV])
     }
 }
 
+// The blocks of a launch that share a sum, and which of them this one is.
+struct SumBlocks {
+    int block, blocks;
+    __device__ __forceinline__ SumBlocks() : block((int)blockIdx.x), blocks((int)gridDim.x) {}
+    __device__ __forceinline__ SumBlocks(int b, int n) : block(b), blocks(n) {}
+};
+
 // Writes this block's sums to `partials`; returns true, in every thread of
 // the block, for the last block to finish.
 template <int NV>
-__device__ __forceinline__ bool publish_partials(double (&v)[NV], double* partials, unsigned int* counter)
+__device__ __forceinline__ bool publish_partials(double (&v)[NV], double* partials, unsigned int* counter,
+                                                 SumBlocks at = SumBlocks())
 {
     block_sum<NV>(v);
     __shared__ bool last;
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int k = 0; k < NV; ++k) partials[blockIdx.x * NV + k] = v[k];
+        for (int k = 0; k < NV; ++k) partials[at.block * NV + k] = v[k];
         __threadfence();
         const unsigned int done = atomicAdd(counter, 1u);
-        last = (done == gridDim.x - 1);
+        last = ((int)done == at.blocks - 1);
     }
     __syncthreads();
     return last;
@@ -148,14 +156,15 @@ __device__ __forceinline__ bool publish_partials(double (&v)[NV], double* partia
 // last block to finish adds them up in a fixed order with all its threads.
 // Returns true in thread 0 of that block, with the sums in `out`.
 template <int NV>
-__device__ __forceinline__ bool grid_sum(double (&v)[NV], double* partials, unsigned int* counter, double (&out)[NV])
+__device__ __forceinline__ bool grid_sum(double (&v)[NV], double* partials, unsigned int* counter, double (&out)[NV],
+                                         SumBlocks at = SumBlocks())
 {
-    if (!publish_partials<NV>(v, partials, counter)) return false;
+    if (!publish_partials<NV>(v, partials, counter, at)) return false;
     __threadfence();
     double acc[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) acc[k] = 0.0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
+    for (int b = threadIdx.x; b < at.blocks; b += blockDim.x)
 #pragma unroll
         for (int k = 0; k < NV; ++k) acc[k] += ((volatile double*)partials)[b * NV + k];
     __syncthreads();

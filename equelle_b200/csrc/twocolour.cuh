@@ -770,17 +770,15 @@ __global__ void __launch_bounds__(kThreads) rb_gather_kernel(RbGrid g, int bb, i
 // 25 : 1 of its pressure as soon as there was flow (33x31x17: 14 iterations a
 // solve with the pressure's pairs, 18 with those).
 template <int B>
-__global__ void __launch_bounds__(kThreads) rb_strength_kernel(RbGrid g, int nd, const double* __restrict__ a,
-                                                               double* partials, unsigned int* counter, double* out)
+__device__ __forceinline__ void strengths(const RbGrid& g, int nd, const double* __restrict__ a, double* partials,
+                                          unsigned int* counter, double* out, const SumBlocks& at)
 {
     constexpr int bb = B * B;
     const RbMatrix<const double> m(a, nd, bb, g.n, g.nr);
     double sum[3 * B];
 #pragma unroll
     for (int t = 0; t < 3 * B; ++t) sum[t] = 0.0;
-    GRID_STRIDE(P64, g.n)
-    {
-        const int P = (int)P64;
+    for (int P = at.block * kThreads + (int)threadIdx.x; P < g.n; P += at.blocks * kThreads) {
         const bool red = P < g.nr;
         const int rows = red ? g.nr : g.n - g.nr, q = red ? P : P - g.nr;
 #pragma unroll
@@ -799,7 +797,7 @@ __global__ void __launch_bounds__(kThreads) rb_strength_kernel(RbGrid g, int nd,
         }
     }
     double s[3 * B];
-    if (grid_sum<3 * B>(sum, partials, counter, s)) {
+    if (grid_sum<3 * B>(sum, partials, counter, s, at)) {
         double most = -1.0;
 #pragma unroll
         for (int c = 0; c < B; ++c) {
@@ -811,18 +809,41 @@ __global__ void __launch_bounds__(kThreads) rb_strength_kernel(RbGrid g, int nd,
     }
 }
 
+template <int B>
+__global__ void __launch_bounds__(kThreads) rb_strength_kernel(RbGrid g, int nd, const double* __restrict__ a,
+                                                               double* partials, unsigned int* counter, double* out)
+{
+    strengths<B>(g, nd, a, partials, counter, out, SumBlocks());
+}
+
+// The strengths of the fine matrix by the blocks from `first` on of the launch
+// that makes the first coarse one (with a launch of their own a step of heat
+// 64x64 took 577 to 583 us, so 575 to 578).
+struct StrengthPart {
+    int first = 0, blocks = 0;
+    double* partials = nullptr;
+    unsigned int* counter = nullptr;
+    double* out = nullptr;
+};
+
 // The coarse matrix R A R^T of a 0/1 aggregation, one thread per value of a
 // coarse cell: the blocks of its members that cross each of its faces, and
 // its diagonal block with the couplings inside it, summed in the order of
 // the members and directions.
-__global__ void __launch_bounds__(kThreads) rb_galerkin_kernel(Aggregates a, int bb, int nd, const double* __restrict__ fa,
-                                                               double* __restrict__ ca)
+template <int B>
+__global__ void __launch_bounds__(kThreads) rb_galerkin_kernel(Aggregates a, int nd, const double* __restrict__ fa,
+                                                               double* __restrict__ ca, StrengthPart sp)
 {
+    constexpr int bb = B * B;
+    if (sp.blocks && (int)blockIdx.x >= sp.first) {
+        strengths<B>(a.fine, nd, fa, sp.partials, sp.counter, sp.out, SumBlocks((int)blockIdx.x - sp.first, sp.blocks));
+        return;
+    }
     const RbGrid &f = a.fine, &g = a.coarse;
     const RbMatrix<const double> F(fa, nd, bb, f.n, f.nr);
     const RbMatrix<double> G(ca, nd, bb, g.n, g.nr);
-    GRID_STRIDE(x, (int64_t)g.n * bb)
-    {
+    for (int64_t x = (int64_t)blockIdx.x * kThreads + threadIdx.x; x < (int64_t)g.n * bb;
+         x += (int64_t)(gridDim.x - sp.blocks) * kThreads) {
         const int c = (int)(x / bb), e = (int)(x - (int64_t)c * bb);
         const Cell C = cell_at(g, c);
         const bool red = ((C.i + C.j + C.k) & 1) == 0;

@@ -230,13 +230,20 @@ void rb_setup(Core& c, SolverAnalysis& an, const double* jval, bool mixed)
     const int bs = an.rb_bs, bb = bs * bs, nd = an.rb_nd;
     int* status = an.factor_status->as<int>();
     rb_gather(c, an, jval);
-    if (an.rb_directions > 1) rb_strengths(c, an);
     for (size_t l = 0; l + 1 < an.rb.size(); ++l) {
         const RbLevel &F = an.rb[l], &C = an.rb[l + 1];
-        launch(c, "mg_galerkin", [&] {
-            rb_galerkin_kernel<<<blocksFor((int64_t)C.g.n * bb), kThreads, 0, c.stream>>>(
-                F.agg, bb, nd, F.a64->as<double>(), C.a64->as<double>());
-        }, 8.0 * bb * (nd + 1) * ((double)F.g.n + C.g.n));
+        StrengthPart sp;
+        sp.first = blocksFor((int64_t)C.g.n * bb);
+        if (l == 0 && an.rb_directions > 1) {
+            sp.blocks = blocksFor(F.g.n, kThreads, kRedBlocks);
+            sp.partials = an.partials->as<double>();
+            sp.counter = an.counter->as<unsigned int>();
+            sp.out = an.factor_status->as<double>() + 1;
+        }
+        WITH_BS(bs, launch(c, "mg_galerkin", [&] {
+                    rb_galerkin_kernel<BS><<<sp.first + sp.blocks, kThreads, 0, c.stream>>>(
+                        F.agg, nd, F.a64->as<double>(), C.a64->as<double>(), sp);
+                }, 8.0 * bb * (nd + 1) * ((double)F.g.n + C.g.n)));
     }
     // the levels' factors, and beside them the coarsest one's inverse: one
     // block's chain of n steps (183 us for n = 128, 67 us for n = 60) that the
