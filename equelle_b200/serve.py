@@ -119,6 +119,13 @@ class Server:
     def _run_one(self, req, t0):
         start = time.perf_counter() - t0
         args = req.args + ["output_values=%s" % self.output_values, "host_threads=%d" % self.host_threads]
+        # Solver kernels that start while the one before them ends (same
+        # results) hold SMs while they wait, which is free for one request
+        # and taken from the others of many: 192 2D two-phase instances, 40
+        # steps each, 32 at once 508 instance-steps/s with and 579 without,
+        # 8 at once 472 and 551 (means of six runs that spread by a fifth).
+        if self.slots > 1 and not any(a.startswith("linsolver_pdl=") for a in args):
+            args.append("linsolver_pdl=0")
         if self.output_values == "last":
             args.append("output_dir=%s/" % req.workdir)
         err = ""
