@@ -142,11 +142,13 @@ void rb_levels(Core& c, SolverAnalysis& an)
 
 // The two-colour hierarchy of a system of `bs` unknowns per cell of the
 // Cartesian grid, built on the device; false when its pattern couples cells
-// that are no neighbours, or the form has no room for it.
+// that are no neighbours, or the form has no room for it, or there is no black
+// cell (a missing neighbour's value is read from a cell of the other colour).
 bool rb_analyse(Core& c, SolverAnalysis& an, const Pattern& p, int bs, int coarsest, const double* jval)
 {
     const int nd = c.nz > 1 ? 6 : 4, bb = bs * bs;
-    if (!two_colour_fits((int64_t)c.nx * c.ny * c.nz, nd, bb)) return false;
+    const int64_t cells = (int64_t)c.nx * c.ny * c.nz;
+    if (cells < 2 || !two_colour_fits(cells, nd, bb)) return false;
     an.rb_bs = bs;
     an.rb_nd = nd;
     an.rb_coarsest = coarsest;
