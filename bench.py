@@ -37,13 +37,16 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 SPMV_KERNEL = "rb_spmv_omega"
-# DRAM bytes (read + write) that ncu measured for one launch of a kernel
-# against its algorithmic bytes, on the FP64 2 x 2 block layout of the
-# two-phase 128x128x48 case (profiles/solver_kernels_twophase_128x128x48.md,
+# DRAM bytes (read + write) that ncu measured for one launch of a kernel (the
+# two-colour form's: the launches of one V-cycle together) against its
+# algorithmic bytes, on the FP64 2 x 2 blocks of the two-phase 128x128x48 case
+# (profiles/two_colour_solver.md, profiles/solver_kernels_twophase_128x128x48.md,
 # profiles/bilu_upper_kernel_twophase_128x128x48.md).
 # Both scale with the number of blocks, so a launch of the same layout on
 # another grid moves this ratio times its algorithmic bytes.
 TRAFFIC_RATIO = {
+    "rb_y": 176.5 / 188.4,
+    "rb_post": 216.2 / 230.3,
     "bicg_spmv_omega": 242.5 / 237.0,
     "mg_residual": 245.5 / 237.0,
     "bilu_lower": 114.8 / 118.5,
