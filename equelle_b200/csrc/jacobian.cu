@@ -116,9 +116,9 @@ __device__ __forceinline__ double opmat_row(int64_t i, const int* __restrict__ m
 // entry per thread these kernels ran at 1.6 to 2.5 TB/s and waited for that
 // chain in 22 to 33 of the 27 to 38 cycles between two instructions of a warp,
 // so the loads of each link are issued for all of a thread's entries before
-// the next link.  Two-phase, 128x128x64 (12.5 M entries on faces): elementwise
-// 153 -> 105 us, product 79 -> 39 us, all residuals of a step 15.9 -> 11.9 ms
-// (two entries: 12.6 ms).
+// the next link.  Two-phase, 128x128x64 (12.5 M entries on faces), one entry and
+// four: elementwise 153 and 105 us, product 79 and 39 us, all residuals of a step
+// 15.9 and 11.9 ms.
 constexpr int kEntries = 4;
 
 // rule_weights of kEntries rows: the rule is looked at once, the row values
@@ -222,12 +222,14 @@ inline int entry_blocks(int64_t n) { return blocksFor((n + kEntries - 1) / kEntr
 
 // The values that go with a Jacobian, by the blocks from `first` on of the
 // launch that computes it: small systems wait for launches, not for their
-// kernels.  Residuals of a step, apart and joint: two-phase 48x40 1.96 -> 1.60
-// ms (982 -> 847 launches), 33x31x17 2.09 -> 1.65, 512x512 (524k faces) 3.70 ->
-// 3.56; but heat 1000x701 (1.4 M faces) 0.57 -> 0.62 and two-phase 128x128x64
-// (3.1 M) 12.1 -> 13.1: there the values' kernels, which fill an SM with four
+// kernels; for many rows the values' own kernels, which fill an SM with four
 // times as many warps as fit beside the Jacobian's registers, are worth their
-// launch.  Hence the line between them.
+// launch.  Microseconds of a residual, all values apart, all joint and with
+// this line: two-phase 48x40 395, 307, 305; 400x400 (319 k faces) 604, 549, 548;
+// 560x560 (626 k) 830, 801, 807; 620x620 (768 k) 928, 909, 897; 720x720 (1.04 M)
+// 1128, 1143, 1111; 80x80x80 (1.5 M) 1380, 1438, 1362; heat 600x600 191, 190,
+// 188; 1000x701 283, 300, 281.  The lines from 2^19 to 2^20 rows are equal
+// within 2%.
 constexpr int64_t kJointRows = 1 << 19;
 
 struct ValuePart {

@@ -1239,14 +1239,10 @@ __device__ __forceinline__ double select_of(const double (&v)[N], int i)
 // step k, the inverse has a[p_k][j] in row k, column p_j.  A zero or
 // non-finite pivot sets *status.
 //
-// Bound: the chain of two barriers, a reduction and a division per step.
-// n = 128: 586 us with the matrix in shared memory and row swaps (three
-// barriers, a 2 x 128 KB sweep and an index division per entry and step),
-// 196 us from registers with rows t, t + 4, ... a thread, which read the
-// column in single values and picked the pivot's row in 32 dependent
-// selections, 183 us so (with the two-colour form's dense fill, 6 us); n = 60:
-// 91 and 67 us (warps without a row or column of the matrix only take part in
-// the barriers).
+// Bound: the chain of two barriers, a reduction and a division per step.  With
+// the matrix in shared memory and row swaps, and so: n = 128 586 and 183 us
+// (with the two-colour form's dense fill), n = 60 227 and 67 us (warps without
+// a row or column of the matrix only take part in the barriers).
 constexpr int kInverseThreads = 512;
 
 __device__ __forceinline__ void dense_inverse_block(int n, double* __restrict__ a, int* status)

@@ -15,13 +15,13 @@
 // The V-cycle's block ILU(0) sweeps read the same factors (D_b, the black
 // diagonal block of the factorization, is A_bb less the diagonal blocks of
 // L U).  With right-hand side (r_r, r_b) and iterate z_b,
-//   y   = r_r - U z_b                       (rb_y_rows)
+//   y   = r_r - U z_b                       (rb_y_kernel)
 //   t_b = r_b - A_bb z_b - L y              (the residual; red rows: 0)
-//   z_b += D_b^-1 t_b                       (rb_post_rows)
-//   z_r = D_r^-1 (r_r - U z_b)              (rb_fin_rows)
+//   z_b += D_b^-1 t_b                       (rb_post_kernel)
+//   z_r = D_r^-1 (r_r - U z_b)              (rb_fin_kernel)
 // is one sweep from any z_b: the red part of the iterate is never needed
 // before the last line, the residual of the down-leg is summed straight into
-// the coarse right-hand side (rb_res_rows), and the coarse level's last two
+// the coarse right-hand side (rb_res_kernel), and the coarse level's last two
 // steps add alpha times their rows to the fine black cells (UpRow).  A
 // level with pre-smoothing (Level::pre) takes six half products of its
 // factors, one without three; level 0 needs no red rows at all.
@@ -36,14 +36,11 @@
 // blocks.
 //
 // Bound: HBM on the fine levels (32 bytes per 2 x 2 FP64 block), latency of
-// dependent steps on the coarse ones.  Measured on one time step, against the
-// full-length form over stages with 2 x 2 x 2 aggregates only and against
-// this form on the block sliced layout (stored columns and lengths): Krylov
-// time of two-phase 128x128x64, 150 (203 iterations) -> 59 -> 51 ms (90; the
-// iterations by pairing along z alone on the first two levels); 512x512, 26.5
-// -> 16.6 -> 11.6 ms; 33x31x17, 20.6 -> 9.7 -> 7.9 ms; impes 97x83x41, 31.6 ->
-// 12.6 -> 10.4 ms.  First step of a new 128x128x64 runtime, with the analysis
-// on the host, then on the device: 526 -> 180 ms.
+// dependent steps on the coarse ones.  Krylov time of one time step in the
+// general form with 2 x 2 x 2 aggregates and in this one: two-phase 128x128x64
+// 150 ms (203 iterations) and 44 (90), 512x512 26.5 and 8.9, 33x31x17 20.6 and
+// 6.2, impes 97x83x41 31.6 and 8.6.  First step of a new 128x128x64 runtime,
+// with the analysis on the host and on the device: 756 and 154 ms.
 
 // Division by a run-time constant, exact for 0 <= n < 2^31: with l =
 // ceil(log2 d) and m = floor(2^(31+l) / d) + 1, floor(n / d) = floor(n m /
@@ -902,7 +899,10 @@ struct RbFactorLevel {
     int first = 0, blocks = 0;
 };
 
-constexpr int kMaxRbLevels = 32;  // every one has at most half the cells of the one before
+// Every level pairs a direction, so there are at most the sum of ceil(log2
+// side) of them below level 0: in 3D less than log2(cells) + 3, and
+// two_colour_fits gives cells < 2^31 / 7; in 2D less.
+constexpr int kMaxRbLevels = 32;
 
 struct RbFactorParams {
     int nlev = 0;
@@ -1032,15 +1032,13 @@ __global__ void __launch_bounds__(kInverseThreads, 1)
 // memory of one thread-block cluster: every block holds the matrix rows and
 // the vector entries of its share of each level's cells, neighbours' values are
 // read from the other blocks' shared memory, and a cluster barrier ends a step.
-// A step through global memory was two or three round trips to L2 of some
-// 1000 cycles each and a barrier that waits for the stores to reach it: 2.4k
-// to 9k cycles; from distributed shared memory 1.2k to 2.5k, most of it index
-// arithmetic and FP64 latency.  (Every step has one call site: inlined once more
-// for the first level, its code was fetched anew and took 8k to 10k.)  The cycle
-// from the 32x32x4 level of two-phase 128x128x64: 33 -> 19 us, from the 64x64
-// level of 512x512 22 us.  The smallest levels
-// are block 0's alone (solo), with block barriers; the dense solve's rows are
-// shared out again.  The matrices are copied in at every launch, before the
+// A step takes 1.2k to 2.5k cycles, most of it index arithmetic and FP64
+// latency (through global memory, two or three round trips to L2 and a barrier
+// that waits for the stores to reach it: 2.4k to 9k).  Every step has one call
+// site: another copy of its code would be fetched anew, 8k to 10k cycles.  The
+// cycle from the 32x32x4 level of two-phase 128x128x64: 33 us through global
+// memory, 19 so.  The smallest levels are block 0's alone (solo), with block
+// barriers; the dense solve's rows are shared out again.  The matrices are copied in at every launch, before the
 // wait for the previous kernel.  Products and sums are those of the one-step
 // kernels, in their order; where those add alpha zc to the finer level's z
 // (UpRow), the finer level here reads both (z0_at): the same bits.
@@ -1138,7 +1136,7 @@ struct RbTailView {
     }
 };
 
-// stencil_dot over a block's rows, the neighbours' values from get(neighbour's
+// StencilRow::dot over a block's rows, the neighbours' values from get(neighbour's
 // cell, its number, value).
 template <int B, int ND, class M, class Get>
 __device__ __forceinline__ void tail_dot(const RbGrid& g, const Cell& e, int q, int others, const M* a, int rows, int ql,
@@ -1198,7 +1196,7 @@ __device__ __forceinline__ void tail_down(const RbTailView<B, ND, M>& V, const R
     const RbGrid& g = L.g;
     const int nk = g.n - g.nr;
     if (L.pre) {
-        for (int q = V.lo + tid; q < V.hi(1); q += nth) {  // rb_pre_rows
+        for (int q = V.lo + tid; q < V.hi(1); q += nth) {  // rb_pre_kernel
             const int ql = q - V.lo;
             M dv[BB];
             double acc[B], v[B], x[B];
@@ -1215,7 +1213,7 @@ __device__ __forceinline__ void tail_down(const RbTailView<B, ND, M>& V, const R
             store_vec<B>(V.z, q, x);
         }
         sync();
-        for (int q = V.lo + tid; q < V.hi(0); q += nth) {  // rb_y_rows
+        for (int q = V.lo + tid; q < V.hi(0); q += nth) {  // rb_y_kernel
             double acc[B], v[B];
 #pragma unroll
             for (int t = 0; t < B; ++t) acc[t] = v[t] = 0.0;
@@ -1227,7 +1225,7 @@ __device__ __forceinline__ void tail_down(const RbTailView<B, ND, M>& V, const R
             store_vec<B>(V.y, q, v);
         }
         sync();
-        for (int q = V.lo + tid; q < V.hi(1); q += nth) {  // the residual of rb_res_rows
+        for (int q = V.lo + tid; q < V.hi(1); q += nth) {  // the residual of rb_res_kernel
             const int ql = q - V.lo;
             M av[BB];
             double acc[B], az[B], z[B], t[B];
@@ -1252,7 +1250,7 @@ __device__ __forceinline__ void tail_down(const RbTailView<B, ND, M>& V, const R
         if (q >= C.hi(colour)) continue;
         const Cell e = cell_of(G, colour, q);
         double s[B];
-        if (L.pre) {  // the butterfly sum of rb_res_rows
+        if (L.pre) {  // the butterfly sum of rb_res_kernel
             double w[4][B];
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
@@ -1266,7 +1264,7 @@ __device__ __forceinline__ void tail_down(const RbTailView<B, ND, M>& V, const R
                 s[t] = L.agg.g == 1 ? w[0][t]
                                     : L.agg.g == 2 ? __dadd_rn(w[0][t], w[1][t])
                                                    : __dadd_rn(__dadd_rn(w[0][t], w[1][t]), __dadd_rn(w[2][t], w[3][t]));
-        } else {  // rb_restrict_rows
+        } else {  // rb_restrict_kernel
             const Aggregates& a = L.agg;
 #pragma unroll
             for (int t = 0; t < B; ++t) s[t] = 0.0;
@@ -1301,7 +1299,7 @@ __device__ __forceinline__ void tail_up(const RbTailParams<M>& p, const RbTailVi
     const RbTailLevel<M>& L = V.L;
     const RbGrid& g = L.g;
     const int nk = g.n - g.nr;
-    for (int q = V.lo + tid; q < V.hi(0); q += nth) {  // rb_y_rows
+    for (int q = V.lo + tid; q < V.hi(0); q += nth) {  // rb_y_kernel
         double acc[B], v[B];
 #pragma unroll
         for (int t = 0; t < B; ++t) acc[t] = v[t] = 0.0;
@@ -1313,7 +1311,7 @@ __device__ __forceinline__ void tail_up(const RbTailParams<M>& p, const RbTailVi
         store_vec<B>(V.y, q, v);
     }
     sync();
-    for (int q = V.lo + tid; q < V.hi(1); q += nth) {  // rb_post_rows
+    for (int q = V.lo + tid; q < V.hi(1); q += nth) {  // rb_post_kernel
         const int ql = q - V.lo;
         const Cell e = cell_of(g, 1, q);
         M av[BB], dv[BB];
@@ -1343,7 +1341,7 @@ __device__ __forceinline__ void tail_up(const RbTailParams<M>& p, const RbTailVi
     }
     if (!need_red) return;
     sync();
-    for (int q = V.lo + tid; q < V.hi(0); q += nth) {  // rb_fin_rows
+    for (int q = V.lo + tid; q < V.hi(0); q += nth) {  // rb_fin_kernel
         const int ql = q - V.lo;
         const Cell e = cell_of(g, 0, q);
         M dv[BB];

@@ -27,10 +27,20 @@ RbMatrix<const M> rb_matrix(const SolverAnalysis& an, const RbLevel& L)
 // Levels are coarsened only along the directions at least 1 / kSemiCoarsen
 // as strong as the strongest one: the point smoothers do not reduce error
 // that varies slowly along a strong direction and quickly along a weak one.
-// BiCGStab iterations of a two-phase solve on 48 x 48 x 32 cells of 10 x 10 x
-// 2 m (strengths 25 : 1 : 1): 38 with 2 x 2 x 2 aggregates on every level, 21
-// with one z-pairing level first, 17 with two (then 2 x 2 x 2 at 6.25 : 1),
-// 18 with three.  At 4 : 1 one z-pairing level and none are equal.
+// Krylov ms of two time steps at lines of 4, 6.5, 9 and 13 (before: with
+// 2 x 2 x 2 aggregates in the general form), cells of 10 x 10 x dz m:
+//   48x48x32    dz 5    13.9  14.1  14.0  14.0  (24.4)
+//               dz 3.9  15.6  16.0  15.9  16.0  (27.5)
+//               dz 3    15.3  17.2  16.7  20.1  (33.5)
+//               dz 2    19.2  16.2  16.3  20.5  (50.7)
+//               dz 1    28.8  23.9  23.8  21.4  (101)
+//   33x31x17    dz 2    12.9  11.5  11.6  11.6
+//   97x83x41    dz 2    37.5  30.9  30.6  38.3
+//   256x256  10 x 3.9   10.4  10.0   9.9   9.9  (21.5)
+//            10 x 2     23.7  18.2  17.9  20.1  (66.7)
+//            10 x 1     43.4  31.8  31.9  30.3  (176)
+// 6.5 and 9 choose alike on all of these; 4 pairs one direction too long, 13
+// gives up too early.
 constexpr double kSemiCoarsen = 6.5;
 
 // The directions that the next level pairs, bit d for direction d, from the
@@ -123,6 +133,9 @@ void rb_levels(Core& c, SolverAnalysis& an)
             F.agg = aggregates_of(F.g, an.rb_pairs[l]);
             const int cut = F.agg.sx + F.agg.sy + F.agg.sz;
             F.alpha = c.param_d("linsolver_mg_alpha", cut == 2 && c.nz == 1 ? kMgAlpha2d : kMgAlpha3d);
+            // pairs only: no sweep before the correction.  With it, fewer
+            // iterations and more time (48x48x32, dz 2: 120 in 16.4 ms against
+            // 132 in 16.2; dz 1: 157 in 26.1 against 172 in 23.9)
             F.pre = cut > 1;
             C.g = F.agg.coarse;
         }
@@ -354,9 +367,11 @@ int plan_rb_tail(Core& c, const SolverAnalysis& an, int cl, int& bytes, RbTailPa
                                        : (int64_t)(2 * an.rb_nd + 3) * t.rows * bs * bs;
         const int64_t need = al(mat * (int64_t)sizeof(M)) + 5 * (int64_t)t.vec +
                              (L.coarsest ? al((int64_t)L.n * sizeof(double)) : 0);
-        // more rows than half the threads of a block are better spread over the
-        // whole GPU, one launch per step (two-phase 255x257 mixed, whose
-        // 128x129 level would be 516 rows a block: 6.6 against 6.4 ms a step)
+        // levels of more rows are spread over the whole GPU, one launch per
+        // step.  Microseconds an iteration with lines of 128, 256, 512 and 4096
+        // rows: two-phase 97x83x41 mixed 215, 215, 224, 223; 512x512 mixed 173,
+        // 171, 174, 175; 255x257 mixed 132, 128, 128, 138; 128x128 mixed 91, 91,
+        // 83, 83; heat 1000x701 217, 217, 212, 214; 400x300 131, 124, 122, 124
         if (!alone && !L.coarsest && t.rows > kTailThreads / 2 && cl > 1) break;
         if (off + need > kRbTailSmem) break;
         t.so_m = (int)off;

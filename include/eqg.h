@@ -130,11 +130,13 @@ const char* eqg_backend_name(void);
  * linsolver_mg_alpha (factor of the coarse-grid correction z += alpha P zc;
  * 1.9 for 2 x 2 aggregates of 2D grids, else 1.4), linsolver_mg_ap_rows
  * (40000: levels with more unknowns correct their residual through A P
- * instead of recomputing r - A z; where the sweeps run over more than two
- * stages), linsolver_mg_coarsest (128: coarsening stops at
+ * instead of recomputing r - A z; in the general form with FP64 vectors: not
+ * in the two-colour form of default solves, nor with refine),
+ * linsolver_mg_coarsest (128: coarsening stops at
  * this many unknowns, at most 128; that level is solved with a dense
  * inverse), linsolver_pdl (1: the BiCGStab iteration's kernels
- * as programmatic dependent launches; 0: plain launches),
+ * as programmatic dependent launches, which start while the one before them
+ * ends; 0: plain launches, better where several runtimes share the GPU),
  * linsolver_mg_local (1: that kernel keeps its coarsest levels in one thread
  * block's shared memory; 0: off),
  * linsolver_tail_trace (0; 1: print the SM clock cycles of every step of the
