@@ -120,6 +120,13 @@ __device__ __forceinline__ double opmat_row(int64_t i, const int* __restrict__ m
 // four: elementwise 153 and 105 us, product 79 and 39 us, all residuals of a step
 // 15.9 and 11.9 ms.
 constexpr int kEntries = 4;
+// Products of at most this many entries take one per thread: they leave most of
+// the GPU idle, and a thread of four waits for its longest chain.  Divergence
+// of a flux, one and four entries per thread: 16x16x16 (54 k entries) 7.4 and
+// 8.4 us, with a deferred rule 8.7 and 9.7; 24x24x24 (187 k) 8.4 and 8.7;
+// 33x31x17 (235 k) 8.6 and 8.7; 255x257 (653 k) 11.9 and 10.8.  Extension to all
+// faces: 100x100 (79 k) 8.6 and 8.7, 33x31x17 (200 k) 10.3 and 8.7.
+constexpr int64_t kOneEntry = 1 << 17;
 
 // rule_weights of kEntries rows: the rule is looked at once, the row values
 // of all entries are loaded before they are used.
@@ -211,14 +218,13 @@ __device__ __forceinline__ void apply_deferred_of(const Deferred& d, const int (
     }
 }
 
-// This thread's entries: e + u blockDim for u < kEntries, e from the loop;
-// past the end the last entry (its result is not stored).  vp: the launch's
-// ValuePart.
-#define ENTRY_STRIDE(e, n)                                                                                  \
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x * kEntries + threadIdx.x; e < (n);                    \
-         e += (int64_t)(gridDim.x - vp.blocks) * blockDim.x * kEntries)
+// This thread's entries: e + u blockDim for u < E, e from the loop; past the
+// end the last entry (its result is not stored).  vp: the launch's ValuePart.
+#define ENTRY_STRIDE(E, e, n)                                                                        \
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x * (E) + threadIdx.x; e < (n);                  \
+         e += (int64_t)(gridDim.x - vp.blocks) * blockDim.x * (E))
 
-inline int entry_blocks(int64_t n) { return blocksFor((n + kEntries - 1) / kEntries); }
+inline int entry_blocks(int64_t n, int per_thread = kEntries) { return blocksFor((n + per_thread - 1) / per_thread); }
 
 // The values that go with a Jacobian, by the blocks from `first` on of the
 // launch that computes it: small systems wait for launches, not for their
@@ -433,6 +439,7 @@ __global__ void spgemm_plan_kernel(int n_out, const int* __restrict__ mptr, cons
     }
 }
 
+template <int E>
 __global__ void __launch_bounds__(kThreads) spgemm_planned_kernel(int64_t nnz, const int* __restrict__ start,
                                                                   const int* __restrict__ contrib,
                                                                   const int* __restrict__ jrow,
@@ -443,39 +450,39 @@ __global__ void __launch_bounds__(kThreads) spgemm_planned_kernel(int64_t nnz, c
                                                                   const double* __restrict__ mw, const ValuePart vp)
 {
     if (value_blocks(vp, [&](int64_t i) { vp.out[i] = opmat_row(i, mptr, msrc, mw, vp.a); })) return;
-    ENTRY_STRIDE(e0, nnz)
+    ENTRY_STRIDE(E, e0, nnz)
     {
-        int k[kEntries], k1[kEntries];
-        double acc[kEntries];
+        int k[E], k1[E];
+        double acc[E];
         bool more = false;
 #pragma unroll
-        for (int u = 0; u < kEntries; ++u) {
+        for (int u = 0; u < E; ++u) {
             const int64_t e = min(e0 + (int64_t)u * blockDim.x, nnz - 1);
             k[u] = start[e];
             k1[u] = start[e + 1];
             acc[u] = 0.0;
         }
         do {  // the next contribution of every entry (each has at least one)
-            int q[kEntries], row[kEntries];
-            double x[kEntries];
+            int q[E], row[E];
+            double x[E];
 #pragma unroll
-            for (int u = 0; u < kEntries; ++u) {
+            for (int u = 0; u < E; ++u) {
                 const int at = max(min(k[u], k1[u] - 1), 0);
                 q[u] = contrib[at];
                 row[u] = dj.n ? jrow[at] : 0;
             }
 #pragma unroll
-            for (int u = 0; u < kEntries; ++u) x[u] = jval[q[u] & kPlanMask];
-            if (dj.n) apply_deferred_of<kEntries>(dj, row, x);
+            for (int u = 0; u < E; ++u) x[u] = jval[q[u] & kPlanMask];
+            if (dj.n) apply_deferred_of<E>(dj, row, x);
             more = false;
 #pragma unroll
-            for (int u = 0; u < kEntries; ++u) {
+            for (int u = 0; u < E; ++u) {
                 if (k[u] < k1[u]) acc[u] += q[u] < 0 ? -x[u] : x[u];
                 more |= ++k[u] < k1[u];
             }
         } while (more);
 #pragma unroll
-        for (int u = 0; u < kEntries; ++u) {
+        for (int u = 0; u < E; ++u) {
             const int64_t e = e0 + (int64_t)u * blockDim.x;
             if (e < nnz) oval[e] = acc[u];
         }
@@ -554,7 +561,7 @@ __global__ void __launch_bounds__(kThreads) ew_flat_kernel(Rule r, const int* __
                                                              const ValuePart vp)
 {
     if (ew_values(vp, r.rule)) return;
-    ENTRY_STRIDE(e0, nnz)
+    ENTRY_STRIDE(kEntries, e0, nnz)
     {
         int i[kEntries];
         double a[kEntries], b[kEntries], wa[kEntries], wb[kEntries], post[kEntries];
@@ -585,7 +592,7 @@ __global__ void __launch_bounds__(kThreads) apply_deferred_kernel(const Deferred
                                                                   double* __restrict__ out, int64_t nnz)
 {
     const ValuePart vp;
-    ENTRY_STRIDE(e0, nnz)
+    ENTRY_STRIDE(kEntries, e0, nnz)
     {
         int i[kEntries];
         double x[kEntries];
@@ -672,7 +679,7 @@ __global__ void __launch_bounds__(kThreads) ew_mapped_kernel(Rule r, const int* 
                                                              const ValuePart vp)
 {
     if (ew_values(vp, r.rule)) return;
-    ENTRY_STRIDE(e0, nnz)
+    ENTRY_STRIDE(kEntries, e0, nnz)
     {
         int i[kEntries], xa[kEntries], xb[kEntries];
         double a[kEntries], b[kEntries], wa[kEntries], wb[kEntries], post[kEntries];
@@ -816,9 +823,10 @@ void spgemm_numeric(Core& c, const OpMatrix& m, const Pattern& jp, const double*
         vp.n = m.n_out;
         vp.a = x;
         vp.out = y;
+        const int per_thread = op.nnz <= kOneEntry ? 1 : kEntries;
         launch(c, "spgemm_planned", [&] {
-            const int grid = vp.grid(entry_blocks(op.nnz));
-            spgemm_planned_kernel<<<grid, kThreads, 0, c.stream>>>(
+            const int grid = vp.grid(entry_blocks(op.nnz, per_thread));
+            (per_thread == 1 ? spgemm_planned_kernel<1> : spgemm_planned_kernel<kEntries>)<<<grid, kThreads, 0, c.stream>>>(
                 op.nnz, op.plan_start->as<int>(), op.plan_contrib->as<int>(), op.plan_jrow->as<int>(), jv, ov, jd,
                 m.ptr->as<int>(), m.src->as<int>(), m.w->as<double>(), vp);
         }, bytes + (y ? 4.0 * (m.n_out + 1) + 12.0 * m.nnz + 8.0 * m.n_src + 8.0 * m.n_out : 0.0));
