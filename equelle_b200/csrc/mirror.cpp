@@ -106,14 +106,14 @@ extern PyTypeObject RuntimeBaseType, CollBaseType, MaskBaseType, SetBaseType;
 
 // An object whose __init__ has not run (or not got that far) lacks what it
 // sets: an error, as for any Python attribute.
-void* lacks(PyObject* o, const char* name)
+__attribute__((noinline, cold)) void* lacks(PyObject* o, const char* name)
 {
     PyErr_Format(PyExc_AttributeError, "'%s' object has no attribute '%s'", Py_TYPE(o)->tp_name, name);
     return nullptr;
 }
 
 // The runtime that a method is called on; null (an error) before its __init__.
-RuntimeObject* rt_of(PyObject* self)
+inline RuntimeObject* rt_of(PyObject* self)
 {
     RuntimeObject* rt = (RuntimeObject*)self;
     if (!rt->bound) return (RuntimeObject*)lacks(self, "lib");
@@ -122,7 +122,7 @@ RuntimeObject* rt_of(PyObject* self)
 }
 
 // The runtime of a handle; null (an error) before the handle's __init__.
-RuntimeObject* rt_of_handle(PyObject* handle)
+inline RuntimeObject* rt_of_handle(PyObject* handle)
 {
     RuntimeObject* rt = ((HandleObject*)handle)->rt;
     return rt ? rt_of((PyObject*)rt) : (RuntimeObject*)lacks(handle, "rt");
@@ -168,7 +168,7 @@ PyObject* as_object(const void* v) { return v ? PyLong_FromVoidPtr((void*)v) : P
 
 // runtime.<hook>(runtime.lib.<name>, args...)
 template <class... A>
-PyObject* call_hook(RuntimeObject* rt, const char* hook, const char* name, A... args)
+__attribute__((noinline, cold)) PyObject* call_hook(RuntimeObject* rt, const char* hook, const char* name, A... args)
 {
     constexpr Py_ssize_t N = 1 + sizeof...(A);
     PyObject* lib = PyObject_GetAttrString((PyObject*)rt, "lib");
@@ -187,7 +187,7 @@ PyObject* call_hook(RuntimeObject* rt, const char* hook, const char* name, A... 
 // runtime class with methods of its own for that (_coll and the like) makes it
 // through them.
 template <class T, class F, class... A>
-PyObject* make(RuntimeObject* rt, F Api::*fn, const char* name, A... args)
+inline __attribute__((always_inline)) PyObject* make(RuntimeObject* rt, F Api::*fn, const char* name, A... args)
 {
     if (rt->hooked) return call_hook(rt, Made<T>::hook, name, args...);
     T* out = nullptr;
@@ -196,19 +196,20 @@ PyObject* make(RuntimeObject* rt, F Api::*fn, const char* name, A... args)
 }
 #define ENTRY(name) &Api::name, "eqg_" #name
 
+// The handle of an object of a handle type.
+inline bool own_handle(PyObject* o, void** h)
+{
+    *h = ((HandleObject*)o)->h;
+    return ((HandleObject*)o)->rt || lacks(o, "h");
+}
+
 // The handle inside a Python object: a handle type's own, or the integer in
 // its attribute `h`.
 bool handle_of(PyObject* o, void** h)
 {
     if (PyObject_TypeCheck(o, &CollBaseType) || PyObject_TypeCheck(o, &SetBaseType) ||
-        PyObject_TypeCheck(o, &MaskBaseType)) {
-        if (!((HandleObject*)o)->rt) {
-            lacks(o, "h");
-            return false;
-        }
-        *h = ((HandleObject*)o)->h;
-        return true;
-    }
+        PyObject_TypeCheck(o, &MaskBaseType))
+        return own_handle(o, h);
     PyObject* v = PyObject_GetAttrString(o, "h");
     if (!v) return false;
     *h = v == Py_None ? nullptr : PyLong_AsVoidPtr(v);
@@ -343,7 +344,7 @@ PyObject* coll_binary(int op, PyObject* left, PyObject* right)
     if (!rt) return nullptr;
     if (l && r) {
         void *a0, *b0;
-        if (!handle_of(left, &a0) || !handle_of(right, &b0)) return nullptr;
+        if (!own_handle(left, &a0) || !own_handle(right, &b0)) return nullptr;
         const eqg_coll *a = (eqg_coll*)a0, *b = (eqg_coll*)b0;
         return make<eqg_coll>(rt, ENTRY(binary), op, a, b);
     }
@@ -374,7 +375,7 @@ PyObject* coll_compare_op(PyObject* self, int op, PyObject* other)
     const eqg_coll* a = (eqg_coll*)((HandleObject*)self)->h;
     if (PyObject_TypeCheck(other, &CollBaseType)) {
         void* b0;
-        if (!handle_of(other, &b0)) return nullptr;
+        if (!own_handle(other, &b0)) return nullptr;
         const eqg_coll* b = (eqg_coll*)b0;
         return make<eqg_mask>(rt, ENTRY(compare), op, a, b);
     }
