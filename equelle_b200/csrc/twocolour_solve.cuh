@@ -135,7 +135,8 @@ void rb_levels(Core& c, SolverAnalysis& an)
             F.alpha = c.param_d("linsolver_mg_alpha", cut == 2 && c.nz == 1 ? kMgAlpha2d : kMgAlpha3d);
             // pairs only: no sweep before the correction.  With it, fewer
             // iterations and more time (48x48x32, dz 2: 120 in 16.4 ms against
-            // 132 in 16.2; dz 1: 157 in 26.1 against 172 in 23.9)
+            // 132 in 16.2; dz 1: 157 in 26.1 against 172 in 23.9; but cells of
+            // 2 x 10 x 10: 116 in 15.7 against 136 in 17.1)
             F.pre = cut > 1;
             C.g = F.agg.coarse;
         }
