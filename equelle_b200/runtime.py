@@ -27,7 +27,7 @@ except ImportError:  # not built yet: a few seconds of the system compiler
     except (ImportError, OSError, RuntimeError) as e:
         import warnings
         warnings.warn("the native module equelle_b200._mirror is not built and cannot be built here (%s); runtime "
-                      "calls go through ctypes, some ten times the host time each" % str(e).splitlines()[0],
+                      "calls go through ctypes, some ten times the host time each" % (str(e).splitlines() or [""])[0],
                       RuntimeWarning, stacklevel=2)
         from . import _mirror_py as _mirror
 
