@@ -926,7 +926,7 @@ __device__ __forceinline__ double block_max(double v, double* scratch)
 
 // Cells that a warp updates per row (its outer lanes are the halo), warps of
 // a block, and the rows of a warp's strip (between the least and the most).
-constexpr int kLanes = 30, kStripWarps = 4, kStripMin = 8, kStripMax = 64;
+constexpr int kLanes = 30, kStripWarps = 4, kStripMax = 64;
 
 // Arrays of a row in a warp's ring of rows in shared memory.
 enum SweRow { R_W, R_HU, R_HV, R_BM, R_BE, R_BW, R_BN, R_BS, R_W0, R_HU0, R_HV0 };
@@ -1073,17 +1073,24 @@ __global__ void __launch_bounds__(32 * kStripWarps, 5)
 
 // The launch of a stage: strips of kLanes columns, of the most rows (a strip
 // costs the side fluxes of two more) that still give every SM four blocks of
-// warps: the walk of a strip is a chain, hidden by other warps only.
+// warps: the walk of a strip is a chain, hidden by other warps only.  Below
+// eight rows only while all strips are resident at once (five blocks an SM),
+// and single rows, a third of whose work is their own, where they leave most
+// of the GPU idle.  Both stages, with 8 rows at least and so (before, windows
+// of 32 x 10 cells): 64 x 48 43.9 and 28.7 us (25.2), 128 x 128 43.2 and 28.3
+// (26.1), 256 x 256 44.3 and 31.9 (29.8), 512 x 512 55.1 and 45.8 (46.5), 4000 x
+// 31 43.0 and 33.3 (32.4); 700 x 700 60.3 both (64.2).
 struct StripGrid {
     int strips_x, rows, blocks;
+    int64_t strips_of(int ny, int r) const { return (int64_t)strips_x * ((ny + r - 1) / r); }
     StripGrid(int nx, int ny)
     {
         strips_x = (nx + kLanes - 1) / kLanes;
-        const int64_t wanted = (int64_t)148 * 4 * kStripWarps;
+        const int64_t wanted = (int64_t)148 * 4 * kStripWarps, resident = (int64_t)148 * 5 * kStripWarps;
         rows = kStripMax;
-        while (rows > kStripMin && (int64_t)strips_x * ((ny + rows - 1) / rows) < wanted) rows /= 2;
-        const int64_t strips = (int64_t)strips_x * ((ny + rows - 1) / rows);
-        blocks = (int)((strips + kStripWarps - 1) / kStripWarps);
+        while (rows > 8 && strips_of(ny, rows) < wanted) rows /= 2;
+        while (rows > 1 && strips_of(ny, rows / 2) <= (rows > 2 ? resident : resident / 4)) rows /= 2;
+        blocks = (int)((strips_of(ny, rows) + kStripWarps - 1) / kStripWarps);
     }
 };
 
