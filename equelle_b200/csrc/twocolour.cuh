@@ -137,8 +137,9 @@ struct RbMatrix {
 };
 
 // One block of a level's matrix, which no kernel of a solve writes: read past
-// L1 (every block is used once per kernel), and where it stands relative to
-// pdl_wait (the assembly statements keep their order).
+// L1 (every block is used once per kernel; 3 x 3 blocks through it, since the
+// lanes' single values share sectors), and where it stands relative to pdl_wait
+// (the assembly statements keep their order).
 template <int BB, class M>
 __device__ __forceinline__ void load_matrix(const M* p, M (&v)[BB])
 {
@@ -148,6 +149,12 @@ __device__ __forceinline__ void load_matrix(const M* p, M (&v)[BB])
     } else if constexpr (BB == 4) {
         asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
                      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p));
+    } else if constexpr (BB == 9 && sizeof(M) == 8) {
+#pragma unroll
+        for (int e = 0; e < BB; ++e) asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v[e]) : "l"(p + e));
+    } else if constexpr (BB == 9) {
+#pragma unroll
+        for (int e = 0; e < BB; ++e) asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v[e]) : "l"(p + e));
     } else if constexpr (sizeof(M) == 8) {
 #pragma unroll
         for (int e = 0; e < BB; ++e) asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v[e]) : "l"(p + e));
@@ -163,10 +170,19 @@ __device__ __forceinline__ void load_matrix(const M* p, M (&v)[BB])
 // the first sum (with a branch per neighbour the compiler waited for each one
 // in turn, in 34 registers): the block of a missing neighbour is stored as
 // zero, and the vector is then read at the row's own number, or the last one.
+//
+// A row of 3 x 3 FP64 blocks is more than fits in registers beside them (rows of
+// six spilled 84 to 780 bytes): half of it comes ahead, the other half after
+// the first half's sums.  With that, and 3 x 3 blocks through L1: an iteration
+// of three species on 96^3 cells 1515 -> 963 us (general form 1335), 64^3 580 ->
+// 417, 600x600 580 -> 440.
 template <int B, int ND, class M>
 struct StencilRow {
-    M av[ND][B * B];
+    static constexpr int G = B * B * ND * (int)sizeof(M) > 256 ? ND / 2 : ND;  // directions ahead
+    M av[G][B * B];
     int nq[ND];
+    const M* rest;  // the blocks of direction G
+    int stride;     // rows of the colour
     // row q of `rows`, cell e
     __device__ __forceinline__ void load(const RbGrid& g, const Cell& e, int q, int rows, const M* a)
     {
@@ -174,20 +190,35 @@ struct StencilRow {
 #pragma unroll
         for (int d = 0; d < ND; ++d) {
             if (!neighbour(g, e, d, nq[d])) nq[d] = own;
-            load_matrix<B * B, M>(a + ((size_t)d * rows + q) * (B * B), av[d]);
+            if (d < G) load_matrix<B * B, M>(a + ((size_t)d * rows + q) * (B * B), av[d]);
         }
+        rest = a + ((size_t)G * rows + q) * (B * B);
+        stride = rows;
     }
     __device__ __forceinline__ void dot(const double* x, double (&acc)[B]) const
     {
-        double xv[ND][B];
+        sums(0, av, x, acc);
+        if constexpr (G < ND) {
+            M bv[ND - G][B * B];
 #pragma unroll
-        for (int d = 0; d < ND; ++d) load_bvec<B, double>(x, nq[d], xv[d]);
+            for (int d = G; d < ND; ++d) load_matrix<B * B, M>(rest + (size_t)(d - G) * stride * (B * B), bv[d - G]);
+            sums(G, bv, x, acc);
+        }
+    }
+
+private:
+    template <int N>
+    __device__ __forceinline__ void sums(int d0, const M (&v)[N][B * B], const double* x, double (&acc)[B]) const
+    {
+        double xv[N][B];
 #pragma unroll
-        for (int d = 0; d < ND; ++d)
+        for (int d = 0; d < N; ++d) load_bvec<B, double>(x, nq[d0 + d], xv[d]);
+#pragma unroll
+        for (int d = 0; d < N; ++d)
 #pragma unroll
             for (int i = 0; i < B; ++i)
 #pragma unroll
-                for (int j = 0; j < B; ++j) acc[i] = __fma_rn((double)av[d][i * B + j], xv[d][j], acc[i]);
+                for (int j = 0; j < B; ++j) acc[i] = __fma_rn((double)v[d][i * B + j], xv[d][j], acc[i]);
     }
 };
 
